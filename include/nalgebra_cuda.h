@@ -95,6 +95,13 @@ int nacu_device_count(int* count);
  * nacu_free synchronizes the device (cudaFree). */
 int nacu_malloc(void** ptr, size_t bytes);
 int nacu_free(void* ptr);
+/* Scratch in stream order (cudaMallocFromPoolAsync on a pool of the library's
+ * own): usable by work queued on `stream` after the call, released by the free
+ * once the work queued before it has run; neither synchronizes.  The pool
+ * keeps up to 4 GiB between calls and gives them back when nacu_malloc needs
+ * them.  Inside a stream capture both become nodes of the graph. */
+int nacu_malloc_async(void** ptr, size_t bytes, nacu_stream_t stream);
+int nacu_free_async(void* ptr, nacu_stream_t stream);
 /* Page-locked host memory (lets nacu_memcpy and the *_host entry points
  * overlap copies with kernels). */
 int nacu_host_alloc(void** ptr, size_t bytes);
@@ -568,6 +575,18 @@ int nacu_dgesv_mixed_ir(int n, const double* A, int64_t lda, const double* b, do
 int nacu_dgemm(int m, int n, int k, double alpha, const double* A, int64_t lda, const double* B, int64_t ldb,
                double beta, double* C, int64_t ldc, nacu_stream_t stream);
 
+/* nacu_dgemm with scratch, which lets large products run on the tensor cores:
+ * A and B scaled to integers of up to 62 bits, multiplied exactly modulo 16
+ * small numbers in BF16, the integer product put together by the Chinese
+ * remainder theorem.  Its error is below nacu_dgemm's; output tiles where
+ * |A||B| cancels strongly, and NaN, infinities and extreme exponents, are
+ * computed by nacu_dgemm's kernel.  Where nacu_dgemm_workspace_bytes is 0 (small
+ * products) the call is nacu_dgemm and the workspace may be NULL. */
+size_t nacu_dgemm_workspace_bytes(int m, int n, int k);
+int nacu_dgemm_ws(int m, int n, int k, double alpha, const double* A, int64_t lda, const double* B, int64_t ldb,
+                  double beta, double* C, int64_t ldc, void* workspace, size_t workspace_bytes,
+                  nacu_stream_t stream);
+
 /* Many independent products in one launch: C_s = alpha * A_s * B_s + beta *
  * C_s for s < batch, each m x k by k x n, column-major with leading dimensions
  * lda / ldb / ldc, product s at A + s*strideA, B + s*strideB, C + s*strideC.
@@ -596,7 +615,7 @@ int nacu_dgemm_split_bf16(int m, int n, int k, double alpha, const double* A, in
                           int64_t ldb, double beta, double* C, int64_t ldc, int slices, void* workspace,
                           size_t workspace_bytes, nacu_stream_t stream);
 
-/* 1 when a split-GEMM kernel gave up waiting on a pipeline barrier (its
+/* 1 when a kernel of nacu_dgemm_split_bf16 or nacu_dgemm_ws gave up waiting on a pipeline barrier (its
  * results are then invalid), else 0; synchronous. */
 int nacu_split_gemm_error(int* flag_out);
 

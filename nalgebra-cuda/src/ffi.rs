@@ -17,6 +17,8 @@ extern "C" {
     pub fn nacu_device_count(count: *mut c_int) -> c_int;
     pub fn nacu_malloc(ptr: *mut *mut c_void, bytes: usize) -> c_int;
     pub fn nacu_free(ptr: *mut c_void) -> c_int;
+    pub fn nacu_malloc_async(ptr: *mut *mut c_void, bytes: usize, s: Stream) -> c_int;
+    pub fn nacu_free_async(ptr: *mut c_void, s: Stream) -> c_int;
     pub fn nacu_host_alloc(ptr: *mut *mut c_void, bytes: usize) -> c_int;
     pub fn nacu_host_free(ptr: *mut c_void) -> c_int;
     pub fn nacu_memcpy(dst: *mut c_void, src: *const c_void, bytes: usize, s: Stream) -> c_int;
@@ -119,6 +121,10 @@ extern "C" {
                               ws: *mut c_void, ws_bytes: usize, flags: c_int, s: Stream) -> c_int;
     pub fn nacu_dgemm(m: c_int, n: c_int, k: c_int, alpha: f64, a: *const f64, lda: i64,
                       b: *const f64, ldb: i64, beta: f64, c: *mut f64, ldc: i64, s: Stream) -> c_int;
+    pub fn nacu_dgemm_workspace_bytes(m: c_int, n: c_int, k: c_int) -> usize;
+    pub fn nacu_dgemm_ws(m: c_int, n: c_int, k: c_int, alpha: f64, a: *const f64, lda: i64,
+                         b: *const f64, ldb: i64, beta: f64, c: *mut f64, ldc: i64, ws: *mut c_void,
+                         ws_bytes: usize, s: Stream) -> c_int;
     pub fn nacu_dgemm_batched(m: c_int, n: c_int, k: c_int, alpha: f64, a: *const f64, lda: i64, stride_a: i64,
                               b: *const f64, ldb: i64, stride_b: i64, beta: f64, c: *mut f64, ldc: i64,
                               stride_c: i64, batch: c_int, flags: c_int, s: Stream) -> c_int;

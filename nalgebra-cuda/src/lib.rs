@@ -263,10 +263,22 @@ impl DeviceMatrix {
         assert!(a.ncols == b.nrows, "gemm: dimensions mismatch for multiplication.");
         assert!(self.nrows == a.nrows && self.ncols == b.ncols, "gemm: dimensions mismatch for addition.");
         let (m, n, k) = (a.nrows as c_int, b.ncols as c_int, a.ncols as c_int);
-        check(unsafe {
-            ffi::nacu_dgemm(m, n, k, alpha, a.data.as_ptr(), m.max(1) as i64, b.data.as_ptr(), k.max(1) as i64, beta,
-                            self.data.as_mut_ptr(), m.max(1) as i64, std::ptr::null_mut())
-        });
+        let bytes = unsafe { ffi::nacu_dgemm_workspace_bytes(m, n, k) };
+        let mut ws = std::ptr::null_mut();
+        // large products run on the tensor cores; without scratch, on the FP64 units
+        let scratch = bytes > 0 && unsafe { ffi::nacu_malloc_async(&mut ws, bytes, std::ptr::null_mut()) } == 0;
+        let rc = unsafe {
+            if scratch {
+                ffi::nacu_dgemm_ws(m, n, k, alpha, a.data.as_ptr(), m.max(1) as i64, b.data.as_ptr(), k.max(1) as i64,
+                                   beta, self.data.as_mut_ptr(), m.max(1) as i64, ws, bytes, std::ptr::null_mut())
+            } else {
+                ffi::nacu_dgemm(m, n, k, alpha, a.data.as_ptr(), m.max(1) as i64, b.data.as_ptr(), k.max(1) as i64,
+                                beta, self.data.as_mut_ptr(), m.max(1) as i64, std::ptr::null_mut())
+            }
+        };
+        let freed = unsafe { ffi::nacu_free_async(ws, std::ptr::null_mut()) };
+        check(rc);
+        check(freed);
     }
 
     /// The precision form for one system (no nalgebra counterpart): FP32 LU

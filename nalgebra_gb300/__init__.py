@@ -644,15 +644,22 @@ def gemm(c: DeviceMatrix, alpha: float, a: DeviceMatrix, b: DeviceMatrix, beta: 
     m, k = a.shape
     k2, n = b.shape
     assert k == k2 and c.shape == (m, n), "gemm dimension mismatch"
+    L = _lib.load()
+    sizes = (m, n, k, float(alpha), a.data.data_ptr(), max(m, 1), b.data.data_ptr(), max(k, 1), float(beta),
+             c.data.data_ptr(), max(m, 1))
     if split_slices:
-        wsb = _lib.load().nacu_gemm_split_workspace_bytes(m, n, k)
-        ws = _bytes(wsb + 1024)
-        wp = (ws.data_ptr() + 1023) // 1024 * 1024
-        _lib.call("nacu_dgemm_split_bf16", m, n, k, float(alpha), a.data.data_ptr(), max(m, 1), b.data.data_ptr(),
-                  max(k, 1), float(beta), c.data.data_ptr(), max(m, 1), int(split_slices), wp, wsb, _stream_ptr())
-    else:
-        _lib.call("nacu_dgemm", m, n, k, float(alpha), a.data.data_ptr(), max(m, 1), b.data.data_ptr(), max(k, 1),
-                  float(beta), c.data.data_ptr(), max(m, 1), _stream_ptr())
+        wsb = L.nacu_gemm_split_workspace_bytes(m, n, k)
+        with _dev.scratch(wsb + 1024) as ws:
+            _lib.call("nacu_dgemm_split_bf16", *sizes, int(split_slices), (ws + 1023) // 1024 * 1024, wsb,
+                      _stream_ptr())
+        return c
+    wsb = L.nacu_dgemm_workspace_bytes(m, n, k)
+    if wsb:  # a large product: on the tensor cores where the scratch is to be had
+        with _dev.scratch(wsb, required=False) as ws:
+            if ws:
+                _lib.call("nacu_dgemm_ws", *sizes, ws, wsb, _stream_ptr())
+                return c
+    _lib.call("nacu_dgemm", *sizes, _stream_ptr())
     return c
 
 

@@ -312,6 +312,22 @@ class DeviceBuffer:
             pass
 
 
+@contextlib.contextmanager
+def scratch(nbytes: int, required: bool = True):
+    """The address of ``nbytes`` of device scratch for calls queued on the
+    current stream inside the block (nacu_malloc_async / nacu_free_async: stream
+    order, no synchronization).  0 where the memory is not to be had and not
+    ``required``."""
+    p, s = C.c_void_p(), current_stream()
+    rc = _lib.load().nacu_malloc_async(C.byref(p), int(nbytes), s)
+    if required:
+        _lib.check(rc, "nacu_malloc_async")
+    try:
+        yield p.value or 0
+    finally:
+        _lib.call("nacu_free_async", p.value, s)
+
+
 def empty(shape, dtype=np.float64) -> DeviceBuffer:
     return DeviceBuffer.empty(shape, dtype)
 

@@ -36,6 +36,8 @@ SIGNATURES = {
     "nacu_device_count": (_i, [C.POINTER(C.c_int)]),
     "nacu_malloc": (_i, [C.POINTER(C.c_void_p), _sz]),
     "nacu_free": (_i, [_vp]),
+    "nacu_malloc_async": (_i, [C.POINTER(C.c_void_p), _sz, _vp]),
+    "nacu_free_async": (_i, [_vp, _vp]),
     "nacu_host_alloc": (_i, [C.POINTER(C.c_void_p), _sz]),
     "nacu_host_free": (_i, [_vp]),
     "nacu_memcpy": (_i, [_vp, _vp, _sz, _vp]),
@@ -100,6 +102,8 @@ SIGNATURES = {
     "nacu_dgesv_mixed_ir": (_i, [_i, _vp, _i64, _vp, _vp, _d, _i, C.POINTER(C.c_int), C.POINTER(C.c_double),
                                  C.POINTER(C.c_int), _vp, _sz, _vp]),
     "nacu_dgemm": (_i, [_i, _i, _i, _d, _vp, _i64, _vp, _i64, _d, _vp, _i64, _vp]),
+    "nacu_dgemm_workspace_bytes": (_sz, [_i, _i, _i]),
+    "nacu_dgemm_ws": (_i, [_i, _i, _i, _d, _vp, _i64, _vp, _i64, _d, _vp, _i64, _vp, _sz, _vp]),
     "nacu_dgemm_batched": (_i, [_i, _i, _i, _d, _vp, _i64, _i64, _vp, _i64, _i64, _d, _vp, _i64, _i64, _i, _i, _vp]),
     "nacu_gemm_split_workspace_bytes": (_sz, [_i, _i, _i]),
     "nacu_dgemm_split_bf16": (_i, [_i, _i, _i, _d, _vp, _i64, _vp, _i64, _d, _vp, _i64, _i, _vp, _sz, _vp]),

