@@ -18,13 +18,12 @@ int dgemm_fp64_run(int m, int n, int k, double alpha, const double* A, int64_t l
                    double beta, double* C, int64_t ldc, const int* tile_flags, int flag_ld, cudaStream_t stream);
 
 // FP64 GEMM by residues on the tensor cores (gemm_crt.cu): whether it is the
-// faster one at these sizes, its scratch, the product.  guarded = false skips
-// the test that hands tiles with strongly cancelling |A||B| to the FP64 kernel.
+// faster one at these sizes, its scratch, the product.
 bool crt_gemm_pays(int m, int n, int k);
 size_t crt_gemm_workspace_bytes(int m, int n, int k);
 int crt_gemm_run(int m, int n, int k, double alpha, const double* A, int64_t lda, const double* B, int64_t ldb,
-                 double beta, double* C, int64_t ldc, bool guarded, void* workspace, size_t workspace_bytes,
-                 cudaStream_t stream, const char* name);
+                 double beta, double* C, int64_t ldc, void* workspace, size_t workspace_bytes, cudaStream_t stream,
+                 const char* name);
 // Whether one of its kernels gave up on a barrier since the library was loaded.
 int crt_gemm_error(int* flag);
 

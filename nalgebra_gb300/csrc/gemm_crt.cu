@@ -38,14 +38,16 @@
 // 128 x 256 tile on one CTA), persistent over (plane, tile) units.  Warp 0:
 // TMA producer, warp 1 (of the leading CTA): MMA issuer, warps 2-9: epilogue,
 // 128 columns x 1 row per thread, reducing one TMEM accumulator (256 of the 512
-// columns) while the next chunk's MMAs run in the other.  Every barrier wait is
-// bounded.
+// columns) while the next chunk's MMAs run in the other and storing its residues
+// as 128-byte rows by TMA.  Every barrier wait is bounded.
 //
-// What bounds it: the tensor pipe, 17 BF16 products instead of one.  Measured
-// (GB300, scratch warm): 8192^3 878 -> 16.5 ms (53x; 17 planes at 1.50 of the
-// 1.90 PFLOP/s a BF16 GEMM reaches), 1000 x 777 x 1333 2.69 -> 0.15 ms, 256^3
-// 266 -> 55 us.  Error against sums in short blocks, N(0,1) entries: 3.9e-16
-// relative at 4096^3 where the FP64 loop has 2.2e-15.
+// What bounds it: the tensor pipe, 17 BF16 products instead of one; for K in the
+// hundreds the epilogue (156 us for the 17 planes of 4096 x 4096 x 128; 186 with
+// byte stores from registers).  Measured (GB300, scratch warm): 8192^3 878 ->
+// 16.1 ms (55x; 17 planes at 1.50 of the 1.90 PFLOP/s a BF16 GEMM reaches),
+// 1000 x 777 x 1333 2.69 -> 0.15 ms, 256^3 266 -> 59 us.  Error against sums in
+// short blocks, N(0,1) entries: 3.9e-16 relative at 4096^3 where the FP64 loop
+// has 2.2e-15.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -57,12 +59,13 @@ namespace nacu {
 namespace {
 
 constexpr int kMod = 16;               // moduli
-constexpr int kLimbs = 6;              // 21-bit limbs of P and P / p
-constexpr int kLimbBits = 21;
+constexpr int kDigits = 15;            // base-256 digits of P / p (117.8 bits), balanced
+constexpr int kKMax = 8;               // |sum_p y_p / p| <= 8: the multiples of P to subtract
 constexpr int kPM = 256, kPN = 256;    // tile of a CTA pair
 constexpr int kKB = 64;                // K of one stage: 128-byte rows, 128-byte swizzle
 constexpr int kChunkBlocks = 16;       // k-blocks per exact FP32 sum: 1024 products
 constexpr int kStagesC = 6;
+constexpr uint32_t kStoreBytes = 32 * 128;  // one epilogue warp's residues: 32 rows x 128 columns
 constexpr uint32_t kHalfTile = 128 * kKB * 2;       // 16 KB: one CTA's share of an operand tile
 constexpr uint32_t kStageBytesC = 2 * kHalfTile;
 constexpr int kCrtThreads = 320;       // producer, MMA issuer, eight epilogue warps
@@ -80,10 +83,15 @@ struct CrtTables {
   int magic[kMod];      // round-up(2^38 / p)
   int wa[kMod][3];      // residues of q, q 2^21, q 2^42 with q = (P/p)^-1 mod p (for A), balanced
   int wb[kMod][3];      // residues of 1, 2^21, 2^42 (for B), balanced
-  int limb[kMod][kLimbs];  // P / p in balanced base-2^21 digits
-  int plimb[kLimbs];       // P
-  float pinv;              // 2^105 / P
+  uint32_t digit[kMod / 4][kDigits];  // digit d of P / p for four moduli, a byte each
+  uint32_t quot[kMod / 4];            // round(2^14 / p), a byte each
 };
+
+// k P + the digit sums' bias, k = -8 .. 8, as 128-bit numbers
+struct CrtMultiples {
+  uint4 v[2 * kKMax + 1];
+};
+constexpr int kDigitBias = 1 << 18;  // |16 digits x 128| < 2^18 keeps every digit sum positive
 
 constexpr int balanced(long long v, int p) {
   long long r = v % p;
@@ -94,25 +102,26 @@ constexpr int balanced(long long v, int p) {
 constexpr CrtTables make_tables() {
   CrtTables t{};
   const int ps[kMod] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193};
-  for (int i = 0; i <= kMod; ++i) {  // i == kMod: P itself
-    long long d[kLimbs + 1] = {1, 0, 0, 0, 0, 0, 0};
+  for (int i = 0; i < kMod; ++i) {
+    long long d[kDigits + 2] = {1};
     for (int j = 0; j < kMod; ++j) {
       if (j == i) continue;
       long long carry = 0;
-      for (int l = 0; l <= kLimbs; ++l) {
+      for (int l = 0; l < kDigits + 2; ++l) {
         const long long v = d[l] * ps[j] + carry;
-        d[l] = v & ((1ll << kLimbBits) - 1);
-        carry = v >> kLimbBits;
+        d[l] = v & 255;
+        carry = v >> 8;
       }
     }
-    for (int l = 0; l < kLimbs - 1; ++l)  // balanced digits: |d| <= 2^20
-      if (d[l] >= (1ll << (kLimbBits - 1))) {
-        d[l] -= 1ll << kLimbBits;
+    for (int l = 0; l < kDigits; ++l) {
+      if (d[l] >= 128) {
+        d[l] -= 256;
         d[l + 1] += 1;
       }
-    for (int l = 0; l < kLimbs; ++l) (i < kMod ? t.limb[i][l] : t.plimb[l]) = (int)d[l];
+      t.digit[i / 4][l] |= (uint32_t)(d[l] & 255) << (8 * (i % 4));
+    }
+    t.quot[i / 4] |= (uint32_t)(((1 << 15) / ps[i] + 1) / 2) << (8 * (i % 4));
   }
-  t.pinv = (float)(1.0 / ((double)t.plimb[kLimbs - 1] + (double)t.plimb[kLimbs - 2] / (1 << kLimbBits)));
   for (int i = 0; i < kMod; ++i) {
     const int p = ps[i];
     long long r = 1;
@@ -135,6 +144,35 @@ constexpr CrtTables make_tables() {
   return t;
 }
 __constant__ CrtTables kT = make_tables();
+
+constexpr CrtMultiples make_multiples() {
+  CrtMultiples t{};
+  const int ps[kMod] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193};
+  long long d[16] = {1};  // P in base 256
+  for (int j = 0; j < kMod; ++j) {
+    long long carry = 0;
+    for (int l = 0; l < 16; ++l) {
+      const long long v = d[l] * ps[j] + carry;
+      d[l] = v & 255;
+      carry = v >> 8;
+    }
+  }
+  for (int k = -kKMax; k <= kKMax; ++k) {
+    uint32_t w[4] = {};
+    long long carry = 0;
+    for (int l = 0; l < 16; ++l) {
+      const long long v = k * d[l] + (l < kDigits + 1 ? kDigitBias : 0) + carry;
+      w[l / 4] |= (uint32_t)(v & 255) << (8 * (l % 4));
+      carry = v >> 8;
+    }
+    t.v[k + kKMax].x = w[0];
+    t.v[k + kKMax].y = w[1];
+    t.v[k + kKMax].z = w[2];
+    t.v[k + kKMax].w = w[3];
+  }
+  return t;
+}
+__constant__ CrtMultiples kP = make_multiples();
 
 // ---- scaling ------------------------------------------------------------------------------------------------
 
@@ -231,7 +269,7 @@ __global__ void __launch_bounds__(128) crt_row_stats_kernel(int m, int k, const 
 // k tile also write the row scales.
 __global__ void __launch_bounds__(256) crt_split_a_kernel(int m, int k, const double* __restrict__ A, int64_t lda,
                                                           const int2* __restrict__ part, int nparts, int mp, int kp,
-                                                          int planes, int* __restrict__ rscale,
+                                                          int* __restrict__ rscale,
                                                           uint32_t* __restrict__ out) {
   __shared__ long long t[64][33];
   __shared__ int s_scale[32];
@@ -269,17 +307,15 @@ __global__ void __launch_bounds__(256) crt_split_a_kernel(int m, int k, const do
     uint32_t* o = out + ((size_t)(i0 + r) * kp + k0) / 2 + lane;
 #pragma unroll
     for (int i = 0; i < kMod; ++i) o[i * plane] = pack_hi(residue_bits(a0, kT.wa[i], i), residue_bits(a1, kT.wa[i], i));
-    if (planes > kMod) {
-      const bool bad = s_scale[r] == kBadScale;
-      o[kMod * plane] = pack_hi(abs_bits(v0, bad), abs_bits(v1, bad));
-    }
+    const bool bad = s_scale[r] == kBadScale;
+    o[kMod * plane] = pack_hi(abs_bits(v0, bad), abs_bits(v1, bad));
   }
 }
 
 // B (columns contiguous along K) -> residue planes [plane][np][kp] and the
 // column scales; one CTA per (padded) column.
 __global__ void __launch_bounds__(256) crt_split_b_kernel(int k, int n, const double* __restrict__ B, int64_t ldb, int np,
-                                                          int kp, int planes, int* __restrict__ cscale,
+                                                          int kp, int* __restrict__ cscale,
                                                           uint32_t* __restrict__ out) {
   __shared__ int s_e[8];
   __shared__ float s_s[8];
@@ -317,7 +353,7 @@ __global__ void __launch_bounds__(256) crt_split_b_kernel(int k, int n, const do
     uint32_t* o = out + ((size_t)j * kp + c) / 2;
 #pragma unroll
     for (int i = 0; i < kMod; ++i) o[i * plane] = pack_hi(residue_bits(b0, kT.wb[i], i), residue_bits(b1, kT.wb[i], i));
-    if (planes > kMod) o[kMod * plane] = pack_hi(abs_bits(v0, bad), abs_bits(v1, bad));
+    o[kMod * plane] = pack_hi(abs_bits(v0, bad), abs_bits(v1, bad));
   }
 }
 
@@ -349,6 +385,11 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m
       "l"(map), "r"(x), "r"(y), "r"(bar)
       : "memory");
 }
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, const void* src) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x), "r"(y),
+               "r"(smem_u32(src))
+               : "memory");
+}
 __device__ __forceinline__ void mma_pair(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accum) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
@@ -374,8 +415,7 @@ struct CrtArgs {
   int m, n;            // valid rows / columns of this block
   int mp, np;          // padded to 256
   int kblocks;         // kp / 64
-  int planes;          // kMod, or kMod + 1 with the ratio plane
-  int8_t* R;           // [kMod][np][mp] residues of the product
+  int8_t* R;           // [kMod][mp][np] residues of the product, a row's columns contiguous
   const int* rscale;
   const int* cscale;
   int* flags;          // [np / 128][mp / 128]
@@ -392,8 +432,29 @@ __device__ __forceinline__ void unit_tile(int u, int tiles, int tm, int tn, int*
   *ni = in / h;
 }
 
+// Sixteen FP32 integers -> their balanced residues mod p as bytes (p = 256:
+// 128 wraps to -128, the same residue).
+__device__ __forceinline__ uint4 reduce_pack16(const uint32_t* v, float p, float inv) {
+  uint32_t w[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint32_t b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float x = __uint_as_float(v[4 * j + i]);
+      const float k = fmaf(x, inv, 12582912.f) - 12582912.f;
+      b[i] = __float_as_uint(fmaf(-p, k, x) + 12582912.f);  // the integer in the low mantissa bits
+    }
+    w[j] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// ONE_CHUNK: K <= 1024, one exact sum per output and no register accumulators.
+template <bool ONE_CHUNK>
 __global__ void __launch_bounds__(kCrtThreads, 1) __cluster_dims__(2, 1, 1)
-    crt_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const CrtArgs g) {
+    crt_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
+                    const __grid_constant__ CUtensorMap mapR, const CrtArgs g) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t full_bar[kStagesC], empty_bar[kStagesC], acc_full[2], acc_empty[2];
@@ -401,7 +462,7 @@ __global__ void __launch_bounds__(kCrtThreads, 1) __cluster_dims__(2, 1, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = blockIdx.x & 1;
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
-  const int tm = g.mp / kPM, tn = g.np / kPN, tiles = tm * tn, units = tiles * g.planes;
+  const int tm = g.mp / kPM, tn = g.np / kPN, tiles = tm * tn, units = tiles * (kMod + 1);
   const int nchunks = (g.kblocks + kChunkBlocks - 1) / kChunkBlocks;
 
   if (threadIdx.x == 0) {
@@ -487,6 +548,8 @@ __global__ void __launch_bounds__(kCrtThreads, 1) __cluster_dims__(2, 1, 1)
     // epilogue: TMEM lanes 32 (warp mod 4) .. + 31 (this CTA's rows), 128 of the 256 columns
     const int q = warp & 3, half = (warp - 2) >> 2;
     const int row_in = (int)rank * 128 + q * 32 + lane;
+    unsigned char* stage_warp = smem + (size_t)kStagesC * kStageBytesC + (size_t)(warp - 2) * kStoreBytes;
+    unsigned char* stage = stage_warp + lane * 128;
     int gc = 0;
     bool ok = true;
     for (int u = pair; u < units && ok; u += npairs) {
@@ -494,9 +557,18 @@ __global__ void __launch_bounds__(kCrtThreads, 1) __cluster_dims__(2, 1, 1)
       unit_tile(u, tiles, tm, tn, &plane, &mi, &ni);
       const bool residue = plane < kMod;
       const float p = residue ? kT.pf[plane] : 0.f, inv = residue ? kT.inv[plane] : 0.f;
+      const int row = mi * kPM + row_in, col0 = ni * kPN + half * 128;
+      // this warp's staging: row `lane`, 16-byte column groups swizzled by the
+      // row (the tensor map's 128-byte swizzle); its last store has been read
+      if (residue) {
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        __syncwarp();
+      }
       float acc[128];
+      if constexpr (!ONE_CHUNK) {
 #pragma unroll
-      for (int i = 0; i < 128; ++i) acc[i] = 0.f;
+        for (int i = 0; i < 128; ++i) acc[i] = 0.f;
+      }
       for (int ch = 0; ch < nchunks; ++ch, ++gc) {
         const int slot = gc & 1;
         if (!mbar_wait(&acc_full[slot], (uint32_t)(gc >> 1) & 1u)) {
@@ -515,11 +587,20 @@ __global__ void __launch_bounds__(kCrtThreads, 1) __cluster_dims__(2, 1, 1)
               : "r"(taddr + (uint32_t)c0));
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           // x - p round(x / p), exact (integers up to 2^24; p = 0 on the ratio plane: x itself)
+          if constexpr (ONE_CHUNK) {
+            if (residue) {
+              *reinterpret_cast<uint4*>(stage + (((c0 / 16) ^ (lane & 7)) << 4)) = reduce_pack16(v, p, inv);
+            } else {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const float x = __uint_as_float(v[i]);
-            const float k = fmaf(x, inv, 12582912.f) - 12582912.f;
-            acc[c0 + i] += fmaf(-p, k, x);
+              for (int i = 0; i < 16; ++i) acc[c0 + i] = __uint_as_float(v[i]);
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const float x = __uint_as_float(v[i]);
+              const float k = fmaf(x, inv, 12582912.f) - 12582912.f;
+              acc[c0 + i] += fmaf(-p, k, x);
+            }
           }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -527,14 +608,18 @@ __global__ void __launch_bounds__(kCrtThreads, 1) __cluster_dims__(2, 1, 1)
         if (lane == 0) remote_arrive(mapa_u32(smem_u32(&acc_empty[slot]), 0));
       }
       if (!ok) break;
-      const int row = mi * kPM + row_in, col0 = ni * kPN + half * 128;
       if (residue) {
-        int8_t* out = g.R + ((size_t)plane * g.np + col0) * g.mp + row;
+        if constexpr (!ONE_CHUNK) {
 #pragma unroll
-        for (int i = 0; i < 128; ++i) {
-          const float k = fmaf(acc[i], inv, 12582912.f) - 12582912.f;
-          // the balanced residue as an integer in the low mantissa bits; 128 (p = 256) wraps to -128
-          out[(size_t)i * g.mp] = (int8_t)__float_as_int(fmaf(-p, k, acc[i]) + 12582912.f);
+          for (int c0 = 0; c0 < 128; c0 += 16)
+            *reinterpret_cast<uint4*>(stage + (((c0 / 16) ^ (lane & 7)) << 4)) =
+                reduce_pack16(reinterpret_cast<uint32_t*>(acc + c0), p, inv);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_2d(&mapR, col0, plane * g.mp + row, stage_warp);
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
       } else {
         bool bad = false;
@@ -550,6 +635,7 @@ __global__ void __launch_bounds__(kCrtThreads, 1) __cluster_dims__(2, 1, 1)
         if (bad) g.flags[(col0 / kFlagTile) * (g.mp / kFlagTile) + row / kFlagTile] = 1;
       }
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -560,62 +646,134 @@ __global__ void __launch_bounds__(kCrtThreads, 1) __cluster_dims__(2, 1, 1)
 // ---- residues -> C ------------------------------------------------------------------------------------------
 __device__ __forceinline__ double pow2d(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
 
-// One thread: four consecutive rows of one column.  P / 4 bounds |X|, so the
-// multiple of P to subtract is the nearest integer of a float quotient.
-__global__ void __launch_bounds__(256) crt_combine_kernel(CrtArgs g, double alpha, double beta, double* __restrict__ C,
-                                                          int64_t ldc, int check) {
-  const int i0 = (blockIdx.x * 64 + (threadIdx.x & 63)) * 4, j = blockIdx.y * 4 + (threadIdx.x >> 6);
-  if (i0 >= g.m || j >= g.n) return;
-  if (check && g.flags[(j / kFlagTile) * (g.mp / kFlagTile) + i0 / kFlagTile]) return;  // the FP64 kernel's tile
-  uint32_t y[kMod];
-  const uint32_t* r = reinterpret_cast<const uint32_t*>(g.R + (size_t)j * g.mp + i0);
-  const size_t plane = (size_t)g.np * g.mp / 4;
+// x 2^e for a signed 128-bit x (x.w the top word), rounded to nearest even by
+// integer instructions: conversions and multiplies would each take the FP64
+// pipe, which issues two lanes per cycle and SM.
+__device__ __forceinline__ double scaled_double(uint4 x, int e) {
+  const uint32_t sign = (uint32_t)((int)x.w >> 31);
+  {  // |x|
+    asm("{\n .reg .u32 c;\n and.b32 c, %4, 1;\n xor.b32 %0, %0, %4;\n xor.b32 %1, %1, %4;\n xor.b32 %2, %2, %4;\n"
+        " xor.b32 %3, %3, %4;\n add.cc.u32 %0, %0, c;\n addc.cc.u32 %1, %1, 0;\n addc.cc.u32 %2, %2, 0;\n"
+        " addc.u32 %3, %3, 0;\n}"
+        : "+r"(x.x), "+r"(x.y), "+r"(x.z), "+r"(x.w)
+        : "r"(sign));
+  }
+  // the leading one into the top word: whole words first (rare: |x| < 2^96)
+  int lead = 127;
+  while (x.w == 0u) {
+    if ((x.x | x.y | x.z) == 0u) return 0.0;
+    x.w = x.z;
+    x.z = x.y;
+    x.y = x.x;
+    x.x = 0u;
+    lead -= 32;
+  }
+  const int z = __clz((int)x.w);
+  const uint32_t t1 = __funnelshift_l(x.z, x.w, z), t0 = __funnelshift_l(x.y, x.z, z);
+  const uint32_t rest = (t0 & 0x7ffu) | (((x.y << z) | x.x) != 0u ? 1u : 0u);
+  uint32_t hi = t1 >> 11, lo = __funnelshift_r(t0, t1, 11);
+  const uint32_t up = (rest + (lo & 1u)) > 0x400u ? 1u : 0u;
+  asm("add.cc.u32 %0, %0, %2;\n addc.u32 %1, %1, 0;" : "+r"(lo), "+r"(hi) : "r"(up));
+  const int ex = 1023 + lead - z + e;  // biased exponent of the leading one
+  if (ex > 0 && ex < 2046)  // hi's leading one adds the last 1; a carry moves on
+    return __hiloint2double((int)((hi + ((uint32_t)(ex - 1) << 20)) | (sign & 0x80000000u)), (int)lo);
+  // over- or underflow in the result: the scaling in two exact halves
+  const double v = (double)(((unsigned long long)hi << 32) | lo);
+  const int e0 = ex - 1023 - 52, e1 = e0 / 2;
+  const double r = v * pow2d(max(min(e1, 1000), -1000)) * pow2d(max(min(e0 - e1, 1000), -1000));
+  return sign ? -r : r;
+}
+
+// The digits of X for four elements at a time: byte dot products of the
+// residues with the digits of P / p (dp4a, four moduli each), the sums carried
+// into a 128-bit number, the nearest multiple of P subtracted (|X| < P / 4, so
+// the quotient sum y_p / p needs no more than 14-bit weights).
+//
+// One thread: 4 rows x 4 columns, a warp 16 x 32 (32-byte pieces of R's rows
+// and of C's columns).  Bound by instruction issue: 200 per element, 112 us for
+// 4096 x 4096 (with 21-bit limbs in 64-bit words and FP64 conversions 280 and
+// 200 us; the bytes would take 100).
+__global__ void __launch_bounds__(128) crt_combine_kernel(CrtArgs g, double alpha, double beta, double* __restrict__ C,
+                                                          int64_t ldc) {
+  __shared__ uint4 s_mult[2 * kKMax + 1];
+  if (threadIdx.x < 2 * kKMax + 1) s_mult[threadIdx.x] = kP.v[threadIdx.x];
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i0 = blockIdx.x * 64 + warp * 16 + (lane >> 3), j0 = blockIdx.y * 32 + (lane & 7) * 4;
+  if (j0 >= g.n) return;
+  if (g.flags[(j0 / kFlagTile) * (g.mp / kFlagTile) + i0 / kFlagTile]) return;  // the FP64 kernel's tile
+  const size_t plane = (size_t)g.mp * g.np / 4;
+  const int4 cs = *reinterpret_cast<const int4*>(g.cscale + j0);
+#pragma unroll 1
+  for (int r = 0; r < 4; ++r) {
+    const int i = i0 + 4 * r;
+    if (i >= g.m) return;
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(g.R) + ((size_t)i * g.np + j0) / 4;
+    uint32_t y[kMod];
 #pragma unroll
-  for (int p = 0; p < kMod; ++p) y[p] = r[p * plane];
-  const int cs = g.cscale[j];
-  const double sc = cs < kZeroScale ? pow2d(-cs) : 0.0;
+    for (int p = 0; p < kMod; ++p) y[p] = src[p * plane];
+    const int rs = g.rscale[i];
+    // 4 x 4 byte transposes: y[4 h + c] = the residues of column c for moduli 4 h .. 4 h + 3
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const int i = i0 + e;
-    int acc[kLimbs] = {0, 0, 0, 0, 0, 0};
-#pragma unroll
-    for (int p = 0; p < kMod; ++p) {
-      const int v = (int)(y[p] << (24 - 8 * e)) >> 24;
-#pragma unroll
-      for (int l = 0; l < kLimbs; ++l) acc[l] += v * kT.limb[p][l];
+    for (int h = 0; h < kMod; h += 4) {
+      const uint32_t a = __byte_perm(y[h], y[h + 1], 0x5140), b = __byte_perm(y[h], y[h + 1], 0x7362);
+      const uint32_t c = __byte_perm(y[h + 2], y[h + 3], 0x5140), d = __byte_perm(y[h + 2], y[h + 3], 0x7362);
+      y[h] = __byte_perm(a, c, 0x5410);
+      y[h + 1] = __byte_perm(a, c, 0x7632);
+      y[h + 2] = __byte_perm(b, d, 0x5410);
+      y[h + 3] = __byte_perm(b, d, 0x7632);
     }
-    const float z = ((float)acc[5] + (float)acc[4] * 4.76837158203125e-07f) * kT.pinv;
-    const int kq = __float2int_rn(z);
 #pragma unroll
-    for (int l = 0; l < kLimbs; ++l) acc[l] -= kq * kT.plimb[l];
-    // carries through the low limbs, then two 63-bit halves
-    long long lo = (long long)acc[0] + ((long long)acc[1] << kLimbBits);
-    long long mid = (long long)acc[2] + (lo >> (2 * kLimbBits));
-    lo &= (1ll << (2 * kLimbBits)) - 1;
-    lo |= (mid & ((1ll << kLimbBits) - 1)) << (2 * kLimbBits);
-    const long long hi = (mid >> kLimbBits) + (long long)acc[3] + ((long long)acc[4] << kLimbBits) +
-                         ((long long)acc[5] << (2 * kLimbBits));
-    const double x = fma((double)hi, 9223372036854775808.0, (double)lo);  // X
-    if (i < g.m) {
-      const int rs = g.rscale[i];
-      const double sr = rs < kZeroScale ? pow2d(-rs) : 0.0;
-      double* cp = C + (size_t)j * ldc + i;
-      const double v = x * sr * sc;
-      *cp = (beta == 0.0) ? alpha * v : fma(alpha, v, beta * *cp);
+    for (int c = 0; c < 4; ++c) {
+      int q = 1 << 13;
+      uint32_t t[8];
+#pragma unroll
+      for (int h = 0; h < kMod / 4; ++h) q = __dp4a((int)y[4 * h + c], (int)kT.quot[h], q);
+#pragma unroll
+      for (int l = 0; l < 16; l += 2) {
+        int s0 = kDigitBias, s1 = kDigitBias;
+#pragma unroll
+        for (int h = 0; h < kMod / 4; ++h) {
+          s0 = __dp4a((int)y[4 * h + c], (int)kT.digit[h][l], s0);
+          if (l + 1 < kDigits) s1 = __dp4a((int)y[4 * h + c], (int)kT.digit[h][l + 1], s1);
+        }
+        t[l / 2] = (uint32_t)s0 + ((uint32_t)s1 << 8);
+      }
+      const uint4 kp = s_mult[(q >> 14) + kKMax];
+      unsigned long long u[4];
+#pragma unroll
+      for (int l = 0; l < 4; ++l) u[l] = (unsigned long long)t[2 * l + 1] * 65536ull + t[2 * l];
+      uint4 x;
+      x.x = (uint32_t)u[0];
+      asm("add.cc.u32 %0, %3, %4;\n addc.cc.u32 %1, %5, %6;\n addc.u32 %2, %7, %8;"
+          : "=&r"(x.y), "=&r"(x.z), "=&r"(x.w)
+          : "r"((uint32_t)(u[0] >> 32)), "r"((uint32_t)u[1]), "r"((uint32_t)(u[1] >> 32)), "r"((uint32_t)u[2]),
+            "r"((uint32_t)(u[2] >> 32)), "r"((uint32_t)u[3]));
+      asm("sub.cc.u32 %0, %0, %4;\n subc.cc.u32 %1, %1, %5;\n subc.cc.u32 %2, %2, %6;\n subc.u32 %3, %3, %7;"
+          : "+r"(x.x), "+r"(x.y), "+r"(x.z), "+r"(x.w)
+          : "r"(kp.x), "r"(kp.y), "r"(kp.z), "r"(kp.w));
+      // an all-zero row or column has X = 0, whatever its scale's code
+      const double v = scaled_double(x, -(rs + (c == 0 ? cs.x : c == 1 ? cs.y : c == 2 ? cs.z : cs.w)));
+      if (j0 + c < g.n) {
+        double* cp = C + (size_t)(j0 + c) * ldc + i;
+        if (beta == 0.0) *cp = alpha == 1.0 ? v : alpha * v;
+        else if (beta == 1.0) *cp = fma(alpha, v, *cp);
+        else *cp = fma(alpha, v, beta * *cp);
+      }
     }
   }
 }
 
-int make_plane_map(CUtensorMap* map, void* base, uint64_t rows, uint64_t kp) {
+int make_map(CUtensorMap* map, CUtensorMapDataType type, uint64_t elem, void* base, uint64_t rows, uint64_t cols,
+             uint32_t box_rows, uint32_t box_cols) {
   EncodeTiledFn f = encode_fn();
   if (!f) return record_arg_error(-100, "dgemm: cuTensorMapEncodeTiled unavailable");
-  const cuuint64_t dims[2] = {kp, rows};
-  const cuuint64_t strides[1] = {kp * 2};
-  const cuuint32_t box[2] = {kKB, 128};
+  const cuuint64_t dims[2] = {cols, rows};
+  const cuuint64_t strides[1] = {cols * elem};
+  const cuuint32_t box[2] = {box_cols, box_rows};
   const cuuint32_t estr[2] = {1, 1};
-  CUresult r = f(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr,
-                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = f(map, type, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? NACU_SUCCESS : record_arg_error(-101, "dgemm: cuTensorMapEncodeTiled failed");
 }
 
@@ -665,7 +823,7 @@ size_t crt_gemm_workspace_bytes(int m, int n, int k) {
 // CTA pairs the device keeps resident (a die whose SM count is odd leaves one SM without a partner).
 static int crt_max_pairs(size_t smem) {
   static int pairs = 0;
-  if (pairs == 0) {
+  if (pairs == 0 && ensure_dynamic_smem(crt_gemm_kernel<false>, smem) == cudaSuccess) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)sm_count() & ~1u);
     cfg.blockDim = dim3(kCrtThreads);
@@ -677,19 +835,18 @@ static int crt_max_pairs(size_t smem) {
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     int c = 0;
-    if (cudaOccupancyMaxActiveClusters(&c, crt_gemm_kernel, &cfg) != cudaSuccess || c < 1) {
+    if (cudaOccupancyMaxActiveClusters(&c, crt_gemm_kernel<false>, &cfg) != cudaSuccess || c < 1) {
       (void)cudaGetLastError();
       c = std::max(1, sm_count() / 2);
     }
     pairs = c;
   }
-  return pairs;
+  return std::max(pairs, 1);
 }
 
-// guarded: form the ratio plane and hand tiles it rejects to the FP64 kernel.
 int crt_gemm_run(int m, int n, int k, double alpha, const double* A, int64_t lda, const double* B, int64_t ldb,
-                 double beta, double* C, int64_t ldc, bool guarded, void* workspace, size_t workspace_bytes,
-                 cudaStream_t s, const char* name) {
+                 double beta, double* C, int64_t ldc, void* workspace, size_t workspace_bytes, cudaStream_t s,
+                 const char* name) {
   const CrtLayout L = crt_layout(m, n, k);
   if (!workspace || workspace_bytes < L.total) return record_arg_error(-13, "dgemm: workspace too small");
   unsigned char* ws = reinterpret_cast<unsigned char*>(round_up(reinterpret_cast<uintptr_t>(workspace), 1024));
@@ -699,9 +856,10 @@ int crt_gemm_run(int m, int n, int k, double alpha, const double* A, int64_t lda
   int* rs = reinterpret_cast<int*>(ws + L.rs_off);
   int* cs = reinterpret_cast<int*>(ws + L.cs_off);
   int* flags = reinterpret_cast<int*>(ws + L.flag_off);
-  const int planes = guarded ? kMod + 1 : kMod;
-  constexpr size_t smem = (size_t)kStagesC * kStageBytesC + 1024;
-  cudaError_t e = ensure_dynamic_smem(crt_gemm_kernel, smem);
+  constexpr int planes = kMod + 1;  // and the ratio plane
+  constexpr size_t smem = (size_t)kStagesC * kStageBytesC + 8 * kStoreBytes + 1024;
+  const auto kern = std::min(k, kBlockK) <= kChunkBlocks * kKB ? crt_gemm_kernel<true> : crt_gemm_kernel<false>;
+  cudaError_t e = ensure_dynamic_smem(kern, smem);
   if (e != cudaSuccess) return record_cuda_error(e, name);
   const int pairs = crt_max_pairs(smem);
   for (int k0 = 0; k0 < k; k0 += kBlockK) {
@@ -709,29 +867,30 @@ int crt_gemm_run(int m, int n, int k, double alpha, const double* A, int64_t lda
     const double bt = k0 == 0 ? beta : 1.0;
     for (int n0 = 0; n0 < n; n0 += kBlockMN) {
       const int nc = std::min(kBlockMN, n - n0), np = (int)round_up((size_t)nc, kPN);
-      crt_split_b_kernel<<<np, 256, 0, s>>>(kc, nc, B + (size_t)n0 * ldb + k0, ldb, np, kp, planes, cs, bp);
+      crt_split_b_kernel<<<np, 256, 0, s>>>(kc, nc, B + (size_t)n0 * ldb + k0, ldb, np, kp, cs, bp);
       for (int m0 = 0; m0 < m; m0 += kBlockMN) {
         const int mc = std::min(kBlockMN, m - m0), mp = (int)round_up((size_t)mc, kPM);
         const double* a = A + (size_t)k0 * lda + m0;
         double* c = C + (size_t)n0 * ldc + m0;
         const int nparts = (kc + kStatChunk - 1) / kStatChunk;
         crt_row_stats_kernel<<<dim3((mc + 127) / 128, nparts), 128, 0, s>>>(mc, kc, a, lda, part);
-        crt_split_a_kernel<<<dim3(kp / 64, mp / 32), 256, 0, s>>>(mc, kc, a, lda, part, nparts, mp, kp, planes, rs, ap);
+        crt_split_a_kernel<<<dim3(kp / 64, mp / 32), 256, 0, s>>>(mc, kc, a, lda, part, nparts, mp, kp, rs, ap);
         const int nflags = (mp / kFlagTile) * (np / kFlagTile);
-        if (guarded) {
-          e = cudaMemsetAsync(flags, 0, (size_t)nflags * 4, s);
-          if (e != cudaSuccess) return record_cuda_error(e, name);
-        }
-        CUtensorMap mapA, mapB;
-        int rc = make_plane_map(&mapA, ap, (uint64_t)planes * mp, kp);
-        if (rc == NACU_SUCCESS) rc = make_plane_map(&mapB, bp, (uint64_t)planes * np, kp);
+        e = cudaMemsetAsync(flags, 0, (size_t)nflags * 4, s);
+        if (e != cudaSuccess) return record_cuda_error(e, name);
+        CUtensorMap mapA, mapB, mapR;
+        int rc = make_map(&mapA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ap, (uint64_t)planes * mp, kp, 128, kKB);
+        if (rc == NACU_SUCCESS)
+          rc = make_map(&mapB, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, bp, (uint64_t)planes * np, kp, 128, kKB);
+        if (rc == NACU_SUCCESS)
+          rc = make_map(&mapR, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, ws + L.r_off, (uint64_t)kMod * mp, np, 32, 128);
         if (rc != NACU_SUCCESS) return rc;
-        CrtArgs g{mc, nc, mp, np, kp / kKB, planes, reinterpret_cast<int8_t*>(ws + L.r_off), rs, cs, flags};
+        CrtArgs g{mc, nc, mp, np, kp / kKB, reinterpret_cast<int8_t*>(ws + L.r_off), rs, cs, flags};
         const int units = (mp / kPM) * (np / kPN) * planes;
-        crt_gemm_kernel<<<2 * std::min(units, pairs), kCrtThreads, smem, s>>>(mapA, mapB, g);
-        crt_combine_kernel<<<dim3((mc + 255) / 256, (nc + 3) / 4), 256, 0, s>>>(g, alpha, bt, c, ldc, guarded ? 1 : 0);
+        kern<<<2 * std::min(units, pairs), kCrtThreads, smem, s>>>(mapA, mapB, mapR, g);
+        crt_combine_kernel<<<dim3((mc + 63) / 64, (nc + 31) / 32), 128, 0, s>>>(g, alpha, bt, c, ldc);
         rc = check_launch(name);
-        if (rc == NACU_SUCCESS && guarded)
+        if (rc == NACU_SUCCESS)
           rc = dgemm_fp64_run(mc, nc, kc, alpha, a, lda, B + (size_t)n0 * ldb + k0, ldb, bt, c, ldc, flags,
                               mp / kFlagTile, s);
         if (rc != NACU_SUCCESS) return rc;

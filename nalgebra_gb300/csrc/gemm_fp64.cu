@@ -149,6 +149,6 @@ extern "C" int nacu_dgemm_ws(int m, int n, int k, double alpha, const double* A,
     return dgemm_fp64_run(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, nullptr, 0, (cudaStream_t)stream);
   if (!workspace || workspace_bytes < need)
     return record_arg_error(-13, "dgemm_ws: workspace smaller than nacu_dgemm_workspace_bytes (argument 13)");
-  return crt_gemm_run(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, true, workspace, workspace_bytes,
-                      (cudaStream_t)stream, "nacu_dgemm_ws");
+  return crt_gemm_run(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, workspace, workspace_bytes, (cudaStream_t)stream,
+                      "nacu_dgemm_ws");
 }
