@@ -11,8 +11,10 @@
 //      column (candidate pivots published; pivot row swapped);
 //   2. the panel's row swaps applied to the columns left and right of it;
 //   3. U12 = L11^-1 A12 (unit lower triangular solve, one thread per column);
-//   4. A22 -= L21 U12 by the GEMM kernels (FP64 DFMA, or the BF16-split
-//      tensor-core GEMM for the FP32 factor).
+//   4. A22 -= L21 U12 by the GEMM kernels: residues on the tensor cores for
+//      FP64 (gemm_crt.cu; n = 8192: 330 -> 117 ms, n = 1000: 4.6 -> 4.2 ms against
+//      the FP64 pipe, whose error is the larger one), the BF16-split tensor-core
+//      GEMM for the FP32 factor.
 // The triangular solves for the right-hand side run as one cooperative kernel
 // per triangle: the diagonal block of each step is solved by CTA 0 while all
 // CTAs then apply it to the remaining rows (coalesced GEMV), one grid barrier
@@ -1132,10 +1134,36 @@ int getrs_one(int n, const T* LU, int64_t lda, const int32_t* ipiv, T* x, int32_
   return check_launch(name);
 }
 
-int update_fp64(int m, int n, int k, const void* L21, const void* U12, void* A22, int64_t lda, void*, int,
+struct Update64Ctx {
+  void* ws[2];  // scratch of the tensor-core product, one per concurrent update (slot); null: the FP64 kernel
+  size_t ws_bytes[2];
+};
+
+int update_fp64(int m, int n, int k, const void* L21, const void* U12, void* A22, int64_t lda, void* ctx, int slot,
                 cudaStream_t s) {
-  return nacu_dgemm(m, n, k, -1.0, static_cast<const double*>(L21), lda, static_cast<const double*>(U12), lda, 1.0,
-                    static_cast<double*>(A22), lda, s);
+  const Update64Ctx* c = static_cast<const Update64Ctx*>(ctx);
+  const double *a = static_cast<const double*>(L21), *b = static_cast<const double*>(U12);
+  double* d = static_cast<double*>(A22);
+  if (c && c->ws[slot] && c->ws_bytes[slot] >= crt_gemm_workspace_bytes(m, n, k))
+    return crt_gemm_run(m, n, k, -1.0, a, lda, b, lda, 1.0, d, lda, c->ws[slot], c->ws_bytes[slot], s, "nacu_dgetrf");
+  return nacu_dgemm(m, n, k, -1.0, a, lda, b, lda, 1.0, d, lda, s);
+}
+
+constexpr int kNb64 = 64;  // panel width of the FP64 factorization
+
+// The FP64 factorization's workspace: the panel's exchange area, then the
+// scratch of the two concurrent updates.
+struct Getrf64Layout {
+  size_t slot[2], bytes[2], total;
+};
+Getrf64Layout getrf64_layout(int n) {
+  Getrf64Layout L;
+  L.bytes[0] = crt_gemm_workspace_bytes(n, kNb64, kNb64);
+  L.bytes[1] = crt_gemm_workspace_bytes(n, n, kNb64);
+  L.slot[0] = getrf_ws_bytes();
+  L.slot[1] = L.slot[0] + L.bytes[0];
+  L.total = L.slot[1] + L.bytes[1];
+  return L;
 }
 
 // ---------------------------------------------------------------------------
@@ -1596,7 +1624,7 @@ int nacu_dgesv_mixed_ir(int n, const double* A, int64_t lda, const double* b, do
     // FP64 fallback on a copy of A
     fallback = 1;
     cudaMemcpy2DAsync(A64, (size_t)n * 8, A, (size_t)lda * 8, (size_t)n * 8, n, cudaMemcpyDeviceToDevice, s);
-    rc = nacu_dgetrf(n, A64, n, ipiv, info, cand, getrf_ws_bytes(), stream);
+    rc = getrf_blocked<double>(n, A64, n, ipiv, info, cand, kNb64, update_fp64, nullptr, s, "nacu_dgesv_mixed_ir");
     if (rc != NACU_SUCCESS) return rc;
     cudaMemcpyAsync(x, b, (size_t)n * 8, cudaMemcpyDeviceToDevice, s);
     rc = nacu_dgetrs(n, A64, n, ipiv, x, info + 1, cand, getrf_ws_bytes(), stream);
@@ -1616,7 +1644,7 @@ int nacu_dgesv_mixed_ir(int n, const double* A, int64_t lda, const double* b, do
 }
 
 size_t nacu_getrf_workspace_bytes(int n) {
-  return std::max(nacu::getrf_ws_bytes(), nacu::trsv_sync_bytes(n < 0 ? 0 : n));
+  return std::max(nacu::getrf64_layout(n < 0 ? 0 : n).total, nacu::trsv_sync_bytes(n < 0 ? 0 : n));
 }
 
 int nacu_dgetrf(int n, double* A, int64_t lda, int32_t* ipiv, int32_t* info, void* workspace, size_t workspace_bytes,
@@ -1629,7 +1657,10 @@ int nacu_dgetrf(int n, double* A, int64_t lda, int32_t* ipiv, int32_t* info, voi
   if (!ipiv || !info) return record_arg_error(-4, "dgetrf: null ipiv or info");
   if (!workspace || workspace_bytes < nacu_getrf_workspace_bytes(n))
     return record_arg_error(-6, "dgetrf: workspace too small");
-  return getrf_blocked<double>(n, A, lda, ipiv, info, workspace, 64, update_fp64, nullptr, (cudaStream_t)stream,
+  const Getrf64Layout L = getrf64_layout(n);
+  unsigned char* ws = static_cast<unsigned char*>(workspace);
+  Update64Ctx ctx{{ws + L.slot[0], ws + L.slot[1]}, {L.bytes[0], L.bytes[1]}};
+  return getrf_blocked<double>(n, A, lda, ipiv, info, workspace, kNb64, update_fp64, &ctx, (cudaStream_t)stream,
                                "nacu_dgetrf");
 }
 
