@@ -39,7 +39,9 @@ __device__ __forceinline__ bool chol_pivot(T d, int has_subst, double subst, T* 
     *denom = sqrt(v);
     *rcp = T(1) / *denom;
   } else {
-    const T r = rsqrt(v);
+    T r;
+    if constexpr (sizeof(T) == 8) r = rsqrt_halley(v);
+    else r = rsqrt(v);
     *rcp = r;
     *denom = v * r;
   }

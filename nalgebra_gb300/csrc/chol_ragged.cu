@@ -20,11 +20,18 @@
 // factor is bit-identical to nalgebra's.  The triangular solves are blocked by
 // 32 rows: one warp solves each diagonal block out of registers with shuffles,
 // the whole CTA applies the block to the remaining rows.
+//
+// That panel form spends its time on the FP64 pipe (0.70 of its peak).  In the
+// FMA form, orders above 32 go to chol_tc.cuh instead, which takes the trailing
+// updates and the back solve to the tensor cores: 20000 systems of order 8..256
+// with four right-hand sides 37.7 -> 16.9 ms, 3000 of order 256 19.0 -> 7.0 ms
+// (a quarter of the FP64 instructions; the pipe is 46% busy, instruction issue 41%,
+// the rest is the serial heads' latency with two matrices on an SM).
 #include <atomic>
 #include <algorithm>
 #include <vector>
 
-#include "chol_device.cuh"
+#include "chol_tc.cuh"
 
 namespace nacu {
 namespace {
@@ -150,6 +157,99 @@ __global__ void __launch_bounds__(THREADS, MINB) chol_ragged_kernel(CholArgs g) 
   }
 }
 
+// The same system through chol_tc.cuh (FMA form, factor wanted): up to
+// kTcMaxRhs right-hand sides take their forward solve along, more are solved
+// from the factor.
+template <int THREADS, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) chol_tc_kernel(CholArgs g) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int s_item, s_info, s_next;
+  __shared__ double s_part[THREADS / 32];
+  __shared__ uint8_t s_packed[136];
+  const int tid = threadIdx.x;
+  for (int e = tid; e < 136; e += THREADS) s_packed[e] = (uint8_t)tc_packed(e);
+  const int ride = g.nrhs <= kTcMaxRhs && g.B ? g.nrhs : 0;
+  const int cols = ride ? ride : (g.nrhs > 0 ? kRhsChunk : 0);
+  const int ldx = g.n_max | 1;
+  unsigned char* SL = smem_raw;
+  double* X = reinterpret_cast<double*>(smem_raw + (size_t)kSlices * tc_slice_bytes(g.n_max));
+  double* rdiag = X + (size_t)ldx * cols;
+  double* Hd = rdiag + ((ldx + 1) & ~1);
+  int* ex = reinterpret_cast<int*>(Hd + 272);
+  const int start = g.range ? g.range[0] : 0;
+  const int end = g.range ? g.range[1] : g.count;
+  for (;;) {
+    if (tid == 0) s_item = g.counter ? atomicAdd(g.counter, 1) : (int)blockIdx.x;
+    __syncthreads();
+    const int idx = start + s_item;
+    if (idx >= end) break;
+    const int s = g.order ? g.order[idx] : idx;
+    const int n = g.ns ? g.ns[s] : g.n_max;
+    if (n < 0 || n > g.n_max) {
+      if (tid == 0) {
+        if (g.info) g.info[s] = -1;
+        if (g.logdet) g.logdet[s] = __longlong_as_double(0x7ff8000000000000ll);
+      }
+    } else {
+      double* a = g.A + (g.aoff ? g.aoff[s] : (int64_t)s * g.astride);
+      double* b = g.B ? g.B + (g.boff ? g.boff[s] : (int64_t)s * g.bstride) : nullptr;
+      if (tid == 0) s_info = 0;
+      for (int e = tid; e < n * ride; e += THREADS) {
+        const int c = e / n, r = e - c * n;
+        X[(size_t)c * ldx + r] = b[e];
+      }
+      __syncthreads();
+      chol_tc_cta(n, a, g.n_max, ride, X, ldx, SL, rdiag, Hd, ex, s_packed, &s_info, &s_next, g.has_subst, g.subst);
+      const int inf = s_info;
+      if (inf == 0) {
+        if (ride) {
+          chol_tc_backward_cta(n, a, g.n_max, ride, X, ldx, SL, rdiag, Hd, ex);
+          for (int e = tid; e < n * ride; e += THREADS) {
+            const int c = e / n, r = e - c * n;
+            b[e] = X[(size_t)c * ldx + r];
+          }
+        } else if (b) {
+          for (int c0 = 0; c0 < g.nrhs; c0 += kRhsChunk) {
+            const int nr = min(kRhsChunk, g.nrhs - c0);
+            for (int e = tid; e < n * nr; e += THREADS) {
+              const int c = e / n, r = e - c * n;
+              X[(size_t)c * ldx + r] = b[(size_t)c0 * n + e];
+            }
+            __syncthreads();
+            chol_forward_cta<false, double>(n, a, X, ldx, nr, rdiag);
+            chol_backward_fast_cta<double>(n, a, X, ldx, nr, rdiag);
+            for (int e = tid; e < n * nr; e += THREADS) {
+              const int c = e / n, r = e - c * n;
+              b[(size_t)c0 * n + e] = X[(size_t)c * ldx + r];
+            }
+            __syncthreads();
+          }
+        }
+        if (g.logdet) {
+          double part = 0.0;
+          for (int i = tid; i < n; i += THREADS) {
+            const double d = a[(size_t)i * n + i];
+            part += log(d * d);
+          }
+          part = warp_sum(part);
+          if ((tid & 31) == 0) s_part[tid >> 5] = part;
+          __syncthreads();
+          if (tid == 0) {
+            double sum = 0.0;
+            for (int w = 0; w < THREADS / 32; ++w) sum += s_part[w];
+            g.logdet[s] = sum;
+          }
+        }
+      } else if (tid == 0 && g.logdet) {
+        g.logdet[s] = __longlong_as_double(0x7ff8000000000000ll);
+      }
+      if (tid == 0 && g.info) g.info[s] = inf;
+    }
+    __syncthreads();
+    if (!g.counter) break;
+  }
+}
+
 // The tiles the autotuner chooses from (threads per matrix, panel width).
 struct CholTile {
   int threads, nb;
@@ -181,12 +281,45 @@ size_t chol_smem_bytes(int n_max, int nb = kNB) {
   return (size_t)ldp * (nb + kRhsChunk + 1) * sizeof(double);
 }
 
-// One launch of one tile over g.range (or the whole batch).
-int chol_launch_tile(CholArgs g, int tile, bool exact, cudaStream_t stream, bool persistent, const char* name) {
+// Orders above kTcMinOrder factor on the tensor cores in the FMA form.  At or
+// below it a matrix has two blocks of 16 and the panel form is as fast (20000
+// systems of order 32: 1.31 ms; of order 40: 2.32 ms on the panel form, 1.80 here).
+constexpr int kTcMinOrder = 32;
+bool chol_on_tensor_cores(const CholArgs& g, bool exact) { return !exact && g.do_factor && g.n_max > kTcMinOrder; }
+
+// Threads per matrix of that form.  Small orders have too few 16 x 32 units per
+// block for more warps, large ones leave room for two CTAs in shared memory.
+// Measured, 4 right-hand sides: 16000 x 64 2.22 ms with 64 threads, 2.62 with
+// 32; 8000 x 128 4.40 with 128, 4.66 with 64; 6000 x 160 4.85 with 128, 5.63 with
+// 256; 3000 x 256 6.96 with 256, 7.42 with 128.
+CholKernel chol_tc_choose(int n_max, int* threads) {
+  *threads = n_max <= 64 ? 64 : n_max <= 192 ? 128 : 256;
+  if (n_max <= 64) return chol_tc_kernel<64, 8>;
+  if (n_max <= 128) return chol_tc_kernel<128, 5>;
+  if (n_max <= 192) return chol_tc_kernel<128, 4>;
+  return chol_tc_kernel<256, 2>;
+}
+
+// The launch's kernel, threads per CTA and shared memory.
+CholKernel chol_choose(const CholArgs& g, int tile, bool exact, bool tiles_only, int* threads, size_t* smem) {
+  if (!tiles_only && chol_on_tensor_cores(g, exact)) {
+    const int cols = g.B == nullptr || g.nrhs <= 0 ? 0 : g.nrhs <= kTcMaxRhs ? g.nrhs : kRhsChunk;
+    *smem = tc_smem_bytes(g.n_max, cols);
+    return chol_tc_choose(g.n_max, threads);
+  }
   if (tile < 0 || tile >= NACU_RAGGED_TILES) tile = kDefaultTile;
-  CholKernel kern = chol_kernel(exact, tile);
-  const int threads = kCholTiles[tile].threads;
-  const size_t smem = chol_smem_bytes(g.n_max, kCholTiles[tile].nb);
+  *threads = kCholTiles[tile].threads;
+  *smem = chol_smem_bytes(g.n_max, kCholTiles[tile].nb);
+  return chol_kernel(exact, tile);
+}
+
+// One launch over g.range (or the whole batch); tile: the panel form's.
+// tiles_only (the autotuner): the panel form whatever the order.
+int chol_launch_tile(CholArgs g, int tile, bool exact, cudaStream_t stream, bool persistent, const char* name,
+                     bool tiles_only = false) {
+  int threads = 0;
+  size_t smem = 0;
+  CholKernel kern = chol_choose(g, tile, exact, tiles_only, &threads, &smem);
   cudaError_t e = ensure_dynamic_smem(kern, smem);
   if (e != cudaSuccess) return record_cuda_error(e, name);
   int grid = 1;
@@ -377,13 +510,12 @@ int chol_uniform_posv(int n, double* A, int64_t strideA, int nrhs, double* B, in
   while (b < NACU_RAGGED_BUCKETS - 1 && n > kBucketHi[b]) ++b;
   CholArgs g{batch, n, nullptr, nullptr, A, nrhs, nullptr, B, info, logdet, nullptr, nullptr, 0, 0.0, 1, nullptr,
              strideA, strideB};
-  int tile = g_tuning[b];
-  if (tile < 0 || tile >= NACU_RAGGED_TILES) tile = kDefaultTile;
-  CholKernel kern = chol_kernel(false, tile);
-  const size_t smem = chol_smem_bytes(n, kCholTiles[tile].nb);
+  int threads = 0;
+  size_t smem = 0;
+  CholKernel kern = chol_choose(g, g_tuning[b], false, false, &threads, &smem);
   cudaError_t e = ensure_dynamic_smem(kern, smem);
   if (e != cudaSuccess) return record_cuda_error(e, name);
-  kern<<<batch, kCholTiles[tile].threads, smem, s>>>(g);
+  kern<<<batch, threads, smem, s>>>(g);
   return check_launch(name);
 }
 
@@ -580,7 +712,8 @@ extern "C" int nacu_dposv_ragged_noalloc(int count, int n_max, const int32_t* ns
 }
 
 // ---------------------------------------------------------------------------
-// Autotuner of the bucketed launch: per size bucket, every tile is timed on a
+// Autotuner of the bucketed launch's panel form (every order in the EXACT form
+// and in solves from factors, orders up to 32 otherwise): per size bucket, every tile is timed on a
 // synthetic batch of that bucket (CUDA events, best of three after a warm-up)
 // and the fastest becomes the bucket's tile.
 // ---------------------------------------------------------------------------
@@ -722,7 +855,7 @@ int nacu_ragged_autotune(int per_bucket, int nrhs, int flags, int32_t* table_out
         CholArgs g{per_bucket, hi, buf.ns, buf.aoff, buf.A, nrhs, buf.boff, buf.B, buf.info, nullptr, nullptr,
                    buf.head, 0, 0.0, 1, nullptr};
         cudaEventRecord(e0, s);
-        rc = chol_launch_tile(g, t, exact, s, true, "nacu_ragged_autotune");
+        rc = chol_launch_tile(g, t, exact, s, true, "nacu_ragged_autotune", true);
         cudaEventRecord(e1, s);
         e = cudaEventSynchronize(e1);
         if (e != cudaSuccess) rc = record_cuda_error(e, "nacu_ragged_autotune");
