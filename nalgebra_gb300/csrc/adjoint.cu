@@ -28,7 +28,7 @@
 // pair-folded index over the lower triangle (column c paired with column
 // m-1-c fills an (m+1) x ceil(m/2) rectangle), so no lane idles on the
 // triangle's empty half.
-#include "common.cuh"
+#include "chol_tc.cuh"
 
 namespace nacu {
 namespace {
@@ -337,6 +337,230 @@ __global__ void __launch_bounds__(kAdjThreads) adj_backward_kernel(int n, const 
   }
 }
 
+// ---------------------------------------------------------------------------
+// FP64 backward on the tensor cores (slices.cuh), orders above kAdjTcMinOrder.
+//
+// With X = L^-T stored by rows (row i = column i of L^-1) the inverse is the
+// product of X's rows, (A^-1)_ij = sum_k X_ik X_jk, and X is the forward solve
+// of the identity: its rows ride along below the factor's rows, as right-hand
+// sides do in chol_tc.cuh.  So one sweep over blocks of 16 columns does
+// everything: the rows' 16 entries are solved against the block's head (one
+// thread per row, FP64), cut into slices, and 16-deep products of the slices
+//   - update the factor's remaining columns (recompute form only),
+//   - update X's remaining columns,
+//   - accumulate A^-1,
+//   - take w along: z = L^-1 w, then v = A^-1 w = X z.
+// Everything lives in the output dA (L2): A^-1 and, ahead of it, the trailing
+// matrix in the lower triangle (an entry's factor value is dead once its
+// block is sliced, A^-1_ij starts at block i), X in the strict upper one.
+//
+// What bounds it: the FP64 pipe still (the rows' solves, one subtraction per
+// product), then latency.  2048 x 128: 4.45 -> 1.46 ms with the factor stored,
+// 6.27 -> 2.20 ms recomputing it; 4000 x 40: 0.71 -> 0.44 ms. At or below order 32 (two
+// blocks) the shared-memory kernel above keeps the call.
+// ---------------------------------------------------------------------------
+constexpr int kAdjTcThreads = 128;
+constexpr int kAdjTcMinOrder = 32;
+
+constexpr size_t adj_tc_smem(int n) {
+  const size_t slots = (size_t)(n + 15) / 16 * 16 + 8;
+  return slots * (kSlices * kSliceRow + 4) + (size_t)(272 + 2 * ((n + 1) & ~1) + 16) * sizeof(double);
+}
+
+// One 16 x 8 tile of slice products added to (sign +) or subtracted from the
+// destination p(i), i = 0..3 the fragment's elements (null: none); fresh: the
+// destination starts at zero.
+template <typename F>
+__device__ __forceinline__ void adj_tile(const unsigned char* sa, const int* ea, const unsigned char* sc, const int* ec, int sb,
+                                         int lane, bool add, bool fresh, F dest) {
+  const int g = lane >> 2, t = lane & 3;
+  double* p[4];
+  double v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    p[i] = dest(g + (i >> 1) * 8, 2 * t + (i & 1));
+    v[i] = (p[i] && !fresh) ? *p[i] : 0.0;
+  }
+  float acc[kSlices][4];
+  slice_products(sa, sc, sb, lane, acc);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const double x = slice_value(acc, i, ea[g + (i >> 1) * 8] + ec[2 * t + (i & 1)]);
+    if (p[i]) *p[i] = v[i] + (add ? x : -x);
+  }
+}
+
+template <bool RECOMPUTE>
+__global__ void __launch_bounds__(kAdjTcThreads, 4)
+    adj_tc_backward_kernel(int n, const double* __restrict__ AL, int64_t strideA, const double* __restrict__ X,
+                           const double* __restrict__ Wt, const double* __restrict__ Glog, double* __restrict__ dA,
+                           double* __restrict__ db, int32_t* __restrict__ info) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int s_info, s_next;
+  __shared__ uint8_t s_packed[136];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr int nw = kAdjTcThreads / 32;
+  const int np = (n + 15) / 16 * 16, slots = np + 8, sb = slots * kSliceRow;
+  unsigned char* SL = smem_raw;
+  double* Hd = reinterpret_cast<double*>(SL + (size_t)kSlices * sb);
+  double* z = Hd + 272;            // w, then L^-1 w block by block
+  double* v = z + ((n + 1) & ~1);  // A^-1 w
+  double* rd = v + ((n + 1) & ~1); // 1 / L_jj of the current block
+  int* ex = reinterpret_cast<int*>(rd + 16);
+  const int s = blockIdx.x;
+  const double* al = AL + (size_t)s * strideA;
+  double* g = dA + (size_t)s * strideA;
+  for (int e = tid; e < 136; e += kAdjTcThreads) s_packed[e] = (uint8_t)tc_packed(e);
+  if (tid == 0) s_info = 0;
+  if (RECOMPUTE)
+    for (int c = warp; c < n; c += nw)
+      for (int r = c + lane; r < n; r += 32) g[(size_t)c * n + r] = al[(size_t)c * n + r];
+  for (int i = tid; i < n; i += kAdjTcThreads) {
+    z[i] = Wt[(size_t)s * n + i];
+    v[i] = 0.0;
+  }
+  __syncthreads();
+  // the head at J0: factored in place (recompute), or read from the stored factor
+  auto head = [&](int J0) {
+    if (RECOMPUTE) {
+      tc_head(n, g, J0, Hd, rd - J0, s_packed, &s_info, 0, 0.0, lane);
+    } else {
+      const int w = min(16, n - J0);
+      for (int e = lane; e < 256; e += 32) {
+        const int c = e >> 4, r = e & 15;
+        Hd[e] = (r < w && c <= r) ? al[(size_t)(J0 + c) * n + J0 + r] : 0.0;
+      }
+      if (lane < w) rd[lane] = 1.0 / al[(size_t)(J0 + lane) * (n + 1)];
+    }
+  };
+  if (warp == 0) head(0);
+  __syncthreads();
+  for (int J0 = 0; J0 < n; J0 += 16) {
+    if (RECOMPUTE && s_info != 0) break;
+    const int j1 = J0 + 16, w = min(16, n - J0), blk = J0 >> 4;
+    const int mp = np - j1, mt = mp >> 4;  // rows below, padded
+    // rows: slots [0, mp) the factor's, [mp, np) X's, np: z; the solve against
+    // the head, the slices
+    for (int q = tid; q < slots; q += kAdjTcThreads) {
+      unsigned char* s0 = SL + q * kSliceRow;
+      const int c = q - mp;  // X's row
+      if (q < mp ? j1 + q >= n : c < j1 ? c >= n : q > np) {
+        slice_zero_row(s0, sb);
+        ex[q] = 1;
+        continue;
+      }
+      double x[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        if (q < mp) x[j] = j < w ? (RECOMPUTE ? g : al)[(size_t)(J0 + j) * n + j1 + q] : 0.0;
+        else if (q == np) x[j] = j < w ? z[J0 + j] : 0.0;
+        else if (c >= J0) x[j] = c - J0 == j ? 1.0 : 0.0;
+        else x[j] = j < w ? g[(size_t)(J0 + j) * n + c] : 0.0;
+      }
+      if (RECOMPUTE || q >= mp) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          x[j] *= j < w ? rd[j] : 0.0;
+#pragma unroll
+          for (int k = j + 1; k < 16; ++k) x[k] = fma(-x[j], Hd[j * 16 + k], x[k]);
+        }
+      }
+      ex[q] = slice_row(x, s0, sb);
+    }
+    if (tid == 0) s_next = nw - 1;
+    __syncthreads();
+    auto lower = [&](int rt, int c0) {  // the factor's trailing columns
+      adj_tile(SL + 16 * rt * kSliceRow, ex + 16 * rt, SL + c0 * kSliceRow, ex + c0, sb, lane, false, false,
+               [&](int i, int k) -> double* {
+                 const int r = j1 + 16 * rt + i, c = j1 + c0 + k;
+                 return r < n && c <= r ? g + (size_t)c * n + r : nullptr;
+               });
+    };
+    if (RECOMPUTE && mt > 0) {
+      for (int rt = warp; rt < mt; rt += nw)
+        for (int c0 = 0; c0 < 16; c0 += 8) lower(rt, c0);
+      __syncthreads();
+    }
+    // units of 16 rows x 32 columns: X against the factor's rows, X against X
+    // (row tile i: ceil((i + 1) / 2)), every row against z, the factor's rest
+    const int ux = (blk + 1) * ((mt + 1) >> 1);
+    const int k1 = (blk + 1) >> 1, us = (blk + 1) & 1 ? (k1 + 1) * (k1 + 1) : k1 * (k1 + 1);
+    const int uz = np >> 4;
+    const int ul = RECOMPUTE ? ((mt & 1) ? (mt >> 1) * ((mt >> 1) + 1) : (mt >> 1) * (mt >> 1)) : 0;
+    const int units = ux + us + uz + ul;
+    int u = warp - 1;
+    if (warp == 0) {
+      if (mt > 0) head(j1);
+      if (lane == 0) u = atomicAdd(&s_next, 1);
+      u = __shfl_sync(0xffffffffu, u, 0);
+    }
+    while (u < units) {
+      int q = u;
+      if (q < ux) {
+        const int rt = q % (blk + 1), c0 = 32 * (q / (blk + 1));
+        for (int c = c0; c < min(c0 + 32, mp); c += 8)
+          adj_tile(SL + (mp + 16 * rt) * kSliceRow, ex + mp + 16 * rt, SL + c * kSliceRow, ex + c, sb, lane, false, rt == blk,
+                   [&](int i, int k) -> double* {
+                     const int r = j1 + c + k;
+                     return r < n ? g + (size_t)r * n + 16 * rt + i : nullptr;
+                   });
+      } else if ((q -= ux) < us) {
+        // row tiles 2 k and 2 k + 1 have k + 1 units each: k (k + 1) before them
+        int k = (int)((sqrtf(1.0f + 4.0f * (float)q) - 1.0f) * 0.5f);
+        if (k * (k + 1) > q) --k;
+        if ((k + 1) * (k + 2) <= q) ++k;
+        const int rem = q - k * (k + 1);
+        const int rt = rem <= k ? 2 * k : 2 * k + 1, c0 = 32 * (rem <= k ? rem : rem - k - 1);
+        for (int c = c0; c < min(c0 + 32, 16 * rt + 16); c += 8)
+          adj_tile(SL + (mp + 16 * rt) * kSliceRow, ex + mp + 16 * rt, SL + (mp + c) * kSliceRow, ex + mp + c, sb, lane, true,
+                   rt == blk, [&](int i, int kk) -> double* {
+                     const int r = 16 * rt + i, cc = c + kk;
+                     return r < n && cc <= r ? g + (size_t)cc * n + r : nullptr;
+                   });
+      } else if ((q -= us) < uz) {
+        const bool fac = 16 * q < mp;  // the factor's rows: z; X's: v
+        adj_tile(SL + 16 * q * kSliceRow, ex + 16 * q, SL + np * kSliceRow, ex + np, sb, lane, !fac, false,
+                 [&](int i, int kk) -> double* {
+                   const int r = fac ? j1 + 16 * q + i : 16 * q - mp + i;
+                   return kk == 0 && r < n ? (fac ? z : v) + r : nullptr;
+                 });
+      } else {
+        q -= uz;
+        int k = (int)((1.0f + sqrtf(1.0f + 4.0f * (float)q)) * 0.5f);
+        if (k * (k - 1) > q) --k;
+        if (k * (k + 1) <= q) ++k;
+        const int rem = q - k * (k - 1);
+        const int rt = rem < k ? 2 * k - 1 : 2 * k, c0 = 16 + 32 * (rem < k ? rem : rem - k);
+        for (int c = c0; c < min(c0 + 32, 16 * rt + 16); c += 8) lower(rt, c);
+      }
+      if (lane == 0) u = atomicAdd(&s_next, 1);
+      u = __shfl_sync(0xffffffffu, u, 0);
+    }
+    __syncthreads();
+  }
+  const int inf = RECOMPUTE ? s_info : 0;
+  if (inf == 0) {
+    double* xs = Hd;  // the forward solution, over the head and z (both done)
+    for (int i = tid; i < n; i += kAdjTcThreads) {
+      xs[i] = X[(size_t)s * n + i];
+      db[(size_t)s * n + i] = v[i];
+    }
+    __syncthreads();
+    const double gl = Glog ? Glog[s] : 1.0, gl2 = 2.0 * gl;
+    for (int c = warp; c < n; c += nw) {
+      const double vc = v[c], xc = xs[c];
+      double* col = g + (size_t)c * n;
+      for (int r = lane; r < n; r += 32) {
+        double val = 0.0;
+        if (r > c) val = fma(-v[r], xc, fma(-vc, xs[r], gl2 * col[r]));
+        else if (r == c) val = fma(-vc, xc, gl * col[r]);
+        col[r] = val;
+      }
+    }
+  }
+  if (tid == 0 && info) info[s] = inf;
+}
+
 template <typename T>
 int adj_launch_forward(int n, const T* A, int64_t strideA, const T* B, T* X, T* Lout, T* logdet, int32_t* info,
                        int batch, cudaStream_t stream, const char* name) {
@@ -360,6 +584,16 @@ int adj_launch_backward(int n, const T* AL, int64_t strideA, int recompute, cons
   if (batch == 0) return NACU_SUCCESS;
   if (!AL || !X || !W || !dA || !db) return record_arg_error(-2, "posv_logdet_backward: null argument");
   if (strideA < (int64_t)n * n) return record_arg_error(-3, "posv_logdet_backward: strideA < n*n");
+  if constexpr (sizeof(T) == 8) {
+    if (n > kAdjTcMinOrder) {
+      const auto kern = recompute ? adj_tc_backward_kernel<true> : adj_tc_backward_kernel<false>;
+      const size_t bytes = adj_tc_smem(n);
+      cudaError_t e = ensure_dynamic_smem(kern, bytes);
+      if (e != cudaSuccess) return record_cuda_error(e, name);
+      kern<<<batch, kAdjTcThreads, bytes, stream>>>(n, AL, strideA, X, W, G, dA, db, info);
+      return check_launch(name);
+    }
+  }
   const size_t smem = ((size_t)n * (n + 1) / 2 + 5 * (size_t)n) * sizeof(T);
   cudaError_t e = ensure_dynamic_smem(adj_backward_kernel<T>, smem);
   if (e != cudaSuccess) return record_cuda_error(e, name);
