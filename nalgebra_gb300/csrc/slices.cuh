@@ -1,4 +1,4 @@
-// FP64 products of short rows on the BF16 tensor cores, for the batched
+// FP64 products of short rows on the FP16 tensor cores, for the batched
 // factorizations: rows of 16 doubles are cut into seven 8-bit digits each, the
 // digit products summed exactly by mma.sync, the sums put together with integer
 // instructions.
@@ -13,9 +13,11 @@
 // applications", with digits instead of floating-point slices): row r with
 // largest exponent E_r becomes integers I = rint(v 2^(54 - E_r)), |I| <= 2^55,
 // in balanced base-256 digits d_0 .. d_6 (d_0 in [-128, 128], the others in
-// [-128, 127]), exact in BF16.  Level l collects the products d_p d_q with
+// [-128, 127]), exact in FP16.  (FP16 and not BF16: with 11 significant bits a
+// byte b placed under the exponent of 1024 is 1024 + b, so two digits take one
+// byte permute and one packed subtraction.)  Level l collects the products d_p d_q with
 // p + q = l; levels 0..6 are kept.  A sum of 16 * 7 such products stays below
-// 2^21, so with the accumulator starting at 1.5 2^23 every partial sum is an
+// 2^21 (of 32: below 2^22), so with the accumulator starting at 1.5 2^23 every partial sum is an
 // integer of FP32 and the low mantissa bits of the result are the sum itself.
 //
 // Error of one 16-deep product against 64 bits: rounding of I 2^-56 2^E of each
@@ -32,60 +34,66 @@ constexpr int kSlices = 7;
 constexpr int kSliceRow = 32;            // bytes of one row's digits in one slice
 constexpr int kBadRow = 1 << 20;         // exponent code of a row with inf or NaN
 
-__device__ __forceinline__ void mma_bf16_16x8x16(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+__device__ __forceinline__ void mma_f16_16x8x16(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
   asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// A row's 16 doubles -> its seven slices at s0 + p * slice_bytes (32 bytes each,
-// digits in the doubles' order) and its biased exponent code.  Eight values at
-// a time, which keeps the registers under the row solve's own.
-__device__ __forceinline__ int slice_row(const double (&v)[16], unsigned char* s0, int slice_bytes) {
-  int em = 0;
+// The digits of two values with common exponent code em (slice_exponent), one
+// word of two FP16 digits per slice.  em 2047 (inf or NaN in the row): zeros.
+__device__ __forceinline__ int slice_exponent(double v) { return max((__double2hiint(v) >> 20) & 0x7ff, 1); }
+__device__ __forceinline__ void slice_pair(double v0, double v1, int em, uint32_t (&w)[kSlices]) {
+  uint32_t lo[2], hi[2];
 #pragma unroll
-  for (int k = 0; k < 16; ++k) em = max(em, (__double2hiint(v[k]) >> 20) & 0x7ff);
-  const bool bad = em == 0x7ff;
-  em = max(em, 1);
+  for (int k = 0; k < 2; ++k) {
+    const long long b = __double_as_longlong(k ? v1 : v0);
+    const int ex = (int)((b >> 52) & 0x7ff);
+    const long long m = (b & 0xfffffffffffffll) | (ex ? 0x10000000000000ll : 0ll);
+    const int sh = em - max(ex, 1);  // >= 0: I = m 2^(2 - sh)
+    long long i = (sh > 60 || em == 0x7ff) ? 0 : ((((m << 3) >> sh) + 1) >> 1);
+    // plus 128 in every digit: the bytes (the top one nine bits) are digit + 128
+    i = (b < 0 ? -i : i) + 0x0080808080808080ll;
+    lo[k] = (uint32_t)i;
+    hi[k] = (uint32_t)(i >> 32);
+  }
+  auto minus = [](uint32_t x) {  // 1024 + 128 off both halves
+    uint32_t r;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(0x64806480u));
+    return r;
+  };
+  w[0] = minus(__byte_perm(hi[0], hi[1], 0x7632) | 0x64006400u);
+  const uint32_t t54 = __byte_perm(hi[0], hi[1], 0x5140);  // bytes 4, 4, 5, 5 of the two values
+  const uint32_t t32 = __byte_perm(lo[0], lo[1], 0x7362), t10 = __byte_perm(lo[0], lo[1], 0x5140);
+  w[1] = minus(__byte_perm(t54, 0x64646464u, 0x4342));
+  w[2] = minus(__byte_perm(t54, 0x64646464u, 0x4140));
+  w[3] = minus(__byte_perm(t32, 0x64646464u, 0x4342));
+  w[4] = minus(__byte_perm(t32, 0x64646464u, 0x4140));
+  w[5] = minus(__byte_perm(t10, 0x64646464u, 0x4342));
+  w[6] = minus(__byte_perm(t10, 0x64646464u, 0x4140));
+}
+// A row's exponent code from its largest exponent: inf and NaN poison the row.
+__device__ __forceinline__ int slice_code(int em) { return em == 0x7ff ? kBadRow : em; }
+
+// A row's 16 doubles -> its seven slices at s0 + p * slice_bytes (32 bytes each,
+// digits in the doubles' order) and its exponent code.
+__device__ __forceinline__ int slice_row(const double (&v)[16], unsigned char* s0, int slice_bytes) {
+  int em = 1;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) em = max(em, slice_exponent(v[k]));
 #pragma unroll
   for (int h = 0; h < 16; h += 8) {
-    // rint(v 2^(54 - E)) plus 128 in each of the six low digits: the bytes are digit + 128
-    uint32_t lo[8], hi[8];
+    uint32_t w0[kSlices], w1[kSlices], w2[kSlices], w3[kSlices];
+    slice_pair(v[h], v[h + 1], em, w0);
+    slice_pair(v[h + 2], v[h + 3], em, w1);
+    slice_pair(v[h + 4], v[h + 5], em, w2);
+    slice_pair(v[h + 6], v[h + 7], em, w3);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const long long b = __double_as_longlong(v[h + k]);
-      const int ex = (int)((b >> 52) & 0x7ff);
-      const long long m = (b & 0xfffffffffffffll) | (ex ? 0x10000000000000ll : 0ll);
-      const int sh = max(ex, 1) - em;  // <= 0: I = m 2^(2 + sh)
-      long long i = sh < -60 ? 0 : ((((m << 3) >> (-sh)) + 1) >> 1);
-      i = (b < 0 ? -i : i) + 0x0000808080808080ll;
-      if (bad) i = 0x0000808080808080ll;
-      lo[k] = (uint32_t)i;
-      hi[k] = (uint32_t)(i >> 32);
-    }
-#pragma unroll
-    for (int p = 0; p < kSlices; ++p) {
-      uint32_t w[4];
-#pragma unroll
-      for (int k = 0; k < 8; k += 2) {
-        float f[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          if (p == 0) {
-            f[u] = __int_as_float(0x4b400000 + ((int)hi[k + u] >> 16)) - 12582912.0f;
-          } else {  // byte 6 - p
-            const int byte = 6 - p;
-            const uint32_t x = __byte_perm(byte >= 4 ? hi[k + u] : lo[k + u], 0x4b000000u, 0x7650u | (byte & 3));
-            f[u] = __uint_as_float(x) - 8388736.0f;  // 2^23 + 128
-          }
-        }
-        w[k / 2] = __byte_perm(__float_as_uint(f[0]), __float_as_uint(f[1]), 0x7632);
-      }
-      *reinterpret_cast<uint4*>(s0 + p * slice_bytes + h * 2) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
+    for (int p = 0; p < kSlices; ++p)
+      *reinterpret_cast<uint4*>(s0 + p * slice_bytes + h * 2) = make_uint4(w0[p], w1[p], w2[p], w3[p]);
   }
-  return bad ? kBadRow : em;
+  return slice_code(em);
 }
 __device__ __forceinline__ void slice_zero_row(unsigned char* s0, int slice_bytes) {
 #pragma unroll
@@ -117,8 +125,20 @@ __device__ __forceinline__ void slice_products(const unsigned char* sa, const un
     const uint2 w1 = *reinterpret_cast<const uint2*>(sa + p * slice_bytes + off + 8 * kSliceRow);
     const uint32_t a[4] = {w0.x, w1.x, w0.y, w1.y};
 #pragma unroll
-    for (int q = 0; q < kSlices - p; ++q) mma_bf16_16x8x16(acc[p + q], a, b[q]);
+    for (int q = 0; q < kSlices - p; ++q) mma_f16_16x8x16(acc[p + q], a, b[q]);
   }
+}
+
+__device__ __forceinline__ void mma_f16_16x8x8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(b0));
+}
+__device__ __forceinline__ void slice_sums_start(float (&acc)[kSlices][4]) {
+#pragma unroll
+  for (int l = 0; l < kSlices; ++l)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[l][i] = 12582912.0f;
 }
 
 __device__ __noinline__ double slice_value_slow(long long w, int e) {
@@ -130,25 +150,30 @@ __device__ __noinline__ double slice_value_slow(long long w, int e) {
 
 // One product from its level sums (the accumulators' bit images); e the sum of
 // the two rows' exponent codes.  W = sum_l S_l 2^(44 - 8 l), the value W 2^(e -
-// 2046 - 56), rounded to 53 bits from the integer.
+// 2046 - 56), rounded to 53 bits from the integer.  DEPTH 32: sums of up to 32
+// products per level and slice pair (7 * 32 * 2^14 < 2^22 still fits the offset
+// accumulators), W one bit shorter to stay below 2^63.
+template <int DEPTH = 16>
 __device__ __forceinline__ double slice_value(const float (&acc)[kSlices][4], int i, int e) {
+  constexpr int kDrop = DEPTH > 16 ? 1 : 0;
   const uint32_t s0 = __float_as_uint(acc[0][i]), s1 = __float_as_uint(acc[1][i]), s2 = __float_as_uint(acc[2][i]);
   const uint32_t s3 = __float_as_uint(acc[3][i]), s4 = __float_as_uint(acc[4][i]), s5 = __float_as_uint(acc[5][i]);
   const uint32_t s6 = __float_as_uint(acc[6][i]);
   constexpr uint32_t kM = 0x4b400000u, kM2 = kM * 256u + kM;  // the offset in one sum, and in 256 x + y
   const int a = (int)(s0 * 256u + s1 - kM2), b = (int)(s2 * 256u + s3 - kM2), c = (int)(s4 * 256u + s5 - kM2);
-  const int d = (int)(s6 - kM) >> 4;
-  const long long w = (long long)b * (1ll << 20) + ((long long)c * 16 + d) + ((long long)((unsigned long long)(uint32_t)a << 36));
+  const int d = (int)(s6 - kM) >> (4 + kDrop);
+  const long long w = (long long)b * (1ll << (20 - kDrop)) + ((long long)c * (16 >> kDrop) + d) +
+                      ((long long)((unsigned long long)(uint32_t)a << (36 - kDrop)));
   const uint32_t sign = (uint32_t)((unsigned long long)w >> 63);
   unsigned long long m = (unsigned long long)(sign ? -w : w);
   if (m == 0) {
-    return e < (kBadRow >> 1) ? 0.0 : slice_value_slow(w, e);
+    return e < (kBadRow >> 1) ? 0.0 : slice_value_slow(w, e + kDrop);
   }
   const int z = __clzll((long long)m);  // >= 1: |w| < 2^63
   m <<= z - 1;                           // leading one at bit 62
   m += 0x200ull;                         // round to 53 bits (a carry to bit 63 moves into the exponent)
-  const int ex = 63 - z + e - 1079;
-  if ((unsigned)(ex - 1) >= 2044u) return slice_value_slow(w, e);
+  const int ex = 63 - z + e - 1079 + kDrop;
+  if ((unsigned)(ex - 1) >= 2044u) return slice_value_slow(w, e + kDrop);
   const uint32_t h = (uint32_t)(m >> 42) + ((uint32_t)(ex - 1) << 20) + (sign << 31);
   return __hiloint2double((int)h, (int)(uint32_t)(m >> 10));
 }
