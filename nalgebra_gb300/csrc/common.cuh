@@ -217,6 +217,14 @@ __device__ __forceinline__ double rsqrt_halley(double d) {
   return fma(r, fma(0.375, e, 0.5) * e, r);
 }
 
+// sqrt(d) from the same: d r and one Newton correction, within an ulp.
+__device__ __forceinline__ double sqrt_halley(double d) {
+  const long long b = __double_as_longlong(d);
+  if (b < 0x0010000000000000ll || b >= 0x7ff0000000000000ll) return sqrt(d);
+  const double r = rsqrt_halley(d), s = d * r;
+  return fma(0.5 * r, fma(-s, s, d), s);
+}
+
 // A lower bound of |x| in binary32 for norm sums, from the high word alone:
 // the fraction truncated to 20 bits, magnitudes below 2^-127 counted as 0 and
 // above the binary32 range clamped just under FLT_MAX (a smaller ||A|| only
