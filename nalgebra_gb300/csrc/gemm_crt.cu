@@ -74,7 +74,10 @@ constexpr float kMinCos = 0.0078125f;  // 2^-7
 constexpr int kMaxExp = 800;           // exponents of a row's / column's largest entry
 constexpr int kBadScale = 0x40000000;  // a row / column for the FP64 kernel
 constexpr int kZeroScale = 0x20000000; // an all-zero row / column: its products are exact zeros
-constexpr int kStatChunk = 128;        // columns of A per thread of the row statistics
+// Columns of A per thread of the row statistics: a thread's loads are one
+// dependent chain, so a short product (K = 128: 25 us with all of it on one
+// thread) takes few; a long one fewer, larger partial sums to merge.
+constexpr int stat_chunk(int k) { return k <= 512 ? 16 : 128; }
 
 // ---- tables -------------------------------------------------------------------------------------------------
 struct CrtTables {
@@ -251,16 +254,17 @@ __device__ __forceinline__ uint32_t abs_bits(long long v, bool bad) {
   return __float_as_uint((float)llabs(v) * 2.168404344971009e-19f) + 0x8000u;  // 2^-62, rounded to BF16
 }
 
-// Partial row norms of A: thread per row, kStatChunk columns; part[chunk][row].
+// Partial row norms of A: thread per row and chunk of columns; part[chunk][row].
 __global__ void __launch_bounds__(128) crt_row_stats_kernel(int m, int k, const double* __restrict__ A, int64_t lda,
+                                                            int chunk, const double* __restrict__ bal, int64_t bstride,
                                                             int2* __restrict__ part) {
   const int i = blockIdx.x * 128 + threadIdx.x;
   if (i >= m) return;
-  const int c0 = blockIdx.y * kStatChunk, c1 = min(k, c0 + kStatChunk);
+  const int c0 = blockIdx.y * chunk, c1 = min(k, c0 + chunk);
   Norm nm;
   const double* a = A + (size_t)c0 * lda + i;
 #pragma unroll 4
-  for (int c = c0; c < c1; ++c, a += lda) nm.add(*a);
+  for (int c = c0; c < c1; ++c, a += lda) nm.add(bal ? shift_exp(*a, plain_exponent(bal[c * bstride])) : *a);
   part[(size_t)blockIdx.y * m + i] = make_int2(nm.e, __float_as_int(nm.s));
 }
 
@@ -269,8 +273,8 @@ __global__ void __launch_bounds__(128) crt_row_stats_kernel(int m, int k, const 
 // k tile also write the row scales.
 __global__ void __launch_bounds__(256) crt_split_a_kernel(int m, int k, const double* __restrict__ A, int64_t lda,
                                                           const int2* __restrict__ part, int nparts, int mp, int kp,
-                                                          int* __restrict__ rscale,
-                                                          uint32_t* __restrict__ out) {
+                                                          const double* __restrict__ bal, int64_t bstride,
+                                                          int* __restrict__ rscale, uint32_t* __restrict__ out) {
   __shared__ long long t[64][33];
   __shared__ int s_scale[32];
   const int i0 = blockIdx.y * 32, k0 = blockIdx.x * 64;
@@ -293,7 +297,9 @@ __global__ void __launch_bounds__(256) crt_split_a_kernel(int m, int k, const do
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const int kk = (tid >> 5) + 8 * u;
-      t[kk][r] = (live && k0 + kk < k) ? scaled_int(A[(size_t)(k0 + kk) * lda + i0 + r], sc) : 0ll;
+      double x = (live && k0 + kk < k) ? A[(size_t)(k0 + kk) * lda + i0 + r] : 0.0;
+      if (bal && k0 + kk < k) x = shift_exp(x, plain_exponent(bal[(k0 + kk) * bstride]));
+      t[kk][r] = scaled_int(x, live ? sc : 0);
     }
   }
   __syncthreads();
@@ -315,16 +321,18 @@ __global__ void __launch_bounds__(256) crt_split_a_kernel(int m, int k, const do
 // B (columns contiguous along K) -> residue planes [plane][np][kp] and the
 // column scales; one CTA per (padded) column.
 __global__ void __launch_bounds__(256) crt_split_b_kernel(int k, int n, const double* __restrict__ B, int64_t ldb, int np,
-                                                          int kp, int* __restrict__ cscale,
+                                                          int kp, const double* __restrict__ bal, int64_t bstride,
+                                                          int* __restrict__ cscale,
                                                           uint32_t* __restrict__ out) {
   __shared__ int s_e[8];
   __shared__ float s_s[8];
   __shared__ int s_scale;
   const int j = blockIdx.x, tid = threadIdx.x;
   const double* col = B + (size_t)j * ldb;
+  auto at = [&](int c) { return bal ? shift_exp(col[c], -plain_exponent(bal[c * bstride])) : col[c]; };
   Norm nm;
   if (j < n)
-    for (int c = tid; c < k; c += 256) nm.add(col[c]);
+    for (int c = tid; c < k; c += 256) nm.add(at(c));
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
     const int e2 = __shfl_xor_sync(0xffffffffu, nm.e, off);
@@ -347,8 +355,8 @@ __global__ void __launch_bounds__(256) crt_split_b_kernel(int k, int n, const do
   const bool live = j < n && sc < kZeroScale, bad = sc == kBadScale;
   const size_t plane = (size_t)np * kp / 2;
   for (int c = 2 * tid; c < kp; c += 512) {
-    const long long v0 = (live && c < k) ? scaled_int(col[c], sc) : 0ll;
-    const long long v1 = (live && c + 1 < k) ? scaled_int(col[c + 1], sc) : 0ll;
+    const long long v0 = (live && c < k) ? scaled_int(at(c), sc) : 0ll;
+    const long long v1 = (live && c + 1 < k) ? scaled_int(at(c + 1), sc) : 0ll;
     const Chunks b0(v0), b1(v1);
     uint32_t* o = out + ((size_t)j * kp + c) / 2;
 #pragma unroll
@@ -798,7 +806,7 @@ CrtLayout crt_layout(int m, int n, int k) {
   L.a_off = take((size_t)(kMod + 1) * L.mb * L.kb * 2);
   L.b_off = take((size_t)(kMod + 1) * L.nb * L.kb * 2);
   L.r_off = take((size_t)kMod * L.mb * L.nb);
-  L.part_off = take((size_t)((L.kb + kStatChunk - 1) / kStatChunk) * L.mb * sizeof(int2));
+  L.part_off = take((size_t)((L.kb + stat_chunk(L.kb) - 1) / stat_chunk(L.kb)) * L.mb * sizeof(int2));
   L.rs_off = take((size_t)L.mb * 4);
   L.cs_off = take((size_t)L.nb * 4);
   L.flag_off = take((size_t)(L.mb / kFlagTile) * (L.nb / kFlagTile) * 4);
@@ -846,7 +854,7 @@ static int crt_max_pairs(size_t smem) {
 
 int crt_gemm_run(int m, int n, int k, double alpha, const double* A, int64_t lda, const double* B, int64_t ldb,
                  double beta, double* C, int64_t ldc, void* workspace, size_t workspace_bytes, cudaStream_t s,
-                 const char* name) {
+                 const char* name, const double* balance, int64_t balance_stride) {
   const CrtLayout L = crt_layout(m, n, k);
   if (!workspace || workspace_bytes < L.total) return record_arg_error(-13, "dgemm: workspace too small");
   unsigned char* ws = reinterpret_cast<unsigned char*>(round_up(reinterpret_cast<uintptr_t>(workspace), 1024));
@@ -865,16 +873,17 @@ int crt_gemm_run(int m, int n, int k, double alpha, const double* A, int64_t lda
   for (int k0 = 0; k0 < k; k0 += kBlockK) {
     const int kc = std::min(kBlockK, k - k0), kp = (int)round_up((size_t)kc, kKB);
     const double bt = k0 == 0 ? beta : 1.0;
+    const double* bal = balance ? balance + k0 * balance_stride : nullptr;
     for (int n0 = 0; n0 < n; n0 += kBlockMN) {
       const int nc = std::min(kBlockMN, n - n0), np = (int)round_up((size_t)nc, kPN);
-      crt_split_b_kernel<<<np, 256, 0, s>>>(kc, nc, B + (size_t)n0 * ldb + k0, ldb, np, kp, cs, bp);
+      crt_split_b_kernel<<<np, 256, 0, s>>>(kc, nc, B + (size_t)n0 * ldb + k0, ldb, np, kp, bal, balance_stride, cs, bp);
       for (int m0 = 0; m0 < m; m0 += kBlockMN) {
         const int mc = std::min(kBlockMN, m - m0), mp = (int)round_up((size_t)mc, kPM);
         const double* a = A + (size_t)k0 * lda + m0;
         double* c = C + (size_t)n0 * ldc + m0;
-        const int nparts = (kc + kStatChunk - 1) / kStatChunk;
-        crt_row_stats_kernel<<<dim3((mc + 127) / 128, nparts), 128, 0, s>>>(mc, kc, a, lda, part);
-        crt_split_a_kernel<<<dim3(kp / 64, mp / 32), 256, 0, s>>>(mc, kc, a, lda, part, nparts, mp, kp, rs, ap);
+        const int chunk = stat_chunk(L.kb), nparts = (kc + chunk - 1) / chunk;
+        crt_row_stats_kernel<<<dim3((mc + 127) / 128, nparts), 128, 0, s>>>(mc, kc, a, lda, chunk, bal, balance_stride, part);
+        crt_split_a_kernel<<<dim3(kp / 64, mp / 32), 256, 0, s>>>(mc, kc, a, lda, part, nparts, mp, kp, bal, balance_stride, rs, ap);
         const int nflags = (mp / kFlagTile) * (np / kFlagTile);
         e = cudaMemsetAsync(flags, 0, (size_t)nflags * 4, s);
         if (e != cudaSuccess) return record_cuda_error(e, name);

@@ -12,9 +12,15 @@
 //   2. the panel's row swaps applied to the columns left and right of it;
 //   3. U12 = L11^-1 A12 (unit lower triangular solve, one thread per column);
 //   4. A22 -= L21 U12 by the GEMM kernels: residues on the tensor cores for
-//      FP64 (gemm_crt.cu; n = 8192: 330 -> 117 ms, n = 1000: 4.6 -> 4.2 ms against
-//      the FP64 pipe, whose error is the larger one), the BF16-split tensor-core
-//      GEMM for the FP32 factor.
+//      FP64 (gemm_crt.cu), the BF16-split tensor-core GEMM for the FP32 factor.
+// Orders up to 8192 take 128 columns per block, panels in registers and 32-deep
+// updates inside the block; above, a block is one panel of 64 (FP64) or 128.
+// Measured, FP64 (all on the FP64 pipe -> residue updates with 64-wide panels ->
+// register panels): n = 8192 328 -> 114 -> 65 ms, 4096 50 -> 24.6 -> 20.0, 2000 11.6 ->
+// 9.4 -> 8.7, 1000 4.62 -> 4.20 -> 4.08.  FP32 factor with refinement, n = 4096: 15.8
+// -> 14.6 ms.  The panels bound it: a column costs about 4900 cycles at n = 1000
+// (pivot search 420, the candidate's push 1200, cluster barrier 1000, the
+// winner 350, the FP64 update 1900).
 // The triangular solves for the right-hand side run as one cooperative kernel
 // per triangle: the diagonal block of each step is solved by CTA 0 while all
 // CTAs then apply it to the remaining rows (coalesced GEMV), one grid barrier
@@ -24,7 +30,7 @@
 #include <algorithm>
 #include <cmath>
 
-#include "common.cuh"
+#include "slices.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -49,8 +55,10 @@ struct PanelPub {
   int idx[2][kPanelMaxG];
   T row[2][kPanelMaxG][kPanelMaxNb];
   T diag[2][kPanelMaxNb];
-  // the panel's swaps as one row mapping: row pdst[k] takes old row psrc[k]
+  // the panel's swaps as one row mapping: row pdst[k] takes old row psrc[k];
+  // the register panels of an outer block one list each, in order
   int npairs;
+  int nlist[kPanelMaxNb / 32];
   int pdst[2 * kPanelMaxNb];
   int psrc[2 * kPanelMaxNb];
 };
@@ -516,6 +524,332 @@ __global__ void __launch_bounds__(kPanelThreads) lu_panel_cluster_kernel(PanelAr
 }
 
 // ---------------------------------------------------------------------------
+// narrow panels in registers
+//
+// The cluster form above pays about six CTA barriers and one cluster barrier
+// per column (2.5 us, 4.2 us for FP64 at 6000 rows, where 64-wide panels also
+// hold the FP64 pipe).  Here a panel is 32 columns wide and a thread keeps one
+// row of it in registers, so a column costs one CTA barrier (the warps' pivot
+// candidates) and one cluster barrier (the CTAs' candidates, each pushed with
+// its row into every CTA's shared memory by the warp that holds it):
+//   - rows never move.  Each thread tracks the position its row has under
+//     nalgebra's swaps (icamax compares positions, src/base/min_max.rs:221-240;
+//     a pivot's row takes position c, the row that was there the pivot's old
+//     one) and writes its row there at the end;
+//   - the registers shift by one column per step, so the loop over columns
+//     stays rolled; finished multipliers and pivot rows wait in shared memory;
+//   - the cluster then applies the swaps to the outer block's other columns and
+//     solves their 32 rows of U, a warp per column.
+// Panels of 128 columns are made of four of these, each followed by the 32-deep
+// update of the block's remaining columns.
+// ---------------------------------------------------------------------------
+constexpr int kRegThreads = 512;
+constexpr int kRegNb = 32;
+constexpr int kRegMaxRows = kRegThreads * kClusterMaxCtas;  // 8192
+
+struct alignas(16) RegMeta {
+  unsigned long long key;  // |pivot candidate|'s bit image
+  double rcp;              // its reciprocal
+  int pos, pad[3];
+};
+template <typename T>
+struct RegPanelArgs {
+  int n;
+  T* A;
+  int64_t lda;
+  int j0, nb, chunk;  // panel columns, rows per CTA
+  int c_lo, c_hi;     // the outer block's columns
+  int list;           // this panel's place in the block
+  int32_t* ipiv;
+  int32_t* info;
+  PanelPub<T>* pub;
+};
+template <typename T>
+struct RegPanelSmem {
+  RegMeta meta[2][kClusterMaxCtas];
+  T slot[2][kClusterMaxCtas][kRegNb];
+  T rows[kRegNb][kRegThreads];
+  T l11[kRegNb][kRegNb + 1];
+  unsigned long long wkey[2][kRegThreads / 32];
+  int wpos[2][kRegThreads / 32];
+  int dst[2 * kRegNb], src[2 * kRegNb];
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kRegThreads, 1) lu_panel_reg_kernel(RegPanelArgs<T> g) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  RegPanelSmem<T>& sm = *reinterpret_cast<RegPanelSmem<T>*>(smem_raw);
+  constexpr int kWarps = kRegThreads / 32;
+  cg::cluster_group cl = cg::this_cluster();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int G = (int)cl.num_blocks(), b = (int)cl.block_rank();
+  const int rb = g.j0 + b * g.chunk;
+  const int nr = max(0, min(g.n - rb, g.chunk));
+  const bool valid = tid < nr;
+  const int row = rb + tid;
+  int pos = row;
+  bool done = !valid;
+  T x[kRegNb];
+#pragma unroll
+  for (int k = 0; k < kRegNb; ++k) x[k] = (valid && k < g.nb) ? g.A[(size_t)(g.j0 + k) * g.lda + row] : T(0);
+  int* const npairs = &g.pub->nlist[g.list];
+  int *const pdst = g.pub->pdst + 2 * kRegNb * g.list, *const psrc = g.pub->psrc + 2 * kRegNb * g.list;
+  if (b == 0 && tid == 0) *npairs = 0;
+  cl.sync();  // every CTA of the cluster runs before anything is pushed to it
+  for (int j = 0; j < g.nb; ++j) {
+    const int c = g.j0 + j, par = j & 1, left = g.nb - j;
+    uint64_t key = done ? 0ull : pivot_key(x[0], pos == c);
+    int idx = done ? 0x7fffffff : pos;
+    warp_argmax(key, idx);
+    if (lane == 0) {
+      sm.wkey[par][warp] = key;
+      sm.wpos[par][warp] = idx;
+    }
+    __syncthreads();
+    key = lane < kWarps ? sm.wkey[par][lane] : 0ull;
+    idx = lane < kWarps ? sm.wpos[par][lane] : 0x7fffffff;
+    warp_argmax(key, idx);
+    // the warp that holds this CTA's candidate pushes it (warp 0 where there is none)
+    const bool cand = !done && pos == idx;
+    if (__any_sync(0xffffffffu, cand) || (idx == 0x7fffffff && warp == 0)) {
+      RegMeta* m = &sm.meta[par][b];
+      T* mine = sm.slot[par][b];
+      if (cand) {
+#pragma unroll
+        for (int k = 0; k < kRegNb; ++k)
+          if (k < left) mine[k] = x[k];
+        m->rcp = (double)pivot_rcp(x[0]);
+      }
+      if (lane == 0) {
+        m->key = key;
+        m->pos = idx == 0x7fffffff ? -1 : idx;
+      }
+      __syncwarp();
+      constexpr int kV = 16 / (int)sizeof(T);
+      const int nv = (left + kV - 1) / kV, per = nv + 2;  // row vectors, then the meta's two
+      for (int e = lane; e < G * per; e += 32) {
+        const int q = e / per, v = e - q * per;
+        if (q == b) continue;
+        const float4* from = v < nv ? reinterpret_cast<const float4*>(mine) + v : reinterpret_cast<const float4*>(m) + (v - nv);
+        float4* to = v < nv ? reinterpret_cast<float4*>(cl.map_shared_rank(mine, q)) + v
+                            : reinterpret_cast<float4*>(cl.map_shared_rank(m, q)) + (v - nv);
+        *to = *from;
+      }
+    }
+    cluster_arrive_release();
+    cluster_wait_acquire();
+    // the pivot, the same in every warp
+    int w = 0;
+    {
+      const RegMeta* m = &sm.meta[par][lane < G ? lane : 0];
+      const int p = lane < G ? m->pos : -1;
+      key = p >= 0 ? m->key : 0ull;
+      idx = p >= 0 ? p : 0x7fffffff;
+      warp_argmax(key, idx);
+      const unsigned holder = __ballot_sync(0xffffffffu, p >= 0 && p == idx);
+      w = holder ? __ffs(holder) - 1 : 0;
+    }
+    const bool zero = idx == 0x7fffffff || key == 0;  // all |x| == 0: skipped, lu.rs:107-110
+    if (b == 0 && tid == 0) {
+      g.ipiv[c] = zero ? c : idx;
+      if (zero) atomicMin(g.info, c + 1);
+    }
+    if (!done) {
+      if (pos == (zero ? c : idx)) {  // this row is row c of U
+        done = true;
+        pos = c;
+#pragma unroll
+        for (int k = 0; k < kRegNb; ++k)
+          if (k < left) sm.rows[j + k][tid] = x[k];
+      } else {
+        if (!zero && pos == c) pos = idx;
+        const T l = zero ? x[0] : x[0] * (T)sm.meta[par][w].rcp;
+        sm.rows[j][tid] = l;
+        const T* u = sm.slot[par][w];
+#pragma unroll
+        for (int k0 = 0; k0 < kRegNb; k0 += 4)
+          if (k0 < left - 1)  // uniform; past the panel's end the values are never used
+#pragma unroll
+            for (int k = k0; k < k0 + 4; ++k)
+              if (k + 1 < kRegNb) x[k] = zero ? x[k + 1] : axpy1<false>(x[k + 1], -u[k + 1], l);
+      }
+    }
+  }
+  if (valid) {
+    for (int k = 0; k < g.nb; ++k) g.A[(size_t)(g.j0 + k) * g.lda + pos] = sm.rows[k][tid];
+    if (pos != row) {
+      const int q = atomicAdd(npairs, 1);
+      pdst[q] = pos;
+      psrc[q] = row;
+    }
+  }
+  __threadfence();
+  cl.sync();
+  const int np = min(__ldcg(npairs), 2 * kRegNb);
+  for (int k = tid; k < np; k += kRegThreads) {
+    sm.dst[k] = __ldcg(&pdst[k]);
+    sm.src[k] = __ldcg(&psrc[k]);
+  }
+  for (int e = tid; e < g.nb * g.nb; e += kRegThreads) {
+    const int k = e / g.nb, i = e - k * g.nb;
+    sm.l11[k][i] = __ldcg(&g.A[(size_t)(g.j0 + k) * g.lda + g.j0 + i]);
+  }
+  __syncthreads();
+  const int others = g.c_hi - g.c_lo - g.nb;
+  for (int q = b * kWarps + warp; q < others; q += G * kWarps) {
+    const int cc = g.c_lo + q < g.j0 ? g.c_lo + q : g.c_lo + q + g.nb;
+    T* col = g.A + (size_t)cc * g.lda;
+    T v[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (lane + 32 * u < np) v[u] = col[sm.src[lane + 32 * u]];
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (lane + 32 * u < np) col[sm.dst[lane + 32 * u]] = v[u];
+    __syncwarp();
+    if (cc > g.j0) {  // U12 = L11^-1 A12
+      T y = lane < g.nb ? col[g.j0 + lane] : T(0);
+      for (int k = 0; k + 1 < g.nb; ++k) {
+        const T yk = __shfl_sync(0xffffffffu, y, k);
+        if (lane > k && lane < g.nb) y = axpy1<false>(y, -sm.l11[k][lane], yk);
+      }
+      if (lane < g.nb) col[g.j0 + lane] = y;
+    }
+  }
+}
+
+// A22 -= L21 U12 for the outer block's remaining columns (at most 96), 32 deep:
+// FP32, a thread per row with its 32 multipliers in registers, four column
+// phases; U in shared memory.
+__global__ void __launch_bounds__(256) lu_inner_update_kernel(int n, float* __restrict__ A, int64_t lda, int j0, int nb,
+                                                              int c_hi) {
+  __shared__ __align__(16) float U[96][kRegNb];
+  const int j1 = j0 + nb, w = c_hi - j1;
+  for (int e = threadIdx.x; e < w * kRegNb; e += 256) {
+    const int c = e >> 5, k = e & 31;
+    U[c][k] = k < nb ? A[(size_t)(j1 + c) * lda + j0 + k] : 0.f;
+  }
+  __syncthreads();
+  const int r = j1 + blockIdx.x * 64 + (threadIdx.x & 63);
+  if (r >= n) return;
+  float l[kRegNb];
+#pragma unroll
+  for (int k = 0; k < kRegNb; ++k) l[k] = k < nb ? A[(size_t)(j0 + k) * lda + r] : 0.f;
+  for (int c = threadIdx.x >> 6; c < w; c += 4) {
+    float* p = A + (size_t)(j1 + c) * lda + r;
+    float acc = *p;
+#pragma unroll
+    for (int k = 0; k < kRegNb; ++k) acc = fmaf(-l[k], U[c][k], acc);
+    *p = acc;
+  }
+}
+
+// The same in FP64 by digit slices (slices.cuh): rows j0 + nb .. r_hi - 1 times
+// columns c_lo .. c_hi - 1, 64 x 96 of them per CTA, the 32 products of an
+// output in one exact sum.  L's columns are scaled by the exponents of their
+// pivots and U's rows by the reverse: L D has the scale of its rows' entries of
+// A in every column and D^-1 U is near one, so rows of very different scale keep
+// their precision, as they do in the FP64 loop.
+constexpr int kInnerRows = 64, kInnerCols = 96;
+constexpr int kInnerSlots = kInnerRows + kInnerCols;
+constexpr size_t kInnerSmem = (size_t)2 * kSlices * kInnerSlots * kSliceRow + kInnerSlots * 4;
+__global__ void __launch_bounds__(128) lu_inner_update_kernel(int r_hi, double* __restrict__ A, int64_t lda, int j0, int nb,
+                                                              int c_lo, int c_hi) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int sb = kInnerSlots * kSliceRow;
+  unsigned char* SL = smem_raw;  // [half][slice][slot]
+  int* ex = reinterpret_cast<int*>(smem_raw + (size_t)2 * kSlices * sb);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int r0 = j0 + nb + blockIdx.x * kInnerRows, cb = c_lo + blockIdx.y * kInnerCols;
+  const int w = min(kInnerCols, c_hi - cb);
+  __shared__ int pe[kRegNb];  // the pivots' exponents
+  if (tid < kRegNb) pe[tid] = tid < nb ? plain_exponent(A[(size_t)(j0 + tid) * (lda + 1)]) : 0;
+  __syncthreads();
+  for (int s = tid; s < kInnerRows + ((w + 7) & ~7); s += 128) {
+    const bool lrow = s < kInnerRows;
+    const int r = r0 + s, c = s - kInnerRows;
+    const bool on = lrow ? r < r_hi : c < w;
+    const double* p = lrow ? A + (size_t)j0 * lda + r : A + (size_t)(cb + c) * lda + j0;
+    const int64_t st = lrow ? lda : 1;
+    double v[kRegNb];
+    int em = 1;
+#pragma unroll
+    for (int k = 0; k < kRegNb; ++k) {
+      v[k] = on && k < nb ? shift_exp(p[k * st], lrow ? pe[k] : -pe[k]) : 0.0;
+      em = max(em, slice_exponent(v[k]));
+    }
+#pragma unroll
+    for (int k = 0; k < kRegNb; k += 4) {
+      uint32_t w0[kSlices], w1[kSlices];
+      slice_pair(v[k], v[k + 1], em, w0);
+      slice_pair(v[k + 2], v[k + 3], em, w1);
+#pragma unroll
+      for (int q = 0; q < kSlices; ++q)
+        *reinterpret_cast<uint2*>(SL + (size_t)((k >> 4) * kSlices + q) * sb + s * kSliceRow + (k & 15) * 2) =
+            make_uint2(w0[q], w1[q]);
+    }
+    ex[s] = slice_code(em);
+  }
+  __syncthreads();
+  const int rt = warp * 16;  // this warp's 16 rows
+  const int e0 = ex[rt + g], e1 = ex[rt + g + 8];
+  for (int c = 0; c < w; c += 8) {
+    double* p[4];
+    double v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = r0 + rt + g + (i >> 1) * 8, cc = c + 2 * t + (i & 1);
+      p[i] = r < r_hi && cc < w ? A + (size_t)(cb + cc) * lda + r : nullptr;
+      v[i] = p[i] ? *p[i] : 0.0;
+    }
+    float acc[kSlices][4];
+    slice_sums_start(acc);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      slice_products_add(SL + (size_t)h * kSlices * sb + rt * kSliceRow,
+                         SL + (size_t)h * kSlices * sb + (kInnerRows + c) * kSliceRow, sb, lane, acc);
+    const int f0 = ex[kInnerRows + c + 2 * t], f1 = ex[kInnerRows + c + 2 * t + 1];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const double x = slice_value<32>(acc, i, (i >> 1 ? e1 : e0) + (i & 1 ? f1 : f0));
+      if (p[i]) *p[i] = v[i] - x;
+    }
+  }
+}
+
+// The outer block's swaps on the columns outside it: the panels' lists in
+// order, a warp per column.
+template <typename T>
+__global__ void __launch_bounds__(256) lu_swap_lists_kernel(int n, T* A, int64_t lda, const PanelPub<T>* __restrict__ pub,
+                                                            int lists, int j0, int nb) {
+  __shared__ int s_dst[2 * kPanelMaxNb], s_src[2 * kPanelMaxNb], s_np[kPanelMaxNb / kRegNb];
+  for (int k = threadIdx.x; k < 2 * kRegNb * lists; k += blockDim.x) {
+    s_dst[k] = pub->pdst[k];
+    s_src[k] = pub->psrc[k];
+  }
+  if (threadIdx.x < (unsigned)lists) s_np[threadIdx.x] = pub->nlist[threadIdx.x];
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int c = blockIdx.x * 8 + warp;
+  if (c >= j0) c += nb;
+  if (c >= n) return;
+  T* col = A + (size_t)c * lda;
+  for (int l = 0; l < lists; ++l) {
+    const int np = s_np[l], o = 2 * kRegNb * l;
+    T v[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (lane + 32 * u < np) v[u] = col[s_src[o + lane + 32 * u]];
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (lane + 32 * u < np) col[s_dst[o + lane + 32 * u]] = v[u];
+    __syncwarp();
+  }
+}
+
+// ---------------------------------------------------------------------------
 // row swaps of the panel applied to the other columns; unit-lower TRSM
 // ---------------------------------------------------------------------------
 template <typename T>
@@ -598,6 +932,27 @@ __global__ void __launch_bounds__(256) lu_trsm_kernel(int n, T* A, int64_t lda, 
 #pragma unroll
       for (int m = 0; m < M; ++m) A[(size_t)col * lda + j0 + m * 32 + lane] = v[c][m];
   }
+}
+
+// The solve with one unit lower triangle of at most 32 rows at p0 for columns
+// c0 .. n - 1: a warp per column, a row per lane.
+__global__ void __launch_bounds__(256) lu_trsm_piece_kernel(int n, double* __restrict__ A, int64_t lda, int p0, int nb,
+                                                            int c0) {
+  __shared__ double L[32][33];
+  for (int e = threadIdx.x; e < nb * nb; e += 256) {
+    const int k = e / nb, i = e - k * nb;
+    L[k][i] = A[(size_t)(p0 + k) * lda + p0 + i];
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, c = c0 + blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (c >= n) return;
+  double* col = A + (size_t)c * lda + p0;
+  double y = lane < nb ? col[lane] : 0.0;
+  for (int k = 0; k + 1 < nb; ++k) {
+    const double yk = __shfl_sync(0xffffffffu, y, k);
+    if (lane > k && lane < nb) y = axpy1<false>(y, -L[k][lane], yk);
+  }
+  if (lane < nb) col[lane] = y;
 }
 
 // The same for a panel width without a register-tiled instance: L11 in shared
@@ -995,6 +1350,99 @@ int panel_cluster_ctas() {
   return ctas;
 }
 
+// CTAs of a register panel's cluster: rows spread over as many as there are 64
+// rows for (an FP64 update is bound by its SMs' FP64 pipes), at most 16.
+inline int reg_panel_ctas(int rows) {
+  int g = 1;
+  while (g < kClusterMaxCtas && rows > 64 * g) g *= 2;
+  return g;
+}
+
+// An outer block of jb columns at j0 by panels of kRegNb (swaps and U inside
+// the block included); the panels' swap lists stay in pub.
+template <typename T>
+int reg_block(int n, T* A, int64_t lda, int j0, int jb, int32_t* ipiv, int32_t* info, PanelPub<T>* pub, cudaStream_t s,
+              const char* name) {
+  for (int p0 = j0; p0 < j0 + jb; p0 += kRegNb) {
+    const int nb = std::min(kRegNb, j0 + jb - p0), rows = n - p0;
+    const int G = reg_panel_ctas(rows);
+    RegPanelArgs<T> pa{n, A, lda, p0, nb, (rows + G - 1) / G, j0, j0 + jb, (p0 - j0) / kRegNb, ipiv, info, pub};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(G);
+    cfg.blockDim = dim3(kRegThreads);
+    cfg.dynamicSmemBytes = sizeof(RegPanelSmem<T>);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = G;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, lu_panel_reg_kernel<T>, pa);
+    if (e != cudaSuccess) return record_cuda_error(e, name);
+    const int below = rows - nb;
+    if (p0 + nb < j0 + jb && below > 0) {
+      if constexpr (sizeof(T) == 8)
+        lu_inner_update_kernel<<<(below + kInnerRows - 1) / kInnerRows, 128, kInnerSmem, s>>>(n, A, lda, p0, nb, p0 + nb,
+                                                                                              j0 + jb);
+      else
+        lu_inner_update_kernel<<<(below + 63) / 64, 256, 0, s>>>(n, A, lda, p0, nb, j0 + jb);
+    }
+  }
+  return check_launch(name);
+}
+
+// Whether this device runs the register panels for order n: a cluster of 16
+// with their shared memory, and no more rows than its threads.
+template <typename T>
+bool reg_panels(int n) {
+  static int ok = -1;
+  if (ok < 0) {
+    ok = 0;
+    auto kern = lu_panel_reg_kernel<T>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kClusterMaxCtas);
+    cfg.blockDim = dim3(kRegThreads);
+    cfg.dynamicSmemBytes = sizeof(RegPanelSmem<T>);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kClusterMaxCtas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int nclusters = 0;
+    bool good = ensure_dynamic_smem(kern, sizeof(RegPanelSmem<T>)) == cudaSuccess &&
+                cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg) == cudaSuccess && nclusters >= 1;
+    if constexpr (sizeof(T) == 8) {
+      void (*upd)(int, double*, int64_t, int, int, int, int) = lu_inner_update_kernel;
+      good = good && ensure_dynamic_smem(upd, kInnerSmem) == cudaSuccess;
+    }
+    if (!good) cudaGetLastError();
+    ok = good ? 1 : 0;
+  }
+  return ok == 1 && n <= kRegMaxRows;
+}
+
+// U12 = L11^-1 A12 in FP64 for an outer block, 32 rows at a time: the solve with
+// the piece's triangle, then its update of the block's rows below by digit
+// slices.  A quarter of the solve's FP64 instructions (2048 columns: 94 us in one
+// kernel; seven launches of 6 to 10 us here).
+cudaError_t trsm_by_pieces(int n, double* A, int64_t lda, int j0, int jb, cudaStream_t s) {
+  const int c0 = j0 + jb, rest = n - c0;
+  for (int p0 = j0; p0 < c0; p0 += kRegNb) {
+    const int nb = std::min(kRegNb, c0 - p0);
+    lu_trsm_piece_kernel<<<(rest + 7) / 8, 256, 0, s>>>(n, A, lda, p0, nb, c0);
+    const int below = c0 - p0 - nb;
+    if (below > 0)
+      lu_inner_update_kernel<<<dim3((below + kInnerRows - 1) / kInnerRows, (rest + kInnerCols - 1) / kInnerCols), 128,
+                               kInnerSmem, s>>>(c0, A, lda, p0, nb, c0, n);
+  }
+  return cudaGetLastError();
+}
+
 // Blocked LU with look-ahead: step k's panel chain (panel, row swaps, TRSM,
 // and the update of the next panel's columns) runs on the panel stream; the
 // rest of step k's trailing update runs on the update stream while panel k+1
@@ -1004,7 +1452,8 @@ template <typename T>
 int getrf_blocked(int n, T* A, int64_t lda, int32_t* ipiv, int32_t* info, void* ws, int nb, UpdateFn update,
                   void* ctx, cudaStream_t s, const char* name) {
   cudaError_t e;
-  if (nb > kPanelMaxNb) nb = kPanelMaxNb;
+  const bool by_registers = reg_panels<T>(n);
+  nb = by_registers ? kPanelMaxNb : std::min(nb, kPanelMaxNb);
   const void* pk = reinterpret_cast<const void*>(lu_panel_grid_kernel<T>);
   e = ensure_dynamic_smem(pk, kPanelMaxSmem);
   if (e != cudaSuccess) return record_cuda_error(e, name);
@@ -1024,6 +1473,10 @@ int getrf_blocked(int n, T* A, int64_t lda, int32_t* ipiv, int32_t* info, void* 
     const int jb = std::min(nb, n - j0);
     const int rows = n - j0;
     PanelArgs<T> pa{n, A, lda, j0, jb, 0, ipiv, info, reinterpret_cast<PanelPub<T>*>(ws)};
+    if (by_registers) {
+      rc = reg_block<T>(n, A, lda, j0, jb, ipiv, info, pa.pub, sp, name);
+      if (rc != NACU_SUCCESS) return rc;
+    } else {
     const int cchunk = cluster ? (rows + cluster - 1) / cluster : 0;
     const size_t csmem = cluster_pub_bytes<T>(jb) + (size_t)(cchunk | 1) * jb * sizeof(T);
     if (cluster && csmem <= kPanelMaxSmem) {
@@ -1053,15 +1506,20 @@ int getrf_blocked(int n, T* A, int64_t lda, int32_t* ipiv, int32_t* info, void* 
       e = cudaLaunchCooperativeKernel(pk, G, kPanelThreads, args, (size_t)(chunk | 1) * jb * sizeof(T), sp);
       if (e != cudaSuccess) return record_cuda_error(e, name);
     }
+    }
     if (rest_pending) {  // the swaps below touch the columns the previous update is still writing
       e = cudaStreamWaitEvent(sp, la->rest_done, 0);
       if (e != cudaSuccess) return record_cuda_error(e, name);
       rest_pending = false;
     }
-    if (n > jb) lu_swap_kernel<T><<<(n - jb + 7) / 8, 256, 0, sp>>>(n, A, lda, pa.pub, j0, jb);
+    if (n > jb && by_registers)
+      lu_swap_lists_kernel<T><<<(n - jb + 7) / 8, 256, 0, sp>>>(n, A, lda, pa.pub, (jb + kRegNb - 1) / kRegNb, j0, jb);
+    else if (n > jb)
+      lu_swap_kernel<T><<<(n - jb + 7) / 8, 256, 0, sp>>>(n, A, lda, pa.pub, j0, jb);
     const int rest = n - j0 - jb;
     if (rest > 0) {
-      e = launch_trsm<T>(n, A, lda, j0, jb, rest, sp);
+      if (by_registers && sizeof(T) == 8) e = trsm_by_pieces(n, reinterpret_cast<double*>(A), lda, j0, jb, sp);
+      else e = launch_trsm<T>(n, A, lda, j0, jb, rest, sp);
       if (e != cudaSuccess) return record_cuda_error(e, name);
       const T* L21 = A + (size_t)j0 * lda + j0 + jb;
       const T* U12 = A + (size_t)(j0 + jb) * lda + j0;
@@ -1145,11 +1603,13 @@ int update_fp64(int m, int n, int k, const void* L21, const void* U12, void* A22
   const double *a = static_cast<const double*>(L21), *b = static_cast<const double*>(U12);
   double* d = static_cast<double*>(A22);
   if (c && c->ws[slot] && c->ws_bytes[slot] >= crt_gemm_workspace_bytes(m, n, k))
-    return crt_gemm_run(m, n, k, -1.0, a, lda, b, lda, 1.0, d, lda, c->ws[slot], c->ws_bytes[slot], s, "nacu_dgetrf");
+    // the pivots: the diagonal of the block above L21 (k columns to the left of it)
+    return crt_gemm_run(m, n, k, -1.0, a, lda, b, lda, 1.0, d, lda, c->ws[slot], c->ws_bytes[slot], s, "nacu_dgetrf",
+                        a - k, lda + 1);
   return nacu_dgemm(m, n, k, -1.0, a, lda, b, lda, 1.0, d, lda, s);
 }
 
-constexpr int kNb64 = 64;  // panel width of the FP64 factorization
+constexpr int kNb64 = 64;  // panel width of the FP64 factorization past the register panels
 
 // The FP64 factorization's workspace: the panel's exchange area, then the
 // scratch of the two concurrent updates.
@@ -1158,8 +1618,10 @@ struct Getrf64Layout {
 };
 Getrf64Layout getrf64_layout(int n) {
   Getrf64Layout L;
-  L.bytes[0] = crt_gemm_workspace_bytes(n, kNb64, kNb64);
-  L.bytes[1] = crt_gemm_workspace_bytes(n, n, kNb64);
+  // either panel width: the device decides between them
+  const int nb = kPanelMaxNb;
+  L.bytes[0] = crt_gemm_workspace_bytes(n, nb, nb);
+  L.bytes[1] = crt_gemm_workspace_bytes(n, n, nb);
   L.slot[0] = getrf_ws_bytes();
   L.slot[1] = L.slot[0] + L.bytes[0];
   L.total = L.slot[1] + L.bytes[1];

@@ -103,32 +103,6 @@ __device__ __forceinline__ void slice_zero_row(unsigned char* s0, int slice_byte
   }
 }
 
-// Level sums of a 16 x 8 tile: rows sa .. sa + 15 against rows sb .. sb + 7
-// (pointers to the first row's digits in slice 0).  A fragment's lane t holds
-// the 16 products' terms 4 t .. 4 t + 3 (one 8-byte load), the same for both
-// operands: the order of the terms is free.
-__device__ __forceinline__ void slice_products(const unsigned char* sa, const unsigned char* sb, int slice_bytes, int lane,
-                                               float (&acc)[kSlices][4]) {
-  const int off = (lane >> 2) * kSliceRow + (lane & 3) * 8;
-  uint32_t b[kSlices][2];
-#pragma unroll
-  for (int q = 0; q < kSlices; ++q) {
-    const uint2 w = *reinterpret_cast<const uint2*>(sb + q * slice_bytes + off);
-    b[q][0] = w.x;
-    b[q][1] = w.y;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) acc[q][i] = 12582912.0f;
-  }
-#pragma unroll
-  for (int p = 0; p < kSlices; ++p) {
-    const uint2 w0 = *reinterpret_cast<const uint2*>(sa + p * slice_bytes + off);
-    const uint2 w1 = *reinterpret_cast<const uint2*>(sa + p * slice_bytes + off + 8 * kSliceRow);
-    const uint32_t a[4] = {w0.x, w1.x, w0.y, w1.y};
-#pragma unroll
-    for (int q = 0; q < kSlices - p; ++q) mma_f16_16x8x16(acc[p + q], a, b[q]);
-  }
-}
-
 __device__ __forceinline__ void mma_f16_16x8x8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
   asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
@@ -139,6 +113,35 @@ __device__ __forceinline__ void slice_sums_start(float (&acc)[kSlices][4]) {
   for (int l = 0; l < kSlices; ++l)
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[l][i] = 12582912.0f;
+}
+
+// Level sums of a 16 x 8 tile: rows sa .. sa + 15 against rows sb .. sb + 7
+// (pointers to the first row's digits in slice 0).  A fragment's lane t holds
+// the 16 products' terms 4 t .. 4 t + 3 (one 8-byte load), the same for both
+// operands: the order of the terms is free.
+__device__ __forceinline__ void slice_products_add(const unsigned char* sa, const unsigned char* sb, int slice_bytes,
+                                                   int lane, float (&acc)[kSlices][4]) {
+  const int off = (lane >> 2) * kSliceRow + (lane & 3) * 8;
+  uint32_t b[kSlices][2];
+#pragma unroll
+  for (int q = 0; q < kSlices; ++q) {
+    const uint2 w = *reinterpret_cast<const uint2*>(sb + q * slice_bytes + off);
+    b[q][0] = w.x;
+    b[q][1] = w.y;
+  }
+#pragma unroll
+  for (int p = 0; p < kSlices; ++p) {
+    const uint2 w0 = *reinterpret_cast<const uint2*>(sa + p * slice_bytes + off);
+    const uint2 w1 = *reinterpret_cast<const uint2*>(sa + p * slice_bytes + off + 8 * kSliceRow);
+    const uint32_t a[4] = {w0.x, w1.x, w0.y, w1.y};
+#pragma unroll
+    for (int q = 0; q < kSlices - p; ++q) mma_f16_16x8x16(acc[p + q], a, b[q]);
+  }
+}
+__device__ __forceinline__ void slice_products(const unsigned char* sa, const unsigned char* sb, int slice_bytes, int lane,
+                                               float (&acc)[kSlices][4]) {
+  slice_sums_start(acc);
+  slice_products_add(sa, sb, slice_bytes, lane, acc);
 }
 
 __device__ __noinline__ double slice_value_slow(long long w, int e) {

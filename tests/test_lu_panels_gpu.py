@@ -1,0 +1,82 @@
+"""GPU checks of the large LU's register panels: orders around the 32-wide panels,
+the 128-wide outer blocks and the cluster sizes, ties, zero columns, NaN, rows
+and columns of extreme scale.
+
+Pivots are compared with the oracle's (nalgebra's icamax rule); factors by
+||P A - L U||_F / (||A||_F n eps) <= 10 as the other LU tests."""
+import numpy as np
+import pytest
+
+import oracle as O
+from tests.test_getrf_large_gpu import _getrf
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [129, 159, 160, 161, 192, 255, 256, 257, 300, 383, 385, 640, 1025])
+def test_orders_at_panel_and_block_edges(cuda, n):
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((n, n))
+    lu, ipiv, info, _, _ = _getrf(cuda, a)
+    _, ipiv_o, _ = O.lu(a)
+    assert info == 0 and np.array_equal(ipiv, ipiv_o)
+    assert O.lu_reconstruction(a, lu, ipiv) <= 10.0
+
+
+def test_ties_take_the_first_position(cuda):
+    """Small integers: equal magnitudes in most columns, resolved by the position
+    the rows have after the swaps so far.  The eliminations stay exact while the
+    entries are dyadic; the first panel is compared in full."""
+    rng = np.random.default_rng(4)
+    n = 200
+    a = rng.choice([-1.0, 1.0], size=(n, n))
+    lu, ipiv, info, _, _ = _getrf(cuda, a)
+    lu_o, ipiv_o, _ = O.lu(a)
+    assert np.array_equal(ipiv[:4], ipiv_o[:4])
+    assert O.lu_reconstruction(a, lu, ipiv) <= 10.0
+    p = np.eye(n)[:, ::-1] * 3.0  # an exchange matrix: a swap at every step of the first half
+    lu, ipiv, info, _, _ = _getrf(cuda, p)
+    lu_o, ipiv_o, _ = O.lu(p)
+    assert np.array_equal(ipiv, ipiv_o) and np.array_equal(lu, lu_o)
+
+
+@pytest.mark.parametrize("cols", [[0], [31, 32], [127, 128, 129], [299]])
+def test_zero_columns(cuda, cols):
+    n = 300
+    rng = np.random.default_rng(5)
+    a = rng.standard_normal((n, n))
+    a[:, cols] = 0.0
+    lu, ipiv, info, _, _ = _getrf(cuda, a)
+    _, ipiv_o, _ = O.lu(a)
+    assert info == cols[0] + 1 and np.array_equal(ipiv, ipiv_o)
+    assert O.lu_reconstruction(a, lu, ipiv) <= 10.0
+
+
+def test_zero_block_and_row_scales(cuda):
+    n = 420
+    rng = np.random.default_rng(6)
+    a = rng.standard_normal((n, n)) * 2.0 ** rng.integers(-200, 201, size=(n, 1))
+    lu, ipiv, info, _, _ = _getrf(cuda, a)
+    _, ipiv_o, _ = O.lu(a)
+    assert info == 0 and np.array_equal(ipiv, ipiv_o)
+    b = np.zeros((n, n))
+    b[:100, :100] = rng.standard_normal((100, 100))
+    lu, ipiv, info, _, _ = _getrf(cuda, b)
+    _, ipiv_o, _ = O.lu(b)
+    assert info == 101 and np.array_equal(ipiv[:100], ipiv_o[:100])
+    assert np.all(lu[:, 100:] == 0.0) and O.lu_reconstruction(b, lu, ipiv) <= 10.0
+
+
+def test_nan_is_a_pivot_only_in_first_position(cuda):
+    n = 180
+    rng = np.random.default_rng(7)
+    a = rng.standard_normal((n, n))
+    a[90, 0] = np.nan  # below the first position: not chosen
+    _, ipiv, _, _, _ = _getrf(cuda, a)
+    _, ipiv_o, _ = O.lu(a)
+    assert ipiv[0] == ipiv_o[0] != 90
+    a[90, 0] = 1.0
+    a[0, 0] = np.nan  # the first: it wins
+    _, ipiv, _, _, _ = _getrf(cuda, a)
+    _, ipiv_o, _ = O.lu(a)
+    assert ipiv[0] == ipiv_o[0] == 0
