@@ -69,6 +69,16 @@ def _bytes(k: int) -> DeviceBuffer:
     return _dev.empty(max(int(k), 1), np.uint8)
 
 
+def _info():
+    """One call's status word in scratch: read it inside the block."""
+    return _dev.scratch_array(1, np.int32, zero=True)
+
+
+def _work(nbytes: int):
+    """One call's workspace in scratch."""
+    return _dev.scratch_array(max(int(nbytes), 1), np.uint8)
+
+
 def _padded_i32(v, n: int) -> DeviceBuffer:
     return _dev.from_numpy(np.append(np.asarray(v).astype(np.int32), np.zeros(max(n, 1) - n, np.int32)))
 
@@ -118,17 +128,17 @@ class DeviceMatrix:
         overwritten."""
         n = self.nrows
         assert self.is_square() and b.nrows == n, "triangular solve dimension mismatch"
-        info = _i32(1)
-        if n > 128:
-            ws = _bytes(_lib.load().nacu_trsv_workspace_bytes(n))
-            _lib.call("nacu_dtrsv", n, b.ncols, int(upper), int(trans), int(diag is not None),
-                      float(diag if diag is not None else 0.0), self.data.data_ptr(), n, b.data.data_ptr(), n,
-                      info.data_ptr(), ws.data_ptr(), ws.numel(), flags, _stream_ptr())
+        with _info() as info:
+            if n > 128:
+                with _work(_lib.load().nacu_trsv_workspace_bytes(n)) as ws:
+                    _lib.call("nacu_dtrsv", n, b.ncols, int(upper), int(trans), int(diag is not None),
+                              float(diag if diag is not None else 0.0), self.data.data_ptr(), n, b.data.data_ptr(), n,
+                              info.data_ptr(), ws.data_ptr(), ws.numel(), flags, _stream_ptr())
+            else:
+                _lib.call("nacu_dtrsv_batched", n, b.ncols, int(upper), int(trans), int(diag is not None),
+                          float(diag if diag is not None else 0.0), self.data.data_ptr(), n * n, b.data.data_ptr(),
+                          n * b.ncols, info.data_ptr(), 1, flags, _stream_ptr())
             return int(info.item()) == 0
-        _lib.call("nacu_dtrsv_batched", n, b.ncols, int(upper), int(trans), int(diag is not None),
-                  float(diag if diag is not None else 0.0), self.data.data_ptr(), n * n, b.data.data_ptr(),
-                  n * b.ncols, info.data_ptr(), 1, flags, _stream_ptr())
-        return int(info.item()) == 0
 
     def solve_lower_triangular_mut(self, b: "DeviceMatrix", flags: int = 0) -> bool:
         """Matrix::solve_lower_triangular_mut (src/linalg/solve.rs:55-101)."""
@@ -215,9 +225,9 @@ class LU:
         self.info = _i32(2)
         self.large = n > 128
         if self.large:
-            self._ws = _bytes(_lib.load().nacu_getrf_workspace_bytes(n))
-            _lib.call("nacu_dgetrf", n, m.data.data_ptr(), n, self.ipiv.data_ptr(), self.info.data_ptr(),
-                      self._ws.data_ptr(), self._ws.numel(), _stream_ptr())
+            with _work(_lib.load().nacu_getrf_workspace_bytes(n)) as ws:
+                _lib.call("nacu_dgetrf", n, m.data.data_ptr(), n, self.ipiv.data_ptr(), self.info.data_ptr(),
+                          ws.data_ptr(), ws.numel(), _stream_ptr())
         else:
             _lib.call("nacu_dgetrf_batched", n, m.data.data_ptr(), n * n, self.ipiv.data_ptr(),
                       self.info.data_ptr(), 1, flags, _stream_ptr())
@@ -226,18 +236,19 @@ class LU:
         """LU::solve_mut (src/linalg/lu.rs:242-260)."""
         n = self.lu.nrows
         assert b.nrows == n, "LU solve matrix dimension mismatch."
-        info = _i32(1)
-        if self.large:
+        with _info() as info:
+            if not self.large:
+                _lib.call("nacu_dgetrs_batched", n, b.ncols, self.lu.data.data_ptr(), n * n, self.ipiv.data_ptr(),
+                          b.data.data_ptr(), n * b.ncols, info.data_ptr(), 1, self.flags, _stream_ptr())
+                return int(info.item()) == 0
             ok = True
-            for c in range(b.ncols):
-                _lib.call("nacu_dgetrs", n, self.lu.data.data_ptr(), n, self.ipiv.data_ptr(),
-                          b.data.data_ptr() + c * n * 8, info.data_ptr(), self._ws.data_ptr(), self._ws.numel(),
-                          _stream_ptr())
-                ok = ok and int(info.item()) == 0
+            with _work(_lib.load().nacu_getrf_workspace_bytes(n)) as ws:
+                for c in range(b.ncols):
+                    _lib.call("nacu_dgetrs", n, self.lu.data.data_ptr(), n, self.ipiv.data_ptr(),
+                              b.data.data_ptr() + c * n * 8, info.data_ptr(), ws.data_ptr(), ws.numel(),
+                              _stream_ptr())
+                    ok = ok and int(info.item()) == 0
             return ok
-        _lib.call("nacu_dgetrs_batched", n, b.ncols, self.lu.data.data_ptr(), n * n, self.ipiv.data_ptr(),
-                  b.data.data_ptr(), n * b.ncols, info.data_ptr(), 1, self.flags, _stream_ptr())
-        return int(info.item()) == 0
 
     def solve(self, b: DeviceMatrix):
         """LU::solve (src/linalg/lu.rs:221-236): a new matrix, or None."""
@@ -267,10 +278,10 @@ class LU:
         if self.large:
             raise NotImplementedError("try_inverse: n <= 128 (the batched kernels)")
         out = DeviceMatrix(_dev.empty(n * n, np.float64), n, n)
-        info = _i32(1)
-        _lib.call("nacu_dgetri_batched", n, self.lu.data.data_ptr(), n * n, self.ipiv.data_ptr(), out.data.data_ptr(),
-                  n * n, info.data_ptr(), 1, self.flags, _stream_ptr())
-        return out if int(info.item()) == 0 else None
+        with _info() as info:
+            _lib.call("nacu_dgetri_batched", n, self.lu.data.data_ptr(), n * n, self.ipiv.data_ptr(),
+                      out.data.data_ptr(), n * n, info.data_ptr(), 1, self.flags, _stream_ptr())
+            return out if int(info.item()) == 0 else None
 
     def l(self) -> np.ndarray:
         lu = self.lu.to_numpy()
@@ -293,8 +304,6 @@ class LU:
         obj.ipiv = _padded_i32(ipiv, n)
         zero = np.nonzero(np.diag(lu) == 0)[0]
         obj.info = _dev.from_numpy(np.array([int(zero[0]) + 1 if len(zero) else 0, 0], np.int32))
-        if obj.large:
-            obj._ws = _bytes(_lib.load().nacu_getrf_workspace_bytes(n))
         return obj
 
 
@@ -314,13 +323,13 @@ class FullPivLU:
 
     def _solve_cols(self, b: DeviceMatrix) -> bool:
         n = self.lu.nrows
-        info = _i32(1)
-        for c0 in range(0, b.ncols, 16):
-            k = min(16, b.ncols - c0)
-            _lib.call("nacu_dfullpivlu_solve_batched", n, k, self.lu.data.data_ptr(), n * n, self.ipiv.data_ptr(),
-                      self.jpiv.data_ptr(), b.data.data_ptr() + c0 * n * 8, n * k, info.data_ptr(), 1, self.flags,
-                      _stream_ptr())
-        return int(info.item()) == 0
+        with _info() as info:
+            for c0 in range(0, b.ncols, 16):
+                k = min(16, b.ncols - c0)
+                _lib.call("nacu_dfullpivlu_solve_batched", n, k, self.lu.data.data_ptr(), n * n, self.ipiv.data_ptr(),
+                          self.jpiv.data_ptr(), b.data.data_ptr() + c0 * n * 8, n * k, info.data_ptr(), 1, self.flags,
+                          _stream_ptr())
+            return int(info.item()) == 0
 
     def solve_mut(self, b: DeviceMatrix) -> bool:
         """FullPivLU::solve_mut (src/linalg/full_piv_lu.rs:185-211)."""
@@ -414,18 +423,18 @@ class QR:
 
     def _solve_cols(self, b: DeviceMatrix) -> bool:
         m, n = self.qr.shape
-        info = _i32(1)
-        if self.large:
-            ws = _bytes(_lib.load().nacu_qr_solve_workspace_bytes(n))
-            _lib.call("nacu_dqr_solve", m, n, b.ncols, self.qr.data.data_ptr(), max(m, 1), self.diag.data_ptr(),
-                      b.data.data_ptr(), max(m, 1), info.data_ptr(), ws.data_ptr(), ws.numel(), self.flags,
-                      _stream_ptr())
+        with _info() as info:
+            if self.large:
+                with _work(_lib.load().nacu_qr_solve_workspace_bytes(n)) as ws:
+                    _lib.call("nacu_dqr_solve", m, n, b.ncols, self.qr.data.data_ptr(), max(m, 1),
+                              self.diag.data_ptr(), b.data.data_ptr(), max(m, 1), info.data_ptr(), ws.data_ptr(),
+                              ws.numel(), self.flags, _stream_ptr())
+            else:
+                for c0 in range(0, b.ncols, 16):
+                    k = min(16, b.ncols - c0)
+                    _lib.call("nacu_dqr_solve_batched", n, k, self.qr.data.data_ptr(), n * n, self.diag.data_ptr(),
+                              b.data.data_ptr() + c0 * n * 8, n * k, info.data_ptr(), 1, self.flags, _stream_ptr())
             return int(info.item()) == 0
-        for c0 in range(0, b.ncols, 16):
-            k = min(16, b.ncols - c0)
-            _lib.call("nacu_dqr_solve_batched", n, k, self.qr.data.data_ptr(), n * n, self.diag.data_ptr(),
-                      b.data.data_ptr() + c0 * n * 8, n * k, info.data_ptr(), 1, self.flags, _stream_ptr())
-        return int(info.item()) == 0
 
     def solve_mut(self, b: DeviceMatrix) -> bool:
         """QR::solve_mut (src/linalg/qr.rs:204-222), square factors: b is
@@ -512,13 +521,13 @@ class ColPivQR:
 
     def _solve_cols(self, b: DeviceMatrix) -> bool:
         n = self.qr.nrows
-        info = _i32(1)
-        for c0 in range(0, b.ncols, 16):
-            k = min(16, b.ncols - c0)
-            _lib.call("nacu_dcolpivqr_solve_batched", n, k, self.qr.data.data_ptr(), n * n, self.diag.data_ptr(),
-                      self.jpiv.data_ptr(), b.data.data_ptr() + c0 * n * 8, n * k, info.data_ptr(), 1, self.flags,
-                      _stream_ptr())
-        return int(info.item()) == 0
+        with _info() as info:
+            for c0 in range(0, b.ncols, 16):
+                k = min(16, b.ncols - c0)
+                _lib.call("nacu_dcolpivqr_solve_batched", n, k, self.qr.data.data_ptr(), n * n, self.diag.data_ptr(),
+                          self.jpiv.data_ptr(), b.data.data_ptr() + c0 * n * 8, n * k, info.data_ptr(), 1, self.flags,
+                          _stream_ptr())
+            return int(info.item()) == 0
 
     def solve_mut(self, b: DeviceMatrix) -> bool:
         """ColPivQR::solve_mut (src/linalg/col_piv_qr.rs:227-247): b is
@@ -593,11 +602,11 @@ def solve_refined(a: DeviceMatrix, b: DeviceMatrix, tol_units: float = 1.0, max_
     n = a.nrows
     assert a.is_square() and b.nrows == n and b.ncols == 1, "one n x n system with one right-hand side"
     x = DeviceMatrix(_dev.empty(n, np.float64), n, 1)
-    ws = _bytes(_lib.load().nacu_gesv_mixed_workspace_bytes(n))
     it, berr, fb = C.c_int(0), C.c_double(0.0), C.c_int(0)
-    _lib.call("nacu_dgesv_mixed_ir", n, a.data.data_ptr(), n, b.data.data_ptr(), x.data.data_ptr(),
-              float(tol_units), int(max_iter), C.byref(it), C.byref(berr), C.byref(fb), ws.data_ptr(), ws.numel(),
-              _stream_ptr())
+    with _work(_lib.load().nacu_gesv_mixed_workspace_bytes(n)) as ws:
+        _lib.call("nacu_dgesv_mixed_ir", n, a.data.data_ptr(), n, b.data.data_ptr(), x.data.data_ptr(),
+                  float(tol_units), int(max_iter), C.byref(it), C.byref(berr), C.byref(fb), ws.data_ptr(), ws.numel(),
+                  _stream_ptr())
     return x, {"iters": it.value, "berr": berr.value, "fallback": fb.value == 1, "gmres": fb.value == 2}
 
 

@@ -328,6 +328,16 @@ def scratch(nbytes: int, required: bool = True):
         _lib.call("nacu_free_async", p.value, s)
 
 
+@contextlib.contextmanager
+def scratch_array(shape, dtype, zero: bool = False):
+    """A DeviceBuffer of scratch for calls queued on the current stream inside
+    the block (``scratch``; a plain allocation where that is not to be had)."""
+    nbytes = math.prod(_shape(shape)) * np.dtype(dtype).itemsize
+    with scratch(nbytes, required=False) as p:
+        buf = DeviceBuffer(p, shape, dtype) if p else DeviceBuffer.empty(shape, dtype)
+        yield buf.zero_() if zero else buf
+
+
 def empty(shape, dtype=np.float64) -> DeviceBuffer:
     return DeviceBuffer.empty(shape, dtype)
 
