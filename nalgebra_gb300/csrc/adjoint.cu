@@ -561,6 +561,336 @@ __global__ void __launch_bounds__(kAdjTcThreads, 4)
   if (tid == 0 && info) info[s] = inf;
 }
 
+// ---------------------------------------------------------------------------
+// FP32 in blocks of 16 columns, orders above kAdjF32MinOrder.
+//
+// The column-by-column kernels above take three barriers and an integer
+// division per element for every column; FP32 itself is far from its limits.
+// Here the matrix sits in shared memory as a square (odd leading dimension) and
+// a block of 16 columns takes three barriers: warp 0 factors the 16 x 16 head in
+// registers, a thread per row solves its 16 entries against it and leaves them
+// k-major in S, and warps apply 16-deep products in 16 x 32 tiles of 4 x 4 per
+// lane.  The backward pass is the FP64 one's sweep (adj_tc_backward_kernel): X =
+// L^-T rides below the factor, A^-1 = X X^T accumulates in the lower triangle.
+// 1000 x 97, factor recomputed: forward 385 -> 117, backward 615 -> 210 us.
+// ---------------------------------------------------------------------------
+constexpr int kAdjF32Threads = 128;
+// At order 4 both take 95 us forward (20,000 matrices; 10,000 of order 6: 72
+// against 59); below it the 16 x 16 head is mostly padding (order 1: 40 against 92).
+constexpr int kAdjF32MinOrder = 4;
+
+__host__ __device__ constexpr int adj_f32_slots(int n) { return (n + 15) / 16 * 16 + 4; }  // rows of S, and one vector
+constexpr size_t adj_f32_smem(int n) {
+  return ((size_t)((n * (n | 1) + 3) & ~3) + 16 * (size_t)adj_f32_slots(n) + 256 + 16 + 2 * (size_t)((n + 3) & ~3)) *
+         sizeof(float);
+}
+struct AdjF32 {
+  float *M, *S, *Hd, *rd, *z, *v;
+  int n, ld, slots;
+  __device__ AdjF32(int n_, unsigned char* smem) : n(n_), ld(n_ | 1), slots(adj_f32_slots(n_)) {
+    M = reinterpret_cast<float*>(smem);
+    S = M + ((n * ld + 3) & ~3);
+    Hd = S + 16 * slots;
+    rd = Hd + 256;
+    z = rd + 16;
+    v = z + ((n + 3) & ~3);
+  }
+  // the head at J0 of the matrix in M, factored in place by one warp: Hd[j * 16 + r], 1 / L_jj in rd
+  __device__ void head(int J0, int* s_info, int lane) const {
+    const int w = min(16, n - J0), r = lane & 15, h = lane >> 4;
+    float a[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int c = 2 * i + h;
+      a[i] = (r < w && c <= r) ? M[(J0 + c) * ld + J0 + r] : (r == c ? 1.f : 0.f);
+    }
+    int fail = 0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int ij = j >> 1, hj = (j & 1) * 16;
+      const float d = __shfl_sync(0xffffffffu, a[ij], j + hj);
+      if (!pos_or_inf(d) && fail == 0) fail = J0 + j + 1;
+      const float rcp = rsqrt(d);
+      if (h == (j & 1)) a[ij] = r > j ? a[ij] * rcp : (r == j ? d * rcp : a[ij]);
+      if (lane == 0) rd[j] = rcp;
+      const float x = __shfl_sync(0xffffffffu, a[ij], r + hj);
+#pragma unroll
+      for (int i = ij; i < 8; ++i) {
+        const int c = 2 * i + h;
+        const float l = __shfl_sync(0xffffffffu, a[ij], (c & 15) + hj);
+        if (c > j && r >= c) a[i] = fmaf(-x, l, a[i]);
+      }
+    }
+    if (fail && lane == 0) *s_info = fail;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int c = 2 * i + h;
+      Hd[c * 16 + r] = a[i];
+      if (r < w && c <= r) M[(J0 + c) * ld + J0 + r] = a[i];
+    }
+  }
+  // x against the head (w <= 16 columns)
+  __device__ void solve(float (&x)[16], int w) const {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      x[j] *= j < w ? rd[j] : 0.f;
+#pragma unroll
+      for (int k = j + 1; k < 16; ++k) x[k] = fmaf(-x[j], Hd[j * 16 + k], x[k]);
+    }
+  }
+  // One tile: slots r0 .. r0 + 15 times slots c0 .. c0 + 31 (multiples of 4),
+  // dest(i, k) its elements' places.  A lane's rows are four apart and its
+  // columns adjacent, so a warp's places lie in 32 different banks (odd ld).
+  template <typename F>
+  __device__ void tile(int r0, int c0, int lane, bool add, bool fresh, F dest) const {
+    const int rg = r0 + (lane & 3), cg = c0 + 4 * (lane >> 2);
+    float acc[4][4] = {};
+    if (cg < slots) {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        const float4 b = *reinterpret_cast<const float4*>(S + k * slots + cg);
+        const float bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float a = S[k * slots + rg + 4 * i];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) acc[i][q] = fmaf(a, bv[q], acc[i][q]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        float* p = dest((lane & 3) + 4 * i, cg - c0 + q);
+        if (p) *p = (fresh ? 0.f : *p) + (add ? acc[i][q] : -acc[i][q]);
+      }
+  }
+  // dot product of two slots' 16 entries
+  __device__ float dot(int p, int q) const {
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) s = fmaf(S[k * slots + p], S[k * slots + q], s);
+    return s;
+  }
+  __device__ void keep(const float (&x)[16], int slot) const {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) S[k * slots + slot] = x[k];
+  }
+};
+
+__global__ void __launch_bounds__(kAdjF32Threads) adj_f32_forward_kernel(int n, const float* __restrict__ A, int64_t strideA,
+                                                                         const float* __restrict__ B, float* __restrict__ X,
+                                                                         float* __restrict__ Lout, float* __restrict__ logdet,
+                                                                         int32_t* __restrict__ info) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int s_info;
+  __shared__ float s_part[kAdjF32Threads / 32];
+  const AdjF32 m(n, smem_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, s = blockIdx.x;
+  constexpr int nw = kAdjF32Threads / 32;
+  float* y = m.z;
+  const float* a = A + (size_t)s * strideA;
+  for (int c = warp; c < n; c += nw)
+    for (int r = c + lane; r < n; r += 32) m.M[c * m.ld + r] = a[(size_t)c * n + r];
+  for (int i = tid; i < n; i += kAdjF32Threads) y[i] = B[(size_t)s * n + i];
+  if (tid == 0) s_info = 0;
+  __syncthreads();
+  for (int J0 = 0; J0 < n; J0 += 16) {
+    if (warp == 0) m.head(J0, &s_info, lane);
+    __syncthreads();
+    if (s_info != 0) break;
+    const int j1 = J0 + 16, w = min(16, n - J0), mp = max(0, (n - j1 + 15) / 16 * 16);
+    for (int q = tid; q <= mp; q += kAdjF32Threads) {  // rows below, then y
+      float x[16];
+      const bool vec = q == mp, on = vec || j1 + q < n;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) x[j] = (on && j < w) ? (vec ? y[J0 + j] : m.M[(J0 + j) * m.ld + j1 + q]) : 0.f;
+      m.solve(x, w);
+      m.keep(x, q);
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (on && j < w) (vec ? y[J0 + j] : m.M[(J0 + j) * m.ld + j1 + q]) = x[j];
+    }
+    __syncthreads();
+    const int mt = mp >> 4;
+    for (int u = warp, rt = 0; rt < mt; u -= rt / 2 + 1, ++rt) {  // row tile rt: rt / 2 + 1 groups of 32 columns
+      for (; u < rt / 2 + 1; u += nw)
+        m.tile(16 * rt, 32 * u, lane, false, false, [&](int i, int k) -> float* {
+          const int r = j1 + 16 * rt + i, c = j1 + 32 * u + k;
+          return r < n && c <= r ? m.M + c * m.ld + r : nullptr;
+        });
+    }
+    for (int r = j1 + tid; r < n; r += kAdjF32Threads) y[r] -= m.dot(r - j1, mp);
+    __syncthreads();
+  }
+  const int inf = s_info;
+  if (inf == 0) {
+    // x = L^-T y in blocks of 16 rows from the bottom
+    for (int J0 = (n - 1) / 16 * 16; J0 >= 0; J0 -= 16) {
+      const int w = min(16, n - J0);
+      if (warp == 0) {
+        float v = lane < w ? y[J0 + lane] : 0.f;
+        for (int j = w - 1; j >= 0; --j) {
+          const float xj = __shfl_sync(0xffffffffu, v, j) / m.M[(J0 + j) * m.ld + J0 + j];
+          if (lane == j) v = xj;
+          if (lane < j) v = fmaf(-xj, m.M[(J0 + lane) * m.ld + J0 + j], v);
+        }
+        if (lane < w) y[J0 + lane] = v;
+      }
+      __syncthreads();
+      for (int i = tid; i < J0; i += kAdjF32Threads) {
+        float v = y[i];
+        for (int r = 0; r < w; ++r) v = fmaf(-m.M[i * m.ld + J0 + r], y[J0 + r], v);
+        y[i] = v;
+      }
+      __syncthreads();
+    }
+    float part = 0.f;
+    for (int i = tid; i < n; i += kAdjF32Threads) {
+      X[(size_t)s * n + i] = y[i];
+      const float d = m.M[i * m.ld + i];
+      part += logf(d * d);
+    }
+    part = warp_sum(part);
+    if (lane == 0) s_part[warp] = part;
+    __syncthreads();
+    if (tid == 0) {
+      float sum = 0.f;
+      for (int u = 0; u < nw; ++u) sum += s_part[u];
+      logdet[s] = sum;
+    }
+    if (Lout)
+      for (int c = warp; c < n; c += nw)
+        for (int r = lane; r < n; r += 32) Lout[(size_t)s * strideA + (size_t)c * n + r] = r >= c ? m.M[c * m.ld + r] : 0.f;
+  }
+  if (tid == 0 && info) info[s] = inf;
+}
+
+template <bool RECOMPUTE>
+__global__ void __launch_bounds__(kAdjF32Threads)
+    adj_f32_backward_kernel(int n, const float* __restrict__ AL, int64_t strideA, const float* __restrict__ X,
+                            const float* __restrict__ Wt, const float* __restrict__ Glog, float* __restrict__ dA,
+                            float* __restrict__ db, int32_t* __restrict__ info) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int s_info;
+  const AdjF32 m(n, smem_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, s = blockIdx.x;
+  constexpr int nw = kAdjF32Threads / 32;
+  const int np = (n + 15) / 16 * 16;
+  const float* al = AL + (size_t)s * strideA;
+  if (RECOMPUTE)
+    for (int c = warp; c < n; c += nw)
+      for (int r = c + lane; r < n; r += 32) m.M[c * m.ld + r] = al[(size_t)c * n + r];
+  for (int i = tid; i < n; i += kAdjF32Threads) {
+    m.z[i] = Wt[(size_t)s * n + i];
+    m.v[i] = 0.f;
+  }
+  if (tid == 0) s_info = 0;
+  __syncthreads();
+  for (int J0 = 0; J0 < n; J0 += 16) {
+    const int j1 = J0 + 16, w = min(16, n - J0), blk = J0 >> 4, mp = np - j1, mt = mp >> 4;
+    if (warp == 0) {
+      if (RECOMPUTE) {
+        m.head(J0, &s_info, lane);
+      } else {
+        for (int e = lane; e < 256; e += 32) {
+          const int c = e >> 4, r = e & 15;
+          m.Hd[e] = (r < w && c <= r) ? al[(size_t)(J0 + c) * n + J0 + r] : 0.f;
+        }
+        if (lane < w) m.rd[lane] = 1.f / al[(size_t)(J0 + lane) * (n + 1)];
+      }
+    }
+    __syncthreads();
+    if (RECOMPUTE && s_info != 0) break;
+    // slots [0, mp): the factor's rows below; [mp, np): X's rows; np: z
+    for (int q = tid; q <= np; q += kAdjF32Threads) {
+      const int c = q - mp;
+      float x[16];
+      const bool on = q < mp ? j1 + q < n : q == np || c < n;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        x[j] = 0.f;
+        if (on && j < w) {
+          if (q < mp) x[j] = RECOMPUTE ? m.M[(J0 + j) * m.ld + j1 + q] : al[(size_t)(J0 + j) * n + j1 + q];
+          else if (q == np) x[j] = m.z[J0 + j];
+          else if (c >= J0) x[j] = c - J0 == j ? 1.f : 0.f;
+          else x[j] = m.M[(J0 + j) * m.ld + c];
+        }
+      }
+      if (RECOMPUTE || q >= mp) m.solve(x, w);
+      m.keep(x, q);
+    }
+    __syncthreads();
+    // X against the factor's rows; X against X; the factor's rest; z and v
+    const int ux = (blk + 1) * ((mt + 1) >> 1);
+    const int k1 = (blk + 1) >> 1, us = (blk + 1) & 1 ? (k1 + 1) * (k1 + 1) : k1 * (k1 + 1);
+    const int k2 = mt >> 1, ul = !RECOMPUTE ? 0 : mt & 1 ? (k2 + 1) * (k2 + 1) : k2 * (k2 + 1);
+    // tiles 2 k and 2 k + 1 of a triangle have k + 1 units each
+    auto triangle = [](int q, int* rt, int* c0) {
+      int k = (int)((sqrtf(1.0f + 4.0f * (float)q) - 1.0f) * 0.5f);
+      if (k * (k + 1) > q) --k;
+      if ((k + 1) * (k + 2) <= q) ++k;
+      const int rem = q - k * (k + 1);
+      *rt = rem <= k ? 2 * k : 2 * k + 1;
+      *c0 = 32 * (rem <= k ? rem : rem - k - 1);
+    };
+    for (int u = warp; u < ux + us + ul; u += nw) {
+      int rt, c0;
+      if (u < ux) {
+        rt = u % (blk + 1);
+        c0 = 32 * (u / (blk + 1));
+        m.tile(mp + 16 * rt, c0, lane, false, rt == blk, [&](int i, int k) -> float* {
+          const int r = j1 + c0 + k, c = 16 * rt + i;
+          return c0 + k < mp && r < n && c < n ? m.M + r * m.ld + c : nullptr;
+        });
+      } else if (u < ux + us) {
+        triangle(u - ux, &rt, &c0);
+        m.tile(mp + 16 * rt, mp + c0, lane, true, rt == blk, [&](int i, int k) -> float* {
+          const int r = 16 * rt + i, c = c0 + k;
+          return r < n && c <= r ? m.M + c * m.ld + r : nullptr;
+        });
+      } else {
+        triangle(u - ux - us, &rt, &c0);
+        m.tile(16 * rt, c0, lane, false, false, [&](int i, int k) -> float* {
+          const int r = j1 + 16 * rt + i, c = j1 + c0 + k;
+          return r < n && c <= r ? m.M + c * m.ld + r : nullptr;
+        });
+      }
+    }
+    for (int q = tid; q < np; q += kAdjF32Threads) {
+      const int r = q < mp ? j1 + q : q - mp;
+      if (r < n) {
+        if (q < mp) m.z[r] -= m.dot(q, np);
+        else m.v[r] += m.dot(q, np);
+      }
+    }
+    __syncthreads();
+  }
+  const int inf = RECOMPUTE ? s_info : 0;
+  if (inf == 0) {
+    float* xs = m.z;
+    for (int i = tid; i < n; i += kAdjF32Threads) {
+      xs[i] = X[(size_t)s * n + i];
+      db[(size_t)s * n + i] = m.v[i];
+    }
+    __syncthreads();
+    const float gl = Glog ? Glog[s] : 1.f, gl2 = 2.f * gl;
+    for (int c = warp; c < n; c += nw) {
+      const float vc = m.v[c], xc = xs[c];
+      const float* col = m.M + c * m.ld;
+      float* out = dA + (size_t)s * strideA + (size_t)c * n;
+      for (int r = lane; r < n; r += 32) {
+        float val = 0.f;
+        if (r > c) val = fmaf(-m.v[r], xc, fmaf(-vc, xs[r], gl2 * col[r]));
+        else if (r == c) val = fmaf(-vc, xc, gl * col[r]);
+        out[r] = val;
+      }
+    }
+  }
+  if (tid == 0 && info) info[s] = inf;
+}
+
 template <typename T>
 int adj_launch_forward(int n, const T* A, int64_t strideA, const T* B, T* X, T* Lout, T* logdet, int32_t* info,
                        int batch, cudaStream_t stream, const char* name) {
@@ -569,6 +899,15 @@ int adj_launch_forward(int n, const T* A, int64_t strideA, const T* B, T* X, T* 
   if (batch == 0) return NACU_SUCCESS;
   if (!A || !B || !X || !logdet) return record_arg_error(-2, "posv_logdet_forward: null A, B, X or logdet");
   if (strideA < (int64_t)n * n) return record_arg_error(-3, "posv_logdet_forward: strideA < n*n");
+  if constexpr (sizeof(T) == 4) {
+    if (n > kAdjF32MinOrder) {
+      const size_t bytes = adj_f32_smem(n);
+      cudaError_t e = ensure_dynamic_smem(adj_f32_forward_kernel, bytes);
+      if (e != cudaSuccess) return record_cuda_error(e, name);
+      adj_f32_forward_kernel<<<batch, kAdjF32Threads, bytes, stream>>>(n, A, strideA, B, X, Lout, logdet, info);
+      return check_launch(name);
+    }
+  }
   const size_t smem = ((size_t)n * (n + 1) / 2 + n) * sizeof(T);
   cudaError_t e = ensure_dynamic_smem(adj_forward_kernel<T>, smem);
   if (e != cudaSuccess) return record_cuda_error(e, name);
@@ -584,7 +923,16 @@ int adj_launch_backward(int n, const T* AL, int64_t strideA, int recompute, cons
   if (batch == 0) return NACU_SUCCESS;
   if (!AL || !X || !W || !dA || !db) return record_arg_error(-2, "posv_logdet_backward: null argument");
   if (strideA < (int64_t)n * n) return record_arg_error(-3, "posv_logdet_backward: strideA < n*n");
-  if constexpr (sizeof(T) == 8) {
+  if constexpr (sizeof(T) == 4) {
+    if (n > kAdjF32MinOrder) {
+      const auto kern = recompute ? adj_f32_backward_kernel<true> : adj_f32_backward_kernel<false>;
+      const size_t bytes = adj_f32_smem(n);
+      cudaError_t e = ensure_dynamic_smem(kern, bytes);
+      if (e != cudaSuccess) return record_cuda_error(e, name);
+      kern<<<batch, kAdjF32Threads, bytes, stream>>>(n, AL, strideA, X, W, G, dA, db, info);
+      return check_launch(name);
+    }
+  } else {
     if (n > kAdjTcMinOrder) {
       const auto kern = recompute ? adj_tc_backward_kernel<true> : adj_tc_backward_kernel<false>;
       const size_t bytes = adj_tc_smem(n);

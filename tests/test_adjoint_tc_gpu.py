@@ -43,6 +43,30 @@ def test_gradient_at_block_edges(cuda, n, recompute):
         assert np.all(np.triu(got, 1) == 0.0)
 
 
+@pytest.mark.parametrize("recompute", [0, 1])
+@pytest.mark.parametrize("n", [4, 5, 6, 15, 16, 17, 31, 32, 33, 48, 97, 112, 127, 128])
+def test_f32_gradient_at_block_edges(cuda, n, recompute):
+    """The FP32 form in blocks of 16: the same bound with FP32's rounding."""
+    eps32 = 2.0 ** -23
+    rng = np.random.default_rng(n)
+    count = 2
+    f = rng.standard_normal((count, n, n))
+    a = (f @ np.transpose(f, (0, 2, 1)) + np.array([n, 4.0])[:, None, None] * np.eye(n)).astype(np.float32)
+    b, w = rng.standard_normal((count, n)).astype(np.float32), rng.standard_normal((count, n)).astype(np.float32)
+    X, logdet, dA, db, info = _gpu(cuda, a.reshape(count, n * n), b, w, n, np.float32, recompute)
+    assert np.all(info == 0)
+    for s in range(count):
+        ad, bd, wd = a[s].astype(np.float64), b[s].astype(np.float64), w[s].astype(np.float64)
+        g, v = _reference(ad, bd, wd)
+        x = np.linalg.solve(ad, bd)
+        tol = 8 * n * eps32 * np.linalg.cond(ad)
+        assert np.max(np.abs(X[s] - x)) <= tol * np.max(np.abs(x))
+        assert abs(logdet[s] - np.linalg.slogdet(ad)[1]) <= tol * n
+        assert np.max(np.abs(db[s] - v)) <= tol * np.max(np.abs(v))
+        assert np.max(np.abs(dA[s] - g)) <= tol * np.max(np.abs(g))
+        assert np.all(np.triu(dA[s], 1) == 0.0)
+
+
 def test_not_spd_in_the_recompute_form(cuda):
     n, count = 80, 4
     rng = np.random.default_rng(0)
@@ -50,5 +74,6 @@ def test_not_spd_in_the_recompute_form(cuda):
     a = f @ np.transpose(f, (0, 2, 1)) + n * np.eye(n)
     a[2, 40, 40] = -1.0
     b, w = rng.standard_normal((count, n)), rng.standard_normal((count, n))
-    *_, info = _gpu(cuda, a.reshape(count, n * n), b, w, n, np.float64, 1)
-    assert list(info) == [0, 0, 41, 0]
+    for dtype in (np.float64, np.float32):
+        *_, info = _gpu(cuda, a.reshape(count, n * n), b, w, n, dtype, 1)
+        assert list(info) == [0, 0, 41, 0]
