@@ -816,12 +816,20 @@ CrtLayout crt_layout(int m, int n, int k) {
 
 }  // namespace
 
-// Six dependent launches cost about 50 us whatever the size; the FP64 kernel
-// takes 1.05 us per unit of k before it fills the chip.  Measured: 256^3 266
-// against 55 us, 2000 x 2000 x 64 461 against 155 us.  Below 64 products per
-// output, or on thin products, the FP64 kernel keeps the call.
+// The two forms' times in us, from measurements.  The FP64 kernel: 1.05 per unit
+// of k until its tiles fill the chip, then 1.22 TFLOP/s.  The residues: six
+// dependent launches a block, about 50 us, then 18 planes of each operand to
+// write and read and 16 of the product.  Measured, FP64 against residues: 64^3 70
+// and 47, 64 x 64 x 32 38 and 46, 256^3 266 and 55, 1 x 1 x 8192 8266 and 156,
+// 8192 x 1 x 8192 8523 and 1945, 20000 x 4 x 64 197 and 256, 64 x 8192 x 64 72 and
+// 132, 8192 x 8192 x 32 3589 and 1199.
 bool crt_gemm_pays(int m, int n, int k) {
-  return m >= 128 && n >= 128 && k >= 64 && (double)m * n * k >= 3.0e7;
+  if (m <= 0 || n <= 0 || k <= 0) return false;
+  const auto blocks = [](int x, int b) { return (double)((x + b - 1) / b); };
+  const double mn = (double)m * n, fp64 = fmax(1.05 * k, 1.64e-6 * mn * k);
+  const double crt = 55 * blocks(m, kBlockMN) * blocks(n, kBlockMN) * blocks(k, kBlockK) +
+                     3e-5 * ((double)m * k + (double)k * n) + 2e-5 * mn;
+  return crt < fp64;
 }
 
 size_t crt_gemm_workspace_bytes(int m, int n, int k) {

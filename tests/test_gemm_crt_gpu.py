@@ -52,7 +52,8 @@ def _check(torch, a, b, c, alpha, beta, pad=0, eps=4.0):
 
 
 @pytest.mark.parametrize("m,n,k", [(256, 512, 256), (257, 511, 300), (520, 130, 1024), (301, 260, 1025), (150, 200, 3001),
-                                   (128, 4100, 64)])
+                                   (128, 4100, 200), (1, 1, 64), (64, 64, 64), (1, 300, 700), (4097, 1, 300),
+                                   (33, 1000, 130)])
 @pytest.mark.parametrize("alpha,beta,spread,pad", [(1.0, 0.0, 0, 0), (-0.7, 1.3, 20, 3)])
 def test_products(cuda, m, n, k, alpha, beta, spread, pad):
     rng = np.random.default_rng(m + n + k)
@@ -65,6 +66,12 @@ def test_products(cuda, m, n, k, alpha, beta, spread, pad):
         assert np.all(np.isfinite(got))
         c[:] = 0.0
     _check(cuda, a, b, c, alpha, beta, pad)
+
+
+def test_rule_keeps_short_and_thin_products_native():
+    """Where the FP64 kernel is the faster one the workspace query says none."""
+    query = _lib.load().nacu_dgemm_workspace_bytes
+    assert all(query(*s) == 0 for s in [(64, 64, 32), (500, 500, 32), (8192, 1, 64), (64, 8192, 64), (20000, 4, 64), (1, 1, 1)])
 
 
 def test_integers_are_exact(cuda):
