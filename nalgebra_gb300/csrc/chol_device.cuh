@@ -216,16 +216,13 @@ __device__ void chol_forward_cta(int n, const T* __restrict__ a, T* X, int ldx, 
 #pragma unroll
       for (int c = 0; c < kRhsChunk; ++c) b[c] = (lane < ib && c < nr) ? X[(size_t)c * ldx + I0 + lane] : T(0);
       const T rd = (lane < ib) ? rdiag[I0 + lane] : T(0);
-      if constexpr (EXACT || sizeof(T) != 8) {  // EXACT, and FP32 (latency-bound: the short chain)
+      if constexpr (EXACT) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           if (i < ib) {
 #pragma unroll
             for (int c = 0; c < kRhsChunk; ++c) {
-              if (lane == i) {
-                if constexpr (EXACT) b[c] = b[c] / lrow[i];  // solve.rs:509: b_i / L_ii
-                else b[c] = b[c] * rd;
-              }
+              if (lane == i) b[c] = b[c] / lrow[i];  // solve.rs:509: b_i / L_ii
               const T y = __shfl_sync(0xffffffffu, b[c], i);
               if (lane > i) b[c] = axpy1<EXACT>(b[c], -y, lrow[i]);
             }
@@ -282,92 +279,11 @@ __device__ void chol_forward_cta(int n, const T* __restrict__ a, T* X, int ldx, 
   }
 }
 
-// Back solve L^T x = y, FMA form, FP32: blocked from the bottom, reductions
-// over the rows below each 32-row block (16 sums per lane, one 32-lane
-// reduce-scatter), then a warp solve of the transposed block.
-template <typename T>
-__device__ void chol_backward_fast32_cta(int n, const T* __restrict__ a, T* X, int ldx, int nr, const T* rdiag) {
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  const int warp = tid >> 5, lane = tid & 31, nwarps = nthr >> 5;
-  const int nblocks = (n + 31) / 32;
-  for (int bI = nblocks - 1; bI >= 0; --bI) {
-    const int I0 = bI * 32;
-    const int ib = min(32, n - I0);
-    const int r0 = I0 + ib;
-    if (r0 < n) {
-      // y_i -= sum_{r >= r0} L[r][i] x_r for the block's columns i: warp w owns
-      // 4 columns at a time; each lane accumulates 4 columns x 4 rhs over rows
-      // r = r0+lane, r0+lane+32, ... (coalesced column loads), then a butterfly
-      // reduce-scatter leaves sum k = lane & 15 in lane `lane` (16 adds per lane
-      // instead of 16 separate 5-step warp reductions).
-      for (int cb = warp * 4; cb < ib; cb += nwarps * 4) {
-        T v[16];
-#pragma unroll
-        for (int k = 0; k < 16; ++k) v[k] = T(0);
-        for (int r0l = r0 + lane; r0l < n; r0l += 64) {  // two rows per step: 8 loads in flight
-          T l2[2][4];
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int r = r0l + 32 * h;
-              l2[h][j] = (cb + j < ib && r < n) ? a[(size_t)(I0 + cb + j) * n + r] : T(0);
-            }
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int r = r0l + 32 * h;
-            T xr[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) xr[c] = (c < nr && r < n) ? X[(size_t)c * ldx + r] : T(0);
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-#pragma unroll
-              for (int c = 0; c < 4; ++c) v[j * 4 + c] = fma(l2[h][j], xr[c], v[j * 4 + c]);
-          }
-        }
-#pragma unroll
-        for (int half = 8; half >= 1; half >>= 1) {
-          const bool up = (lane & half) != 0;
-#pragma unroll
-          for (int t = 0; t < half; ++t) {
-            const T keep = up ? v[t + half] : v[t];
-            const T give = up ? v[t] : v[t + half];
-            v[t] = keep + __shfl_xor_sync(0xffffffffu, give, half);
-          }
-        }
-        v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);
-        const int j = (lane & 15) >> 2, c = lane & 3;
-        if (lane < 16 && cb + j < ib && c < nr) X[(size_t)c * ldx + I0 + cb + j] -= v[0];
-      }
-      __syncthreads();
-    }
-    if (warp == 0) {
-      T lcol[32];  // lane j holds column j of the diagonal block
-#pragma unroll
-      for (int i = 0; i < 32; ++i) lcol[i] = (lane < ib && i < ib && i >= lane) ? a[(size_t)(I0 + lane) * n + I0 + i] : T(0);
-      const T rd = (lane < ib) ? rdiag[I0 + lane] : T(0);
-      for (int c = 0; c < nr; ++c) {
-        T y = (lane < ib) ? X[(size_t)c * ldx + I0 + lane] : T(0);
-#pragma unroll
-        for (int i = 31; i >= 0; --i) {
-          if (i < ib) {
-            if (lane == i) y = y * rd;
-            const T xi = __shfl_sync(0xffffffffu, y, i);
-            if (lane < i) y = fma(-xi, lcol[i], y);
-          }
-        }
-        if (lane < ib) X[(size_t)c * ldx + I0 + lane] = y;
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// The same in FP64 with fewer warp-wide FP64 instructions: blocked from the
-// bottom, reductions over the rows below each 32-row block, then a warp solve
+// Back solve L^T x = y, FMA form, bound by the FP64 pipe and so with few
+// warp-wide FP64 instructions: blocked from the bottom, reductions over the rows below each 32-row block, then a warp solve
 // of the transposed block.
 template <typename T>
-__device__ void chol_backward_fast64_cta(int n, const T* __restrict__ a, T* X, int ldx, int nr, const T* rdiag) {
+__device__ void chol_backward_fast_cta(int n, const T* __restrict__ a, T* X, int ldx, int nr, const T* rdiag) {
   const int tid = threadIdx.x, nthr = blockDim.x;
   const int warp = tid >> 5, lane = tid & 31, nwarps = nthr >> 5;
   const int nblocks = (n + 31) / 32;
@@ -452,17 +368,6 @@ __device__ void chol_backward_fast64_cta(int n, const T* __restrict__ a, T* X, i
     }
     __syncthreads();
   }
-}
-
-// Back solve L^T x = y, FMA form.  The FP64 variant is bound by the FP64
-// pipe and minimises its warp-wide FP64 instructions; the FP32 variant (the
-// refinement form's solves) is bound by L2 latency and keeps more loads in
-// flight per lane.
-template <typename T>
-__device__ __forceinline__ void chol_backward_fast_cta(int n, const T* __restrict__ a, T* X, int ldx, int nr,
-                                                       const T* rdiag) {
-  if constexpr (sizeof(T) == 8) chol_backward_fast64_cta<T>(n, a, X, ldx, nr, rdiag);
-  else chol_backward_fast32_cta<T>(n, a, X, ldx, nr, rdiag);
 }
 
 // Back solve L^T x = y in nalgebra's exact order (solve.rs:732-755): for i from
