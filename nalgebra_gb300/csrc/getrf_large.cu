@@ -15,12 +15,12 @@
 //      FP64 (gemm_crt.cu), the BF16-split tensor-core GEMM for the FP32 factor.
 // Orders up to 8192 take 128 columns per block, panels in registers and 32-deep
 // updates inside the block; above, a block is one panel of 64 (FP64) or 128.
-// Measured, FP64 (all on the FP64 pipe -> residue updates with 64-wide panels ->
-// register panels): n = 8192 328 -> 114 -> 65 ms, 4096 50 -> 24.6 -> 20.0, 2000 11.6 ->
-// 9.4 -> 8.7, 1000 4.62 -> 4.20 -> 4.08.  FP32 factor with refinement, n = 4096: 15.8
-// -> 14.6 ms.  The panels bound it: a column costs about 4900 cycles at n = 1000
-// (pivot search 420, the candidate's push 1200, cluster barrier 1000, the
-// winner 350, the FP64 update 1900).
+// Measured, FP64, ms (all on the FP64 pipe -> residue updates with 64-wide panels ->
+// register panels behind a cluster barrier -> as below): n = 8192 328 -> 114 -> 65 -> 63,
+// 4096 50 -> 24.6 -> 20.0 -> 16.8, 2000 11.6 -> 9.4 -> 8.7 -> 6.1, 1000 4.62 -> 4.20 ->
+// 4.08 -> 2.75.  FP32 factor with refinement, n = 4096: 15.8 -> 15.8 -> 14.2 -> 12.6.
+// The chain of panels and inner updates bounds it: at n = 8192 50 ms of the 63 are
+// left when the trailing update beyond the next panel costs nothing.
 // The triangular solves for the right-hand side run as one cooperative kernel
 // per triangle: the diagonal block of each step is solved by CTA 0 while all
 // CTAs then apply it to the remaining rows (coalesced GEMV), one grid barrier
@@ -528,29 +528,43 @@ __global__ void __launch_bounds__(kPanelThreads) lu_panel_cluster_kernel(PanelAr
 //
 // The cluster form above pays about six CTA barriers and one cluster barrier
 // per column (2.5 us, 4.2 us for FP64 at 6000 rows, where 64-wide panels also
-// hold the FP64 pipe).  Here a panel is 32 columns wide and a thread keeps one
-// row of it in registers, so a column costs one CTA barrier (the warps' pivot
-// candidates) and one cluster barrier (the CTAs' candidates, each pushed with
-// its row into every CTA's shared memory by the warp that holds it):
-//   - rows never move.  Each thread tracks the position its row has under
+// hold the FP64 pipe).  Here a panel is 32 columns wide and each row lives in the
+// registers of TPR threads, so a column costs one CTA barrier (the warps' pivot
+// candidates) and one exchange between the CTAs: the warp that holds a CTA's
+// candidate stores its row into every CTA's shared memory, and the stores
+// themselves count on the barrier there that the reader waits for.
+//   - Rows never move.  Each thread tracks the position its row has under
 //     nalgebra's swaps (icamax compares positions, src/base/min_max.rs:221-240;
 //     a pivot's row takes position c, the row that was there the pivot's old
-//     one) and writes its row there at the end;
-//   - the registers shift by one column per step, so the loop over columns
-//     stays rolled; finished multipliers and pivot rows wait in shared memory;
-//   - the cluster then applies the swaps to the outer block's other columns and
+//     one) and writes its row there at the end.
+//   - A warp-wide FP64 FMA holds its quarter of an SM for 64 cycles, whatever the
+//     lanes in use, and the chain through a column is all there is to hide it
+//     under.  So a row's columns are dealt to TPR threads (column j to thread j mod
+//     TPR) as long as the CTA has threads left, and a pivot's update of the columns
+//     beyond the next one is put off until the next column's candidates are under
+//     way.  The candidate's own row is brought up to date first, a lane per column.
+//   - The registers shift as columns finish, so the loop over columns stays
+//     rolled; finished multipliers and pivot rows wait in shared memory.
+//   - The cluster then applies the swaps to the outer block's other columns and
 //     solves their 32 rows of U, a warp per column.
 // Panels of 128 columns are made of four of these, each followed by the 32-deep
-// update of the block's remaining columns.
+// update of the block's remaining columns.  Cycles a column, FP64, before (a
+// cluster barrier, one thread a row, the whole update at once) and now: n = 1000
+// 4870 and 2770 (search 580, send 250, deferred update 700, wait 260, select 530,
+// next column 450); n = 8192 6400 and 6300, of them 4250 the update: there the 16
+// SMs' FP64 pipes bound it.
 // ---------------------------------------------------------------------------
 constexpr int kRegThreads = 512;
 constexpr int kRegNb = 32;
 constexpr int kRegMaxRows = kRegThreads * kClusterMaxCtas;  // 8192
+constexpr int kRegInfoTimeout = -1000;                      // info when a wait ran out
+constexpr int kRegPollLimit = 1 << 20;
 
 struct alignas(16) RegMeta {
   unsigned long long key;  // |pivot candidate|'s bit image
-  double rcp;              // its reciprocal
-  int pos, pad[3];
+  int pos, pad;
+  double rcp;  // its reciprocal (of the panel's type)
+  double pad2;
 };
 template <typename T>
 struct RegPanelArgs {
@@ -564,43 +578,119 @@ struct RegPanelArgs {
   int32_t* info;
   PanelPub<T>* pub;
 };
+// Three slots: a CTA's stores for column j + 1 may arrive while this one still
+// reads column j - 1's pivot row, but not those for j + 2 (they follow this CTA's
+// own for j + 1).
 template <typename T>
 struct RegPanelSmem {
-  RegMeta meta[2][kClusterMaxCtas];
-  T slot[2][kClusterMaxCtas][kRegNb];
+  RegMeta meta[3][kClusterMaxCtas];
+  T slot[3][kClusterMaxCtas][kRegNb];
+  T stage[kRegNb];
   T rows[kRegNb][kRegThreads];
   T l11[kRegNb][kRegNb + 1];
+  unsigned long long bar[3];
   unsigned long long wkey[2][kRegThreads / 32];
   int wpos[2][kRegThreads / 32];
   int dst[2 * kRegNb], src[2 * kRegNb];
 };
 
+// |x| from its bit image, and a reciprocal of |x| given x's sign
 template <typename T>
+__device__ __forceinline__ T from_bits(unsigned long long key) {
+  if constexpr (sizeof(T) == 8) return __longlong_as_double((long long)key);
+  else return __uint_as_float((unsigned)key);
+}
+__device__ __forceinline__ double with_sign(double r, double x) {
+  return __hiloint2double(__double2hiint(r) ^ (__double2hiint(x) & 0x80000000), __double2loint(r));
+}
+__device__ __forceinline__ float with_sign(float r, float x) {
+  return __uint_as_float(__float_as_uint(r) ^ (__float_as_uint(x) & 0x80000000u));
+}
+// warp_argmax, cut short where one lane alone holds the largest leading word
+template <typename T>
+__device__ __forceinline__ void panel_argmax(uint64_t& key, int& idx) {
+  const unsigned lead = sizeof(T) == 8 ? (unsigned)(key >> 32) : (unsigned)key;
+  const unsigned m = __reduce_max_sync(0xffffffffu, lead);
+  const unsigned who = __ballot_sync(0xffffffffu, lead == m);
+  if (__popc(who) == 1) {
+    const int from = __ffs(who) - 1;
+    key = __shfl_sync(0xffffffffu, key, from);
+    idx = __shfl_sync(0xffffffffu, idx, from);
+  } else {
+    warp_argmax(key, idx);
+  }
+}
+__device__ __forceinline__ unsigned cluster_addr(const void* p, int rank) {
+  unsigned a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void store_async(unsigned dst, float4 v, unsigned bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
+               "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w)),
+               "r"(bar)
+               : "memory");
+}
+// false when the limit is reached
+__device__ __forceinline__ bool bar_wait(const void* bar, unsigned parity, int limit) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(bar);
+  for (int it = 0; it < limit; ++it) {
+    unsigned ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(a), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
+template <typename T, int TPR>
 __global__ void __launch_bounds__(kRegThreads, 1) lu_panel_reg_kernel(RegPanelArgs<T> g) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RegPanelSmem<T>& sm = *reinterpret_cast<RegPanelSmem<T>*>(smem_raw);
-  constexpr int kWarps = kRegThreads / 32;
+  constexpr int kWarps = kRegThreads / 32, kPer = kRegNb / TPR;
+  constexpr int kV = 16 / (int)sizeof(T), kVecs = kRegNb / kV;
   cg::cluster_group cl = cg::this_cluster();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int G = (int)cl.num_blocks(), b = (int)cl.block_rank();
   const int rb = g.j0 + b * g.chunk;
   const int nr = max(0, min(g.n - rb, g.chunk));
-  const bool valid = tid < nr;
-  const int row = rb + tid;
+  const int rl = tid / TPR, sub = tid % TPR;  // the row's place in the CTA, and which of its threads
+  const bool valid = rl < nr;
+  const int row = rb + rl;
   int pos = row;
   bool done = !valid;
-  T x[kRegNb];
+  T x[kPer];  // columns j + ((sub - j) mod TPR) + TPR k at step j
 #pragma unroll
-  for (int k = 0; k < kRegNb; ++k) x[k] = (valid && k < g.nb) ? g.A[(size_t)(g.j0 + k) * g.lda + row] : T(0);
+  for (int k = 0; k < kPer; ++k)
+    x[k] = (valid && sub + TPR * k < g.nb) ? g.A[(size_t)(g.j0 + sub + TPR * k) * g.lda + row] : T(0);
   int* const npairs = &g.pub->nlist[g.list];
   int *const pdst = g.pub->pdst + 2 * kRegNb * g.list, *const psrc = g.pub->psrc + 2 * kRegNb * g.list;
   if (b == 0 && tid == 0) *npairs = 0;
-  cl.sync();  // every CTA of the cluster runs before anything is pushed to it
-  for (int j = 0; j < g.nb; ++j) {
+  if (tid == 0) {
+    for (int q = 0; q < 3; ++q)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(&sm.bar[q])));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  cl.sync();  // every CTA of the cluster runs, its barriers ready, before anything is stored to it
+  int w = 0;          // the CTA that held the last pivot
+  bool pend = false;  // column j - 1's update of columns j + 1.. is still to come
+  T lp = T(0);        // with this row's multiplier
+  bool late = false;  // a wait ran out: an error, and nothing more is written
+  for (int j = 0, now = 0, last = 2, phase = 0; j < g.nb; ++j) {
     const int c = g.j0 + j, par = j & 1, left = g.nb - j;
-    uint64_t key = done ? 0ull : pivot_key(x[0], pos == c);
-    int idx = done ? 0x7fffffff : pos;
-    warp_argmax(key, idx);
+    const int s0 = j % TPR, d = (sub - s0) & (TPR - 1);  // x[k] is column j + d + TPR k
+    if (tid == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(&sm.bar[now])),
+                   "r"(G * ((left + kV - 1) / kV * 16 + (int)sizeof(RegMeta)))
+                   : "memory");
+    uint64_t key = done || d != 0 ? 0ull : pivot_key(x[0], pos == c);
+    int idx = done || d != 0 ? 0x7fffffff : pos;
+    panel_argmax<T>(key, idx);
     if (lane == 0) {
       sm.wkey[par][warp] = key;
       sm.wpos[par][warp] = idx;
@@ -608,79 +698,104 @@ __global__ void __launch_bounds__(kRegThreads, 1) lu_panel_reg_kernel(RegPanelAr
     __syncthreads();
     key = lane < kWarps ? sm.wkey[par][lane] : 0ull;
     idx = lane < kWarps ? sm.wpos[par][lane] : 0x7fffffff;
+    const int wp = idx;
     warp_argmax(key, idx);
-    // the warp that holds this CTA's candidate pushes it (warp 0 where there is none)
-    const bool cand = !done && pos == idx;
-    if (__any_sync(0xffffffffu, cand) || (idx == 0x7fffffff && warp == 0)) {
-      RegMeta* m = &sm.meta[par][b];
-      T* mine = sm.slot[par][b];
+    const bool none = idx == 0x7fffffff;
+    const int holder = none ? 0 : __ffs(__ballot_sync(0xffffffffu, wp == idx)) - 1;
+    const T* const up = sm.slot[last][w];
+    // the warp that holds this CTA's candidate sends its row, brought up to date
+    // a lane per column; another warp takes the reciprocal and sends the rest
+    if (warp == holder) {
+      const bool cand = !done && pos == idx;
       if (cand) {
 #pragma unroll
-        for (int k = 0; k < kRegNb; ++k)
-          if (k < left) mine[k] = x[k];
-        m->rcp = (double)pivot_rcp(x[0]);
+        for (int k = 0; k < kPer; ++k) sm.stage[(d + TPR * k) & (kRegNb - 1)] = x[k];
       }
-      if (lane == 0) {
-        m->key = key;
-        m->pos = idx == 0x7fffffff ? -1 : idx;
-      }
+      const unsigned who = __ballot_sync(0xffffffffu, cand);
+      const T l = __shfl_sync(0xffffffffu, lp, who ? __ffs(who) - 1 : 0);
       __syncwarp();
-      constexpr int kV = 16 / (int)sizeof(T);
-      const int nv = (left + kV - 1) / kV, per = nv + 2;  // row vectors, then the meta's two
-      for (int e = lane; e < G * per; e += 32) {
-        const int q = e / per, v = e - q * per;
-        if (q == b) continue;
-        const float4* from = v < nv ? reinterpret_cast<const float4*>(mine) + v : reinterpret_cast<const float4*>(m) + (v - nv);
-        float4* to = v < nv ? reinterpret_cast<float4*>(cl.map_shared_rank(mine, q)) + v
-                            : reinterpret_cast<float4*>(cl.map_shared_rank(m, q)) + (v - nv);
-        *to = *from;
-      }
+      if (pend && lane > 0 && lane < left) sm.stage[lane] = axpy1<false>(sm.stage[lane], -up[lane + 1], l);
+      __syncwarp();
+      const int v = lane % kVecs;
+      const float4 val = reinterpret_cast<const float4*>(sm.stage)[v];
+      if (v * kV < left)
+        for (int q = lane / kVecs; q < G; q += 32 / kVecs)
+          store_async(cluster_addr(&sm.slot[now][b][v * kV], q), val, cluster_addr(&sm.bar[now], q));
+    } else if (warp == (holder ^ 1)) {
+      union {
+        RegMeta m;
+        float4 f[2];
+      } u;
+      u.m.key = key;
+      u.m.pos = none ? -1 : idx;
+      *reinterpret_cast<T*>(&u.m.rcp) = pivot_rcp(from_bits<T>(key));
+      if ((lane >> 1) < G)
+        store_async(cluster_addr(reinterpret_cast<const float4*>(&sm.meta[now][b]) + (lane & 1), lane >> 1),
+                    lane & 1 ? u.f[1] : u.f[0], cluster_addr(&sm.bar[now], lane >> 1));
     }
-    cluster_arrive_release();
-    cluster_wait_acquire();
+    // on the way meanwhile: the rest of column j - 1's update
+    if (pend && !done) {
+#pragma unroll
+      for (int k = 0; k < kPer; ++k)
+        if (TPR * k < left && (TPR > 1 || (k > 0 && k + 1 < kPer))) {  // past the panel's end the values are never used
+          if (TPR == 1 || k > 0 || d > 0) x[k] = axpy1<false>(x[k], -up[(d + TPR * k + 1) & (kRegNb - 1)], lp);
+        }
+    }
+    if (!late) late = !bar_wait(&sm.bar[now], phase, kRegPollLimit);
     // the pivot, the same in every warp
-    int w = 0;
     {
-      const RegMeta* m = &sm.meta[par][lane < G ? lane : 0];
-      const int p = lane < G ? m->pos : -1;
+      const RegMeta* m = &sm.meta[now][lane < G ? lane : 0];
+      const int p = lane < G && m->pos >= c && m->pos < g.n ? m->pos : -1;
       key = p >= 0 ? m->key : 0ull;
       idx = p >= 0 ? p : 0x7fffffff;
-      warp_argmax(key, idx);
-      const unsigned holder = __ballot_sync(0xffffffffu, p >= 0 && p == idx);
-      w = holder ? __ffs(holder) - 1 : 0;
+      panel_argmax<T>(key, idx);
+      const unsigned from = __ballot_sync(0xffffffffu, p >= 0 && p == idx);
+      w = from ? __ffs(from) - 1 : 0;
     }
     const bool zero = idx == 0x7fffffff || key == 0;  // all |x| == 0: skipped, lu.rs:107-110
     if (b == 0 && tid == 0) {
       g.ipiv[c] = zero ? c : idx;
       if (zero) atomicMin(g.info, c + 1);
     }
-    if (!done) {
-      if (pos == (zero ? c : idx)) {  // this row is row c of U
+    if (!__all_sync(0xffffffffu, done)) {
+      const T* u = sm.slot[now][w];
+      const bool mine = !done && pos == (zero ? c : idx);  // this row is row c of U
+      if (mine) {
         done = true;
         pos = c;
 #pragma unroll
-        for (int k = 0; k < kRegNb; ++k)
-          if (k < left) sm.rows[j + k][tid] = x[k];
-      } else {
+        for (int k = 0; k < kPer; ++k)
+          if (d + TPR * k < left) sm.rows[j + d + TPR * k][rl] = x[k];
+      }
+      T l = x[0];
+      if (!zero) l *= with_sign(*reinterpret_cast<const T*>(&sm.meta[now][w].rcp), u[0]);
+      if (TPR > 1) l = __shfl_sync(0xffffffffu, l, (lane & ~(TPR - 1)) | s0);
+      lp = l;
+      if (!done) {
         if (!zero && pos == c) pos = idx;
-        const T l = zero ? x[0] : x[0] * (T)sm.meta[par][w].rcp;
-        sm.rows[j][tid] = l;
-        const T* u = sm.slot[par][w];
+        if (d == 0) {
+          sm.rows[j][rl] = l;
 #pragma unroll
-        for (int k0 = 0; k0 < kRegNb; k0 += 4)
-          if (k0 < left - 1)  // uniform; past the panel's end the values are never used
-#pragma unroll
-            for (int k = k0; k < k0 + 4; ++k)
-              if (k + 1 < kRegNb) x[k] = zero ? x[k + 1] : axpy1<false>(x[k + 1], -u[k + 1], l);
+          for (int k = 0; k + 1 < kPer; ++k) x[k] = x[k + 1];
+        }
+        if (!zero && d == (TPR > 1 ? 1 : 0)) x[0] = axpy1<false>(x[0], -u[1], l);
       }
     }
+    pend = !zero;
+    last = now;
+    now = now == 2 ? 0 : now + 1;
+    if (now == 0) phase ^= 1;
   }
-  if (valid) {
-    for (int k = 0; k < g.nb; ++k) g.A[(size_t)(g.j0 + k) * g.lda + pos] = sm.rows[k][tid];
-    if (pos != row) {
+  if (late) atomicMin(g.info, kRegInfoTimeout);
+  __syncwarp();
+  if (valid && !late) {
+    for (int k = sub; k < g.nb; k += TPR) g.A[(size_t)(g.j0 + k) * g.lda + pos] = sm.rows[k][rl];
+    if (pos != row && sub == 0) {
       const int q = atomicAdd(npairs, 1);
-      pdst[q] = pos;
-      psrc[q] = row;
+      if (q < 2 * kRegNb) {
+        pdst[q] = pos;
+        psrc[q] = row;
+      }
     }
   }
   __threadfence();
@@ -746,16 +861,20 @@ __global__ void __launch_bounds__(256) lu_inner_update_kernel(int n, float* __re
 }
 
 // The same in FP64 by digit slices (slices.cuh): rows j0 + nb .. r_hi - 1 times
-// columns c_lo .. c_hi - 1, 64 x 96 of them per CTA, the 32 products of an
+// columns c_lo .. c_hi - 1, 64 x 32 of them per CTA, the 32 products of an
 // output in one exact sum.  L's columns are scaled by the exponents of their
 // pivots and U's rows by the reverse: L D has the scale of its rows' entries of
 // A in every column and D^-1 U is near one, so rows of very different scale keep
 // their precision, as they do in the FP64 loop.
-constexpr int kInnerRows = 64, kInnerCols = 96;
+// It sits between two panels, so its own latency counts and little else: four
+// threads cut a row, a warp has one 16 x 8 tile, its 4 elements loaded first.  With
+// 128 threads on 64 x 96 it took 17 us (3500 instructions in a row) at 1900 rows;
+// the factorization at n = 2000 7.1 ms, so 6.1.
+constexpr int kInnerRows = 64, kInnerCols = 32, kInnerThreads = 512;
 constexpr int kInnerSlots = kInnerRows + kInnerCols;
 constexpr size_t kInnerSmem = (size_t)2 * kSlices * kInnerSlots * kSliceRow + kInnerSlots * 4;
-__global__ void __launch_bounds__(128) lu_inner_update_kernel(int r_hi, double* __restrict__ A, int64_t lda, int j0, int nb,
-                                                              int c_lo, int c_hi) {
+__global__ void __launch_bounds__(kInnerThreads) lu_inner_update_kernel(int r_hi, double* __restrict__ A, int64_t lda, int j0,
+                                                                        int nb, int c_lo, int c_hi) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int sb = kInnerSlots * kSliceRow;
   unsigned char* SL = smem_raw;  // [half][slice][slot]
@@ -763,58 +882,66 @@ __global__ void __launch_bounds__(128) lu_inner_update_kernel(int r_hi, double* 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int r0 = j0 + nb + blockIdx.x * kInnerRows, cb = c_lo + blockIdx.y * kInnerCols;
   const int w = min(kInnerCols, c_hi - cb);
-  __shared__ int pe[kRegNb];  // the pivots' exponents
-  if (tid < kRegNb) pe[tid] = tid < nb ? plain_exponent(A[(size_t)(j0 + tid) * (lda + 1)]) : 0;
-  __syncthreads();
-  for (int s = tid; s < kInnerRows + ((w + 7) & ~7); s += 128) {
+  const int rt = (warp & 3) * 16, c = (warp >> 2) * 8;  // this warp's tile
+  double* p[4];
+  double v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = r0 + rt + g + (i >> 1) * 8, cc = c + 2 * t + (i & 1);
+    p[i] = r < r_hi && cc < w ? A + (size_t)(cb + cc) * lda + r : nullptr;
+    v[i] = p[i] ? *p[i] : 0.0;
+  }
+  constexpr int kPart = kRegNb / 4;  // a thread's elements of its slot
+  if (tid < 4 * kInnerSlots) {
+    const int s = tid >> 2, k0 = (tid & 3) * kPart;
     const bool lrow = s < kInnerRows;
-    const int r = r0 + s, c = s - kInnerRows;
-    const bool on = lrow ? r < r_hi : c < w;
-    const double* p = lrow ? A + (size_t)j0 * lda + r : A + (size_t)(cb + c) * lda + j0;
+    const int r = r0 + s, cc = s - kInnerRows;
+    const bool on = lrow ? r < r_hi : cc < w;
+    const double* src = lrow ? A + (size_t)j0 * lda + r : A + (size_t)(cb + cc) * lda + j0;
     const int64_t st = lrow ? lda : 1;
-    double v[kRegNb];
+    double x[kPart], d[kPart];
+#pragma unroll
+    for (int k = 0; k < kPart; ++k) {
+      const bool in = on && k0 + k < nb;
+      x[k] = in ? src[(k0 + k) * st] : 0.0;
+      d[k] = in ? A[(size_t)(j0 + k0 + k) * (lda + 1)] : 1.0;  // the pivot
+    }
     int em = 1;
 #pragma unroll
-    for (int k = 0; k < kRegNb; ++k) {
-      v[k] = on && k < nb ? shift_exp(p[k * st], lrow ? pe[k] : -pe[k]) : 0.0;
-      em = max(em, slice_exponent(v[k]));
+    for (int k = 0; k < kPart; ++k) {
+      const int pe = k0 + k < nb ? plain_exponent(d[k]) : 0;
+      x[k] = shift_exp(x[k], lrow ? pe : -pe);
+      em = max(em, slice_exponent(x[k]));
     }
+    em = max(em, __shfl_xor_sync(0xffffffffu, em, 1));
+    em = max(em, __shfl_xor_sync(0xffffffffu, em, 2));
 #pragma unroll
-    for (int k = 0; k < kRegNb; k += 4) {
+    for (int k = 0; k < kPart; k += 4) {
       uint32_t w0[kSlices], w1[kSlices];
-      slice_pair(v[k], v[k + 1], em, w0);
-      slice_pair(v[k + 2], v[k + 3], em, w1);
+      slice_pair(x[k], x[k + 1], em, w0);
+      slice_pair(x[k + 2], x[k + 3], em, w1);
+      const int kk = k0 + k;
 #pragma unroll
       for (int q = 0; q < kSlices; ++q)
-        *reinterpret_cast<uint2*>(SL + (size_t)((k >> 4) * kSlices + q) * sb + s * kSliceRow + (k & 15) * 2) =
+        *reinterpret_cast<uint2*>(SL + (size_t)((kk >> 4) * kSlices + q) * sb + s * kSliceRow + (kk & 15) * 2) =
             make_uint2(w0[q], w1[q]);
     }
-    ex[s] = slice_code(em);
+    if (k0 == 0) ex[s] = slice_code(em);
   }
   __syncthreads();
-  const int rt = warp * 16;  // this warp's 16 rows
+  if (c >= w) return;
+  float acc[kSlices][4];
+  slice_sums_start(acc);
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    slice_products_add(SL + (size_t)h * kSlices * sb + rt * kSliceRow,
+                       SL + (size_t)h * kSlices * sb + (kInnerRows + c) * kSliceRow, sb, lane, acc);
   const int e0 = ex[rt + g], e1 = ex[rt + g + 8];
-  for (int c = 0; c < w; c += 8) {
-    double* p[4];
-    double v[4];
+  const int f0 = ex[kInnerRows + c + 2 * t], f1 = ex[kInnerRows + c + 2 * t + 1];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = r0 + rt + g + (i >> 1) * 8, cc = c + 2 * t + (i & 1);
-      p[i] = r < r_hi && cc < w ? A + (size_t)(cb + cc) * lda + r : nullptr;
-      v[i] = p[i] ? *p[i] : 0.0;
-    }
-    float acc[kSlices][4];
-    slice_sums_start(acc);
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-      slice_products_add(SL + (size_t)h * kSlices * sb + rt * kSliceRow,
-                         SL + (size_t)h * kSlices * sb + (kInnerRows + c) * kSliceRow, sb, lane, acc);
-    const int f0 = ex[kInnerRows + c + 2 * t], f1 = ex[kInnerRows + c + 2 * t + 1];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const double x = slice_value<32>(acc, i, (i >> 1 ? e1 : e0) + (i & 1 ? f1 : f0));
-      if (p[i]) *p[i] = v[i] - x;
-    }
+  for (int i = 0; i < 4; ++i) {
+    const double y = slice_value<32>(acc, i, (i >> 1 ? e1 : e0) + (i & 1 ? f1 : f0));
+    if (p[i]) *p[i] = v[i] - y;
   }
 }
 
@@ -1358,6 +1485,15 @@ inline int reg_panel_ctas(int rows) {
   return g;
 }
 
+// The kernel with as many threads to a row as a CTA of `chunk` rows has.
+template <typename T>
+void (*reg_panel_kernel(int chunk))(RegPanelArgs<T>) {
+  if (chunk <= kRegThreads / 8) return lu_panel_reg_kernel<T, 8>;
+  if (chunk <= kRegThreads / 4) return lu_panel_reg_kernel<T, 4>;
+  if (chunk <= kRegThreads / 2) return lu_panel_reg_kernel<T, 2>;
+  return lu_panel_reg_kernel<T, 1>;
+}
+
 // An outer block of jb columns at j0 by panels of kRegNb (swaps and U inside
 // the block included); the panels' swap lists stay in pub.
 template <typename T>
@@ -1379,13 +1515,14 @@ int reg_block(int n, T* A, int64_t lda, int j0, int jb, int32_t* ipiv, int32_t* 
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, lu_panel_reg_kernel<T>, pa);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, reg_panel_kernel<T>(pa.chunk), pa);
     if (e != cudaSuccess) return record_cuda_error(e, name);
     const int below = rows - nb;
     if (p0 + nb < j0 + jb && below > 0) {
       if constexpr (sizeof(T) == 8)
-        lu_inner_update_kernel<<<(below + kInnerRows - 1) / kInnerRows, 128, kInnerSmem, s>>>(n, A, lda, p0, nb, p0 + nb,
-                                                                                              j0 + jb);
+        lu_inner_update_kernel<<<dim3((below + kInnerRows - 1) / kInnerRows,
+                                      (j0 + jb - p0 - nb + kInnerCols - 1) / kInnerCols),
+                                 kInnerThreads, kInnerSmem, s>>>(n, A, lda, p0, nb, p0 + nb, j0 + jb);
       else
         lu_inner_update_kernel<<<(below + 63) / 64, 256, 0, s>>>(n, A, lda, p0, nb, j0 + jb);
     }
@@ -1400,22 +1537,25 @@ bool reg_panels(int n) {
   static int ok = -1;
   if (ok < 0) {
     ok = 0;
-    auto kern = lu_panel_reg_kernel<T>;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kClusterMaxCtas);
-    cfg.blockDim = dim3(kRegThreads);
-    cfg.dynamicSmemBytes = sizeof(RegPanelSmem<T>);
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = kClusterMaxCtas;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int nclusters = 0;
-    bool good = ensure_dynamic_smem(kern, sizeof(RegPanelSmem<T>)) == cudaSuccess &&
-                cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg) == cudaSuccess && nclusters >= 1;
+    bool good = true;
+    for (int chunk = kRegThreads; chunk >= kRegThreads / 8 && good; chunk /= 2) {
+      const auto kern = reg_panel_kernel<T>(chunk);
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(kClusterMaxCtas);
+      cfg.blockDim = dim3(kRegThreads);
+      cfg.dynamicSmemBytes = sizeof(RegPanelSmem<T>);
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = kClusterMaxCtas;
+      at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      int nclusters = 0;
+      good = ensure_dynamic_smem(kern, sizeof(RegPanelSmem<T>)) == cudaSuccess &&
+             cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+             cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg) == cudaSuccess && nclusters >= 1;
+    }
     if constexpr (sizeof(T) == 8) {
       void (*upd)(int, double*, int64_t, int, int, int, int) = lu_inner_update_kernel;
       good = good && ensure_dynamic_smem(upd, kInnerSmem) == cudaSuccess;
@@ -1437,7 +1577,7 @@ cudaError_t trsm_by_pieces(int n, double* A, int64_t lda, int j0, int jb, cudaSt
     lu_trsm_piece_kernel<<<(rest + 7) / 8, 256, 0, s>>>(n, A, lda, p0, nb, c0);
     const int below = c0 - p0 - nb;
     if (below > 0)
-      lu_inner_update_kernel<<<dim3((below + kInnerRows - 1) / kInnerRows, (rest + kInnerCols - 1) / kInnerCols), 128,
+      lu_inner_update_kernel<<<dim3((below + kInnerRows - 1) / kInnerRows, (rest + kInnerCols - 1) / kInnerCols), kInnerThreads,
                                kInnerSmem, s>>>(c0, A, lda, p0, nb, c0, n);
   }
   return cudaGetLastError();
