@@ -16,11 +16,11 @@
 // Orders up to 8192 take 128 columns per block, panels in registers and 32-deep
 // updates inside the block; above, a block is one panel of 64 (FP64) or 128.
 // Measured, FP64, ms (all on the FP64 pipe -> residue updates with 64-wide panels ->
-// register panels behind a cluster barrier -> as below): n = 8192 328 -> 114 -> 65 -> 63,
-// 4096 50 -> 24.6 -> 20.0 -> 16.8, 2000 11.6 -> 9.4 -> 8.7 -> 6.1, 1000 4.62 -> 4.20 ->
-// 4.08 -> 2.75.  FP32 factor with refinement, n = 4096: 15.8 -> 15.8 -> 14.2 -> 12.6.
-// The chain of panels and inner updates bounds it: at n = 8192 50 ms of the 63 are
-// left when the trailing update beyond the next panel costs nothing.
+// register panels behind a cluster barrier -> as below): n = 8192 328 -> 114 -> 65 -> 62,
+// 4096 50 -> 24.6 -> 20.0 -> 16.0, 2000 11.6 -> 9.4 -> 8.7 -> 5.7, 1000 4.62 -> 4.20 ->
+// 4.08 -> 2.55.  FP32 factor with refinement, n = 4096: 15.8 -> 15.8 -> 14.2 -> 10.2.
+// The chain of panels and inner updates bounds it: at n = 8192 50 ms were left of 67
+// when the trailing update beyond the next panel cost nothing.
 // The triangular solves for the right-hand side run as one cooperative kernel
 // per triangle: the diagonal block of each step is solved by CTA 0 while all
 // CTAs then apply it to the remaining rows (coalesced GEMV), one grid barrier
@@ -647,6 +647,28 @@ __device__ __forceinline__ bool bar_wait(const void* bar, unsigned parity, int l
   return false;
 }
 
+// The chain of small kernels between two trailing updates is launched ahead of its
+// predecessors' ends (programmatic stream serialization): each waits for the one
+// before it as its first act, and tells the next to come in: the panel only in its
+// tail, so that nothing idle holds the SMs which the trailing update runs on.
+// n = 1000 2.75 -> 2.55 ms, 4096 16.8 -> 16.0; FP32 with refinement, 4096 10.6 -> 10.2.
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_successor_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... Q>
+cudaError_t launch_chained(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, Q... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 template <typename T, int TPR>
 __global__ void __launch_bounds__(kRegThreads, 1) lu_panel_reg_kernel(RegPanelArgs<T> g) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -663,6 +685,7 @@ __global__ void __launch_bounds__(kRegThreads, 1) lu_panel_reg_kernel(RegPanelAr
   const int row = rb + rl;
   int pos = row;
   bool done = !valid;
+  wait_for_predecessor();
   T x[kPer];  // columns j + ((sub - j) mod TPR) + TPR k at step j
 #pragma unroll
   for (int k = 0; k < kPer; ++k)
@@ -699,7 +722,7 @@ __global__ void __launch_bounds__(kRegThreads, 1) lu_panel_reg_kernel(RegPanelAr
     key = lane < kWarps ? sm.wkey[par][lane] : 0ull;
     idx = lane < kWarps ? sm.wpos[par][lane] : 0x7fffffff;
     const int wp = idx;
-    warp_argmax(key, idx);
+    panel_argmax<T>(key, idx);
     const bool none = idx == 0x7fffffff;
     const int holder = none ? 0 : __ffs(__ballot_sync(0xffffffffu, wp == idx)) - 1;
     const T* const up = sm.slot[last][w];
@@ -786,6 +809,7 @@ __global__ void __launch_bounds__(kRegThreads, 1) lu_panel_reg_kernel(RegPanelAr
     now = now == 2 ? 0 : now + 1;
     if (now == 0) phase ^= 1;
   }
+  let_successor_in();
   if (late) atomicMin(g.info, kRegInfoTimeout);
   __syncwarp();
   if (valid && !late) {
@@ -840,6 +864,8 @@ __global__ void __launch_bounds__(kRegThreads, 1) lu_panel_reg_kernel(RegPanelAr
 __global__ void __launch_bounds__(256) lu_inner_update_kernel(int n, float* __restrict__ A, int64_t lda, int j0, int nb,
                                                               int c_hi) {
   __shared__ __align__(16) float U[96][kRegNb];
+  wait_for_predecessor();
+  let_successor_in();
   const int j1 = j0 + nb, w = c_hi - j1;
   for (int e = threadIdx.x; e < w * kRegNb; e += 256) {
     const int c = e >> 5, k = e & 31;
@@ -883,6 +909,8 @@ __global__ void __launch_bounds__(kInnerThreads) lu_inner_update_kernel(int r_hi
   const int r0 = j0 + nb + blockIdx.x * kInnerRows, cb = c_lo + blockIdx.y * kInnerCols;
   const int w = min(kInnerCols, c_hi - cb);
   const int rt = (warp & 3) * 16, c = (warp >> 2) * 8;  // this warp's tile
+  wait_for_predecessor();
+  let_successor_in();
   double* p[4];
   double v[4];
 #pragma unroll
@@ -1066,6 +1094,8 @@ __global__ void __launch_bounds__(256) lu_trsm_kernel(int n, T* A, int64_t lda, 
 __global__ void __launch_bounds__(256) lu_trsm_piece_kernel(int n, double* __restrict__ A, int64_t lda, int p0, int nb,
                                                             int c0) {
   __shared__ double L[32][33];
+  wait_for_predecessor();
+  let_successor_in();
   for (int e = threadIdx.x; e < nb * nb; e += 256) {
     const int k = e / nb, i = e - k * nb;
     L[k][i] = A[(size_t)(p0 + k) * lda + p0 + i];
@@ -1121,7 +1151,8 @@ cudaError_t launch_trsm_tiled(int n, T* A, int64_t lda, int j0, int rest, cudaSt
 template <typename T>
 cudaError_t launch_trsm(int n, T* A, int64_t lda, int j0, int jb, int rest, cudaStream_t s) {
   if (jb == 64) return launch_trsm_tiled<T, 64>(n, A, lda, j0, rest, s);
-  if (jb == 128) return launch_trsm_tiled<T, 128>(n, A, lda, j0, rest, s);
+  if constexpr (sizeof(T) == 4)  // FP64 blocks of 128 go by pieces
+    if (jb == 128) return launch_trsm_tiled<T, 128>(n, A, lda, j0, rest, s);
   const size_t smem = (size_t)jb * jb * sizeof(T) + (size_t)jb * 64 * sizeof(T);
   if (smem > 48 * 1024) {
     cudaError_t e = ensure_dynamic_smem(lu_trsm_generic_kernel<T>, smem);
@@ -1485,6 +1516,9 @@ inline int reg_panel_ctas(int rows) {
   return g;
 }
 
+using InnerUpdate32 = void (*)(int, float*, int64_t, int, int, int);
+using InnerUpdate64 = void (*)(int, double*, int64_t, int, int, int, int);
+
 // The kernel with as many threads to a row as a CTA of `chunk` rows has.
 template <typename T>
 void (*reg_panel_kernel(int chunk))(RegPanelArgs<T>) {
@@ -1508,23 +1542,27 @@ int reg_block(int n, T* A, int64_t lda, int j0, int jb, int32_t* ipiv, int32_t* 
     cfg.blockDim = dim3(kRegThreads);
     cfg.dynamicSmemBytes = sizeof(RegPanelSmem<T>);
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = G;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     cudaError_t e = cudaLaunchKernelEx(&cfg, reg_panel_kernel<T>(pa.chunk), pa);
     if (e != cudaSuccess) return record_cuda_error(e, name);
     const int below = rows - nb;
     if (p0 + nb < j0 + jb && below > 0) {
       if constexpr (sizeof(T) == 8)
-        lu_inner_update_kernel<<<dim3((below + kInnerRows - 1) / kInnerRows,
-                                      (j0 + jb - p0 - nb + kInnerCols - 1) / kInnerCols),
-                                 kInnerThreads, kInnerSmem, s>>>(n, A, lda, p0, nb, p0 + nb, j0 + jb);
+        e = launch_chained(static_cast<InnerUpdate64>(lu_inner_update_kernel),
+                           dim3((below + kInnerRows - 1) / kInnerRows, (j0 + jb - p0 - nb + kInnerCols - 1) / kInnerCols),
+                           kInnerThreads, kInnerSmem, s, n, A, lda, p0, nb, p0 + nb, j0 + jb);
       else
-        lu_inner_update_kernel<<<(below + 63) / 64, 256, 0, s>>>(n, A, lda, p0, nb, j0 + jb);
+        e = launch_chained(static_cast<InnerUpdate32>(lu_inner_update_kernel), dim3((below + 63) / 64), 256, 0, s, n, A, lda,
+                           p0, nb, j0 + jb);
+      if (e != cudaSuccess) return record_cuda_error(e, name);
     }
   }
   return check_launch(name);
@@ -1557,8 +1595,7 @@ bool reg_panels(int n) {
              cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg) == cudaSuccess && nclusters >= 1;
     }
     if constexpr (sizeof(T) == 8) {
-      void (*upd)(int, double*, int64_t, int, int, int, int) = lu_inner_update_kernel;
-      good = good && ensure_dynamic_smem(upd, kInnerSmem) == cudaSuccess;
+      good = good && ensure_dynamic_smem(static_cast<InnerUpdate64>(lu_inner_update_kernel), kInnerSmem) == cudaSuccess;
     }
     if (!good) cudaGetLastError();
     ok = good ? 1 : 0;
@@ -1574,13 +1611,15 @@ cudaError_t trsm_by_pieces(int n, double* A, int64_t lda, int j0, int jb, cudaSt
   const int c0 = j0 + jb, rest = n - c0;
   for (int p0 = j0; p0 < c0; p0 += kRegNb) {
     const int nb = std::min(kRegNb, c0 - p0);
-    lu_trsm_piece_kernel<<<(rest + 7) / 8, 256, 0, s>>>(n, A, lda, p0, nb, c0);
+    cudaError_t e = launch_chained(lu_trsm_piece_kernel, dim3((rest + 7) / 8), 256, 0, s, n, A, lda, p0, nb, c0);
     const int below = c0 - p0 - nb;
-    if (below > 0)
-      lu_inner_update_kernel<<<dim3((below + kInnerRows - 1) / kInnerRows, (rest + kInnerCols - 1) / kInnerCols), kInnerThreads,
-                               kInnerSmem, s>>>(c0, A, lda, p0, nb, c0, n);
+    if (e == cudaSuccess && below > 0)
+      e = launch_chained(static_cast<InnerUpdate64>(lu_inner_update_kernel),
+                         dim3((below + kInnerRows - 1) / kInnerRows, (rest + kInnerCols - 1) / kInnerCols), kInnerThreads,
+                         kInnerSmem, s, c0, A, lda, p0, nb, c0, n);
+    if (e != cudaSuccess) return e;
   }
-  return cudaGetLastError();
+  return cudaSuccess;
 }
 
 // Blocked LU with look-ahead: step k's panel chain (panel, row swaps, TRSM,
@@ -1617,35 +1656,35 @@ int getrf_blocked(int n, T* A, int64_t lda, int32_t* ipiv, int32_t* info, void* 
       rc = reg_block<T>(n, A, lda, j0, jb, ipiv, info, pa.pub, sp, name);
       if (rc != NACU_SUCCESS) return rc;
     } else {
-    const int cchunk = cluster ? (rows + cluster - 1) / cluster : 0;
-    const size_t csmem = cluster_pub_bytes<T>(jb) + (size_t)(cchunk | 1) * jb * sizeof(T);
-    if (cluster && csmem <= kPanelMaxSmem) {
-      pa.chunk = cchunk;
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(cluster);
-      cfg.blockDim = dim3(kPanelThreads);
-      cfg.dynamicSmemBytes = csmem;
-      cfg.stream = sp;
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = cluster;
-      at[0].val.clusterDim.y = 1;
-      at[0].val.clusterDim.z = 1;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      e = cudaLaunchKernelEx(&cfg, lu_panel_cluster_kernel<T>, pa);
-      if (e != cudaSuccess) return record_cuda_error(e, name);
-    } else {
-      const int max_rows = (int)(kPanelMaxSmem / ((size_t)jb * sizeof(T))) - 1;  // leading dimension chunk | 1
-      int G = std::max((rows + kPanelRowsPerCta - 1) / kPanelRowsPerCta, (rows + max_rows - 1) / max_rows);
-      G = std::max(1, std::min(G, gmax));
-      const int chunk = (rows + G - 1) / G;
-      if (chunk > max_rows) return record_arg_error(-1, "getrf: n too large for the shared-memory panel");
-      pa.chunk = chunk;
-      void* args[] = {&pa};
-      e = cudaLaunchCooperativeKernel(pk, G, kPanelThreads, args, (size_t)(chunk | 1) * jb * sizeof(T), sp);
-      if (e != cudaSuccess) return record_cuda_error(e, name);
-    }
+      const int cchunk = cluster ? (rows + cluster - 1) / cluster : 0;
+      const size_t csmem = cluster_pub_bytes<T>(jb) + (size_t)(cchunk | 1) * jb * sizeof(T);
+      if (cluster && csmem <= kPanelMaxSmem) {
+        pa.chunk = cchunk;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(cluster);
+        cfg.blockDim = dim3(kPanelThreads);
+        cfg.dynamicSmemBytes = csmem;
+        cfg.stream = sp;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = cluster;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        e = cudaLaunchKernelEx(&cfg, lu_panel_cluster_kernel<T>, pa);
+        if (e != cudaSuccess) return record_cuda_error(e, name);
+      } else {
+        const int max_rows = (int)(kPanelMaxSmem / ((size_t)jb * sizeof(T))) - 1;  // leading dimension chunk | 1
+        int G = std::max((rows + kPanelRowsPerCta - 1) / kPanelRowsPerCta, (rows + max_rows - 1) / max_rows);
+        G = std::max(1, std::min(G, gmax));
+        const int chunk = (rows + G - 1) / G;
+        if (chunk > max_rows) return record_arg_error(-1, "getrf: n too large for the shared-memory panel");
+        pa.chunk = chunk;
+        void* args[] = {&pa};
+        e = cudaLaunchCooperativeKernel(pk, G, kPanelThreads, args, (size_t)(chunk | 1) * jb * sizeof(T), sp);
+        if (e != cudaSuccess) return record_cuda_error(e, name);
+      }
     }
     if (rest_pending) {  // the swaps below touch the columns the previous update is still writing
       e = cudaStreamWaitEvent(sp, la->rest_done, 0);
