@@ -258,6 +258,124 @@ __global__ void __launch_bounds__(kLuThreads) lu_batched_kernel(int n, int nrhs,
   }
 }
 
+// b <- L^-1 b (unit lower) and b <- U^-1 b for one right-hand side by one warp, n <=
+// 128: b in registers (lane + 32 k), a step's value by shuffle.  nalgebra's axpy
+// order (solve.rs:106-133, 155-182: coeff = b_i / U_ii, then the rows above), so
+// the same bits as with b in shared memory, where each step of the forward solve
+// cost a CTA barrier and each of the back substitution two trips through shared
+// memory.
+template <typename T, bool EXACT>
+__device__ __forceinline__ void lu_forward(int n, int ld, const T* sa, T* bcol, int lane) {
+  T b[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) b[k] = lane + 32 * k < n ? bcol[lane + 32 * k] : T(0);
+#pragma unroll
+  for (int kb = 0; kb < 4; ++kb) {
+    const int w = min(32, n - 32 * kb);
+#pragma unroll 2
+    for (int i = 0; i < w; ++i) {
+      const T y = __shfl_sync(0xffffffffu, b[kb], i);
+      const T* lcol = sa + (size_t)(32 * kb + i) * ld;
+#pragma unroll
+      for (int k = kb; k < 4; ++k) {
+        const int r = lane + 32 * k;
+        if (32 * k < n && r < n && (k > kb || lane > i)) b[k] = axpy1<EXACT>(b[k], -y, lcol[r]);
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (lane + 32 * k < n) bcol[lane + 32 * k] = b[k];
+}
+template <typename T, bool EXACT>
+__device__ __forceinline__ void lu_backward(int n, int ld, const T* sa, const T* rcp, T* bcol, int lane) {
+  T b[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) b[k] = lane + 32 * k < n ? bcol[lane + 32 * k] : T(0);
+#pragma unroll
+  for (int kb = 3; kb >= 0; --kb) {
+#pragma unroll 2
+    for (int i = min(32, n - 32 * kb) - 1; i >= 0; --i) {
+      const T* ucol = sa + (size_t)(32 * kb + i) * ld;
+      T q;
+      if constexpr (EXACT) q = b[kb] / ucol[32 * kb + i];
+      else q = b[kb] * rcp[32 * kb + i];
+      const T coeff = __shfl_sync(0xffffffffu, q, i);
+      if (lane == i) b[kb] = coeff;
+#pragma unroll
+      for (int k = 0; k <= kb; ++k)
+        if (k < kb || lane < i) b[k] = axpy1<EXACT>(b[k], -coeff, ucol[lane + 32 * k]);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (lane + 32 * k < n) bcol[lane + 32 * k] = b[k];
+}
+
+// Solve from given factors with one right-hand side: a CTA of 128 threads per
+// system, whose last warp swaps the right-hand side's rows while the others load
+// the factors, and whose first one solves.  One system of order 100: 59 -> 40 us,
+// of 128 84 -> 52; 4096 of order 64 (with the copy of B) 211 -> 155, 16384 of order 8
+// 108 -> 79.  With more right-hand sides the CTA-wide form fills its FP64
+// instructions better (8000 of order 32, two of them: 174 against 202 us).
+constexpr int kLuSolveThreads = 128;
+template <typename T, bool EXACT>
+__global__ void __launch_bounds__(kLuSolveThreads, 8) lu_solve_one_kernel(int n, const T* __restrict__ A, int64_t strideA,
+                                                                           const int32_t* __restrict__ ipiv, T* __restrict__ B,
+                                                                           int64_t strideB, int32_t* __restrict__ info) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int ld = n | 1;
+  T* sa = reinterpret_cast<T*>(smem_raw);
+  T* sb = sa + (size_t)ld * n;
+  T* rcp = sb + ld;
+  int* piv = reinterpret_cast<int*>(rcp + n);
+  __shared__ int s_info;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const T* a = A + (size_t)blockIdx.x * strideA;
+  T* b = B + (size_t)blockIdx.x * strideB;
+  constexpr int loaders = kLuSolveThreads - 32;
+  if (warp == loaders / 32) {
+    for (int i = lane; i < n; i += 32) {
+      piv[i] = ipiv[(size_t)blockIdx.x * n + i];
+      sb[i] = b[i];
+    }
+    __syncwarp();
+    if (lane == 0)
+      for (int i = 0; i < n; ++i) {  // permutation_sequence.rs:97-104, in order
+        const int p = piv[i];
+        if (p != i) {
+          const T t = sb[i];
+          sb[i] = sb[p];
+          sb[p] = t;
+        }
+      }
+  } else {
+    for (int e = tid; e < n * n; e += loaders) {
+      const int c = e / n, r = e - c * n;
+      sa[(size_t)c * ld + r] = a[e];
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {
+    lu_forward<T, EXACT>(n, ld, sa, sb, lane);
+  } else if (warp == 1) {  // LAPACK getrf convention: first zero U_ii, 1-based
+    int inf = 0;
+    for (int i0 = 0; i0 < n && inf == 0; i0 += 32) {
+      const int i = i0 + lane;
+      const unsigned zeros = __ballot_sync(0xffffffffu, i < n && is_zero_bits(sa[(size_t)min(i, n - 1) * (ld + 1)]));
+      if (zeros) inf = i0 + __ffs(zeros);
+    }
+    if (lane == 0) s_info = inf;
+  } else if (!EXACT) {
+    for (int i = tid - 64; i < n; i += kLuSolveThreads - 64) rcp[i] = T(1) / sa[(size_t)i * (ld + 1)];
+  }
+  __syncthreads();
+  if (warp == 0 && s_info == 0) lu_backward<T, EXACT>(n, ld, sa, rcp, sb, lane);
+  __syncthreads();
+  for (int i = tid; i < n; i += kLuSolveThreads) b[i] = sb[i];
+  if (tid == 0 && info) info[blockIdx.x] = s_info;
+}
+
 template <typename T>
 size_t lu_smem_bytes(int n, int nrhs) {
   const int ld = n | 1;
@@ -277,6 +395,15 @@ int lu_launch(int n, int nrhs, T* A, int64_t strideA, int32_t* ipiv, T* B, int64
   if (nrhs > 0 && strideB < (int64_t)n * nrhs) return record_arg_error(-7, "lu batched: strideB < n*nrhs");
   const size_t smem = lu_smem_bytes<T>(n, nrhs);
   const bool exact = (flags & NACU_FLAG_EXACT) != 0;
+  if (mode == 2 && nrhs == 1) {
+    auto one = exact ? lu_solve_one_kernel<T, true> : lu_solve_one_kernel<T, false>;
+    if (smem > 48 * 1024) {
+      cudaError_t e = ensure_dynamic_smem(one, smem);
+      if (e != cudaSuccess) return record_cuda_error(e, name);
+    }
+    one<<<batch, kLuSolveThreads, smem, stream>>>(n, A, strideA, ipiv, B, strideB, info);
+    return check_launch(name);
+  }
   auto kern = exact ? lu_batched_kernel<T, true> : lu_batched_kernel<T, false>;
   if (smem > 48 * 1024) {
     cudaError_t e = ensure_dynamic_smem(kern, smem);
