@@ -500,8 +500,10 @@ int nacu_dposv_ragged_noalloc(int count, int n_max, const int32_t* ns, const int
 
 /* ---- LU of one large matrix (blocked, multi-SM) ---------------------------- */
 
-/* Workspace bytes of nacu_dgetrf and nacu_dgetrs (the panel's pivot exchange
- * area; the triangular solves' block flags). */
+/* Workspace bytes of nacu_dgetrf (the panel's pivot exchange area, the trailing
+ * updates' residues; 341 MB at n = 8192) and nacu_dgetrs (its blocks' flags).
+ * Both calls also take the bytes for n = 0 (the exchange area alone, under
+ * 1 MB); nacu_dgetrf then updates on the FP64 pipe, several times slower at large n. */
 size_t nacu_getrf_workspace_bytes(int n);
 
 /* LU with partial pivoting of one n x n matrix (column-major, lda), in place,

@@ -31,6 +31,8 @@ runs the fused kernel, writing the factors as a side effect.
 """
 from __future__ import annotations
 
+import contextlib
+
 import numpy as np
 
 from . import _device as _dev
@@ -225,7 +227,12 @@ class LU:
         self.info = _i32(2)
         self.large = n > 128
         if self.large:
-            with _work(_lib.load().nacu_getrf_workspace_bytes(n)) as ws:
+            bytes_for = _lib.load().nacu_getrf_workspace_bytes
+            with contextlib.ExitStack() as stack:
+                try:
+                    ws = stack.enter_context(_work(bytes_for(n)))
+                except _lib.NacuError:  # no room for the updates' residues: the FP64 pipe
+                    ws = stack.enter_context(_work(bytes_for(0)))
                 _lib.call("nacu_dgetrf", n, m.data.data_ptr(), n, self.ipiv.data_ptr(), self.info.data_ptr(),
                           ws.data_ptr(), ws.numel(), _stream_ptr())
         else:
@@ -242,7 +249,7 @@ class LU:
                           b.data.data_ptr(), n * b.ncols, info.data_ptr(), 1, self.flags, _stream_ptr())
                 return int(info.item()) == 0
             ok = True
-            with _work(_lib.load().nacu_getrf_workspace_bytes(n)) as ws:
+            with _work(_lib.load().nacu_getrf_workspace_bytes(0)) as ws:
                 for c in range(b.ncols):
                     _lib.call("nacu_dgetrs", n, self.lu.data.data_ptr(), n, self.ipiv.data_ptr(),
                               b.data.data_ptr() + c * n * 8, info.data_ptr(), ws.data_ptr(), ws.numel(),

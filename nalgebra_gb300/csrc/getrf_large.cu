@@ -1995,7 +1995,9 @@ inline size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 MixedLuLayout mixed_lu_layout(int n, int nb) {
   MixedLuLayout L;
   size_t o = 0;
-  L.a32 = o;   o = up256(o + (size_t)n * n * 4);
+  // the FP64 fallback's updates keep their residues where the FP32 factor was
+  const Getrf64Layout F = getrf64_layout(n);
+  L.a32 = o;   o = up256(o + std::max((size_t)n * n * 4, F.bytes[0] + F.bytes[1]));
   L.ipiv = o;  o = up256(o + (size_t)n * 4);
   L.perm = o;  o = up256(o + (size_t)n * 4);
   L.info = o;  o = up256(o + 16);
@@ -2265,7 +2267,9 @@ int nacu_dgesv_mixed_ir(int n, const double* A, int64_t lda, const double* b, do
     // FP64 fallback on a copy of A
     fallback = 1;
     cudaMemcpy2DAsync(A64, (size_t)n * 8, A, (size_t)lda * 8, (size_t)n * 8, n, cudaMemcpyDeviceToDevice, s);
-    rc = getrf_blocked<double>(n, A64, n, ipiv, info, cand, kNb64, update_fp64, nullptr, s, "nacu_dgesv_mixed_ir");
+    const Getrf64Layout F = getrf64_layout(n);
+    Update64Ctx fctx{{base + L.a32, base + L.a32 + F.bytes[0]}, {F.bytes[0], F.bytes[1]}};
+    rc = getrf_blocked<double>(n, A64, n, ipiv, info, cand, kNb64, update_fp64, &fctx, s, "nacu_dgesv_mixed_ir");
     if (rc != NACU_SUCCESS) return rc;
     cudaMemcpyAsync(x, b, (size_t)n * 8, cudaMemcpyDeviceToDevice, s);
     rc = nacu_dgetrs(n, A64, n, ipiv, x, info + 1, cand, getrf_ws_bytes(), stream);
@@ -2296,11 +2300,11 @@ int nacu_dgetrf(int n, double* A, int64_t lda, int32_t* ipiv, int32_t* info, voi
   if (!A) return record_arg_error(-2, "dgetrf: null A");
   if (lda < n) return record_arg_error(-3, "dgetrf: lda < n");
   if (!ipiv || !info) return record_arg_error(-4, "dgetrf: null ipiv or info");
-  if (!workspace || workspace_bytes < nacu_getrf_workspace_bytes(n))
-    return record_arg_error(-6, "dgetrf: workspace too small");
+  if (!workspace || workspace_bytes < getrf_ws_bytes()) return record_arg_error(-6, "dgetrf: workspace too small");
   const Getrf64Layout L = getrf64_layout(n);
   unsigned char* ws = static_cast<unsigned char*>(workspace);
   Update64Ctx ctx{{ws + L.slot[0], ws + L.slot[1]}, {L.bytes[0], L.bytes[1]}};
+  if (workspace_bytes < L.total) ctx.ws[0] = ctx.ws[1] = nullptr;  // the updates on the FP64 pipe
   return getrf_blocked<double>(n, A, lda, ipiv, info, workspace, kNb64, update_fp64, &ctx, (cudaStream_t)stream,
                                "nacu_dgetrf");
 }

@@ -47,6 +47,35 @@ def test_orders_where_a_row_gets_fewer_threads(cuda, n):
     assert np.linalg.norm(d) <= 10.0 * np.linalg.norm(a) * n * 2.0 ** -52
 
 
+def test_least_workspace_updates_on_the_fp64_pipe(cuda, monkeypatch):
+    """Without room for the residues: the same pivots, and the mirror does without
+    them by itself."""
+    import nalgebra_gb300 as ng
+    from nalgebra_gb300 import _lib
+
+    n = 300
+    rng = np.random.default_rng(8)
+    a = rng.standard_normal((n, n))
+    _, ipiv_o, _ = O.lu(a)
+    full = _lib.load().nacu_getrf_workspace_bytes(n)
+    real = ng._work
+    sizes = []
+
+    def scarce(nbytes):
+        sizes.append(nbytes)
+        if nbytes >= full:
+            raise _lib.NacuError("out of memory")
+        return real(nbytes)
+
+    monkeypatch.setattr(ng, "_work", scarce)
+    lu = ng.DeviceMatrix.from_numpy(a).lu()
+    x = lu.solve(ng.DeviceMatrix.from_numpy(np.ones((n, 1)))).to_numpy()
+    assert sizes[0] == full and max(sizes[1:]) < full
+    assert np.array_equal(lu.ipiv.to_numpy()[:n], ipiv_o)
+    assert O.lu_reconstruction(a, lu.lu.to_numpy(), ipiv_o) <= 10.0
+    assert O.backward_error(a, x, np.ones((n, 1))) <= 10 * n * 2.0 ** -52
+
+
 def test_ties_take_the_first_position(cuda):
     """Small integers: equal magnitudes in most columns, resolved by the position
     the rows have after the swaps so far.  The eliminations stay exact while the
