@@ -119,6 +119,27 @@ __device__ __forceinline__ bool is_zero_bits(float x) {
   return (u & 0x7fffffffu) == 0u;
 }
 
+// A launch ahead of its predecessor's end in the stream (programmatic stream
+// serialization).  The kernel waits for the predecessor before it touches memory,
+// and may let its own successor in early; every kernel launched so waits, so one
+// that is let in follows all before it.
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_successor_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... Q>
+cudaError_t launch_chained(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, const Q&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // The bit image is taken through an opaque mov: a plain mask of the
 // reinterpreted bits is recognised as fabs and then costs an FP64 add (an
 // FP64 pipe slot) per key, where the key is taken for every updated element.

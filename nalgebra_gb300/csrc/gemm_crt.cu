@@ -257,8 +257,10 @@ __device__ __forceinline__ uint32_t abs_bits(long long v, bool bad) {
 // Partial row norms of A: thread per row and chunk of columns; part[chunk][row].
 __global__ void __launch_bounds__(128) crt_row_stats_kernel(int m, int k, const double* __restrict__ A, int64_t lda,
                                                             int chunk, const double* __restrict__ bal, int64_t bstride,
-                                                            int2* __restrict__ part) {
+                                                            int2* __restrict__ part, int* __restrict__ flags, int nflags) {
+  wait_for_predecessor();
   const int i = blockIdx.x * 128 + threadIdx.x;
+  for (int f = blockIdx.y * gridDim.x * 128 + i; f < nflags; f += gridDim.x * gridDim.y * 128) flags[f] = 0;
   if (i >= m) return;
   const int c0 = blockIdx.y * chunk, c1 = min(k, c0 + chunk);
   Norm nm;
@@ -279,6 +281,7 @@ __global__ void __launch_bounds__(256) crt_split_a_kernel(int m, int k, const do
   __shared__ int s_scale[32];
   const int i0 = blockIdx.y * 32, k0 = blockIdx.x * 64;
   const int tid = threadIdx.x;
+  wait_for_predecessor();
   if (tid < 32) {
     Norm nm;
     if (i0 + tid < m)
@@ -328,6 +331,7 @@ __global__ void __launch_bounds__(256) crt_split_b_kernel(int k, int n, const do
   __shared__ float s_s[8];
   __shared__ int s_scale;
   const int j = blockIdx.x, tid = threadIdx.x;
+  wait_for_predecessor();
   const double* col = B + (size_t)j * ldb;
   auto at = [&](int c) { return bal ? shift_exp(col[c], -plain_exponent(bal[c * bstride])) : col[c]; };
   Norm nm;
@@ -493,6 +497,7 @@ __global__ void __launch_bounds__(kCrtThreads, 1) __cluster_dims__(2, 1, 1)
   cluster_barrier();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base_sh;
+  wait_for_predecessor();
 
   if (warp == 0 && lane == 0) {
     // producer: this CTA's 128 rows of A and 128 columns of B of every k-block
@@ -647,6 +652,7 @@ __global__ void __launch_bounds__(kCrtThreads, 1) __cluster_dims__(2, 1, 1)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  let_successor_in();
   cluster_barrier();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
 }
@@ -709,6 +715,7 @@ __global__ void __launch_bounds__(128) crt_combine_kernel(CrtArgs g, int mode, d
   __shared__ uint4 s_mult[2 * kKMax + 1];
   if (threadIdx.x < 2 * kKMax + 1) s_mult[threadIdx.x] = kP.v[threadIdx.x];
   __syncthreads();
+  wait_for_predecessor();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int i0 = blockIdx.x * 64 + warp * 16 + (lane >> 3), j0 = blockIdx.y * 32 + (lane & 7) * 4;
   if (j0 >= g.n) return;
@@ -826,16 +833,17 @@ CrtLayout crt_layout(int m, int n, int k) {
 
 // The two forms' times in us, from measurements.  The FP64 kernel: 1.05 per unit
 // of k until its tiles fill the chip, then 1.22 TFLOP/s.  The residues: six
-// dependent launches a block, about 50 us, then 18 planes of each operand to
-// write and read and 16 of the product.  Measured, FP64 against residues: 64^3 70
-// and 47, 64 x 64 x 32 38 and 46, 256^3 266 and 55, 1 x 1 x 8192 8266 and 156,
-// 8192 x 1 x 8192 8523 and 1945, 20000 x 4 x 64 197 and 256, 64 x 8192 x 64 72 and
-// 132, 8192 x 8192 x 32 3589 and 1199.
+// dependent launches a block, about 35 us (47 where each waits for the one before
+// to end instead of being launched ahead), then 18 planes of each operand to write
+// and read and 16 of the product.  Measured, FP64 against residues: 128^3 136 and
+// 33, 256^3 266 and 38, 8192 x 1 x 8192 8523 and 1945, 1 x 1 x 8192 8266 and 156;
+// with the launches one by one 64 x 64 x 32 38 and 46, 20000 x 4 x 64 197 and 256,
+// 64 x 8192 x 64 72 and 132.
 bool crt_gemm_pays(int m, int n, int k) {
   if (m <= 0 || n <= 0 || k <= 0) return false;
   const auto blocks = [](int x, int b) { return (double)((x + b - 1) / b); };
   const double mn = (double)m * n, fp64 = fmax(1.05 * k, 1.64e-6 * mn * k);
-  const double crt = 55 * blocks(m, kBlockMN) * blocks(n, kBlockMN) * blocks(k, kBlockK) +
+  const double crt = 42 * blocks(m, kBlockMN) * blocks(n, kBlockMN) * blocks(k, kBlockK) +
                      3e-5 * ((double)m * k + (double)k * n) + 2e-5 * mn;
   return crt < fp64;
 }
@@ -892,16 +900,20 @@ int crt_gemm_run(int m, int n, int k, double alpha, const double* A, int64_t lda
     const double* bal = balance ? balance + k0 * balance_stride : nullptr;
     for (int n0 = 0; n0 < n; n0 += kBlockMN) {
       const int nc = std::min(kBlockMN, n - n0), np = (int)round_up((size_t)nc, kPN);
-      crt_split_b_kernel<<<np, 256, 0, s>>>(kc, nc, B + (size_t)n0 * ldb + k0, ldb, np, kp, bal, balance_stride, cs, bp);
+      e = launch_chained(crt_split_b_kernel, dim3(np), 256, 0, s, kc, nc, B + (size_t)n0 * ldb + k0, ldb, np, kp, bal,
+                         balance_stride, cs, bp);
+      if (e != cudaSuccess) return record_cuda_error(e, name);
       for (int m0 = 0; m0 < m; m0 += kBlockMN) {
         const int mc = std::min(kBlockMN, m - m0), mp = (int)round_up((size_t)mc, kPM);
         const double* a = A + (size_t)k0 * lda + m0;
         double* c = C + (size_t)n0 * ldc + m0;
         const int chunk = stat_chunk(L.kb), nparts = (kc + chunk - 1) / chunk;
-        crt_row_stats_kernel<<<dim3((mc + 127) / 128, nparts), 128, 0, s>>>(mc, kc, a, lda, chunk, bal, balance_stride, part);
-        crt_split_a_kernel<<<dim3(kp / 64, mp / 32), 256, 0, s>>>(mc, kc, a, lda, part, nparts, mp, kp, bal, balance_stride, rs, ap);
         const int nflags = (mp / kFlagTile) * (np / kFlagTile);
-        e = cudaMemsetAsync(flags, 0, (size_t)nflags * 4, s);
+        e = launch_chained(crt_row_stats_kernel, dim3((mc + 127) / 128, nparts), 128, 0, s, mc, kc, a, lda, chunk, bal,
+                           balance_stride, part, flags, nflags);
+        if (e == cudaSuccess)
+          e = launch_chained(crt_split_a_kernel, dim3(kp / 64, mp / 32), 256, 0, s, mc, kc, a, lda, part, nparts, mp, kp, bal,
+                             balance_stride, rs, ap);
         if (e != cudaSuccess) return record_cuda_error(e, name);
         CUtensorMap mapA, mapB, mapR;
         int rc = make_map(&mapA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ap, (uint64_t)planes * mp, kp, 128, kKB);
@@ -915,12 +927,12 @@ int crt_gemm_run(int m, int n, int k, double alpha, const double* A, int64_t lda
         // The large LU's updates (balance) run beside its panels, whose clusters wait
         // for a whole kernel where every SM holds a CTA to its end: two rounds of
         // shorter ones take n = 8192 from 64.5 to 62.2 ms (four rounds 62.1, eight 63.5).
-        kern<<<2 * std::min(units, balance ? 2 * pairs : pairs), kCrtThreads, smem, s>>>(mapA, mapB, mapR, g);
+        e = launch_chained(kern, dim3(2 * std::min(units, balance ? 2 * pairs : pairs)), kCrtThreads, smem, s, mapA, mapB, mapR, g);
         const int mode = bt == 0.0 ? (alpha == 1.0 ? kPlain : kScaled) : bt == 1.0 ? kAdded : kGeneral;
-        crt_combine_kernel<<<dim3((mc + 63) / 64, (nc + 31) / 32), 128, 0, s>>>(g, mode, alpha, bt, c, ldc);
-        rc = check_launch(name);
-        if (rc == NACU_SUCCESS)
-          rc = dgemm_fp64_run(mc, nc, kc, alpha, a, lda, B + (size_t)n0 * ldb + k0, ldb, bt, c, ldc, flags,
+        if (e == cudaSuccess)
+          e = launch_chained(crt_combine_kernel, dim3((mc + 63) / 64, (nc + 31) / 32), 128, 0, s, g, mode, alpha, bt, c, ldc);
+        if (e != cudaSuccess) return record_cuda_error(e, name);
+        rc = dgemm_fp64_run(mc, nc, kc, alpha, a, lda, B + (size_t)n0 * ldb + k0, ldb, bt, c, ldc, flags,
                               mp / kFlagTile, s);
         if (rc != NACU_SUCCESS) return rc;
       }

@@ -160,6 +160,7 @@ __global__ void split_a_kernel(int m, int k, const TI* __restrict__ A, int64_t l
                                int mp, int kp, int slices, __nv_bfloat16* __restrict__ out) {
   __shared__ double t[32][33];
   const int i0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
+  wait_for_predecessor();
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8 threads
   for (int r = ty; r < 32; r += 8) {
     const int i = i0 + tx, c = c0 + r;
@@ -185,6 +186,7 @@ __global__ void __launch_bounds__(256) split_b_kernel(int k, int n, const TI* __
                                                       __nv_bfloat16* __restrict__ out) {
   __shared__ int s_e[8];
   const int j = blockIdx.x;
+  wait_for_predecessor();
   const TI* col = B + (size_t)j * ldb;
   int e = INT_MIN;
   if (j < n)
@@ -257,6 +259,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base_sh;
+  wait_for_predecessor();
 
   if (warp == 0 && lane == 0) {
     // producer: TMA loads of every slice tile of A and B, k-block after
@@ -498,10 +501,12 @@ int split_gemm_run(int m, int n, int k, double alpha, const TI* A, int64_t lda, 
   if (k > 0) {
     row_exp_kernel<TI><<<dim3((m + 255) / 256, (k + kRowExpChunk - 1) / kRowExpChunk), 256, 0, s>>>(m, k, A, lda,
                                                                                                  rexp);
-    split_a_kernel<TI><<<dim3(L.kp / 32, L.mp / 32), 256, 0, s>>>(m, k, A, lda, rexp, L.mp, L.kp, slices, as);
-    split_b_kernel<TI><<<L.np, 256, 0, s>>>(k, n, B, ldb, cexp, L.np, L.kp, slices, bs);
     int rc = check_launch("nacu_dgemm_split_bf16: split");
     if (rc != NACU_SUCCESS) return rc;
+    e = launch_chained(split_a_kernel<TI>, dim3(L.kp / 32, L.mp / 32), 256, 0, s, m, k, A, lda, rexp, L.mp, L.kp, slices, as);
+    if (e == cudaSuccess)
+      e = launch_chained(split_b_kernel<TI>, dim3(L.np), 256, 0, s, k, n, B, ldb, cexp, L.np, L.kp, slices, bs);
+    if (e != cudaSuccess) return record_cuda_error(e, "nacu_dgemm_split_bf16");
   } else {
     e = cudaMemsetAsync(cexp, 0, (size_t)L.np * 4, s);
     if (e != cudaSuccess) return record_cuda_error(e, "nacu_dgemm_split_bf16");
@@ -548,8 +553,8 @@ int split_gemm_run(int m, int n, int k, double alpha, const TI* A, int64_t lda, 
     else
       return record_arg_error(-3, "split gemm: k == 0 is not supported for FP32 output");
   }
-  split_gemm_kernel<TO><<<grid, kSplitThreads, smem, s>>>(mapA, mapB, g);
-  return check_launch("nacu_dgemm_split_bf16");
+  e = launch_chained(split_gemm_kernel<TO>, dim3(grid), kSplitThreads, smem, s, mapA, mapB, g);
+  return e == cudaSuccess ? NACU_SUCCESS : record_cuda_error(e, "nacu_dgemm_split_bf16");
 }
 
 

@@ -17,8 +17,8 @@
 // updates inside the block; above, a block is one panel of 64 (FP64) or 128.
 // Measured, FP64, ms (all on the FP64 pipe -> residue updates with 64-wide panels ->
 // register panels behind a cluster barrier -> as below): n = 8192 328 -> 114 -> 65 ->
-// 57.6, 4096 50 -> 24.6 -> 20.0 -> 15.5, 2000 11.6 -> 9.4 -> 8.7 -> 5.7, 1000 4.62 ->
-// 4.20 -> 4.08 -> 2.51.  FP32 factor with refinement, n = 4096: 15.8 -> 15.8 -> 14.2 -> 10.2.
+// 55.6, 4096 50 -> 24.6 -> 20.0 -> 15.1, 2000 11.6 -> 9.4 -> 8.7 -> 5.4, 1000 4.62 ->
+// 4.20 -> 4.08 -> 2.39.  FP32 factor with refinement, n = 4096: 15.8 -> 15.8 -> 14.2 -> 9.9.
 // The chain of panels and inner updates bounds it: at n = 8192 50 ms were left of 67
 // when the trailing update beyond the next panel cost nothing.
 // The triangular solves for the right-hand side run as one cooperative kernel
@@ -648,27 +648,9 @@ __device__ __forceinline__ bool bar_wait(const void* bar, unsigned parity, int l
 }
 
 // The chain of small kernels between two trailing updates is launched ahead of its
-// predecessors' ends (programmatic stream serialization): each waits for the one
-// before it as its first act, and tells the next to come in: the panel only in its
+// predecessors' ends (launch_chained); the panel lets the next one in only in its
 // tail, so that nothing idle holds the SMs which the trailing update runs on.
 // n = 1000 2.75 -> 2.55 ms, 4096 16.8 -> 16.0; FP32 with refinement, 4096 10.6 -> 10.2.
-__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void let_successor_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-template <typename... P, typename... Q>
-cudaError_t launch_chained(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, Q... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
-}
-
 template <typename T, int TPR>
 __global__ void __launch_bounds__(kRegThreads, 1) lu_panel_reg_kernel(RegPanelArgs<T> g) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
