@@ -45,7 +45,7 @@
 // hundreds the epilogue (156 us for the 17 planes of 4096 x 4096 x 128; 186 with
 // byte stores from registers).  Measured (GB300, scratch warm): 8192^3 878 ->
 // 16.1 ms (55x; 17 planes at 1.50 of the 1.90 PFLOP/s a BF16 GEMM reaches),
-// 1000 x 777 x 1333 2.69 -> 0.15 ms, 256^3 266 -> 59 us.  Error against sums in
+// 1000 x 777 x 1333 2.69 -> 0.13 ms, 256^3 266 -> 38 us.  Error against sums in
 // short blocks, N(0,1) entries: 3.9e-16 relative at 4096^3 where the FP64 loop
 // has 2.2e-15.
 #include <cuda_bf16.h>
