@@ -76,6 +76,30 @@ def test_least_workspace_updates_on_the_fp64_pipe(cuda, monkeypatch):
     assert O.backward_error(a, x, np.ones((n, 1))) <= 10 * n * 2.0 ** -52
 
 
+@pytest.mark.parametrize("n", [160, 700])
+def test_captured_factorization_has_the_same_bits(cuda, n):
+    """Two streams, clusters and launches ahead of their predecessors' ends, as a
+    CUDA graph replayed on new inputs."""
+    import nalgebra_gb300 as ng
+    from nalgebra_gb300 import _lib
+
+    rng = np.random.default_rng(n)
+    a = [np.asfortranarray(rng.standard_normal((n, n))) for _ in range(3)]
+    want = [_getrf(cuda, x)[:2] for x in a]
+    W = ng.DeviceMatrix.from_numpy(a[0])
+    wsb = _lib.load().nacu_getrf_workspace_bytes(n)
+    ws, ipiv, info = (ng.DeviceBuffer.zeros(*x) for x in ((wsb, np.uint8), (n, np.int32), (2, np.int32)))
+    g = ng.Graph()
+    with g.capture():
+        _lib.call("nacu_dgetrf", n, W.data.data_ptr(), n, ipiv.data_ptr(), info.data_ptr(), ws.data_ptr(), wsb,
+                  ng.current_stream())
+    for x, (lu, piv) in zip(a, want):
+        W.data.copy_(x.ravel(order="F"))
+        g.replay()
+        ng.synchronize()
+        assert np.array_equal(ipiv.to_numpy(), piv) and np.array_equal(W.to_numpy(), lu)
+
+
 def test_ties_take_the_first_position(cuda):
     """Small integers: equal magnitudes in most columns, resolved by the position
     the rows have after the swaps so far.  The eliminations stay exact while the
