@@ -205,8 +205,8 @@ __device__ void lu_system(int n, int nrhs, int ld, T* sa, int* s_piv, int* s_inf
 
 // One CTA per system, grid-stride over the batch.  mode: 0 = factor only,
 // 1 = factor + solve, 2 = solve from given factors.
-template <typename T, bool EXACT>
-__global__ void __launch_bounds__(kLuThreads) lu_batched_kernel(int n, int nrhs, T* __restrict__ A,
+template <typename T, bool EXACT, int MINB>
+__global__ void __launch_bounds__(kLuThreads, MINB) lu_batched_kernel(int n, int nrhs, T* __restrict__ A,
                                                                  int64_t strideA, int32_t* __restrict__ ipiv,
                                                                  T* __restrict__ B, int64_t strideB,
                                                                  int32_t* __restrict__ info, int batch,
@@ -221,34 +221,34 @@ __global__ void __launch_bounds__(kLuThreads) lu_batched_kernel(int n, int nrhs,
   const int tid = threadIdx.x;
   for (int s = blockIdx.x; s < batch; s += gridDim.x) {
     const T* a = A + (size_t)s * strideA;
-    for (int e = tid; e < n * n; e += blockDim.x) {
+    for (int e = tid; e < n * n; e += kLuThreads) {
       const int c = e / n, r = e - c * n;
       sa[(size_t)c * ld + r] = a[e];
     }
     if (nrhs > 0) {
       const T* b = B + (size_t)s * strideB;
-      for (int e = tid; e < n * nrhs; e += blockDim.x) {
+      for (int e = tid; e < n * nrhs; e += kLuThreads) {
         const int c = e / n, r = e - c * n;
         sa[(size_t)(n + c) * ld + r] = b[(size_t)c * n + r];
       }
     }
     if (mode == 2)
-      for (int i = tid; i < n; i += blockDim.x) s_piv[i] = ipiv[(size_t)s * n + i];
+      for (int i = tid; i < n; i += kLuThreads) s_piv[i] = ipiv[(size_t)s * n + i];
     __syncthreads();
     lu_system<T, EXACT>(n, nrhs, ld, sa, s_piv, s_info, s_rcp, mode != 2);
     if (mode != 2) {
       if (write_factors) {
         T* aw = A + (size_t)s * strideA;
-        for (int e = tid; e < n * n; e += blockDim.x) {
+        for (int e = tid; e < n * n; e += kLuThreads) {
           const int c = e / n, r = e - c * n;
           aw[e] = sa[(size_t)c * ld + r];
         }
       }
-      for (int i = tid; i < n; i += blockDim.x) ipiv[(size_t)s * n + i] = s_piv[i];
+      for (int i = tid; i < n; i += kLuThreads) ipiv[(size_t)s * n + i] = s_piv[i];
     }
     if (nrhs > 0) {
       T* b = B + (size_t)s * strideB;
-      for (int e = tid; e < n * nrhs; e += blockDim.x) {
+      for (int e = tid; e < n * nrhs; e += kLuThreads) {
         const int c = e / n, r = e - c * n;
         b[(size_t)c * n + r] = sa[(size_t)(n + c) * ld + r];
       }
@@ -404,7 +404,14 @@ int lu_launch(int n, int nrhs, T* A, int64_t strideA, int32_t* ipiv, T* B, int64
     one<<<batch, kLuSolveThreads, smem, stream>>>(n, A, strideA, ipiv, B, strideB, info);
     return check_launch(name);
   }
-  auto kern = exact ? lu_batched_kernel<T, true> : lu_batched_kernel<T, false>;
+  // CTAs an SM, and with them registers a thread: 8 of 32 registers where shared
+  // memory has room for them, 6 of 40 as it has at order 64, 2 of 96 past 97 (room
+  // for 2 or 1).  Against one kernel of 35 registers, us: 16384 of order 16 356 ->
+  // 311, 8000 of 32 409 -> 372, 4096 of 64 830 -> 827, 2000 of 96 1425 -> 1366, 2000 of
+  // 100 1763 -> 1657, 1000 of 128 2165 -> 1990, one of 100 172 -> 163.
+  const int few = n > 97 ? 2 : n > 48 ? 1 : 0;
+  auto kern = exact ? (few == 2 ? lu_batched_kernel<T, true, 2> : few == 1 ? lu_batched_kernel<T, true, 6> : lu_batched_kernel<T, true, 8>)
+                    : (few == 2 ? lu_batched_kernel<T, false, 2> : few == 1 ? lu_batched_kernel<T, false, 6> : lu_batched_kernel<T, false, 8>);
   if (smem > 48 * 1024) {
     cudaError_t e = ensure_dynamic_smem(kern, smem);
     if (e != cudaSuccess) return record_cuda_error(e, name);
