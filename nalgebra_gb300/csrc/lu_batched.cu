@@ -205,8 +205,66 @@ __device__ void lu_system(int n, int nrhs, int ld, T* sa, int* s_piv, int* s_inf
 
 // One CTA per system, grid-stride over the batch.  mode: 0 = factor only,
 // 1 = factor + solve, 2 = solve from given factors.
-template <typename T, bool EXACT, int MINB>
-__global__ void __launch_bounds__(kLuThreads, MINB) lu_batched_kernel(int n, int nrhs, T* __restrict__ A,
+template <typename T, bool EXACT>
+__global__ void __launch_bounds__(kLuThreads) lu_batched_kernel(int n, int nrhs, T* __restrict__ A,
+                                                                 int64_t strideA, int32_t* __restrict__ ipiv,
+                                                                 T* __restrict__ B, int64_t strideB,
+                                                                 int32_t* __restrict__ info, int batch,
+                                                                 int mode, int write_factors) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int ld = n | 1;
+  const int ncols = n + nrhs;
+  T* sa = reinterpret_cast<T*>(smem_raw);
+  T* s_rcp = sa + (size_t)ld * ncols;  // [0]: 1/pivot, [n+1], [n+2]: the step's scalars; [1+i]: 1/U_ii
+  int* s_piv = reinterpret_cast<int*>(s_rcp + n + 3);
+  int* s_info = s_piv + n;
+  const int tid = threadIdx.x;
+  for (int s = blockIdx.x; s < batch; s += gridDim.x) {
+    const T* a = A + (size_t)s * strideA;
+    for (int e = tid; e < n * n; e += blockDim.x) {
+      const int c = e / n, r = e - c * n;
+      sa[(size_t)c * ld + r] = a[e];
+    }
+    if (nrhs > 0) {
+      const T* b = B + (size_t)s * strideB;
+      for (int e = tid; e < n * nrhs; e += blockDim.x) {
+        const int c = e / n, r = e - c * n;
+        sa[(size_t)(n + c) * ld + r] = b[(size_t)c * n + r];
+      }
+    }
+    if (mode == 2)
+      for (int i = tid; i < n; i += blockDim.x) s_piv[i] = ipiv[(size_t)s * n + i];
+    __syncthreads();
+    lu_system<T, EXACT>(n, nrhs, ld, sa, s_piv, s_info, s_rcp, mode != 2);
+    if (mode != 2) {
+      if (write_factors) {
+        T* aw = A + (size_t)s * strideA;
+        for (int e = tid; e < n * n; e += blockDim.x) {
+          const int c = e / n, r = e - c * n;
+          aw[e] = sa[(size_t)c * ld + r];
+        }
+      }
+      for (int i = tid; i < n; i += blockDim.x) ipiv[(size_t)s * n + i] = s_piv[i];
+    }
+    if (nrhs > 0) {
+      T* b = B + (size_t)s * strideB;
+      for (int e = tid; e < n * nrhs; e += blockDim.x) {
+        const int c = e / n, r = e - c * n;
+        b[(size_t)c * n + r] = sa[(size_t)(n + c) * ld + r];
+      }
+    }
+    if (tid == 0 && info) info[s] = *s_info;
+    __syncthreads();
+  }
+}
+
+// The same where shared memory admits two CTAs an SM or one (orders past 97): up to
+// 96 registers a thread, the loops' stride known when compiling and their loads
+// unrolled.  1000 of order 100 with one right-hand side 1151 -> 1038 us (whole call),
+// 1000 of 128 with five 2458 -> 2273, one of 100 172 -> 162.  Where more CTAs fit the
+// longer code costs more than it gives (4096 of order 64 942 -> 950).
+template <typename T, bool EXACT>
+__global__ void __launch_bounds__(kLuThreads, 2) lu_batched_wide_kernel(int n, int nrhs, T* __restrict__ A,
                                                                  int64_t strideA, int32_t* __restrict__ ipiv,
                                                                  T* __restrict__ B, int64_t strideB,
                                                                  int32_t* __restrict__ info, int batch,
@@ -404,14 +462,8 @@ int lu_launch(int n, int nrhs, T* A, int64_t strideA, int32_t* ipiv, T* B, int64
     one<<<batch, kLuSolveThreads, smem, stream>>>(n, A, strideA, ipiv, B, strideB, info);
     return check_launch(name);
   }
-  // CTAs an SM, and with them registers a thread: 8 of 32 registers where shared
-  // memory has room for them, 6 of 40 as it has at order 64, 2 of 96 past 97 (room
-  // for 2 or 1).  Against one kernel of 35 registers, us: 16384 of order 16 356 ->
-  // 311, 8000 of 32 409 -> 372, 4096 of 64 830 -> 827, 2000 of 96 1425 -> 1366, 2000 of
-  // 100 1763 -> 1657, 1000 of 128 2165 -> 1990, one of 100 172 -> 163.
-  const int few = n > 97 ? 2 : n > 48 ? 1 : 0;
-  auto kern = exact ? (few == 2 ? lu_batched_kernel<T, true, 2> : few == 1 ? lu_batched_kernel<T, true, 6> : lu_batched_kernel<T, true, 8>)
-                    : (few == 2 ? lu_batched_kernel<T, false, 2> : few == 1 ? lu_batched_kernel<T, false, 6> : lu_batched_kernel<T, false, 8>);
+  auto kern = n > 97 ? (exact ? lu_batched_wide_kernel<T, true> : lu_batched_wide_kernel<T, false>)
+                     : (exact ? lu_batched_kernel<T, true> : lu_batched_kernel<T, false>);
   if (smem > 48 * 1024) {
     cudaError_t e = ensure_dynamic_smem(kern, smem);
     if (e != cudaSuccess) return record_cuda_error(e, name);
