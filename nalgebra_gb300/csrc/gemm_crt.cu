@@ -444,6 +444,17 @@ __device__ __forceinline__ void unit_tile(int u, int tiles, int tm, int tn, int*
   *ni = in / h;
 }
 
+// Past this K a sum's remainder mod 255 needs a second reduction to fit a byte:
+// 1 / 255 is 5.9e-8 too large in FP32, so from |x| = 8,454,907 on a quotient next to
+// a tie rounds the wrong way and leaves +128.  Sums of 512 products stay below 2^23;
+// the other odd moduli leave at most 127 up to 2^24.
+constexpr int kOnceMaxK = 512;
+
+// x - p round(x / p), exact for integers up to 2^24.
+__device__ __forceinline__ float reduce_once(float x, float p, float inv) {
+  return fmaf(-p, fmaf(x, inv, 12582912.f) - 12582912.f, x);
+}
+
 // Sixteen FP32 integers -> their balanced residues mod p as bytes (p = 256:
 // 128 wraps to -128, the same residue).
 __device__ __forceinline__ uint4 reduce_pack16(const uint32_t* v, float p, float inv) {
@@ -462,8 +473,11 @@ __device__ __forceinline__ uint4 reduce_pack16(const uint32_t* v, float p, float
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// ONE_CHUNK: K <= 1024, one exact sum per output and no register accumulators.
-template <bool ONE_CHUNK>
+// kShort, kOneChunk: K <= 512 and K <= 1024, one exact sum per output and no register
+// accumulators (the second reduction in the short products' code too costs the LU of
+// order 8192, K = 128, 2.7%).
+enum CrtForm { kShort, kOneChunk, kChunks };
+template <CrtForm FORM>
 __global__ void __launch_bounds__(kCrtThreads, 1) __cluster_dims__(2, 1, 1)
     crt_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                     const __grid_constant__ CUtensorMap mapR, const CrtArgs g) {
@@ -578,7 +592,7 @@ __global__ void __launch_bounds__(kCrtThreads, 1) __cluster_dims__(2, 1, 1)
         __syncwarp();
       }
       float acc[128];
-      if constexpr (!ONE_CHUNK) {
+      if constexpr (FORM == kChunks) {
 #pragma unroll
         for (int i = 0; i < 128; ++i) acc[i] = 0.f;
       }
@@ -599,9 +613,13 @@ __global__ void __launch_bounds__(kCrtThreads, 1) __cluster_dims__(2, 1, 1)
                 "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
               : "r"(taddr + (uint32_t)c0));
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          // x - p round(x / p), exact (integers up to 2^24; p = 0 on the ratio plane: x itself)
-          if constexpr (ONE_CHUNK) {
+          // p = 0 on the ratio plane: x itself
+          if constexpr (FORM != kChunks) {
             if (residue) {
+              if (FORM == kOneChunk && p == 255.f) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(reduce_once(__uint_as_float(v[i]), p, inv));
+              }
               *reinterpret_cast<uint4*>(stage + (((c0 / 16) ^ (lane & 7)) << 4)) = reduce_pack16(v, p, inv);
             } else {
 #pragma unroll
@@ -609,11 +627,7 @@ __global__ void __launch_bounds__(kCrtThreads, 1) __cluster_dims__(2, 1, 1)
             }
           } else {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const float x = __uint_as_float(v[i]);
-              const float k = fmaf(x, inv, 12582912.f) - 12582912.f;
-              acc[c0 + i] += fmaf(-p, k, x);
-            }
+            for (int i = 0; i < 16; ++i) acc[c0 + i] += reduce_once(__uint_as_float(v[i]), p, inv);
           }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -622,7 +636,7 @@ __global__ void __launch_bounds__(kCrtThreads, 1) __cluster_dims__(2, 1, 1)
       }
       if (!ok) break;
       if (residue) {
-        if constexpr (!ONE_CHUNK) {
+        if constexpr (FORM == kChunks) {
 #pragma unroll
           for (int c0 = 0; c0 < 128; c0 += 16)
             *reinterpret_cast<uint4*>(stage + (((c0 / 16) ^ (lane & 7)) << 4)) =
@@ -855,7 +869,7 @@ size_t crt_gemm_workspace_bytes(int m, int n, int k) {
 // CTA pairs the device keeps resident (a die whose SM count is odd leaves one SM without a partner).
 static int crt_max_pairs(size_t smem) {
   static int pairs = 0;
-  if (pairs == 0 && ensure_dynamic_smem(crt_gemm_kernel<false>, smem) == cudaSuccess) {
+  if (pairs == 0 && ensure_dynamic_smem(crt_gemm_kernel<kChunks>, smem) == cudaSuccess) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)sm_count() & ~1u);
     cfg.blockDim = dim3(kCrtThreads);
@@ -867,7 +881,7 @@ static int crt_max_pairs(size_t smem) {
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     int c = 0;
-    if (cudaOccupancyMaxActiveClusters(&c, crt_gemm_kernel<false>, &cfg) != cudaSuccess || c < 1) {
+    if (cudaOccupancyMaxActiveClusters(&c, crt_gemm_kernel<kChunks>, &cfg) != cudaSuccess || c < 1) {
       (void)cudaGetLastError();
       c = std::max(1, sm_count() / 2);
     }
@@ -890,7 +904,9 @@ int crt_gemm_run(int m, int n, int k, double alpha, const double* A, int64_t lda
   int* flags = reinterpret_cast<int*>(ws + L.flag_off);
   constexpr int planes = kMod + 1;  // and the ratio plane
   constexpr size_t smem = (size_t)kStagesC * kStageBytesC + 8 * kStoreBytes + 1024;
-  const auto kern = std::min(k, kBlockK) <= kChunkBlocks * kKB ? crt_gemm_kernel<true> : crt_gemm_kernel<false>;
+  const auto kern = k <= kOnceMaxK            ? crt_gemm_kernel<kShort>
+                    : k <= kChunkBlocks * kKB ? crt_gemm_kernel<kOneChunk>
+                                              : crt_gemm_kernel<kChunks>;
   cudaError_t e = ensure_dynamic_smem(kern, smem);
   if (e != cudaSuccess) return record_cuda_error(e, name);
   const int pairs = crt_max_pairs(smem);
