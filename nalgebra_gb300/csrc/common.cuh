@@ -21,13 +21,13 @@ int dgemm_fp64_run(int m, int n, int k, double alpha, const double* A, int64_t l
 // faster one at these sizes, its scratch, the product.
 bool crt_gemm_pays(int m, int n, int k);
 size_t crt_gemm_workspace_bytes(int m, int n, int k);
-// balance (nullable, k values balance[i * balance_stride]): column i of A and row i
-// of B are scaled by its exponent and the reverse before they are cut, which
-// leaves the product and moves no precision to where B's large rows meet A's
-// small columns (an LU's pivots, for rows of very different scale).
+// balance (nullable, k exponents): column i of A is scaled by 2^balance[i] and row i
+// of B by the reverse before they are cut, which leaves the product and moves no
+// precision to where B's large rows meet A's small columns (L and U of a matrix with
+// rows of very different scale).
 int crt_gemm_run(int m, int n, int k, double alpha, const double* A, int64_t lda, const double* B, int64_t ldb,
                  double beta, double* C, int64_t ldc, void* workspace, size_t workspace_bytes, cudaStream_t stream,
-                 const char* name, const double* balance = nullptr, int64_t balance_stride = 0);
+                 const char* name, const int* balance = nullptr);
 // Whether one of its kernels gave up on a barrier since the library was loaded.
 int crt_gemm_error(int* flag);
 
@@ -256,11 +256,6 @@ __device__ __forceinline__ double shift_exp(double x, int e) {
   const int hi = __double2hiint(x), ex = (hi >> 20) & 0x7ff;
   if (ex != 0 && ex != 0x7ff && ex + e > 0 && ex + e < 0x7ff) return __hiloint2double(hi + e * (1 << 20), __double2loint(x));
   return scalbn(x, e);
-}
-// The exponent of a normal number, 0 for zero, subnormal, inf and NaN.
-__device__ __forceinline__ int plain_exponent(double x) {
-  const int ex = (__double2hiint(x) >> 20) & 0x7ff;
-  return ex == 0 || ex == 0x7ff ? 0 : ex - 1023;
 }
 
 // A lower bound of |x| in binary32 for norm sums, from the high word alone:

@@ -185,10 +185,11 @@ __constant__ CrtMultiples kP = make_multiples();
 struct Norm {
   int e = 0;
   float s = 0.f;
-  __device__ __forceinline__ void add(double x) {
+  // x 2^shift; where it falls below the normal numbers, as the smallest of them
+  __device__ __forceinline__ void add(double x, int shift) {
     const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu, lo = (unsigned)__double2loint(x);
     if ((hi | lo) == 0u) return;
-    const int ex = max((int)(hi >> 20), 1);
+    const int ex = hi >= 0x7ff00000u ? 2047 : min(max(max((int)(hi >> 20), 1) + shift, 1), 2047);
     // the mantissa rounded up to 21 bits: never below |x|
     const float f = __uint_as_float(0x3f800000u | ((hi & 0xfffffu) << 3) | 7u);
     if (ex > e) {
@@ -256,7 +257,7 @@ __device__ __forceinline__ uint32_t abs_bits(long long v, bool bad) {
 
 // Partial row norms of A: thread per row and chunk of columns; part[chunk][row].
 __global__ void __launch_bounds__(128) crt_row_stats_kernel(int m, int k, const double* __restrict__ A, int64_t lda,
-                                                            int chunk, const double* __restrict__ bal, int64_t bstride,
+                                                            int chunk, const int* __restrict__ bal,
                                                             int2* __restrict__ part, int* __restrict__ flags, int nflags) {
   wait_for_predecessor();
   const int i = blockIdx.x * 128 + threadIdx.x;
@@ -266,7 +267,7 @@ __global__ void __launch_bounds__(128) crt_row_stats_kernel(int m, int k, const 
   Norm nm;
   const double* a = A + (size_t)c0 * lda + i;
 #pragma unroll 4
-  for (int c = c0; c < c1; ++c, a += lda) nm.add(bal ? shift_exp(*a, plain_exponent(bal[c * bstride])) : *a);
+  for (int c = c0; c < c1; ++c, a += lda) nm.add(*a, bal ? bal[c] : 0);
   part[(size_t)blockIdx.y * m + i] = make_int2(nm.e, __float_as_int(nm.s));
 }
 
@@ -275,7 +276,7 @@ __global__ void __launch_bounds__(128) crt_row_stats_kernel(int m, int k, const 
 // k tile also write the row scales.
 __global__ void __launch_bounds__(256) crt_split_a_kernel(int m, int k, const double* __restrict__ A, int64_t lda,
                                                           const int2* __restrict__ part, int nparts, int mp, int kp,
-                                                          const double* __restrict__ bal, int64_t bstride,
+                                                          const int* __restrict__ bal,
                                                           int* __restrict__ rscale, uint32_t* __restrict__ out) {
   __shared__ long long t[64][33];
   __shared__ int s_scale[32];
@@ -301,7 +302,7 @@ __global__ void __launch_bounds__(256) crt_split_a_kernel(int m, int k, const do
     for (int u = 0; u < 8; ++u) {
       const int kk = (tid >> 5) + 8 * u;
       double x = (live && k0 + kk < k) ? A[(size_t)(k0 + kk) * lda + i0 + r] : 0.0;
-      if (bal && k0 + kk < k) x = shift_exp(x, plain_exponent(bal[(k0 + kk) * bstride]));
+      if (bal && k0 + kk < k) x = shift_exp(x, bal[k0 + kk]);
       t[kk][r] = scaled_int(x, live ? sc : 0);
     }
   }
@@ -324,7 +325,7 @@ __global__ void __launch_bounds__(256) crt_split_a_kernel(int m, int k, const do
 // B (columns contiguous along K) -> residue planes [plane][np][kp] and the
 // column scales; one CTA per (padded) column.
 __global__ void __launch_bounds__(256) crt_split_b_kernel(int k, int n, const double* __restrict__ B, int64_t ldb, int np,
-                                                          int kp, const double* __restrict__ bal, int64_t bstride,
+                                                          int kp, const int* __restrict__ bal,
                                                           int* __restrict__ cscale,
                                                           uint32_t* __restrict__ out) {
   __shared__ int s_e[8];
@@ -333,10 +334,10 @@ __global__ void __launch_bounds__(256) crt_split_b_kernel(int k, int n, const do
   const int j = blockIdx.x, tid = threadIdx.x;
   wait_for_predecessor();
   const double* col = B + (size_t)j * ldb;
-  auto at = [&](int c) { return bal ? shift_exp(col[c], -plain_exponent(bal[c * bstride])) : col[c]; };
+  auto at = [&](int c) { return bal ? shift_exp(col[c], -bal[c]) : col[c]; };
   Norm nm;
   if (j < n)
-    for (int c = tid; c < k; c += 256) nm.add(at(c));
+    for (int c = tid; c < k; c += 256) nm.add(col[c], bal ? -bal[c] : 0);
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
     const int e2 = __shfl_xor_sync(0xffffffffu, nm.e, off);
@@ -892,7 +893,7 @@ static int crt_max_pairs(size_t smem) {
 
 int crt_gemm_run(int m, int n, int k, double alpha, const double* A, int64_t lda, const double* B, int64_t ldb,
                  double beta, double* C, int64_t ldc, void* workspace, size_t workspace_bytes, cudaStream_t s,
-                 const char* name, const double* balance, int64_t balance_stride) {
+                 const char* name, const int* balance) {
   const CrtLayout L = crt_layout(m, n, k);
   if (!workspace || workspace_bytes < L.total) return record_arg_error(-13, "dgemm: workspace too small");
   unsigned char* ws = reinterpret_cast<unsigned char*>(round_up(reinterpret_cast<uintptr_t>(workspace), 1024));
@@ -910,14 +911,14 @@ int crt_gemm_run(int m, int n, int k, double alpha, const double* A, int64_t lda
   cudaError_t e = ensure_dynamic_smem(kern, smem);
   if (e != cudaSuccess) return record_cuda_error(e, name);
   const int pairs = crt_max_pairs(smem);
+  if (balance && k > kBlockK) balance = nullptr;  // one block's depth
   for (int k0 = 0; k0 < k; k0 += kBlockK) {
     const int kc = std::min(kBlockK, k - k0), kp = (int)round_up((size_t)kc, kKB);
     const double bt = k0 == 0 ? beta : 1.0;
-    const double* bal = balance ? balance + k0 * balance_stride : nullptr;
     for (int n0 = 0; n0 < n; n0 += kBlockMN) {
       const int nc = std::min(kBlockMN, n - n0), np = (int)round_up((size_t)nc, kPN);
-      e = launch_chained(crt_split_b_kernel, dim3(np), 256, 0, s, kc, nc, B + (size_t)n0 * ldb + k0, ldb, np, kp, bal,
-                         balance_stride, cs, bp);
+      e = launch_chained(crt_split_b_kernel, dim3(np), 256, 0, s, kc, nc, B + (size_t)n0 * ldb + k0, ldb, np, kp,
+                         balance, cs, bp);
       if (e != cudaSuccess) return record_cuda_error(e, name);
       for (int m0 = 0; m0 < m; m0 += kBlockMN) {
         const int mc = std::min(kBlockMN, m - m0), mp = (int)round_up((size_t)mc, kPM);
@@ -925,11 +926,11 @@ int crt_gemm_run(int m, int n, int k, double alpha, const double* A, int64_t lda
         double* c = C + (size_t)n0 * ldc + m0;
         const int chunk = stat_chunk(L.kb), nparts = (kc + chunk - 1) / chunk;
         const int nflags = (mp / kFlagTile) * (np / kFlagTile);
-        e = launch_chained(crt_row_stats_kernel, dim3((mc + 127) / 128, nparts), 128, 0, s, mc, kc, a, lda, chunk, bal,
-                           balance_stride, part, flags, nflags);
+        e = launch_chained(crt_row_stats_kernel, dim3((mc + 127) / 128, nparts), 128, 0, s, mc, kc, a, lda, chunk,
+                           balance, part, flags, nflags);
         if (e == cudaSuccess)
-          e = launch_chained(crt_split_a_kernel, dim3(kp / 64, mp / 32), 256, 0, s, mc, kc, a, lda, part, nparts, mp, kp, bal,
-                             balance_stride, rs, ap);
+          e = launch_chained(crt_split_a_kernel, dim3(kp / 64, mp / 32), 256, 0, s, mc, kc, a, lda, part, nparts, mp, kp,
+                             balance, rs, ap);
         if (e != cudaSuccess) return record_cuda_error(e, name);
         CUtensorMap mapA, mapB, mapR;
         int rc = make_map(&mapA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ap, (uint64_t)planes * mp, kp, 128, kKB);

@@ -40,7 +40,7 @@ namespace nacu {
 // panel factorization (cooperative, the panel resident in shared memory)
 // ---------------------------------------------------------------------------
 constexpr int kPanelThreads = 256;
-constexpr int kPanelMaxG = 256;          // CTAs of one panel launch
+constexpr int kPanelMaxG = 255;          // CTAs of one panel launch
 constexpr int kPanelMaxNb = 128;         // panel width
 constexpr int kPanelRowsPerCta = 64;     // rows per CTA aimed for
 constexpr size_t kPanelMaxSmem = 200 * 1024;
@@ -61,6 +61,7 @@ struct PanelPub {
   int nlist[kPanelMaxNb / 32];
   int pdst[2 * kPanelMaxNb];
   int psrc[2 * kPanelMaxNb];
+  int balance[kPanelMaxNb];  // of the block's trailing updates (u_row_exponents)
 };
 
 template <typename T>
@@ -868,90 +869,141 @@ __global__ void __launch_bounds__(256) lu_inner_update_kernel(int n, float* __re
   }
 }
 
+// The scales of 32 rows of U, for the balance of the products L U: a CTA's warps hold
+// a column each (lane: row), the first eight right of the block.  The mean of a row's
+// exponents is blind to column scaling, which moves all rows' alike; the pivots' are
+// not.  A row without a sample counts for little: where it is not zero further right,
+// the products' checks send the outputs to the FP64 loop.
+constexpr int kBalanceMax = 400;
+__device__ __forceinline__ int packed_exponent(double x) {  // sum and count in one word, up to 255 of them
+  const int ex = (__double2hiint(x) >> 20) & 0x7ff;
+  return ex == 0x7ff || is_zero_bits(x) ? 0 : ex << 8 | 1;
+}
+__device__ __forceinline__ int mean_exponent(int packed) {
+  if ((packed & 255) == 32) return packed >> 13;
+  return __float2int_rn(__fdividef((float)(packed >> 8), (float)(packed & 255)));
+}
+__device__ __forceinline__ void u_row_exponents(double y, bool on, int nb, int* balance) {
+  __shared__ int s_e[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  s_e[warp][lane] = on ? packed_exponent(y) : 0;
+  __syncthreads();
+  if (warp == 0 && lane < nb) {
+    int e = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) e += s_e[w][lane];
+    balance[lane] = e == 0 ? -kBalanceMax : max(-kBalanceMax, min(kBalanceMax, mean_exponent(e) - 1023));
+  }
+}
+
 // The same in FP64 by digit slices (slices.cuh): rows j0 + nb .. r_hi - 1 times
 // columns c_lo .. c_hi - 1, 64 x 32 of them per CTA, the 32 products of an
-// output in one exact sum.  L's columns are scaled by the exponents of their
-// pivots and U's rows by the reverse: L D has the scale of its rows' entries of
-// A in every column and D^-1 U is near one, so rows of very different scale keep
-// their precision, as they do in the FP64 loop.
+// output in one exact sum.  Where A's rows and columns have scales r_i and c_j, L_ik
+// goes as r_i / r_k and U_kj as r_k c_j; so row k of U is cut against its mean
+// exponent over the CTA's columns and column k of L the other way, which leaves r_i
+// in every term of a row of L and c_j in every one of a column of U: both kinds of
+// scaling keep their precision, as they do in the FP64 loop.  (The exponent of the
+// pivot, r_k c_k, serves rows only: columns scaled by 2^+-20 lost 40 bits.)  What
+// grading is left the meeting test finds, and those outputs take the FP64 loop.
 // It sits between two panels, so its own latency counts and little else: four
 // threads cut a row, a warp has one 16 x 8 tile, its 4 elements loaded first.  With
 // 128 threads on 64 x 96 it took 17 us (3500 instructions in a row) at 1900 rows;
 // the factorization at n = 2000 7.1 ms, so 6.1.
 constexpr int kInnerRows = 64, kInnerCols = 32, kInnerThreads = 512;
 constexpr int kInnerSlots = kInnerRows + kInnerCols;
-constexpr size_t kInnerSmem = (size_t)2 * kSlices * kInnerSlots * kSliceRow + kInnerSlots * 4;
+constexpr int kInnerUWarps = 4 * kInnerCols / 32;  // the warps that hold U
+constexpr size_t kInnerSmem = (size_t)2 * kSlices * kInnerSlots * kSliceRow + (kRegNb * kInnerUWarps + kInnerSlots) * 4;
+// One output by the FP64 loop; out of line, its code would be fetched in vain.
+__device__ __noinline__ void lu_inner_fp64(double* A, int64_t lda, int j0, int nb, int r, int c) {
+  double v = A[(size_t)c * lda + r];
+  for (int k = 0; k < nb; ++k) v = axpy1<false>(v, -A[(size_t)c * lda + j0 + k], A[(size_t)(j0 + k) * lda + r]);
+  A[(size_t)c * lda + r] = v;
+}
 __global__ void __launch_bounds__(kInnerThreads) lu_inner_update_kernel(int r_hi, double* __restrict__ A, int64_t lda, int j0,
                                                                         int nb, int c_lo, int c_hi) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int sb = kInnerSlots * kSliceRow;
   unsigned char* SL = smem_raw;  // [half][slice][slot]
-  int* ex = reinterpret_cast<int*>(smem_raw + (size_t)2 * kSlices * sb);
+  int* uexp = reinterpret_cast<int*>(smem_raw + (size_t)2 * kSlices * sb);  // [row of U][warp]
+  int* ex = uexp + kRegNb * kInnerUWarps;
+  static_assert(kInnerUWarps == 4, "a row's exponents are read as one int4");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int r0 = j0 + nb + blockIdx.x * kInnerRows, cb = c_lo + blockIdx.y * kInnerCols;
   const int w = min(kInnerCols, c_hi - cb);
   const int rt = (warp & 3) * 16, c = (warp >> 2) * 8;  // this warp's tile
   wait_for_predecessor();
   let_successor_in();
-  double* p[4];
+  const int rg = r0 + rt + g, cg = c + 2 * t;  // the element's place: row rg (+ 8), column cb + cg (+ 1)
+  const auto on = [&](int i) { return rg + (i >> 1) * 8 < r_hi && cg + (i & 1) < w; };
   double v[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = r0 + rt + g + (i >> 1) * 8, cc = c + 2 * t + (i & 1);
-    p[i] = r < r_hi && cc < w ? A + (size_t)(cb + cc) * lda + r : nullptr;
-    v[i] = p[i] ? *p[i] : 0.0;
-  }
+  for (int i = 0; i < 4; ++i) v[i] = on(i) ? A[(size_t)(cb + cg + (i & 1)) * lda + rg + (i >> 1) * 8] : 0.0;
   constexpr int kPart = kRegNb / 4;  // a thread's elements of its slot
-  if (tid < 4 * kInnerSlots) {
-    const int s = tid >> 2, k0 = (tid & 3) * kPart;
-    const bool lrow = s < kInnerRows;
+  const int s = tid >> 2, k0 = (tid & 3) * kPart;
+  const bool lrow = s < kInnerRows;
+  double x[kPart];
+  if (s < kInnerSlots) {
     const int r = r0 + s, cc = s - kInnerRows;
-    const bool on = lrow ? r < r_hi : cc < w;
+    const bool in = lrow ? r < r_hi : cc < w;
     const double* src = lrow ? A + (size_t)j0 * lda + r : A + (size_t)(cb + cc) * lda + j0;
     const int64_t st = lrow ? lda : 1;
-    double x[kPart], d[kPart];
 #pragma unroll
-    for (int k = 0; k < kPart; ++k) {
-      const bool in = on && k0 + k < nb;
-      x[k] = in ? src[(k0 + k) * st] : 0.0;
-      d[k] = in ? A[(size_t)(j0 + k0 + k) * (lda + 1)] : 1.0;  // the pivot
+    for (int k = 0; k < kPart; ++k) x[k] = in && k0 + k < nb ? src[(k0 + k) * st] : 0.0;
+    if (!lrow) {
+#pragma unroll
+      for (int k = 0; k < kPart; ++k) {
+        int e = packed_exponent(x[k]);
+        e += __shfl_xor_sync(0xffffffffu, e, 4);
+        e += __shfl_xor_sync(0xffffffffu, e, 8);
+        e += __shfl_xor_sync(0xffffffffu, e, 16);
+        if (lane < 4) uexp[(k0 + k) * kInnerUWarps + (s - kInnerRows) / 8] = e;
+      }
     }
-    int em = 1;
+  }
+  __syncthreads();
+  if (s < kInnerSlots) {
+    int shift[kPart];  // kNoExponent: the row of U is zero, L's entry does not count
+    int em = kNoExponent;
 #pragma unroll
     for (int k = 0; k < kPart; ++k) {
-      const int pe = k0 + k < nb ? plain_exponent(d[k]) : 0;
-      x[k] = shift_exp(x[k], lrow ? pe : -pe);
-      em = max(em, slice_exponent(x[k]));
+      const int4 u = *reinterpret_cast<const int4*>(uexp + (k0 + k) * kInnerUWarps);
+      const int sum = u.x + u.y + u.z + u.w, e = sum ? mean_exponent(sum) : kNoExponent;
+      shift[k] = lrow ? e : -e;
+      em = max(em, shifted_exponent(x[k], shift[k]));
     }
     em = max(em, __shfl_xor_sync(0xffffffffu, em, 1));
     em = max(em, __shfl_xor_sync(0xffffffffu, em, 2));
 #pragma unroll
     for (int k = 0; k < kPart; k += 4) {
       uint32_t w0[kSlices], w1[kSlices];
-      slice_pair(x[k], x[k + 1], em, w0);
-      slice_pair(x[k + 2], x[k + 3], em, w1);
+      slice_digits(x[k], x[k + 1], em - shift[k], em - shift[k + 1], w0);
+      slice_digits(x[k + 2], x[k + 3], em - shift[k + 2], em - shift[k + 3], w1);
       const int kk = k0 + k;
 #pragma unroll
       for (int q = 0; q < kSlices; ++q)
         *reinterpret_cast<uint2*>(SL + (size_t)((kk >> 4) * kSlices + q) * sb + s * kSliceRow + (kk & 15) * 2) =
             make_uint2(w0[q], w1[q]);
     }
-    if (k0 == 0) ex[s] = slice_code(em);
+    if (k0 == 0) ex[s] = em >= kBadRow / 2 ? kBadRow : em <= kNoExponent / 2 ? kNoExponent : em;
   }
   __syncthreads();
   if (c >= w) return;
-  float acc[kSlices][4];
+  float acc[kSlices][4], met[4] = {0.f, 0.f, 0.f, 0.f};
   slice_sums_start(acc);
 #pragma unroll
   for (int h = 0; h < 2; ++h)
-    slice_products_add(SL + (size_t)h * kSlices * sb + rt * kSliceRow,
-                       SL + (size_t)h * kSlices * sb + (kInnerRows + c) * kSliceRow, sb, lane, acc);
+    slice_products_met(SL + (size_t)h * kSlices * sb + rt * kSliceRow,
+                       SL + (size_t)h * kSlices * sb + (kInnerRows + c) * kSliceRow, sb, lane, acc, met);
   const int e0 = ex[rt + g], e1 = ex[rt + g + 8];
   const int f0 = ex[kInnerRows + c + 2 * t], f1 = ex[kInnerRows + c + 2 * t + 1];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const double y = slice_value<32>(acc, i, (i >> 1 ? e1 : e0) + (i & 1 ? f1 : f0));
-    if (p[i]) *p[i] = v[i] - y;
+    const int er = i >> 1 ? e1 : e0, ec = i & 1 ? f1 : f0;
+    const bool bad = er == kBadRow || ec == kBadRow, zero = er == kNoExponent || ec == kNoExponent;
+    const double y = slice_value<32>(acc, i, er + ec);
+    if (!on(i)) continue;
+    if (bad || (!zero && met[i] < kMeet)) lu_inner_fp64(A, lda, j0, nb, rg + (i >> 1) * 8, cb + cg + (i & 1));
+    else A[(size_t)(cb + cg + (i & 1)) * lda + rg + (i >> 1) * 8] = v[i] - y;
   }
 }
 
@@ -1071,10 +1123,17 @@ __global__ void __launch_bounds__(256) lu_trsm_kernel(int n, T* A, int64_t lda, 
   }
 }
 
+__global__ void __launch_bounds__(256) lu_balance_kernel(int n, const double* A, int64_t lda, int p0, int nb, int c0,
+                                                         int* balance) {
+  const int lane = threadIdx.x & 31, c = c0 + (threadIdx.x >> 5);
+  const bool on = c < n && lane < nb;
+  u_row_exponents(on ? A[(size_t)c * lda + p0 + lane] : 0.0, on, nb, balance);
+}
+
 // The solve with one unit lower triangle of at most 32 rows at p0 for columns
-// c0 .. n - 1: a warp per column, a row per lane.
+// c0 .. n - 1: a warp per column, a row per lane.  The first CTA leaves the rows' scales.
 __global__ void __launch_bounds__(256) lu_trsm_piece_kernel(int n, double* __restrict__ A, int64_t lda, int p0, int nb,
-                                                            int c0) {
+                                                            int c0, int* balance) {
   __shared__ double L[32][33];
   wait_for_predecessor();
   let_successor_in();
@@ -1084,14 +1143,15 @@ __global__ void __launch_bounds__(256) lu_trsm_piece_kernel(int n, double* __res
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, c = c0 + blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (c >= n) return;
+  const bool on = c < n && lane < nb;
   double* col = A + (size_t)c * lda + p0;
-  double y = lane < nb ? col[lane] : 0.0;
+  double y = on ? col[lane] : 0.0;
   for (int k = 0; k + 1 < nb; ++k) {
     const double yk = __shfl_sync(0xffffffffu, y, k);
     if (lane > k && lane < nb) y = axpy1<false>(y, -L[k][lane], yk);
   }
-  if (lane < nb) col[lane] = y;
+  if (on) col[lane] = y;
+  if (blockIdx.x == 0) u_row_exponents(y, on, nb, balance);
 }
 
 // The same for a panel width without a register-tiled instance: L11 in shared
@@ -1589,11 +1649,12 @@ bool reg_panels(int n) {
 // the piece's triangle, then its update of the block's rows below by digit
 // slices.  A quarter of the solve's FP64 instructions (2048 columns: 94 us in one
 // kernel; seven launches of 6 to 10 us here).
-cudaError_t trsm_by_pieces(int n, double* A, int64_t lda, int j0, int jb, cudaStream_t s) {
+cudaError_t trsm_by_pieces(int n, double* A, int64_t lda, int j0, int jb, int* balance, cudaStream_t s) {
   const int c0 = j0 + jb, rest = n - c0;
   for (int p0 = j0; p0 < c0; p0 += kRegNb) {
     const int nb = std::min(kRegNb, c0 - p0);
-    cudaError_t e = launch_chained(lu_trsm_piece_kernel, dim3((rest + 7) / 8), 256, 0, s, n, A, lda, p0, nb, c0);
+    cudaError_t e = launch_chained(lu_trsm_piece_kernel, dim3((rest + 7) / 8), 256, 0, s, n, A, lda, p0, nb, c0,
+                                   balance + (p0 - j0));
     const int below = c0 - p0 - nb;
     if (e == cudaSuccess && below > 0)
       e = launch_chained(static_cast<InnerUpdate64>(lu_inner_update_kernel),
@@ -1679,8 +1740,18 @@ int getrf_blocked(int n, T* A, int64_t lda, int32_t* ipiv, int32_t* info, void* 
       lu_swap_kernel<T><<<(n - jb + 7) / 8, 256, 0, sp>>>(n, A, lda, pa.pub, j0, jb);
     const int rest = n - j0 - jb;
     if (rest > 0) {
-      if (by_registers && sizeof(T) == 8) e = trsm_by_pieces(n, reinterpret_cast<double*>(A), lda, j0, jb, sp);
-      else e = launch_trsm<T>(n, A, lda, j0, jb, rest, sp);
+      if constexpr (sizeof(T) == 8) {
+        if (by_registers) {
+          e = trsm_by_pieces(n, A, lda, j0, jb, pa.pub->balance, sp);
+        } else {
+          e = launch_trsm<T>(n, A, lda, j0, jb, rest, sp);
+          for (int p0 = 0; p0 < jb; p0 += kRegNb)
+            lu_balance_kernel<<<1, 256, 0, sp>>>(n, A, lda, j0 + p0, std::min(kRegNb, jb - p0), j0 + jb,
+                                                 pa.pub->balance + p0);
+        }
+      } else {
+        e = launch_trsm<T>(n, A, lda, j0, jb, rest, sp);
+      }
       if (e != cudaSuccess) return record_cuda_error(e, name);
       const T* L21 = A + (size_t)j0 * lda + j0 + jb;
       const T* U12 = A + (size_t)(j0 + jb) * lda + j0;
@@ -1754,6 +1825,7 @@ int getrs_one(int n, const T* LU, int64_t lda, const int32_t* ipiv, T* x, int32_
 }
 
 struct Update64Ctx {
+  const int* balance;  // PanelPub's
   void* ws[2];  // scratch of the tensor-core product, one per concurrent update (slot); null: the FP64 kernel
   size_t ws_bytes[2];
 };
@@ -1764,9 +1836,8 @@ int update_fp64(int m, int n, int k, const void* L21, const void* U12, void* A22
   const double *a = static_cast<const double*>(L21), *b = static_cast<const double*>(U12);
   double* d = static_cast<double*>(A22);
   if (c && c->ws[slot] && c->ws_bytes[slot] >= crt_gemm_workspace_bytes(m, n, k))
-    // the pivots: the diagonal of the block above L21 (k columns to the left of it)
     return crt_gemm_run(m, n, k, -1.0, a, lda, b, lda, 1.0, d, lda, c->ws[slot], c->ws_bytes[slot], s, "nacu_dgetrf",
-                        a - k, lda + 1);
+                        c->balance);
   return nacu_dgemm(m, n, k, -1.0, a, lda, b, lda, 1.0, d, lda, s);
 }
 
@@ -2250,7 +2321,9 @@ int nacu_dgesv_mixed_ir(int n, const double* A, int64_t lda, const double* b, do
     fallback = 1;
     cudaMemcpy2DAsync(A64, (size_t)n * 8, A, (size_t)lda * 8, (size_t)n * 8, n, cudaMemcpyDeviceToDevice, s);
     const Getrf64Layout F = getrf64_layout(n);
-    Update64Ctx fctx{{base + L.a32, base + L.a32 + F.bytes[0]}, {F.bytes[0], F.bytes[1]}};
+    Update64Ctx fctx{reinterpret_cast<PanelPub<double>*>(cand)->balance,
+                     {base + L.a32, base + L.a32 + F.bytes[0]},
+                     {F.bytes[0], F.bytes[1]}};
     rc = getrf_blocked<double>(n, A64, n, ipiv, info, cand, kNb64, update_fp64, &fctx, s, "nacu_dgesv_mixed_ir");
     if (rc != NACU_SUCCESS) return rc;
     cudaMemcpyAsync(x, b, (size_t)n * 8, cudaMemcpyDeviceToDevice, s);
@@ -2285,7 +2358,9 @@ int nacu_dgetrf(int n, double* A, int64_t lda, int32_t* ipiv, int32_t* info, voi
   if (!workspace || workspace_bytes < getrf_ws_bytes()) return record_arg_error(-6, "dgetrf: workspace too small");
   const Getrf64Layout L = getrf64_layout(n);
   unsigned char* ws = static_cast<unsigned char*>(workspace);
-  Update64Ctx ctx{{ws + L.slot[0], ws + L.slot[1]}, {L.bytes[0], L.bytes[1]}};
+  Update64Ctx ctx{reinterpret_cast<PanelPub<double>*>(workspace)->balance,
+                  {ws + L.slot[0], ws + L.slot[1]},
+                  {L.bytes[0], L.bytes[1]}};
   if (workspace_bytes < L.total) ctx.ws[0] = ctx.ws[1] = nullptr;  // the updates on the FP64 pipe
   return getrf_blocked<double>(n, A, lda, ipiv, info, workspace, kNb64, update_fp64, &ctx, (cudaStream_t)stream,
                                "nacu_dgetrf");

@@ -33,6 +33,7 @@ namespace {
 constexpr int kSlices = 7;
 constexpr int kSliceRow = 32;            // bytes of one row's digits in one slice
 constexpr int kBadRow = 1 << 20;         // exponent code of a row with inf or NaN
+constexpr int kNoExponent = -(1 << 20);  // of zero, where rows are told from zero rows
 
 __device__ __forceinline__ void mma_f16_16x8x16(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
   asm volatile(
@@ -41,18 +42,17 @@ __device__ __forceinline__ void mma_f16_16x8x16(float (&c)[4], const uint32_t (&
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// The digits of two values with common exponent code em (slice_exponent), one
-// word of two FP16 digits per slice.  em 2047 (inf or NaN in the row): zeros.
-__device__ __forceinline__ int slice_exponent(double v) { return max((__double2hiint(v) >> 20) & 0x7ff, 1); }
-__device__ __forceinline__ void slice_pair(double v0, double v1, int em, uint32_t (&w)[kSlices]) {
+// The digits of two values against the exponents e0 and e1, one word of two FP16
+// digits per slice.  No digits where a value lies 2^60 below its exponent.
+__device__ __forceinline__ void slice_digits(double v0, double v1, int e0, int e1, uint32_t (&w)[kSlices]) {
   uint32_t lo[2], hi[2];
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     const long long b = __double_as_longlong(k ? v1 : v0);
     const int ex = (int)((b >> 52) & 0x7ff);
     const long long m = (b & 0xfffffffffffffll) | (ex ? 0x10000000000000ll : 0ll);
-    const int sh = em - max(ex, 1);  // >= 0: I = m 2^(2 - sh)
-    long long i = (sh > 60 || em == 0x7ff) ? 0 : ((((m << 3) >> sh) + 1) >> 1);
+    const int sh = (k ? e1 : e0) - max(ex, 1);  // >= 0, but for zeros: I = m 2^(2 - sh)
+    long long i = (unsigned)sh > 60u ? 0 : ((((m << 3) >> sh) + 1) >> 1);
     // plus 128 in every digit: the bytes (the top one nine bits) are digit + 128
     i = (b < 0 ? -i : i) + 0x0080808080808080ll;
     lo[k] = (uint32_t)i;
@@ -72,6 +72,13 @@ __device__ __forceinline__ void slice_pair(double v0, double v1, int em, uint32_
   w[4] = minus(__byte_perm(t32, 0x64646464u, 0x4140));
   w[5] = minus(__byte_perm(t10, 0x64646464u, 0x4342));
   w[6] = minus(__byte_perm(t10, 0x64646464u, 0x4140));
+}
+// The same against a row's common exponent code em (slice_exponent).  em 2047 (inf or
+// NaN in the row): zeros.
+__device__ __forceinline__ int slice_exponent(double v) { return max((__double2hiint(v) >> 20) & 0x7ff, 1); }
+__device__ __forceinline__ void slice_pair(double v0, double v1, int em, uint32_t (&w)[kSlices]) {
+  const int e = em == 0x7ff ? kBadRow : em;
+  slice_digits(v0, v1, e, e, w);
 }
 // A row's exponent code from its largest exponent: inf and NaN poison the row.
 __device__ __forceinline__ int slice_code(int em) { return em == 0x7ff ? kBadRow : em; }
@@ -137,6 +144,36 @@ __device__ __forceinline__ void slice_products_add(const unsigned char* sa, cons
 #pragma unroll
     for (int q = 0; q < kSlices - p; ++q) mma_f16_16x8x16(acc[p + q], a, b[q]);
   }
+}
+
+// ---- products whose factors' rows are graded ----------------------------------------------------------------
+// The digits count from a row's largest entry.  Where the large entries of two rows
+// do not meet, the product is far below that of the largest entries and the digits
+// dropped weigh on it.  So a caller may (1) move powers of two from one factor to
+// the other, term by term, by cutting against shifted exponents, and (2) let the
+// magnitudes' leading digits be multiplied too: where their sum is under kMeet / 2^14
+// = 1/8 of the largest entries' product, the products are to be formed in FP64.  The
+// error, a few 2^-56 of the largest entries' product, is then below 2^-50 of the sum
+// of the magnitudes, inside the bound 32 2^-53 of the FP64 loop's roundings.  Dense
+// rows of one scale have sums of 1 to 4.
+constexpr float kMeet = 2048.f;
+
+// The exponent of v 2^shift; kNoExponent for zero, kBadRow for inf and NaN.
+__device__ __forceinline__ int shifted_exponent(double v, int shift) {
+  const int hi = __double2hiint(v) & 0x7fffffff, ex = hi >> 20;
+  if (ex == 0x7ff) return kBadRow;
+  return (hi | __double2loint(v)) == 0 ? kNoExponent : max(ex, 1) + shift;
+}
+// slice_products_add, and the sums of the leading digits' magnitudes.
+__device__ __forceinline__ void slice_products_met(const unsigned char* sa, const unsigned char* sb, int slice_bytes,
+                                                   int lane, float (&acc)[kSlices][4], float (&met)[4]) {
+  slice_products_add(sa, sb, slice_bytes, lane, acc);
+  const int off = (lane >> 2) * kSliceRow + (lane & 3) * 8;
+  constexpr uint32_t kAbs = 0x7fff7fffu;
+  const uint2 w = *reinterpret_cast<const uint2*>(sb + off);
+  const uint2 w0 = *reinterpret_cast<const uint2*>(sa + off), w1 = *reinterpret_cast<const uint2*>(sa + off + 8 * kSliceRow);
+  const uint32_t a[4] = {w0.x & kAbs, w1.x & kAbs, w0.y & kAbs, w1.y & kAbs}, b[2] = {w.x & kAbs, w.y & kAbs};
+  mma_f16_16x8x16(met, a, b);
 }
 __device__ __forceinline__ void slice_products(const unsigned char* sa, const unsigned char* sb, int slice_bytes, int lane,
                                                float (&acc)[kSlices][4]) {
