@@ -115,9 +115,10 @@ __device__ __forceinline__ void mma_f16_16x8x8(float (&c)[4], uint32_t a0, uint3
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a0), "r"(a1), "r"(b0));
 }
-__device__ __forceinline__ void slice_sums_start(float (&acc)[kSlices][4]) {
+template <int LEVELS>
+__device__ __forceinline__ void slice_sums_start(float (&acc)[LEVELS][4]) {
 #pragma unroll
-  for (int l = 0; l < kSlices; ++l)
+  for (int l = 0; l < LEVELS; ++l)
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[l][i] = 12582912.0f;
 }
@@ -126,8 +127,9 @@ __device__ __forceinline__ void slice_sums_start(float (&acc)[kSlices][4]) {
 // (pointers to the first row's digits in slice 0).  A fragment's lane t holds
 // the 16 products' terms 4 t .. 4 t + 3 (one 8-byte load), the same for both
 // operands: the order of the terms is free.
+template <int LEVELS>
 __device__ __forceinline__ void slice_products_add(const unsigned char* sa, const unsigned char* sb, int slice_bytes,
-                                                   int lane, float (&acc)[kSlices][4]) {
+                                                   int lane, float (&acc)[LEVELS][4]) {
   const int off = (lane >> 2) * kSliceRow + (lane & 3) * 8;
   uint32_t b[kSlices][2];
 #pragma unroll
@@ -142,7 +144,7 @@ __device__ __forceinline__ void slice_products_add(const unsigned char* sa, cons
     const uint2 w1 = *reinterpret_cast<const uint2*>(sa + p * slice_bytes + off + 8 * kSliceRow);
     const uint32_t a[4] = {w0.x, w1.x, w0.y, w1.y};
 #pragma unroll
-    for (int q = 0; q < kSlices - p; ++q) mma_f16_16x8x16(acc[p + q], a, b[q]);
+    for (int q = 0; q < kSlices && p + q < LEVELS; ++q) mma_f16_16x8x16(acc[p + q], a, b[q]);
   }
 }
 
@@ -165,8 +167,9 @@ __device__ __forceinline__ int shifted_exponent(double v, int shift) {
   return (hi | __double2loint(v)) == 0 ? kNoExponent : max(ex, 1) + shift;
 }
 // slice_products_add, and the sums of the leading digits' magnitudes.
+template <int LEVELS>
 __device__ __forceinline__ void slice_products_met(const unsigned char* sa, const unsigned char* sb, int slice_bytes,
-                                                   int lane, float (&acc)[kSlices][4], float (&met)[4]) {
+                                                   int lane, float (&acc)[LEVELS][4], float (&met)[4]) {
   slice_products_add(sa, sb, slice_bytes, lane, acc);
   const int off = (lane >> 2) * kSliceRow + (lane & 3) * 8;
   constexpr uint32_t kAbs = 0x7fff7fffu;
@@ -192,16 +195,19 @@ __device__ __noinline__ double slice_value_slow(long long w, int e) {
 // the two rows' exponent codes.  W = sum_l S_l 2^(44 - 8 l), the value W 2^(e -
 // 2046 - 56), rounded to 53 bits from the integer.  DEPTH 32: sums of up to 32
 // products per level and slice pair (7 * 32 * 2^14 < 2^22 still fits the offset
-// accumulators), W one bit shorter to stay below 2^63.
-template <int DEPTH = 16>
-__device__ __forceinline__ double slice_value(const float (&acc)[kSlices][4], int i, int e) {
+// accumulators), W one bit shorter to stay below 2^63.  With an eighth level, S_7
+// enters after S_6.
+template <int DEPTH = 16, int LEVELS = kSlices>
+__device__ __forceinline__ double slice_value(const float (&acc)[LEVELS][4], int i, int e) {
   constexpr int kDrop = DEPTH > 16 ? 1 : 0;
   const uint32_t s0 = __float_as_uint(acc[0][i]), s1 = __float_as_uint(acc[1][i]), s2 = __float_as_uint(acc[2][i]);
   const uint32_t s3 = __float_as_uint(acc[3][i]), s4 = __float_as_uint(acc[4][i]), s5 = __float_as_uint(acc[5][i]);
   const uint32_t s6 = __float_as_uint(acc[6][i]);
   constexpr uint32_t kM = 0x4b400000u, kM2 = kM * 256u + kM;  // the offset in one sum, and in 256 x + y
   const int a = (int)(s0 * 256u + s1 - kM2), b = (int)(s2 * 256u + s3 - kM2), c = (int)(s4 * 256u + s5 - kM2);
-  const int d = (int)(s6 - kM) >> (4 + kDrop);
+  int d = (int)(s6 - kM) >> (4 + kDrop);
+  if constexpr (LEVELS > kSlices)
+    d = (int)(s6 * 256u + __float_as_uint(acc[kSlices][i]) - kM2) >> (12 + kDrop);
   const long long w = (long long)b * (1ll << (20 - kDrop)) + ((long long)c * (16 >> kDrop) + d) +
                       ((long long)((unsigned long long)(uint32_t)a << (36 - kDrop)));
   const uint32_t sign = (uint32_t)((unsigned long long)w >> 63);
