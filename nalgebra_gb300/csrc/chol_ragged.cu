@@ -157,10 +157,16 @@ __global__ void __launch_bounds__(THREADS, MINB) chol_ragged_kernel(CholArgs g) 
   }
 }
 
+// The back solve of orders up to 128 (SMALL) with few right-hand sides is formed in
+// FP64: its products are too few to pay for cutting L.  Whole call, digits and FP64:
+// 23712 x 100 with one 9.4 and 8.4 ms, with four 9.7 and 8.9; 178000 x 40 16.2 and
+// 13.8, 16.5 and 15.0.  With 8, and from order 192 on with 4, FP64 is 8 to 30% slower.
+constexpr int kTcFp64BackRhs = 4;
+
 // The same system through chol_tc.cuh (FMA form, factor wanted): up to
 // kTcMaxRhs right-hand sides take their forward solve along, more are solved
 // from the factor.
-template <int THREADS, int MINB>
+template <int THREADS, int MINB, bool SMALL>
 __global__ void __launch_bounds__(THREADS, MINB) chol_tc_kernel(CholArgs g) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_item, s_info, s_next;
@@ -176,6 +182,7 @@ __global__ void __launch_bounds__(THREADS, MINB) chol_tc_kernel(CholArgs g) {
   double* rdiag = X + (size_t)ldx * cols;
   double* Hd = rdiag + ((ldx + 1) & ~1);
   int* ex = reinterpret_cast<int*>(Hd + 272);
+  int* rexp = ex + tc_slots(g.n_max);
   const int start = g.range ? g.range[0] : 0;
   const int end = g.range ? g.range[1] : g.count;
   for (;;) {
@@ -199,11 +206,14 @@ __global__ void __launch_bounds__(THREADS, MINB) chol_tc_kernel(CholArgs g) {
         X[(size_t)c * ldx + r] = b[e];
       }
       __syncthreads();
-      chol_tc_cta(n, a, g.n_max, ride, X, ldx, SL, rdiag, Hd, ex, s_packed, &s_info, &s_next, g.has_subst, g.subst);
+      chol_tc_cta(n, a, g.n_max, ride, X, ldx, SL, rdiag, Hd, ex, rexp, s_packed, &s_info, &s_next, g.has_subst, g.subst);
       const int inf = s_info;
       if (inf == 0) {
         if (ride) {
-          chol_tc_backward_cta(n, a, g.n_max, ride, X, ldx, SL, rdiag, Hd, ex);
+          bool fp64 = false;
+          if constexpr (SMALL) fp64 = ride <= kTcFp64BackRhs;
+          if (fp64) chol_tc_backward_fp64_cta(n, a, ride, X, ldx, rdiag, Hd);
+          else chol_tc_backward_cta(n, a, g.n_max, ride, X, ldx, SL, rdiag, Hd, ex, rexp);
           for (int e = tid; e < n * ride; e += THREADS) {
             const int c = e / n, r = e - c * n;
             b[e] = X[(size_t)c * ldx + r];
@@ -294,10 +304,10 @@ bool chol_on_tensor_cores(const CholArgs& g, bool exact) { return !exact && g.do
 // 256; 3000 x 256 6.96 with 256, 7.42 with 128.
 CholKernel chol_tc_choose(int n_max, int* threads) {
   *threads = n_max <= 64 ? 64 : n_max <= 192 ? 128 : 256;
-  if (n_max <= 64) return chol_tc_kernel<64, 8>;
-  if (n_max <= 128) return chol_tc_kernel<128, 5>;
-  if (n_max <= 192) return chol_tc_kernel<128, 4>;
-  return chol_tc_kernel<256, 2>;
+  if (n_max <= 64) return chol_tc_kernel<64, 8, true>;
+  if (n_max <= 128) return chol_tc_kernel<128, 5, true>;
+  if (n_max <= 192) return chol_tc_kernel<128, 4, false>;
+  return chol_tc_kernel<256, 2, false>;
 }
 
 // The launch's kernel, threads per CTA and shared memory.

@@ -25,12 +25,14 @@ namespace {
 constexpr int kTcBlock = 16;
 constexpr int kTcMaxRhs = 16;  // right-hand sides that ride along
 
-__host__ __device__ constexpr int tc_slice_bytes(int n_max) { return ((n_max + 15) / 16 * 16 + 16) * kSliceRow; }
+// Slots of the slices: rows below the first head (of 16) and 16 for the right-hand sides.
+__host__ __device__ constexpr int tc_slots(int n_max) { return (n_max + 15) / 16 * 16; }
+__host__ __device__ constexpr int tc_slice_bytes(int n_max) { return tc_slots(n_max) * kSliceRow; }
 // Shared memory: slices, X (nrhs columns), 1 / L_ii, the head and its scratch,
-// row exponents.
+// the slices' exponents, the factor's row exponents.
 __host__ __device__ constexpr size_t tc_smem_bytes(int n_max, int nrhs) {
   return (size_t)kSlices * tc_slice_bytes(n_max) + ((size_t)(n_max | 1) * (nrhs + 1) + 1 + 16 * 17) * 8 +
-         ((size_t)(n_max + 15) / 16 * 16 + 16) * 4;
+         (size_t)2 * tc_slots(n_max) * 4;
 }
 
 // Element e of a 16 x 16 lower triangle packed by columns: 16 r + c.
@@ -156,10 +158,11 @@ __device__ __noinline__ void tc_update(int n, double* __restrict__ a, double* X,
 }
 
 // Factor the matrix a (n x n, column-major, in place) and, for nrhs <= 16
-// columns in X, the forward solve.  *s_info 0 or the first failing pivot.
+// columns in X, the forward solve.  *s_info 0 or the first failing pivot; rexp the
+// largest exponents of L's rows left of their diagonal blocks, kBadRow past the last.
 __device__ __forceinline__ void chol_tc_cta(int n, double* __restrict__ a, int n_max, int nrhs, double* X, int ldx,
-                                            unsigned char* SL, double* rdiag, double* Hd, int* ex, const uint8_t* packed, int* s_info,
-                                            int* s_next, int has_subst, double subst) {
+                                            unsigned char* SL, double* rdiag, double* Hd, int* ex, int* rexp,
+                                            const uint8_t* packed, int* s_info, int* s_next, int has_subst, double subst) {
   const int tid = threadIdx.x, nthr = blockDim.x, warp = tid >> 5, lane = tid & 31, nw = nthr >> 5;
   const int sb = tc_slice_bytes(n_max);
   if (warp == 0) tc_head(n, a, 0, Hd, rdiag, packed, s_info, has_subst, subst, lane);
@@ -177,6 +180,7 @@ __device__ __forceinline__ void chol_tc_cta(int n, double* __restrict__ a, int n
       if (rhs ? r >= nrhs : r >= n) {
         slice_zero_row(s0, sb);
         ex[s] = 1;
+        if (!rhs) rexp[r] = kBadRow;
         continue;
       }
       double* p = rhs ? X + (size_t)r * ldx + J0 : a + (size_t)J0 * n + r;
@@ -193,7 +197,9 @@ __device__ __forceinline__ void chol_tc_cta(int n, double* __restrict__ a, int n
 #pragma unroll
       for (int j = 0; j < 16; ++j)
         if (j < w) p[j * st] = x[j];
-      ex[s] = slice_row(x, s0, sb);
+      const int em = slice_row(x, s0, sb);
+      ex[s] = em;
+      if (!rhs) rexp[r] = J0 == 0 ? em : max(rexp[r], em);
     }
     if (tid == 0) *s_next = nw - 1;
     __syncthreads();
@@ -241,41 +247,94 @@ __device__ __forceinline__ void chol_tc_cta(int n, double* __restrict__ a, int n
   __syncthreads();
 }
 
-// x = L^-T y for the nrhs <= 16 columns of X, in blocks of 16 rows from the
-// bottom.  Per block: warp 0 solves the 16 x 16 transposed triangle (four
-// right-hand sides at a time, eight lanes of two rows each; the rows pre-scaled
-// by 1 / L_jj, so the chain is one FMA per step) while the other warps cut the
-// block's row of L -- column i's 16 entries are contiguous -- into slices; then
+// One block of the back solve by one warp: the 16 x 16 transposed triangle at J0, four
+// right-hand sides at a time, eight lanes of two rows each; the rows pre-scaled by
+// 1 / L_jj, so the chain is one FMA per step.
+__device__ __forceinline__ void tc_backward_block(int n, const double* __restrict__ a, int J0, int nrhs, double* X, int ldx,
+                                                  const double* rdiag, double* Hd, int lane) {
+  const int w = min(16, n - J0);
+  // Hd[j * 16 + i] = L_ji / L_jj (row j of the block)
+  for (int e = lane; e < 256; e += 32) {
+    const int i = e >> 4, j = e & 15;
+    Hd[j * 16 + i] = (j < w && i < j) ? a[(size_t)(J0 + i) * n + J0 + j] * rdiag[J0 + j] : 0.0;
+  }
+  __syncwarp();
+  for (int c0 = 0; c0 < nrhs; c0 += 4) {
+    const int c = c0 + (lane >> 3), q = lane & 7;
+    double* xc = X + (size_t)min(c, nrhs - 1) * ldx + J0;
+    double y0 = q < w ? xc[q] : 0.0, y1 = q + 8 < w ? xc[q + 8] : 0.0;
+#pragma unroll
+    for (int j = 15; j > 0; --j) {
+      const double yj = __shfl_sync(0xffffffffu, j >= 8 ? y1 : y0, (lane & 24) + (j & 7));
+      y0 = fma(-yj, Hd[j * 16 + q], y0);  // zero for rows >= j
+      if (j > 8) y1 = fma(-yj, Hd[j * 16 + q + 8], y1);
+    }
+    if (c < nrhs) {
+      if (q < w) xc[q] = y0 * rdiag[J0 + q];
+      if (q + 8 < w) xc[q + 8] = y1 * rdiag[J0 + q + 8];
+    }
+  }
+}
+
+// x = L^-T y for the nrhs columns of X, in blocks of 16 rows from the bottom, in FP64:
+// a block solved by warp 0 while the other warps' threads load a row of L above it each
+// (column i's 16 entries are contiguous), then y_i -= sum_r L_ri x_r, a thread per row.
+__device__ __noinline__ void chol_tc_backward_fp64_cta(int n, const double* __restrict__ a, int nrhs, double* X, int ldx,
+                                                       const double* rdiag, double* Hd) {
+  const int tid = threadIdx.x, nthr = blockDim.x, warp = tid >> 5, lane = tid & 31;
+  const int first = warp == 0 ? nthr - 32 + tid : tid - 32;  // this thread's first row
+  for (int J0 = (n - 1) / 16 * 16; J0 >= 0; J0 -= 16) {
+    const int w = min(16, n - J0);
+    double l[16];
+    const auto load = [&](int i) {
+      const double* p = a + (size_t)i * n + J0;
+#pragma unroll
+      for (int r = 0; r < 16; ++r) l[r] = i < J0 && r < w ? p[r] : 0.0;
+    };
+    if (warp == 0) tc_backward_block(n, a, J0, nrhs, X, ldx, rdiag, Hd, lane);
+    else load(first);
+    __syncthreads();
+    for (int i = first; i < J0; i += nthr) {
+      if (warp == 0 || i != first) load(i);
+      for (int c = 0; c < nrhs; ++c) {
+        double* const x = X + (size_t)c * ldx;
+        double s = 0.0;  // summed apart: one rounding of y a block
+#pragma unroll
+        for (int r = 0; r < 16; ++r)
+          if (r < w) s = fma(l[r], x[J0 + r], s);
+        x[i] -= s;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// One sum of the back solve in FP64; out of line, most blocks have none.
+__device__ __noinline__ void tc_backward_fp64(const double* l, const double* x, int w, double* y) {
+  double s = 0.0;
+  for (int r = 0; r < w; ++r) s = fma(l[r], x[r], s);
+  *y -= s;
+}
+
+// The same for the nrhs <= 16 columns with the products on the tensor cores: the other
+// warps cut the block's row of L into slices while warp 0 solves its triangle, then
 // y_i -= sum_r L_ri x_r for all rows i above, 16 x 8 tiles on the tensor cores.
+// For A = D A0 D the entries L_ri go as d_r and x_r as 1 / d_r, where the factor's and
+// the forward solve's slices, along rows, hold one scale each.  So L_ri is cut against
+// row r's largest exponent and x_r the other way; where that leaves sums whose large
+// terms do not meet (slices.cuh; in proportion to the terms where the last block has
+// fewer than 16), an FP64 loop forms them.  (Without it, D of 2^+-20 left 1e-4 of an
+// error of 3e-14.)
 __device__ __forceinline__ void chol_tc_backward_cta(int n, const double* __restrict__ a, int n_max, int nrhs, double* X,
-                                                     int ldx, unsigned char* SL, const double* rdiag, double* Hd, int* ex) {
+                                                     int ldx, unsigned char* SL, const double* rdiag, double* Hd, int* ex,
+                                                     const int* rexp) {
   const int tid = threadIdx.x, nthr = blockDim.x, warp = tid >> 5, lane = tid & 31, nw = nthr >> 5;
   const int sb = tc_slice_bytes(n_max);
   const int rhs_slots = nrhs > 8 ? 16 : 8;
   for (int J0 = (n - 1) / 16 * 16; J0 >= 0; J0 -= 16) {
     const int w = min(16, n - J0);
     if (warp == 0) {
-      // Hd[j * 16 + i] = L_ji / L_jj (row j of the block)
-      for (int e = lane; e < 256; e += 32) {
-        const int i = e >> 4, j = e & 15;
-        Hd[j * 16 + i] = (j < w && i < j) ? a[(size_t)(J0 + i) * n + J0 + j] * rdiag[J0 + j] : 0.0;
-      }
-      __syncwarp();
-      for (int c0 = 0; c0 < nrhs; c0 += 4) {
-        const int c = c0 + (lane >> 3), q = lane & 7;
-        double* xc = X + (size_t)min(c, nrhs - 1) * ldx + J0;
-        double y0 = q < w ? xc[q] : 0.0, y1 = q + 8 < w ? xc[q + 8] : 0.0;
-#pragma unroll
-        for (int j = 15; j > 0; --j) {
-          const double yj = __shfl_sync(0xffffffffu, j >= 8 ? y1 : y0, (lane & 24) + (j & 7));
-          y0 = fma(-yj, Hd[j * 16 + q], y0);  // zero for rows >= j
-          if (j > 8) y1 = fma(-yj, Hd[j * 16 + q + 8], y1);
-        }
-        if (c < nrhs) {
-          if (q < w) xc[q] = y0 * rdiag[J0 + q];
-          if (q + 8 < w) xc[q + 8] = y1 * rdiag[J0 + q + 8];
-        }
-      }
+      tc_backward_block(n, a, J0, nrhs, X, ldx, rdiag, Hd, lane);
       __syncwarp();
       if (lane < rhs_slots && J0 > 0) {  // the solved block as slices
         unsigned char* s0 = SL + (J0 + lane) * kSliceRow;
@@ -283,10 +342,10 @@ __device__ __forceinline__ void chol_tc_backward_cta(int n, const double* __rest
           double x[16];
 #pragma unroll
           for (int r = 0; r < 16; ++r) x[r] = r < w ? X[(size_t)lane * ldx + J0 + r] : 0.0;
-          ex[J0 + lane] = slice_row(x, s0, sb);
+          ex[J0 + lane] = slice_row_raised(x, rexp + J0, s0, sb);
         } else {
           slice_zero_row(s0, sb);
-          ex[J0 + lane] = 1;
+          ex[J0 + lane] = kNoExponent;
         }
       }
     }
@@ -297,21 +356,29 @@ __device__ __forceinline__ void chol_tc_backward_cta(int n, const double* __rest
         double x[16];
 #pragma unroll
         for (int r = 0; r < 16; ++r) x[r] = r < w ? p[r] : 0.0;
-        ex[i] = slice_row(x, SL + i * kSliceRow, sb);
+        ex[i] = slice_row_lowered(x, rexp + J0, SL + i * kSliceRow, sb);
       }
     __syncthreads();
     const int tiles = (J0 >> 4) * (rhs_slots >> 3);
+    const float meet = kMeet / 16.f * (float)w;
     for (int u = warp; u < tiles; u += nw) {
       const int it = rhs_slots > 8 ? u >> 1 : u, c8 = rhs_slots > 8 ? (u & 1) * 8 : 0;
       const int g = lane >> 2, t = lane & 3;
       const int i0 = 16 * it + g, c = c8 + 2 * t;
-      float acc[kSlices][4];
-      slice_products(SL + 16 * it * kSliceRow, SL + (J0 + c8) * kSliceRow, sb, lane, acc);
+      float acc[kSlices + 1][4], met[4] = {0.f, 0.f, 0.f, 0.f};
+      slice_sums_start(acc);
+      slice_products_met(SL + 16 * it * kSliceRow, SL + (J0 + c8) * kSliceRow, sb, lane, acc, met);
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
         const int i = i0 + (v >> 1) * 8, cc = c + (v & 1);
-        const double x = slice_value(acc, v, ex[i] + ex[J0 + cc]);
-        if (cc < nrhs) X[(size_t)cc * ldx + i] -= x;
+        const int el = ex[i], er = ex[J0 + cc];
+        const double x = slice_value(acc, v, el + er);
+        double* const y = X + (size_t)cc * ldx;
+        if (cc >= nrhs) continue;
+        if (er == kBadRow || (met[v] < meet && el != kNoExponent && er != kNoExponent))
+          tc_backward_fp64(a + (size_t)i * n + J0, y + J0, w, y + i);
+        else
+          y[i] -= x;
       }
     }
     __syncthreads();

@@ -987,7 +987,7 @@ __global__ void __launch_bounds__(kInnerThreads) lu_inner_update_kernel(int r_hi
         *reinterpret_cast<uint2*>(SL + (size_t)((kk >> 4) * kSlices + q) * sb + s * kSliceRow + (kk & 15) * 2) =
             make_uint2(w0[q], w1[q]);
     }
-    if (k0 == 0) ex[s] = em >= kBadRow / 2 ? kBadRow : em <= kNoExponent / 2 ? kNoExponent : em;
+    if (k0 == 0) ex[s] = graded_code(em);
   }
   __syncthreads();
   if (c >= w) return;

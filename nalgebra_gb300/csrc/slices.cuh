@@ -166,6 +166,63 @@ __device__ __forceinline__ int shifted_exponent(double v, int shift) {
   if (ex == 0x7ff) return kBadRow;
   return (hi | __double2loint(v)) == 0 ? kNoExponent : max(ex, 1) + shift;
 }
+// Likewise a row's code.
+__device__ __forceinline__ int graded_code(int em) {
+  return em >= kBadRow / 2 ? kBadRow : em <= kNoExponent / 2 ? kNoExponent : em;
+}
+// The digits of 16 elements, element k times 2^-shift[k] in the one factor and
+// 2^shift[k] in the other (shift: 8-byte aligned).  Lowered, shift[k] is at least v[k]'s
+// exponent, kBadRow for no entry and for inf or NaN (which the raised factor's code
+// then tells).
+__device__ __forceinline__ int slice_row_lowered(const double (&v)[16], const int* shift, unsigned char* s0, int slice_bytes) {
+  int e[16], em = 2 * kNoExponent;
+#pragma unroll
+  for (int k = 0; k < 16; k += 2) {
+    const int2 p = *reinterpret_cast<const int2*>(shift + k);
+    e[k] = p.x, e[k + 1] = p.y;
+  }
+#pragma unroll
+  for (int k = 0; k < 16; ++k) em = max(em, slice_exponent(v[k]) - e[k]);
+  uint32_t any = 0;
+#pragma unroll
+  for (int h = 0; h < 16; h += 8) {
+    uint32_t w[4][kSlices];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int k = h + 2 * q;
+      slice_digits(v[k], v[k + 1], em + e[k], em + e[k + 1], w[q]);
+      any |= w[q][0];
+    }
+#pragma unroll
+    for (int p = 0; p < kSlices; ++p)
+      *reinterpret_cast<uint4*>(s0 + p * slice_bytes + h * 2) = make_uint4(w[0][p], w[1][p], w[2][p], w[3][p]);
+  }
+  if (any == 0) {  // no leading digit: a zero row, or its scale is that of its zeros (counted as 2^-1022)
+    bool zero = true;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) zero = zero && is_zero_bits(v[k]);
+    if (zero) return kNoExponent;
+  }
+  return em;
+}
+__device__ __forceinline__ int slice_row_raised(const double (&v)[16], const int* shift, unsigned char* s0, int slice_bytes) {
+  int em = kNoExponent;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) em = max(em, shifted_exponent(v[k], shift[k]));
+#pragma unroll
+  for (int h = 0; h < 16; h += 8) {
+    uint32_t w[4][kSlices];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int k = h + 2 * q;
+      slice_digits(v[k], v[k + 1], em - shift[k], em - shift[k + 1], w[q]);
+    }
+#pragma unroll
+    for (int p = 0; p < kSlices; ++p)
+      *reinterpret_cast<uint4*>(s0 + p * slice_bytes + h * 2) = make_uint4(w[0][p], w[1][p], w[2][p], w[3][p]);
+  }
+  return graded_code(em);
+}
 // slice_products_add, and the sums of the leading digits' magnitudes.
 template <int LEVELS>
 __device__ __forceinline__ void slice_products_met(const unsigned char* sa, const unsigned char* sb, int slice_bytes,
