@@ -138,6 +138,10 @@ __device__ __forceinline__ void qr_apply_reflector(double* col, int rows, const 
 // place for both keep four CTAs on an SM at m = 512 (three with four quarters:
 // 8192 problems of 128..512 x 64 14.4 -> 12.6 ms).
 constexpr int kQrParts = 2;
+// Levels of digit products (slices.cuh).  With seven, rows of falling or rising scale
+// (2^+-20) left 1.4 to 1.5 times the error of the FP64 update; with eight 0.7.  8192
+// problems of 128..512 x 64 (the call) 13.3 -> 13.5 ms.
+constexpr int kQrLevels = kSlices + 1;
 constexpr int kQrSlot = kQrParts * kQrNB * 8 + 16;
 __host__ __device__ constexpr int qr_tc_cols(int n) { return (n + 1 + 15) / 16 * 16; }
 __host__ __device__ constexpr size_t qr_tc_bytes(int n) { return (size_t)qr_tc_cols(n) * (kQrSlot + 4); }
@@ -209,7 +213,7 @@ __device__ __forceinline__ void qr_trailing_tc(ColPtr colptr, int ncol, int rows
         ea[u] = max(ea[u], __shfl_xor_sync(0xffffffffu, ea[u], 1));
         ea[u] = max(ea[u], __shfl_xor_sync(0xffffffffu, ea[u], 2));
       }
-      float acc[kSlices][4];
+      float acc[kQrLevels][4];
       slice_sums_start(acc);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -222,7 +226,7 @@ __device__ __forceinline__ void qr_trailing_tc(ColPtr colptr, int ncol, int rows
         for (int p = 0; p < kSlices; ++p) {
           const uint32_t a[4] = {a0[p], a1[p], a2[p], a3[p]};
 #pragma unroll
-          for (int q = 0; q < kSlices - p; ++q) {
+          for (int q = 0; q < kSlices && p + q < kQrLevels; ++q) {
             const uint32_t bb[2] = {b[h][0][q], b[h][1][q]};
             mma_f16_16x8x16(acc[p + q], a, bb);
           }
@@ -287,7 +291,7 @@ __device__ __forceinline__ void qr_trailing_tc(ColPtr colptr, int ncol, int rows
         p[i] = (r < rows && cc < ncol) ? colptr(cc) + r : nullptr;
         v[i] = p[i] ? *p[i] : 0.0;
       }
-      float acc[kSlices][4];
+      float acc[kQrLevels][4];
       slice_sums_start(acc);
       uint32_t b[kSlices];
 #pragma unroll
@@ -296,7 +300,7 @@ __device__ __forceinline__ void qr_trailing_tc(ColPtr colptr, int ncol, int rows
 #pragma unroll
       for (int p2 = 0; p2 < kSlices; ++p2)
 #pragma unroll
-        for (int q = 0; q < kSlices - p2; ++q) mma_f16_16x8x8(acc[p2 + q], a[0][p2], a[1][p2], b[q]);
+        for (int q = 0; q < kSlices && p2 + q < kQrLevels; ++q) mma_f16_16x8x8(acc[p2 + q], a[0][p2], a[1][p2], b[q]);
       const int e0 = ew[c + 2 * t], e1 = ew[c + 2 * t + 1];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
