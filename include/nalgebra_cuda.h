@@ -509,7 +509,8 @@ size_t nacu_getrf_workspace_bytes(int n);
 /* LU with partial pivoting of one n x n matrix (column-major, lda), in place,
  * nalgebra's packed L\U with per-step pivots ipiv[0..n) (src/linalg/lu.rs:93-122;
  * icamax rule src/base/min_max.rs:221-240; a zero column is skipped,
- * lu.rs:107-110).  *info (device) = 0, or the first skipped column + 1.
+ * lu.rs:107-110).  *info (device) = 0, or the first skipped column + 1 (-1000: an
+ * internal wait between thread blocks ran out; factors and pivots are not valid).
  * Look-ahead: the work forks from `stream` onto two internal streams of the
  * library (per device; the panel chain at the highest stream priority, the
  * bulk of each trailing update concurrently) and joins back before the call
@@ -519,6 +520,13 @@ size_t nacu_getrf_workspace_bytes(int n);
  * threads on one device. */
 int nacu_dgetrf(int n, double* A, int64_t lda, int32_t* ipiv, int32_t* info, void* workspace, size_t workspace_bytes,
                 nacu_stream_t stream);
+
+/* Test hook, no counterpart in nalgebra: nacu_dgetrf whose panels' waits give up
+ * after `poll_limit` polls (0 .. 2^20; nacu_dgetrf has 2^20).  With 0 every wait of a
+ * panel in registers (n <= 8192) runs out at once: *info becomes -1000, the matrix
+ * is not valid and the call ends with the context usable. */
+int nacu_test_dgetrf_wait_limit(int n, double* A, int64_t lda, int32_t* ipiv, int32_t* info, int poll_limit,
+                                void* workspace, size_t workspace_bytes, nacu_stream_t stream);
 
 /* Solve A x = b in place in b from nacu_dgetrf factors
  * (src/linalg/lu.rs:242-260); *info = first zero U_kk + 1, or 0 (-1000: an

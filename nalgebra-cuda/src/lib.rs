@@ -327,7 +327,8 @@ pub struct DeviceLU {
 }
 
 impl DeviceLU {
-    /// `LU::solve_mut` (src/linalg/lu.rs:242-260): false when some U_ii == 0.
+    /// `LU::solve_mut` (src/linalg/lu.rs:242-260): false when some U_ii == 0 (or when
+    /// the factorization failed: a negative `info`).
     pub fn solve_mut(&mut self, b: &mut DeviceMatrix) -> bool {
         let n = self.lu.nrows as c_int;
         assert!(b.nrows == self.lu.nrows, "LU solve matrix dimension mismatch.");
@@ -344,7 +345,8 @@ impl DeviceLU {
                     return false;
                 }
             }
-            return true;
+            // negative: the factorization gave up on an internal wait
+            return self.info.to_vec()[0] >= 0;
         }
         check(unsafe {
             ffi::nacu_dgetrs_batched(n, b.ncols as c_int, self.lu.data.as_mut_ptr(), (n * n) as i64,

@@ -240,22 +240,25 @@ class LU:
                       self.info.data_ptr(), 1, flags, _stream_ptr())
 
     def solve_mut(self, b: DeviceMatrix) -> bool:
-        """LU::solve_mut (src/linalg/lu.rs:242-260)."""
+        """LU::solve_mut (src/linalg/lu.rs:242-260).  False also where the
+        factorization or the solve gave up on an internal wait."""
         n = self.lu.nrows
         assert b.nrows == n, "LU solve matrix dimension mismatch."
-        with _info() as info:
-            if not self.large:
+        if not self.large:
+            with _info() as info:
                 _lib.call("nacu_dgetrs_batched", n, b.ncols, self.lu.data.data_ptr(), n * n, self.ipiv.data_ptr(),
                           b.data.data_ptr(), n * b.ncols, info.data_ptr(), 1, self.flags, _stream_ptr())
                 return int(info.item()) == 0
-            ok = True
-            with _work(_lib.load().nacu_getrf_workspace_bytes(0)) as ws:
-                for c in range(b.ncols):
-                    _lib.call("nacu_dgetrs", n, self.lu.data.data_ptr(), n, self.ipiv.data_ptr(),
-                              b.data.data_ptr() + c * n * 8, info.data_ptr(), ws.data_ptr(), ws.numel(),
-                              _stream_ptr())
-                    ok = ok and int(info.item()) == 0
-            return ok
+        ok = True
+        with _dev.scratch_array(2, np.int32) as status, _work(_lib.load().nacu_getrf_workspace_bytes(0)) as ws:
+            # the factorization's status rides along in the solve's copy
+            _lib.call("nacu_memcpy", status.data_ptr() + 4, self.info.data_ptr(), 4, _stream_ptr())
+            for c in range(b.ncols):
+                _lib.call("nacu_dgetrs", n, self.lu.data.data_ptr(), n, self.ipiv.data_ptr(),
+                          b.data.data_ptr() + c * n * 8, status.data_ptr(), ws.data_ptr(), ws.numel(), _stream_ptr())
+                solved, factored = status.to_numpy()
+                ok = ok and solved == 0 and factored >= 0
+        return bool(ok)
 
     def solve(self, b: DeviceMatrix):
         """LU::solve (src/linalg/lu.rs:221-236): a new matrix, or None."""

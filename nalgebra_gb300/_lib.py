@@ -92,6 +92,7 @@ SIGNATURES = {
     "nacu_getrf_workspace_bytes": (_sz, [_i]),
     "nacu_dgetrf": (_i, [_i, _vp, _i64, _vp, _vp, _vp, _sz, _vp]),
     "nacu_dgetrs": (_i, [_i, _vp, _i64, _vp, _vp, _vp, _vp, _sz, _vp]),
+    "nacu_test_dgetrf_wait_limit": (_i, [_i, _vp, _i64, _vp, _vp, _i, _vp, _sz, _vp]),
     "nacu_test_dgetrs_flag_timeout": (_i, [_i, _vp, _i64, _vp, _vp, _vp, _i, _i, _vp, _sz, _vp]),
     "nacu_test_rcp": (_i, [_i, _vp, _vp, _vp]),
     "nacu_ragged_tuning_layout": (_i, [_vp, _vp, _vp]),

@@ -578,6 +578,7 @@ struct RegPanelArgs {
   int32_t* ipiv;
   int32_t* info;
   PanelPub<T>* pub;
+  int poll_limit;  // polls of one wait
 };
 // Three slots: a CTA's stores for column j + 1 may arrive while this one still
 // reads column j - 1's pivot row, but not those for j + 2 (they follow this CTA's
@@ -685,11 +686,14 @@ __global__ void __launch_bounds__(kRegThreads, 1) lu_panel_reg_kernel(RegPanelAr
   int w = 0;          // the CTA that held the last pivot
   bool pend = false;  // column j - 1's update of columns j + 1.. is still to come
   T lp = T(0);        // with this row's multiplier
-  bool late = false;  // a wait ran out: an error, and nothing more is written
+  // This thread's wait ran out: an error; it waits no more and writes no row, and the
+  // barriers, whose phases may still be open, are armed no more (so the other waits run
+  // out too).  What is read meanwhile is any column's: pivots stay rows of the matrix.
+  bool late = false;
   for (int j = 0, now = 0, last = 2, phase = 0; j < g.nb; ++j) {
     const int c = g.j0 + j, par = j & 1, left = g.nb - j;
     const int s0 = j % TPR, d = (sub - s0) & (TPR - 1);  // x[k] is column j + d + TPR k
-    if (tid == 0)
+    if (tid == 0 && !late)
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
                        (unsigned)__cvta_generic_to_shared(&sm.bar[now])),
                    "r"(G * ((left + kV - 1) / kV * 16 + (int)sizeof(RegMeta)))
@@ -747,7 +751,7 @@ __global__ void __launch_bounds__(kRegThreads, 1) lu_panel_reg_kernel(RegPanelAr
           if (TPR == 1 || k > 0 || d > 0) x[k] = axpy1<false>(x[k], -up[(d + TPR * k + 1) & (kRegNb - 1)], lp);
         }
     }
-    if (!late) late = !bar_wait(&sm.bar[now], phase, kRegPollLimit);
+    if (!late) late = !bar_wait(&sm.bar[now], phase, g.poll_limit);
     // the pivot, the same in every warp
     {
       const RegMeta* m = &sm.meta[now][lane < G ? lane : 0];
@@ -1576,12 +1580,13 @@ void (*reg_panel_kernel(int chunk))(RegPanelArgs<T>) {
 // An outer block of jb columns at j0 by panels of kRegNb (swaps and U inside
 // the block included); the panels' swap lists stay in pub.
 template <typename T>
-int reg_block(int n, T* A, int64_t lda, int j0, int jb, int32_t* ipiv, int32_t* info, PanelPub<T>* pub, cudaStream_t s,
-              const char* name) {
+int reg_block(int n, T* A, int64_t lda, int j0, int jb, int32_t* ipiv, int32_t* info, PanelPub<T>* pub, int poll_limit,
+              cudaStream_t s, const char* name) {
   for (int p0 = j0; p0 < j0 + jb; p0 += kRegNb) {
     const int nb = std::min(kRegNb, j0 + jb - p0), rows = n - p0;
     const int G = reg_panel_ctas(rows);
-    RegPanelArgs<T> pa{n, A, lda, p0, nb, (rows + G - 1) / G, j0, j0 + jb, (p0 - j0) / kRegNb, ipiv, info, pub};
+    RegPanelArgs<T> pa{n, A, lda, p0, nb, (rows + G - 1) / G, j0, j0 + jb, (p0 - j0) / kRegNb, ipiv, info, pub,
+                       poll_limit};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(G);
     cfg.blockDim = dim3(kRegThreads);
@@ -1675,7 +1680,7 @@ cudaError_t trsm_by_pieces(int n, double* A, int64_t lda, int j0, int jb, int* b
 // joins to the caller's stream.
 template <typename T>
 int getrf_blocked(int n, T* A, int64_t lda, int32_t* ipiv, int32_t* info, void* ws, int nb, UpdateFn update,
-                  void* ctx, cudaStream_t s, const char* name) {
+                  void* ctx, cudaStream_t s, const char* name, int poll_limit = kRegPollLimit) {
   cudaError_t e;
   const bool by_registers = reg_panels<T>(n);
   nb = by_registers ? kPanelMaxNb : std::min(nb, kPanelMaxNb);
@@ -1699,7 +1704,7 @@ int getrf_blocked(int n, T* A, int64_t lda, int32_t* ipiv, int32_t* info, void* 
     const int rows = n - j0;
     PanelArgs<T> pa{n, A, lda, j0, jb, 0, ipiv, info, reinterpret_cast<PanelPub<T>*>(ws)};
     if (by_registers) {
-      rc = reg_block<T>(n, A, lda, j0, jb, ipiv, info, pa.pub, sp, name);
+      rc = reg_block<T>(n, A, lda, j0, jb, ipiv, info, pa.pub, poll_limit, sp, name);
       if (rc != NACU_SUCCESS) return rc;
     } else {
       const int cchunk = cluster ? (rows + cluster - 1) / cluster : 0;
@@ -2186,6 +2191,23 @@ int gmres_correction(const GmresBufs& g, const double* r, double* x, int* inner,
   return check_launch("nacu_dgesv_mixed_ir: gmres");
 }
 
+int getrf_run(int n, double* A, int64_t lda, int32_t* ipiv, int32_t* info, void* workspace, size_t workspace_bytes,
+              cudaStream_t stream, int poll_limit, const char* name) {
+  if (n < 0) return record_arg_error(-1, "dgetrf: n < 0");
+  if (n == 0) return NACU_SUCCESS;
+  if (!A) return record_arg_error(-2, "dgetrf: null A");
+  if (lda < n) return record_arg_error(-3, "dgetrf: lda < n");
+  if (!ipiv || !info) return record_arg_error(-4, "dgetrf: null ipiv or info");
+  if (!workspace || workspace_bytes < getrf_ws_bytes()) return record_arg_error(-6, "dgetrf: workspace too small");
+  const Getrf64Layout L = getrf64_layout(n);
+  unsigned char* ws = static_cast<unsigned char*>(workspace);
+  Update64Ctx ctx{reinterpret_cast<PanelPub<double>*>(workspace)->balance,
+                  {ws + L.slot[0], ws + L.slot[1]},
+                  {L.bytes[0], L.bytes[1]}};
+  if (workspace_bytes < L.total) ctx.ws[0] = ctx.ws[1] = nullptr;  // the updates on the FP64 pipe
+  return getrf_blocked<double>(n, A, lda, ipiv, info, workspace, kNb64, update_fp64, &ctx, stream, name, poll_limit);
+}
+
 }  // namespace nacu
 
 extern "C" {
@@ -2352,21 +2374,18 @@ size_t nacu_getrf_workspace_bytes(int n) {
 
 int nacu_dgetrf(int n, double* A, int64_t lda, int32_t* ipiv, int32_t* info, void* workspace, size_t workspace_bytes,
                 nacu_stream_t stream) {
+  return nacu::getrf_run(n, A, lda, ipiv, info, workspace, workspace_bytes, (cudaStream_t)stream, nacu::kRegPollLimit,
+                         "nacu_dgetrf");
+}
+
+int nacu_test_dgetrf_wait_limit(int n, double* A, int64_t lda, int32_t* ipiv, int32_t* info, int poll_limit,
+                                void* workspace, size_t workspace_bytes, nacu_stream_t stream) {
   using namespace nacu;
-  if (n < 0) return record_arg_error(-1, "dgetrf: n < 0");
-  if (n == 0) return NACU_SUCCESS;
-  if (!A) return record_arg_error(-2, "dgetrf: null A");
-  if (lda < n) return record_arg_error(-3, "dgetrf: lda < n");
-  if (!ipiv || !info) return record_arg_error(-4, "dgetrf: null ipiv or info");
-  if (!workspace || workspace_bytes < getrf_ws_bytes()) return record_arg_error(-6, "dgetrf: workspace too small");
-  const Getrf64Layout L = getrf64_layout(n);
-  unsigned char* ws = static_cast<unsigned char*>(workspace);
-  Update64Ctx ctx{reinterpret_cast<PanelPub<double>*>(workspace)->balance,
-                  {ws + L.slot[0], ws + L.slot[1]},
-                  {L.bytes[0], L.bytes[1]}};
-  if (workspace_bytes < L.total) ctx.ws[0] = ctx.ws[1] = nullptr;  // the updates on the FP64 pipe
-  return getrf_blocked<double>(n, A, lda, ipiv, info, workspace, kNb64, update_fp64, &ctx, (cudaStream_t)stream,
-                               "nacu_dgetrf");
+  if (n < 0) return record_arg_error(-1, "test_dgetrf_wait_limit: n < 0");
+  if (poll_limit < 0 || poll_limit > kRegPollLimit)
+    return record_arg_error(-6, "test_dgetrf_wait_limit: poll_limit outside [0, 2^20]");
+  return getrf_run(n, A, lda, ipiv, info, workspace, workspace_bytes, (cudaStream_t)stream, poll_limit,
+                   "nacu_test_dgetrf_wait_limit");
 }
 
 int nacu_dgetrs(int n, const double* LU, int64_t lda, const int32_t* ipiv, double* b, int32_t* info, void* workspace,
