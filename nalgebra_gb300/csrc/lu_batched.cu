@@ -204,13 +204,12 @@ __device__ void lu_system(int n, int nrhs, int ld, T* sa, int* s_piv, int* s_inf
 }
 
 // One CTA per system, grid-stride over the batch.  mode: 0 = factor only,
-// 1 = factor + solve, 2 = solve from given factors.
+// 1 = factor + solve, 2 = solve from given factors.  stride: the CTA's threads.
 template <typename T, bool EXACT>
-__global__ void __launch_bounds__(kLuThreads) lu_batched_kernel(int n, int nrhs, T* __restrict__ A,
-                                                                 int64_t strideA, int32_t* __restrict__ ipiv,
-                                                                 T* __restrict__ B, int64_t strideB,
-                                                                 int32_t* __restrict__ info, int batch,
-                                                                 int mode, int write_factors) {
+__device__ __forceinline__ void lu_batched_body(int n, int nrhs, T* __restrict__ A, int64_t strideA,
+                                                int32_t* __restrict__ ipiv, T* __restrict__ B, int64_t strideB,
+                                                int32_t* __restrict__ info, int batch, int mode, int write_factors,
+                                                int stride) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int ld = n | 1;
   const int ncols = n + nrhs;
@@ -221,34 +220,34 @@ __global__ void __launch_bounds__(kLuThreads) lu_batched_kernel(int n, int nrhs,
   const int tid = threadIdx.x;
   for (int s = blockIdx.x; s < batch; s += gridDim.x) {
     const T* a = A + (size_t)s * strideA;
-    for (int e = tid; e < n * n; e += blockDim.x) {
+    for (int e = tid; e < n * n; e += stride) {
       const int c = e / n, r = e - c * n;
       sa[(size_t)c * ld + r] = a[e];
     }
     if (nrhs > 0) {
       const T* b = B + (size_t)s * strideB;
-      for (int e = tid; e < n * nrhs; e += blockDim.x) {
+      for (int e = tid; e < n * nrhs; e += stride) {
         const int c = e / n, r = e - c * n;
         sa[(size_t)(n + c) * ld + r] = b[(size_t)c * n + r];
       }
     }
     if (mode == 2)
-      for (int i = tid; i < n; i += blockDim.x) s_piv[i] = ipiv[(size_t)s * n + i];
+      for (int i = tid; i < n; i += stride) s_piv[i] = ipiv[(size_t)s * n + i];
     __syncthreads();
     lu_system<T, EXACT>(n, nrhs, ld, sa, s_piv, s_info, s_rcp, mode != 2);
     if (mode != 2) {
       if (write_factors) {
         T* aw = A + (size_t)s * strideA;
-        for (int e = tid; e < n * n; e += blockDim.x) {
+        for (int e = tid; e < n * n; e += stride) {
           const int c = e / n, r = e - c * n;
           aw[e] = sa[(size_t)c * ld + r];
         }
       }
-      for (int i = tid; i < n; i += blockDim.x) ipiv[(size_t)s * n + i] = s_piv[i];
+      for (int i = tid; i < n; i += stride) ipiv[(size_t)s * n + i] = s_piv[i];
     }
     if (nrhs > 0) {
       T* b = B + (size_t)s * strideB;
-      for (int e = tid; e < n * nrhs; e += blockDim.x) {
+      for (int e = tid; e < n * nrhs; e += stride) {
         const int c = e / n, r = e - c * n;
         b[(size_t)c * n + r] = sa[(size_t)(n + c) * ld + r];
       }
@@ -258,62 +257,26 @@ __global__ void __launch_bounds__(kLuThreads) lu_batched_kernel(int n, int nrhs,
   }
 }
 
-// The same where shared memory admits two CTAs an SM or one (orders past 97): up to
-// 96 registers a thread, the loops' stride known when compiling and their loads
-// unrolled.  1000 of order 100 with one right-hand side 1151 -> 1038 us (whole call),
-// 1000 of 128 with five 2458 -> 2273, one of 100 172 -> 162.  Where more CTAs fit the
-// longer code costs more than it gives (4096 of order 64 942 -> 950).
 template <typename T, bool EXACT>
-__global__ void __launch_bounds__(kLuThreads, 2) lu_batched_wide_kernel(int n, int nrhs, T* __restrict__ A,
-                                                                 int64_t strideA, int32_t* __restrict__ ipiv,
-                                                                 T* __restrict__ B, int64_t strideB,
-                                                                 int32_t* __restrict__ info, int batch,
+__global__ void __launch_bounds__(kLuThreads) lu_batched_kernel(int n, int nrhs, T* __restrict__ A, int64_t strideA,
+                                                                 int32_t* __restrict__ ipiv, T* __restrict__ B,
+                                                                 int64_t strideB, int32_t* __restrict__ info, int batch,
                                                                  int mode, int write_factors) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int ld = n | 1;
-  const int ncols = n + nrhs;
-  T* sa = reinterpret_cast<T*>(smem_raw);
-  T* s_rcp = sa + (size_t)ld * ncols;  // [0]: 1/pivot, [n+1], [n+2]: the step's scalars; [1+i]: 1/U_ii
-  int* s_piv = reinterpret_cast<int*>(s_rcp + n + 3);
-  int* s_info = s_piv + n;
-  const int tid = threadIdx.x;
-  for (int s = blockIdx.x; s < batch; s += gridDim.x) {
-    const T* a = A + (size_t)s * strideA;
-    for (int e = tid; e < n * n; e += kLuThreads) {
-      const int c = e / n, r = e - c * n;
-      sa[(size_t)c * ld + r] = a[e];
-    }
-    if (nrhs > 0) {
-      const T* b = B + (size_t)s * strideB;
-      for (int e = tid; e < n * nrhs; e += kLuThreads) {
-        const int c = e / n, r = e - c * n;
-        sa[(size_t)(n + c) * ld + r] = b[(size_t)c * n + r];
-      }
-    }
-    if (mode == 2)
-      for (int i = tid; i < n; i += kLuThreads) s_piv[i] = ipiv[(size_t)s * n + i];
-    __syncthreads();
-    lu_system<T, EXACT>(n, nrhs, ld, sa, s_piv, s_info, s_rcp, mode != 2);
-    if (mode != 2) {
-      if (write_factors) {
-        T* aw = A + (size_t)s * strideA;
-        for (int e = tid; e < n * n; e += kLuThreads) {
-          const int c = e / n, r = e - c * n;
-          aw[e] = sa[(size_t)c * ld + r];
-        }
-      }
-      for (int i = tid; i < n; i += kLuThreads) ipiv[(size_t)s * n + i] = s_piv[i];
-    }
-    if (nrhs > 0) {
-      T* b = B + (size_t)s * strideB;
-      for (int e = tid; e < n * nrhs; e += kLuThreads) {
-        const int c = e / n, r = e - c * n;
-        b[(size_t)c * n + r] = sa[(size_t)(n + c) * ld + r];
-      }
-    }
-    if (tid == 0 && info) info[s] = *s_info;
-    __syncthreads();
-  }
+  lu_batched_body<T, EXACT>(n, nrhs, A, strideA, ipiv, B, strideB, info, batch, mode, write_factors, blockDim.x);
+}
+
+// Where shared memory admits two CTAs an SM or one (FP64, orders past 97; FP32 has room
+// for three at every order): up to 96 registers a thread, the loops' stride known when
+// compiling and their loads unrolled.  1000 of order 100 with one right-hand side 1151
+// -> 1038 us (whole call), 1000 of 128 with five 2458 -> 2273, one of 100 172 -> 162.
+// Where more CTAs fit the longer code costs more than it gives (4096 of order 64 942 ->
+// 950; FP32, 3000 of order 98 1.13 -> 1.37, of 128 2.28 -> 2.43).
+template <bool EXACT>
+__global__ void __launch_bounds__(kLuThreads, 2)
+    lu_batched_wide_kernel(int n, int nrhs, double* __restrict__ A, int64_t strideA, int32_t* __restrict__ ipiv,
+                           double* __restrict__ B, int64_t strideB, int32_t* __restrict__ info, int batch, int mode,
+                           int write_factors) {
+  lu_batched_body<double, EXACT>(n, nrhs, A, strideA, ipiv, B, strideB, info, batch, mode, write_factors, kLuThreads);
 }
 
 // b <- L^-1 b (unit lower) and b <- U^-1 b for one right-hand side by one warp, n <=
@@ -462,8 +425,9 @@ int lu_launch(int n, int nrhs, T* A, int64_t strideA, int32_t* ipiv, T* B, int64
     one<<<batch, kLuSolveThreads, smem, stream>>>(n, A, strideA, ipiv, B, strideB, info);
     return check_launch(name);
   }
-  auto kern = n > 97 ? (exact ? lu_batched_wide_kernel<T, true> : lu_batched_wide_kernel<T, false>)
-                     : (exact ? lu_batched_kernel<T, true> : lu_batched_kernel<T, false>);
+  auto kern = exact ? lu_batched_kernel<T, true> : lu_batched_kernel<T, false>;
+  if constexpr (sizeof(T) == 8)
+    if (n > 97) kern = exact ? lu_batched_wide_kernel<true> : lu_batched_wide_kernel<false>;
   if (smem > 48 * 1024) {
     cudaError_t e = ensure_dynamic_smem(kern, smem);
     if (e != cudaSuccess) return record_cuda_error(e, name);
