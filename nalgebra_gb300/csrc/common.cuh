@@ -122,7 +122,9 @@ __device__ __forceinline__ bool is_zero_bits(float x) {
 // A launch ahead of its predecessor's end in the stream (programmatic stream
 // serialization).  The kernel waits for the predecessor before it touches memory,
 // and may let its own successor in early; every kernel launched so waits, so one
-// that is let in follows all before it.
+// that is let in follows all before it.  What a predecessor writes is read through
+// pointers without `const __restrict__`, which would promise memory that is constant
+// from the kernel's start.
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_successor_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... P, typename... Q>

@@ -256,8 +256,8 @@ __device__ __forceinline__ uint32_t abs_bits(long long v, bool bad) {
 }
 
 // Partial row norms of A: thread per row and chunk of columns; part[chunk][row].
-__global__ void __launch_bounds__(128) crt_row_stats_kernel(int m, int k, const double* __restrict__ A, int64_t lda,
-                                                            int chunk, const int* __restrict__ bal,
+__global__ void __launch_bounds__(128) crt_row_stats_kernel(int m, int k, const double* A, int64_t lda,
+                                                            int chunk, const int* bal,
                                                             int2* __restrict__ part, int* __restrict__ flags, int nflags) {
   wait_for_predecessor();
   const int i = blockIdx.x * 128 + threadIdx.x;
@@ -274,9 +274,9 @@ __global__ void __launch_bounds__(128) crt_row_stats_kernel(int m, int k, const 
 // A -> residue planes [plane][mp][kp], K contiguous: 64 k x 32 rows per CTA,
 // transposed through shared memory as scaled integers.  The CTAs of the first
 // k tile also write the row scales.
-__global__ void __launch_bounds__(256) crt_split_a_kernel(int m, int k, const double* __restrict__ A, int64_t lda,
-                                                          const int2* __restrict__ part, int nparts, int mp, int kp,
-                                                          const int* __restrict__ bal,
+__global__ void __launch_bounds__(256) crt_split_a_kernel(int m, int k, const double* A, int64_t lda,
+                                                          const int2* part, int nparts, int mp, int kp,
+                                                          const int* bal,
                                                           int* __restrict__ rscale, uint32_t* __restrict__ out) {
   __shared__ long long t[64][33];
   __shared__ int s_scale[32];
@@ -324,8 +324,8 @@ __global__ void __launch_bounds__(256) crt_split_a_kernel(int m, int k, const do
 
 // B (columns contiguous along K) -> residue planes [plane][np][kp] and the
 // column scales; one CTA per (padded) column.
-__global__ void __launch_bounds__(256) crt_split_b_kernel(int k, int n, const double* __restrict__ B, int64_t ldb, int np,
-                                                          int kp, const int* __restrict__ bal,
+__global__ void __launch_bounds__(256) crt_split_b_kernel(int k, int n, const double* B, int64_t ldb, int np,
+                                                          int kp, const int* bal,
                                                           int* __restrict__ cscale,
                                                           uint32_t* __restrict__ out) {
   __shared__ int s_e[8];

@@ -156,7 +156,7 @@ __device__ __forceinline__ void split3(double v, int slices, __nv_bfloat16* out)
 // 32 x 32 tiles transposed through shared memory; the grid covers the padded
 // mp x kp extent and writes its zeros too, so the buffer needs no memset.
 template <typename TI>
-__global__ void split_a_kernel(int m, int k, const TI* __restrict__ A, int64_t lda, const int* __restrict__ rexp,
+__global__ void split_a_kernel(int m, int k, const TI* A, int64_t lda, const int* rexp,
                                int mp, int kp, int slices, __nv_bfloat16* __restrict__ out) {
   __shared__ double t[32][33];
   const int i0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
@@ -181,7 +181,7 @@ __global__ void split_a_kernel(int m, int k, const TI* __restrict__ A, int64_t l
 // all-zero or padding column) first, then the split, reading the column a
 // second time from L2.
 template <typename TI>
-__global__ void __launch_bounds__(256) split_b_kernel(int k, int n, const TI* __restrict__ B, int64_t ldb,
+__global__ void __launch_bounds__(256) split_b_kernel(int k, int n, const TI* B, int64_t ldb,
                                                       int* __restrict__ cexp, int np, int kp, int slices,
                                                       __nv_bfloat16* __restrict__ out) {
   __shared__ int s_e[8];
@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
             const int col = n0 + c0 + jj;
             cv[jj] = row < g.m && col < g.n ? crow[(size_t)col * g.ldc] : TO(0);
           }
-          ce = scale_exp(__ldg(&g.cexp[n0 + c0 + lane]));
+          ce = scale_exp(g.cexp[n0 + c0 + lane]);
         };
         TO cv[kEpi], nv[kEpi];
         int ce, ne = 0;
