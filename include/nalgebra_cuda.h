@@ -446,7 +446,7 @@ int nacu_sposv_logdet_forward(int n, const float* A, int64_t strideA, const floa
  * (dA_ii = -v_i x_i + g (A^-1)_ii, dA_ij = -(v_i x_j + v_j x_i) + 2 g (A^-1)_ij
  * for i > j, v = A^-1 w; zeros above).  AL holds the stored factor L
  * (recompute = 0) or the original A (recompute = 1: the factor is rebuilt,
- * trading n^3/3 flops for n^2 stored values per matrix). */
+ * trading n^3/3 flops for n^2 stored values per matrix).  dA may be AL itself. */
 int nacu_dposv_logdet_backward(int n, const double* AL, int64_t strideA, int recompute, const double* X,
                                const double* W, const double* G, double* dA, double* db, int32_t* info,
                                int batch, nacu_stream_t stream);

@@ -273,10 +273,10 @@ __global__ void __launch_bounds__(kAdjThreads) adj_forward_kernel(int n, const T
 // Backward: from L (store form) or A (recompute form) build A^-1 in shared
 // memory, then db = v = A^-1 w and the lower-triangle gradient dA.
 template <typename T>
-__global__ void __launch_bounds__(kAdjThreads) adj_backward_kernel(int n, const T* __restrict__ AL, int64_t strideA,
+__global__ void __launch_bounds__(kAdjThreads) adj_backward_kernel(int n, const T* AL, int64_t strideA,
                                                                    int recompute, const T* __restrict__ X,
                                                                    const T* __restrict__ Wt,
-                                                                   const T* __restrict__ Glog, T* __restrict__ dA,
+                                                                   const T* __restrict__ Glog, T* dA,
                                                                    T* __restrict__ db, int32_t* __restrict__ info,
                                                                    int batch) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -352,7 +352,8 @@ __global__ void __launch_bounds__(kAdjThreads) adj_backward_kernel(int n, const 
 //   - take w along: z = L^-1 w, then v = A^-1 w = X z.
 // Everything lives in the output dA (L2): A^-1 and, ahead of it, the trailing
 // matrix in the lower triangle (an entry's factor value is dead once its
-// block is sliced, A^-1_ij starts at block i), X in the strict upper one.
+// block is sliced, A^-1_ij starts at block i), X in the strict upper one.  So the
+// output may be the stored factor's own buffer, and AL carries no __restrict__.
 //
 // What bounds it: the FP64 pipe still (the rows' solves, one subtraction per
 // product), then latency.  2048 x 128: 4.45 -> 1.46 ms with the factor stored,
@@ -392,8 +393,8 @@ __device__ __forceinline__ void adj_tile(const unsigned char* sa, const int* ea,
 
 template <bool RECOMPUTE>
 __global__ void __launch_bounds__(kAdjTcThreads, 4)
-    adj_tc_backward_kernel(int n, const double* __restrict__ AL, int64_t strideA, const double* __restrict__ X,
-                           const double* __restrict__ Wt, const double* __restrict__ Glog, double* __restrict__ dA,
+    adj_tc_backward_kernel(int n, const double* AL, int64_t strideA, const double* __restrict__ X,
+                           const double* __restrict__ Wt, const double* __restrict__ Glog, double* dA,
                            double* __restrict__ db, int32_t* __restrict__ info) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_info, s_next;
@@ -769,8 +770,8 @@ __global__ void __launch_bounds__(kAdjF32Threads) adj_f32_forward_kernel(int n, 
 
 template <bool RECOMPUTE>
 __global__ void __launch_bounds__(kAdjF32Threads)
-    adj_f32_backward_kernel(int n, const float* __restrict__ AL, int64_t strideA, const float* __restrict__ X,
-                            const float* __restrict__ Wt, const float* __restrict__ Glog, float* __restrict__ dA,
+    adj_f32_backward_kernel(int n, const float* AL, int64_t strideA, const float* __restrict__ X,
+                            const float* __restrict__ Wt, const float* __restrict__ Glog, float* dA,
                             float* __restrict__ db, int32_t* __restrict__ info) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_info;
