@@ -16,28 +16,33 @@
 namespace nacu {
 namespace {
 
-constexpr int kBM = 64, kBN = 64, kBK = 16, kGemmThreads = 256;
+constexpr int kBK = 16, kGemmThreads = 256;
 
-__global__ void __launch_bounds__(kGemmThreads, 3)
+// Tiles of 16 T x 16 T, T x T per thread; the smaller ones for the tiles the modular
+// form leaves over, the same sums in the same order.
+template <int T>
+__global__ void __launch_bounds__(kGemmThreads, T == 4 ? 3 : 4)
     dgemm_kernel(int M, int N, int K, double alpha, const double* __restrict__ A, int64_t lda,
                  const double* __restrict__ B, int64_t ldb, double beta, double* __restrict__ C, int64_t ldc,
                  const int* __restrict__ tile_flags, int flag_ld) {
+  constexpr int kTile = 16 * T, kPerFlag = 128 / kTile;
   // with flags, only the 128 x 128 tiles the modular form (gemm_crt.cu) left to this kernel
-  if (tile_flags && !tile_flags[(blockIdx.y >> 1) * flag_ld + (blockIdx.x >> 1)]) return;
-  __shared__ __align__(16) double As[2][kBK][kBM];
-  __shared__ __align__(16) double Bs[2][kBK][kBN + 2];  // +2: conflict-free column writes
+  if (tile_flags && !tile_flags[(blockIdx.y / kPerFlag) * flag_ld + blockIdx.x / kPerFlag]) return;
+  __shared__ __align__(16) double As[2][kBK][kTile];
+  __shared__ __align__(16) double Bs[2][kBK][kTile + 2];  // +2: conflict-free column writes
   const int tid = threadIdx.x;
   const int tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * kBN;
-  // loader mapping: A slice (64 x 16): 4 elements per thread, rows contiguous
-  const int ar = tid & 63, ak = tid >> 6;   // rows ar, k = ak + 4*u
-  // B slice (16 x 64): k contiguous within a column
+  const int m0 = blockIdx.x * kTile, n0 = blockIdx.y * kTile;
+  // loader mapping: A slice (16 T x 16): T elements per thread, rows contiguous
+  constexpr int kStep = kGemmThreads / kTile;
+  const int ar = tid % kTile, ak = tid / kTile;  // rows ar, k = ak + kStep*u
+  // B slice (16 x 16 T): k contiguous within a column
   const int bk = tid & 15, bc = tid >> 4;   // k = bk, columns bc + 16*u
-  double ra[4], rb[4];
+  double ra[T], rb[T];
   auto load = [&](int k0) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int k = k0 + ak + 4 * u, r = m0 + ar;
+    for (int u = 0; u < T; ++u) {
+      const int k = k0 + ak + kStep * u, r = m0 + ar;
       ra[u] = (r < M && k < K) ? A[(size_t)k * lda + r] : 0.0;
       const int c = n0 + bc + 16 * u, kb = k0 + bk;
       rb[u] = (c < N && kb < K) ? B[(size_t)c * ldb + kb] : 0.0;
@@ -45,16 +50,16 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
   };
   auto store = [&](int buf) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      As[buf][ak + 4 * u][ar] = ra[u];
+    for (int u = 0; u < T; ++u) {
+      As[buf][ak + kStep * u][ar] = ra[u];
       Bs[buf][bk][bc + 16 * u] = rb[u];
     }
   };
-  double acc[4][4];
+  double acc[T][T];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < T; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
+    for (int j = 0; j < T; ++j) acc[i][j] = 0.0;
   load(0);
   store(0);
   __syncthreads();
@@ -64,16 +69,22 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
     if (more) load(k0 + kBK);  // prefetch the next slice into registers
 #pragma unroll
     for (int k = 0; k < kBK; ++k) {
-      const double2 a01 = *reinterpret_cast<const double2*>(&As[buf][k][ty * 4]);
-      const double2 a23 = *reinterpret_cast<const double2*>(&As[buf][k][ty * 4 + 2]);
-      const double a[4] = {a01.x, a01.y, a23.x, a23.y};
-      double b[4];
+      double a[T], b[T];
+      if constexpr (T > 1) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[buf][k][tx + 16 * j];
+        for (int i = 0; i < T; i += 2) {
+          const double2 p = *reinterpret_cast<const double2*>(&As[buf][k][ty * T + i]);
+          a[i] = p.x, a[i + 1] = p.y;
+        }
+      } else {
+        a[0] = As[buf][k][ty];
+      }
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < T; ++j) b[j] = Bs[buf][k][tx + 16 * j];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+      for (int i = 0; i < T; ++i)
+#pragma unroll
+        for (int j = 0; j < T; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
     }
     if (more) {
       store(buf ^ 1);
@@ -81,14 +92,14 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
       buf ^= 1;
     }
   }
-  // epilogue: thread (ty, tx) owns rows m0 + 4ty + i, columns n0 + tx + 16j
+  // epilogue: thread (ty, tx) owns rows m0 + T ty + i, columns n0 + tx + 16j
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
+  for (int j = 0; j < T; ++j) {
     const int c = n0 + tx + 16 * j;
     if (c >= N) continue;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = m0 + ty * 4 + i;
+    for (int i = 0; i < T; ++i) {
+      const int r = m0 + ty * T + i;
       if (r >= M) continue;
       double* cp = C + (size_t)c * ldc + r;
       *cp = (beta == 0.0) ? alpha * acc[i][j] : fma(alpha, acc[i][j], beta * *cp);
@@ -100,9 +111,22 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
 
 int dgemm_fp64_run(int m, int n, int k, double alpha, const double* A, int64_t lda, const double* B, int64_t ldb,
                    double beta, double* C, int64_t ldc, const int* tile_flags, int flag_ld, cudaStream_t stream) {
-  const dim3 grid((m + kBM - 1) / kBM, (n + kBN - 1) / kBN);
-  if (grid.y > 65535) return record_arg_error(-2, "dgemm: n too large for one launch");
-  dgemm_kernel<<<grid, kGemmThreads, 0, stream>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tile_flags, flag_ld);
+  const auto grid = [&](int t) { return dim3((m + 16 * t - 1) / (16 * t), (n + 16 * t - 1) / (16 * t)); };
+  const auto tiles = [&](int t) { return (int64_t)grid(t).x * grid(t).y; };
+  if (grid(4).y > 65535) return record_arg_error(-2, "dgemm: n too large for one launch");
+  // Left-over tiles have paid for the modular form already; a product too small for
+  // its 64 x 64 tiles to fill the chip takes smaller ones, so that diagonal, permutation
+  // and banded operands, which leave every tile, come out no later than by this kernel
+  // alone.  Whole call in us, this kernel alone, modular form and 64 x 64, and as here:
+  // 256^3 266, 298, 68; 64^3 71, 97, 35; 1000 x 777 x 1333 2697, 2817, 2136.  Products
+  // that fill the chip pay 2 to 5% (2048^3 14.29 and 14.65 ms), 3000 x 300 x 64 136 and 160.
+  const int64_t enough = 4 * sm_count();
+  if (tile_flags && tiles(4) < enough && tiles(2) < enough)
+    dgemm_kernel<1><<<grid(1), kGemmThreads, 0, stream>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tile_flags, flag_ld);
+  else if (tile_flags && tiles(4) < enough)
+    dgemm_kernel<2><<<grid(2), kGemmThreads, 0, stream>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tile_flags, flag_ld);
+  else
+    dgemm_kernel<4><<<grid(4), kGemmThreads, 0, stream>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tile_flags, flag_ld);
   return check_launch("nacu_dgemm");
 }
 
