@@ -102,6 +102,9 @@ int nacu_free(void* ptr);
  * them.  Inside a stream capture both become nodes of the graph. */
 int nacu_malloc_async(void** ptr, size_t bytes, nacu_stream_t stream);
 int nacu_free_async(void* ptr, nacu_stream_t stream);
+/* Gives what that pool keeps on the current device, and nobody holds, back to it,
+ * for other allocators of the process; waits for the device. */
+int nacu_release_scratch(void);
 /* Page-locked host memory (lets nacu_memcpy and the *_host entry points
  * overlap copies with kernels). */
 int nacu_host_alloc(void** ptr, size_t bytes);

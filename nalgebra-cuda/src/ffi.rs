@@ -19,6 +19,7 @@ extern "C" {
     pub fn nacu_free(ptr: *mut c_void) -> c_int;
     pub fn nacu_malloc_async(ptr: *mut *mut c_void, bytes: usize, s: Stream) -> c_int;
     pub fn nacu_free_async(ptr: *mut c_void, s: Stream) -> c_int;
+    pub fn nacu_release_scratch() -> c_int;
     pub fn nacu_host_alloc(ptr: *mut *mut c_void, bytes: usize) -> c_int;
     pub fn nacu_host_free(ptr: *mut c_void) -> c_int;
     pub fn nacu_memcpy(dst: *mut c_void, src: *const c_void, bytes: usize, s: Stream) -> c_int;

@@ -35,6 +35,11 @@ fn check(rc: c_int) {
     }
 }
 
+/// Gives the scratch that the library keeps between calls (4 GiB at most) back to the device.
+pub fn release_scratch() {
+    check(unsafe { ffi::nacu_release_scratch() });
+}
+
 /// A device allocation of `len` values of `T` (freed on drop).
 pub struct DeviceBuffer<T> {
     ptr: *mut T,

@@ -38,7 +38,8 @@ import numpy as np
 from . import _device as _dev
 from . import _lib
 from . import factor_format
-from ._device import DeviceBuffer, Graph, Stream, current_stream, pinned_empty, set_stream, stream, synchronize
+from ._device import (DeviceBuffer, Graph, Stream, current_stream, pinned_empty, release_scratch, set_stream, stream,
+                      synchronize)
 from ._lib import FLAG_EXACT, FLAG_NO_FACTORS, FLAG_SUBSTITUTE, NacuError
 
 __all__ = [
@@ -47,6 +48,7 @@ __all__ = [
     "PosvLogdet", "cholesky_solve_refined_host",
     "NacuError", "FLAG_EXACT", "FLAG_NO_FACTORS", "FLAG_SUBSTITUTE", "FullPivLU", "ColPivQR", "QR",
     "DeviceBuffer", "Graph", "Stream", "current_stream", "set_stream", "stream", "synchronize", "pinned_empty",
+    "release_scratch",
 ]
 
 

@@ -338,6 +338,12 @@ def scratch_array(shape, dtype, zero: bool = False):
         yield buf.zero_() if zero else buf
 
 
+def release_scratch() -> None:
+    """Give the scratch that the library keeps between calls (4 GiB at most) back
+    to the device, for other allocators of the process; waits for the device."""
+    _lib.call("nacu_release_scratch")
+
+
 def empty(shape, dtype=np.float64) -> DeviceBuffer:
     return DeviceBuffer.empty(shape, dtype)
 

@@ -38,6 +38,7 @@ SIGNATURES = {
     "nacu_free": (_i, [_vp]),
     "nacu_malloc_async": (_i, [C.POINTER(C.c_void_p), _sz, _vp]),
     "nacu_free_async": (_i, [_vp, _vp]),
+    "nacu_release_scratch": (_i, []),
     "nacu_host_alloc": (_i, [C.POINTER(C.c_void_p), _sz]),
     "nacu_host_free": (_i, [_vp]),
     "nacu_memcpy": (_i, [_vp, _vp, _sz, _vp]),

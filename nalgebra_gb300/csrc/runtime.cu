@@ -45,6 +45,15 @@ cudaError_t scratch_pool(cudaMemPool_t* out, bool create) {
   return cudaSuccess;
 }
 
+// What the pool keeps and nobody holds, back to the device.
+cudaError_t trim_scratch_pool() {
+  cudaMemPool_t pool = nullptr;
+  cudaError_t e = scratch_pool(&pool, false);
+  if (e != cudaSuccess || !pool) return e;
+  e = cudaDeviceSynchronize();
+  return e == cudaSuccess ? cudaMemPoolTrimTo(pool, 0) : e;
+}
+
 }  // namespace
 }  // namespace nacu
 
@@ -69,11 +78,8 @@ int nacu_malloc(void** ptr, size_t bytes) {
   if (bytes == 0) return NACU_SUCCESS;
   cudaError_t e = cudaMalloc(ptr, bytes);
   if (e == cudaErrorMemoryAllocation) {  // what the scratch pool keeps may be what is missing
-    cudaMemPool_t pool = nullptr;
     (void)cudaGetLastError();
-    if (scratch_pool(&pool, false) == cudaSuccess && pool && cudaDeviceSynchronize() == cudaSuccess &&
-        cudaMemPoolTrimTo(pool, 0) == cudaSuccess)
-      e = cudaMalloc(ptr, bytes);
+    if (trim_scratch_pool() == cudaSuccess) e = cudaMalloc(ptr, bytes);
   }
   if (e != cudaSuccess) {
     *ptr = nullptr;
@@ -111,6 +117,14 @@ int nacu_free_async(void* ptr, nacu_stream_t stream) {
   if (!ptr) return NACU_SUCCESS;
   const cudaError_t e = cudaFreeAsync(ptr, (cudaStream_t)stream);
   return e == cudaSuccess ? NACU_SUCCESS : record_cuda_error(e, "nacu_free_async");
+}
+
+int nacu_release_scratch(void) {
+  using namespace nacu;
+  const cudaError_t e = trim_scratch_pool();
+  if (e == cudaSuccess) return NACU_SUCCESS;
+  (void)cudaGetLastError();
+  return record_cuda_error(e, "nacu_release_scratch");
 }
 
 int nacu_host_alloc(void** ptr, size_t bytes) {
