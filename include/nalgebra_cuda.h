@@ -591,9 +591,12 @@ int nacu_dgemm(int m, int n, int k, double alpha, const double* A, int64_t lda, 
 /* nacu_dgemm with scratch, which lets large products run on the tensor cores:
  * A and B scaled to integers of up to 62 bits, multiplied exactly modulo 16
  * small numbers in BF16, the integer product put together by the Chinese
- * remainder theorem.  Its error is below nacu_dgemm's; output tiles where
- * |A||B| cancels strongly, and NaN, infinities and extreme exponents, are
- * computed by nacu_dgemm's kernel.  Where nacu_dgemm_workspace_bytes is 0 (small
+ * remainder theorem.  A and B are rounded against their rows' and columns'
+ * 2-norms, to about 2^-61 of them.  Output tiles with |a|.|b| below 2^-7 |a||b|
+ * for a row a and a column b, and those with NaN, infinities or entries beyond
+ * 2^+-800, are computed by nacu_dgemm's kernel; in the others the error is that of
+ * one rounding of C for every 8192 of k, plus at most sqrt(k) 2^-53 |a|.|b|
+ * (nacu_dgemm's bound is k 2^-53 |a|.|b|).  Where nacu_dgemm_workspace_bytes is 0 (small
  * products) the call is nacu_dgemm and the workspace may be NULL. */
 size_t nacu_dgemm_workspace_bytes(int m, int n, int k);
 int nacu_dgemm_ws(int m, int n, int k, double alpha, const double* A, int64_t lda, const double* B, int64_t ldb,

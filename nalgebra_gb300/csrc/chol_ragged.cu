@@ -24,7 +24,7 @@
 // That panel form spends its time on the FP64 pipe (0.70 of its peak).  In the
 // FMA form, orders above 32 go to chol_tc.cuh instead, which takes the trailing
 // updates and the back solve to the tensor cores: 20000 systems of order 8..256
-// with four right-hand sides 37.7 -> 16.9 ms, 3000 of order 256 19.0 -> 7.0 ms
+// with four right-hand sides 37.0 -> 16.6 ms (the launches; 17.7 the call), 3000 of order 256 19.0 -> 7.0 ms
 // (a quarter of the FP64 instructions; the pipe is 46% busy, instruction issue 41%,
 // the rest is the serial heads' latency with two matrices on an SM).
 #include <atomic>

@@ -15,10 +15,10 @@
 //      FP64 (gemm_crt.cu), the BF16-split tensor-core GEMM for the FP32 factor.
 // Orders up to 8192 take 128 columns per block, panels in registers and 32-deep
 // updates inside the block; above, a block is one panel of 64 (FP64) or 128.
-// Measured, FP64, ms (all on the FP64 pipe -> residue updates with 64-wide panels ->
+// Measured, the factorization alone, FP64, ms (all on the FP64 pipe -> residue updates with 64-wide panels ->
 // register panels behind a cluster barrier -> as below): n = 8192 328 -> 114 -> 65 ->
-// 55.6, 4096 50 -> 24.6 -> 20.0 -> 15.1, 2000 11.6 -> 9.4 -> 8.7 -> 5.4, 1000 4.62 ->
-// 4.20 -> 4.08 -> 2.39.  FP32 factor with refinement, n = 4096: 15.8 -> 15.8 -> 14.2 -> 9.9.
+// 56.0, 4096 50 -> 24.6 -> 20.0 -> 15.3, 2000 11.6 -> 9.4 -> 8.7 -> 5.5, 1000 4.62 ->
+// 4.20 -> 4.08 -> 2.41 (the checks of the digit products are 0.5 to 1.5% of these).  FP32 factor with refinement, n = 4096: 15.8 -> 15.8 -> 14.2 -> 9.9.
 // The chain of panels and inner updates bounds it: at n = 8192 50 ms were left of 67
 // when the trailing update beyond the next panel cost nothing.
 // The triangular solves for the right-hand side run as one cooperative kernel

@@ -30,7 +30,7 @@
 // What bounds it: the FP64 pipe, now mostly the panels (12.6k of the 16.4k
 // warp-wide FP64 instructions of a 320 x 64 problem; 41k when the trailing
 // update was dots and axpys), and the panels' serial steps.  Measured: 8192
-// problems of 128..512 x 64 23.7 -> 12.6 ms, 4096 of 100 x 100 10.0 -> 5.2 ms, 8000 of
+// problems of 128..512 x 64 23.7 -> 12.7 ms (the launch; 13.5 the call), 4096 of 100 x 100 10.0 -> 5.2 ms, 8000 of
 // 20..64 x 16 1.23 -> 1.06 ms, 384 of 261..936 x 124 12.2 -> 4.9 ms.
 #include "householder.cuh"
 #include "slices.cuh"

@@ -16,13 +16,14 @@
 // [-128, 127]), exact in FP16.  (FP16 and not BF16: with 11 significant bits a
 // byte b placed under the exponent of 1024 is 1024 + b, so two digits take one
 // byte permute and one packed subtraction.)  Level l collects the products d_p d_q with
-// p + q = l; levels 0..6 are kept.  A sum of 16 * 7 such products stays below
+// p + q = l; levels 0..6 are kept, 0..7 in the LU and the QR.  A sum of 16 * 7 such products stays below
 // 2^21 (of 32: below 2^22), so with the accumulator starting at 1.5 2^23 every partial sum is an
 // integer of FP32 and the low mantissa bits of the result are the sum itself.
 //
 // Error of one 16-deep product against 64 bits: rounding of I 2^-56 2^E of each
-// factor and the levels left out 2^-54 2^(E_r + E_c) (both relative to the
-// largest entries of the two rows); the FP64 loop's is 2^-53 of the partial
+// factor and the levels left out 2^-54 2^(E_r + E_c), with an eighth level the sum's unit, 2^-56 (both
+// relative to the largest entries of the two rows, so a caller whose depth runs over
+// entries of different scale balances and checks, below); the FP64 loop's is 2^-53 of the partial
 // sums, which contain the updated element itself.
 #pragma once
 #include "common.cuh"
