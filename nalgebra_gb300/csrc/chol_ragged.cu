@@ -24,7 +24,7 @@
 // That panel form spends its time on the FP64 pipe (0.70 of its peak).  In the
 // FMA form, orders above 32 go to chol_tc.cuh instead, which takes the trailing
 // updates and the back solve to the tensor cores: 20000 systems of order 8..256
-// with four right-hand sides 37.0 -> 16.6 ms (the launches; 17.7 the call), 3000 of order 256 19.0 -> 7.0 ms
+// with four right-hand sides 37.0 -> 17.5 ms (the launches; 18.8 the call), 3000 of order 256 19.0 -> 7.5 ms
 // (a quarter of the FP64 instructions; the pipe is 46% busy, instruction issue 41%,
 // the rest is the serial heads' latency with two matrices on an SM).
 #include <atomic>
@@ -183,6 +183,7 @@ __global__ void __launch_bounds__(THREADS, MINB) chol_tc_kernel(CholArgs g) {
   double* Hd = rdiag + ((ldx + 1) & ~1);
   int* ex = reinterpret_cast<int*>(Hd + 272);
   int* rexp = ex + tc_slots(g.n_max);
+  uint32_t* pat = reinterpret_cast<uint32_t*>(rexp + tc_slots(g.n_max));
   const int start = g.range ? g.range[0] : 0;
   const int end = g.range ? g.range[1] : g.count;
   for (;;) {
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(THREADS, MINB) chol_tc_kernel(CholArgs g) {
         X[(size_t)c * ldx + r] = b[e];
       }
       __syncthreads();
-      chol_tc_cta(n, a, g.n_max, ride, X, ldx, SL, rdiag, Hd, ex, rexp, s_packed, &s_info, &s_next, g.has_subst, g.subst);
+      chol_tc_cta(n, a, g.n_max, ride, X, ldx, SL, rdiag, Hd, ex, rexp, pat, s_packed, &s_info, &s_next, g.has_subst, g.subst);
       const int inf = s_info;
       if (inf == 0) {
         if (ride) {

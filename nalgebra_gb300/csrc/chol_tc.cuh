@@ -29,10 +29,10 @@ constexpr int kTcMaxRhs = 16;  // right-hand sides that ride along
 __host__ __device__ constexpr int tc_slots(int n_max) { return (n_max + 15) / 16 * 16; }
 __host__ __device__ constexpr int tc_slice_bytes(int n_max) { return tc_slots(n_max) * kSliceRow; }
 // Shared memory: slices, X (nrhs columns), 1 / L_ii, the head and its scratch,
-// the slices' exponents, the factor's row exponents.
+// the slices' exponents and patterns, the factor's row exponents.
 __host__ __device__ constexpr size_t tc_smem_bytes(int n_max, int nrhs) {
   return (size_t)kSlices * tc_slice_bytes(n_max) + ((size_t)(n_max | 1) * (nrhs + 1) + 1 + 16 * 17) * 8 +
-         (size_t)2 * tc_slots(n_max) * 4;
+         (size_t)3 * tc_slots(n_max) * 4;
 }
 
 // Element e of a 16 x 16 lower triangle packed by columns: 16 r + c.
@@ -123,14 +123,64 @@ __device__ __noinline__ void tc_head(int n, double* __restrict__ a, int J0, doub
   }
 }
 
+// A row's pattern: bit k for a nonzero entry k, and kTcThin where fewer than ten of its 16
+// entries are within 1/16 of the largest.  Rows that are not thin meet in four entries at
+// least: their products hold 1/64 of the largest entries' product, and the digits' error
+// is within the FP64 loop's bound (slices.cuh).  Dense rows are thin once in some hundreds.
+constexpr uint32_t kTcThin = 1u << 16;
+__device__ __forceinline__ uint32_t tc_pattern(const double (&x)[16]) {
+  int h[16], hm = 0, near = 0;
+  uint32_t bits = 0;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    h[k] = __double2hiint(x[k]) & 0x7fffffff;
+    hm = max(hm, h[k]);
+    bits |= (h[k] | __double2loint(x[k])) != 0 ? 1u << k : 0u;
+  }
+#pragma unroll
+  for (int k = 0; k < 16; ++k) near += h[k] >= hm - (4 << 20) ? 1 : 0;
+  return bits | (near < 10 ? kTcThin : 0u);
+}
+
+// The elements of one 16 x 8 tile with a thin row whose large terms do not meet (slices.cuh),
+// by FP64 sums over the entries that both rows hold; a bit for each of a lane's four that
+// are done so.  l: row 0 of the tile's rows at the block's columns.
+__device__ __noinline__ int tc_update_thin(int n, const double* l, int64_t row_stride, int64_t stride, const double* lc,
+                                           double* p, int64_t p_row, int64_t p_col, int on, const unsigned char* sa,
+                                           const unsigned char* sc, const int* ea, const int* ec, const uint32_t* pa,
+                                           const uint32_t* pc, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  float met[4] = {0.f, 0.f, 0.f, 0.f};
+  slice_met(sa, sc, lane, met);
+  int done = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = g + (i >> 1) * 8, c = 2 * t + (i & 1);
+    if (!(on >> i & 1) || met[i] >= kMeet || ea[r] + ec[c] >= kBadRow) continue;
+    double s = 0.0;
+    for (uint32_t b = pa[r] & pc[c] & 0xffffu; b != 0; b &= b - 1) {
+      const int k = __ffs((int)b) - 1;
+      s = fma(l[r * row_stride + k * stride], lc[c + (size_t)k * n], s);
+    }
+    p[r * p_row + c * p_col] -= s;
+    done |= 1 << i;
+  }
+  return done;
+}
+
 // A tile of the trailing update: rows of tile `rt` (16 rows from j1 + 16 rt, or
 // the right-hand sides) against columns c0 .. c1 (relative to j1, multiples of
-// 8), a warp.
+// 8), a warp.  Tiles with thin rows are checked: parts of a system that are coupled
+// weakly, or whose right-hand sides have other scales, keep what the loop in FP64 keeps
+// (a coupling or a right-hand side of 2^-60 beside one of 1 was lost).  The checks take
+// 20,000 systems of 8..256 from 17.7 to 18.8 ms, 600 sparse ones (5% of B in B B^T) of
+// order 256 from 1.5 to 3.9 (all in FP64 4.0); those of right-hand sides alone 18.9.
 __device__ __noinline__ void tc_update(int n, double* __restrict__ a, double* X, int ldx, int nrhs, int j1, int rt,
                                           bool rhs, int rhs_slot, int c0, int c1, const unsigned char* SL, int sb,
-                                          const int* ex, int lane) {
+                                          const int* ex, const uint32_t* pat, int lane) {
   const int g = lane >> 2, t = lane & 3;
   const int slot = rhs ? rhs_slot : 16 * rt;
+  const bool thin = __any_sync(0xffffffffu, pat[slot + (lane & 15)] & kTcThin);
   const unsigned char* sa = SL + slot * kSliceRow;
   const int e0 = ex[slot + g], e1 = ex[slot + g + 8];
   const int r0 = rhs ? g : j1 + slot + g;  // rows r0 and r0 + 8
@@ -145,6 +195,18 @@ __device__ __noinline__ void tc_update(int n, double* __restrict__ a, double* X,
       const bool on = rr < rmax && cc < n && (rhs || cc <= rr);
       p[i] = !on ? nullptr : rhs ? X + (size_t)rr * ldx + cc : a + (size_t)cc * n + rr;
       v[i] = on ? *p[i] : 0.0;
+    }
+    if (thin || __any_sync(0xffffffffu, pat[c + (lane & 7)] & kTcThin)) {
+      const int k0 = j1 - kTcBlock, on = (p[0] ? 1 : 0) | (p[1] ? 2 : 0) | (p[2] ? 4 : 0) | (p[3] ? 8 : 0);
+      const int first = j1 + c;
+      const int done = rhs ? tc_update_thin(n, X + k0, ldx, 1, a + (size_t)k0 * n + first, X + first, ldx, 1, on, sa,
+                                            SL + c * kSliceRow, ex + slot, ex + c, pat + slot, pat + c, lane)
+                           : tc_update_thin(n, a + (size_t)k0 * n + j1 + slot, 1, n, a + (size_t)k0 * n + first,
+                                            a + (size_t)first * n + j1 + slot, 1, n, on, sa, SL + c * kSliceRow,
+                                            ex + slot, ex + c, pat + slot, pat + c, lane);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (done >> i & 1) p[i] = nullptr;
     }
     float acc[kSlices][4];
     slice_products(sa, SL + c * kSliceRow, sb, lane, acc);
@@ -161,7 +223,7 @@ __device__ __noinline__ void tc_update(int n, double* __restrict__ a, double* X,
 // columns in X, the forward solve.  *s_info 0 or the first failing pivot; rexp the
 // largest exponents of L's rows left of their diagonal blocks, kBadRow past the last.
 __device__ __forceinline__ void chol_tc_cta(int n, double* __restrict__ a, int n_max, int nrhs, double* X, int ldx,
-                                            unsigned char* SL, double* rdiag, double* Hd, int* ex, int* rexp,
+                                            unsigned char* SL, double* rdiag, double* Hd, int* ex, int* rexp, uint32_t* pat,
                                             const uint8_t* packed, int* s_info, int* s_next, int has_subst, double subst) {
   const int tid = threadIdx.x, nthr = blockDim.x, warp = tid >> 5, lane = tid & 31, nw = nthr >> 5;
   const int sb = tc_slice_bytes(n_max);
@@ -180,6 +242,7 @@ __device__ __forceinline__ void chol_tc_cta(int n, double* __restrict__ a, int n
       if (rhs ? r >= nrhs : r >= n) {
         slice_zero_row(s0, sb);
         ex[s] = 1;
+        pat[s] = 0;
         if (!rhs) rexp[r] = kBadRow;
         continue;
       }
@@ -199,6 +262,7 @@ __device__ __forceinline__ void chol_tc_cta(int n, double* __restrict__ a, int n
         if (j < w) p[j * st] = x[j];
       const int em = slice_row(x, s0, sb);
       ex[s] = em;
+      pat[s] = tc_pattern(x);
       if (!rhs) rexp[r] = J0 == 0 ? em : max(rexp[r], em);
     }
     if (tid == 0) *s_next = nw - 1;
@@ -206,7 +270,7 @@ __device__ __forceinline__ void chol_tc_cta(int n, double* __restrict__ a, int n
     if (m == 0) break;
     // the next block's columns
     for (int rt = warp; rt < mt + (nrhs > 0 ? 1 : 0); rt += nw)
-      tc_update(n, a, X, ldx, nrhs, j1, rt, rt == mt, rhs_slot, 0, 16, SL, sb, ex, lane);
+      tc_update(n, a, X, ldx, nrhs, j1, rt, rt == mt, rhs_slot, 0, 16, SL, sb, ex, pat, lane);
     __syncthreads();
     // the rest, in units of 16 rows x 32 columns: row tile i > 0 has ceil(i / 2), tiles 2 k - 1 and 2 k
     // together 2 k, so the first 2 k tiles k (k + 1)
@@ -230,10 +294,10 @@ __device__ __forceinline__ void chol_tc_cta(int n, double* __restrict__ a, int n
         if (k * (k + 1) <= u) ++k;
         const int rem = u - k * (k - 1);
         const int i = rem < k ? 2 * k - 1 : 2 * k, grp = rem < k ? rem : rem - k;
-        tc_update(n, a, X, ldx, nrhs, j1, i, false, 0, 16 + 32 * grp, min(48 + 32 * grp, 16 * i + 16), SL, sb, ex, lane);
+        tc_update(n, a, X, ldx, nrhs, j1, i, false, 0, 16 + 32 * grp, min(48 + 32 * grp, 16 * i + 16), SL, sb, ex, pat, lane);
       } else {
         const int c0 = 16 + 32 * (u - tri);
-        tc_update(n, a, X, ldx, nrhs, j1, 0, true, rhs_slot, c0, min(c0 + 32, (m + 7) & ~7), SL, sb, ex, lane);
+        tc_update(n, a, X, ldx, nrhs, j1, 0, true, rhs_slot, c0, min(c0 + 32, (m + 7) & ~7), SL, sb, ex, pat, lane);
       }
       if (nw == 1) {
         ++u;

@@ -224,17 +224,21 @@ __device__ __forceinline__ int slice_row_raised(const double (&v)[16], const int
   }
   return graded_code(em);
 }
-// slice_products_add, and the sums of the leading digits' magnitudes.
-template <int LEVELS>
-__device__ __forceinline__ void slice_products_met(const unsigned char* sa, const unsigned char* sb, int slice_bytes,
-                                                   int lane, float (&acc)[LEVELS][4], float (&met)[4]) {
-  slice_products_add(sa, sb, slice_bytes, lane, acc);
+// The sums of the leading digits' magnitudes.
+__device__ __forceinline__ void slice_met(const unsigned char* sa, const unsigned char* sb, int lane, float (&met)[4]) {
   const int off = (lane >> 2) * kSliceRow + (lane & 3) * 8;
   constexpr uint32_t kAbs = 0x7fff7fffu;
   const uint2 w = *reinterpret_cast<const uint2*>(sb + off);
   const uint2 w0 = *reinterpret_cast<const uint2*>(sa + off), w1 = *reinterpret_cast<const uint2*>(sa + off + 8 * kSliceRow);
   const uint32_t a[4] = {w0.x & kAbs, w1.x & kAbs, w0.y & kAbs, w1.y & kAbs}, b[2] = {w.x & kAbs, w.y & kAbs};
   mma_f16_16x8x16(met, a, b);
+}
+// slice_products_add, and those.
+template <int LEVELS>
+__device__ __forceinline__ void slice_products_met(const unsigned char* sa, const unsigned char* sb, int slice_bytes,
+                                                   int lane, float (&acc)[LEVELS][4], float (&met)[4]) {
+  slice_products_add(sa, sb, slice_bytes, lane, acc);
+  slice_met(sa, sb, lane, met);
 }
 __device__ __forceinline__ void slice_products(const unsigned char* sa, const unsigned char* sb, int slice_bytes, int lane,
                                                float (&acc)[kSlices][4]) {
